@@ -119,14 +119,16 @@ class Noise:
 # Dense models
 # ---------------------------------------------------------------------------------------------------------------------
 def gpt_weights(case, seed):
-    """N(0, 0.02), what adds to the stream divided by the root of twice the full depth, as such models are initialised; a stream that starts at the
-    scale it has behind the first layers of a trained one."""
+    """Linears keep the scale of their input; the feed-forward adds a third of it to a stream that starts at scale 1, as behind the first layers of a
+    trained model.  (With a smaller stream the 8-bit roundings of the layers' inputs would be nearly all of the logits' error, and one rounding in another
+    place would move them by most of it.)"""
     s, noise, out = GPT[case["size"]], Noise(seed), {}
     W, qkv = s["width"], (s["heads"] + 2 * s["groups"]) * s["dim"]
 
     def put(name, *shape):
-        std = 0.5 if name.startswith("embedding") else 0.02 / 8 if name.endswith(("linear_proj.weight", "linear_fc2.weight")) else 0.02
-        out[name] = noise(name, *shape, std=std, mean=1.0 if name.endswith("layernorm.weight") else 0.0)
+        norm = name.endswith("layernorm.weight")
+        std = 0.02 if norm else 1.0 if name.startswith("embedding") else (0.35 if "fc2" in name else 1.0) / math.sqrt(shape[-1])
+        out[name] = noise(name, *shape, std=std, mean=1.0 if norm else 0.0)
 
     put("embedding.word_embeddings.weight", s["vocab"], W)
     for i in range(case["layers"]):
@@ -411,10 +413,11 @@ def hybrid_weights(case, seed):
             parts = [("", mlp["ff"])]
         else:
             columns, groups, _ = routed
-            put(p + "router", columns, W, std=0.2 / math.sqrt(W))
+            put(p + "router", columns, W, std=0.1 / math.sqrt(W))
             out[p + "router"][:, :kept] = 0
             for e in range(columns):
-                out[p + "router"][e, feature_of(i, e, columns, groups)] = 0.6
+                out[p + "router"][e, feature_of(i, e, columns, groups)] = 1.2
+            out[f"l{i}.norm{1 if model == 'maginex' else 2}"][:kept] = off  # (what the router reads is scaled alike for every token)
             if model == "lukarax":
                 put(p + "correction", columns, std=0.002)
             elif model == "maginex":
