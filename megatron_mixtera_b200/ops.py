@@ -114,12 +114,9 @@ def _launch(name: str, *args):
 
 
 def _blob(struct) -> torch.Tensor:
-    """The bytes of a ctypes argument struct as a CPU uint8 tensor sharing its memory (made once per struct)."""
-    t = getattr(struct, "_as_tensor", None)
-    if t is None:
-        t = torch.frombuffer(struct, dtype=torch.uint8)
-        struct._as_tensor = t
-    return t
+    """The bytes of a ctypes argument struct as a CPU uint8 tensor sharing its memory.  (Not kept on the struct: the tensor's storage holds the
+    struct, a cycle that no collector sees, and with it whatever else hangs on the struct - a key/value pool, expanded keys.)"""
+    return torch.frombuffer(struct, dtype=torch.uint8)
 
 
 def set_wait_limit_ns(limit_ns: int) -> None:
