@@ -64,6 +64,13 @@ struct Params {
 };
 constexpr int kGatedSilu = 1, kGatedClamped = 2, kGatedPlain = 3;  // Params::gated
 
+// Many tokens: CTA pairs (gemm_pair.cu).
+namespace pair {
+static bool preferred(int M, int N);
+static int launch_bf16(const void* x, int64_t ldx, const void* w, const void* bias, void* y, int64_t ldy, int M, int N, int K, cudaStream_t stream,
+                       float* partials, bool gated, int act);
+}  // namespace pair
+
 __device__ __forceinline__ float clamped_glu(float g, float u, float limit, float alpha) {
   g = fminf(g, limit);
   u = fminf(fmaxf(u, -limit), limit);
@@ -718,6 +725,15 @@ static int launch(const void* x, int64_t ldx, const void* w, const void* bias, v
   return launch_splitk_reduce(p, stream);
 }
 
+// Bytes of split-K partial sums that the weight-streaming kernels need (0: K is not split).
+static size_t splitk_scratch_bytes(int M, int N, int K) {
+  const int bt = pick_bt(M);
+  const int tiles = ((N + kTileN - 1) / kTileN) * ((M + bt - 1) / bt);
+  const int splits = choose_splits(tiles, (K + kTileK - 1) / kTileK);
+  if (splits == 1) return 0;
+  return static_cast<size_t>(splits) * static_cast<size_t>(M) * N * sizeof(float);
+}
+
 }  // namespace gemm
 }  // namespace b200
 
@@ -736,6 +752,7 @@ int b200_set_gemm_split_policy(int ctas_per_sm, int min_k_blocks_per_split, int 
 int b200_gemm_bf16_swiglu_supported(int M, int N, int K) {
   using namespace b200::gemm;
   if (M <= 0 || N <= 0 || K <= 0 || N % 128 != 0 || K % 8 != 0) return 0;
+  if (pair::preferred(M, N)) return 1;
   const int bt = pick_bt(M);
   const int tiles = (N / kTileN) * ((M + bt - 1) / bt);
   return choose_splits(tiles, (K + kTileK - 1) / kTileK) == 1 ? 1 : 0;
@@ -749,6 +766,7 @@ int b200_gemm_bf16_swiglu(const void* x, int64_t ldx, const void* w, void* y, in
   if (!aligned16(x) || !aligned16(w)) return B200_ERR_ALIGNMENT;
   if (!b200_gemm_bf16_swiglu_supported(M, N, K)) return B200_ERR_INVALID_ARGUMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (gemm::pair::preferred(M, N)) return gemm::pair::launch_bf16(x, ldx, w, nullptr, y, ldy, M, N, K, s, nullptr, true, B200_ACT_NONE);
   switch (gemm::pick_bt(M)) {
     case 32: return gemm::launch<32>(x, ldx, w, nullptr, y, ldy, M, N, K, nullptr, 0, s, true, nullptr, 0, nullptr, true);
     case 64: return gemm::launch<64>(x, ldx, w, nullptr, y, ldy, M, N, K, nullptr, 0, s, true, nullptr, 0, nullptr, true);
@@ -760,6 +778,7 @@ int b200_gemm_bf16_swiglu(const void* x, int64_t ldx, const void* w, void* y, in
 size_t b200_gemm_bf16_splitk_bytes(int M, int N, int K) {
   using namespace b200::gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (pair::preferred(M, N)) return static_cast<size_t>(M) * N * sizeof(float);
   const int bt = pick_bt(M);
   const int tiles = ((N + kTileN - 1) / kTileN) * ((M + bt - 1) / bt);
   return static_cast<size_t>(choose_splits(tiles, (K + kTileK - 1) / kTileK)) * M * N * sizeof(float);
@@ -772,6 +791,11 @@ int b200_gemm_bf16_splitk(const void* x, int64_t ldx, const void* w, int M, int 
   if (K % 8 != 0 || ldx % 8 != 0 || ldx < K) return B200_ERR_ALIGNMENT;
   if (!aligned16(x) || !aligned16(w) || !aligned16(partials)) return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (gemm::pair::preferred(M, N)) {
+    if (partials_bytes < static_cast<size_t>(M) * N * sizeof(float)) return B200_ERR_WORKSPACE;
+    *num_splits = 1;
+    return gemm::pair::launch_bf16(x, ldx, w, nullptr, nullptr, N, M, N, K, s, partials, false, B200_ACT_NONE);
+  }
   switch (gemm::pick_bt(M)) {
     case 32: return gemm::launch<32>(x, ldx, w, nullptr, nullptr, N, M, N, K, nullptr, 0, s, true, partials, partials_bytes, num_splits);
     case 64: return gemm::launch<64>(x, ldx, w, nullptr, nullptr, N, M, N, K, nullptr, 0, s, true, partials, partials_bytes, num_splits);
@@ -783,11 +807,8 @@ int b200_gemm_bf16_splitk(const void* x, int64_t ldx, const void* w, int M, int 
 size_t b200_gemm_bf16_workspace_bytes(int M, int N, int K) {
   using namespace b200::gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const int bt = pick_bt(M);
-  const int tiles = ((N + kTileN - 1) / kTileN) * ((M + bt - 1) / bt);
-  const int splits = choose_splits(tiles, (K + kTileK - 1) / kTileK);
-  if (splits == 1) return 0;
-  return static_cast<size_t>(splits) * static_cast<size_t>(M) * N * sizeof(float);
+  if (pair::preferred(M, N)) return 0;
+  return splitk_scratch_bytes(M, N, K);
 }
 
 int b200_gemm_bf16(const void* x, int64_t ldx, const void* w, const void* bias, void* y, int64_t ldy, int M, int N,
@@ -797,6 +818,7 @@ int b200_gemm_bf16(const void* x, int64_t ldx, const void* w, const void* bias, 
   if (K % 8 != 0 || ldx % 8 != 0 || ldx < K || ldy < N) return B200_ERR_ALIGNMENT;
   if (!aligned16(x) || !aligned16(w)) return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (gemm::pair::preferred(M, N)) return gemm::pair::launch_bf16(x, ldx, w, bias, y, ldy, M, N, K, s, nullptr, false, B200_ACT_NONE);
   switch (gemm::pick_bt(M)) {
     case 32: return gemm::launch<32>(x, ldx, w, bias, y, ldy, M, N, K, workspace, workspace_bytes, s);
     case 64: return gemm::launch<64>(x, ldx, w, bias, y, ldy, M, N, K, workspace, workspace_bytes, s);
@@ -817,6 +839,8 @@ int b200_linear_bf16(const void* x, int64_t ldx, const void* w, void* y, int64_t
   if (gate && (gate_ld < (batch - 1) * y_batch + N || act != B200_ACT_NONE)) return B200_ERR_INVALID_ARGUMENT;
   if (!aligned16(x) || !aligned16(w)) return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (batch == 1 && gate == nullptr && gemm::pair::preferred(M, N))
+    return gemm::pair::launch_bf16(x, ldx, w, nullptr, y, ldy, M, N, K, s, nullptr, false, act);
   switch (gemm::pick_bt(M)) {
     case 32: return gemm::launch<32>(x, ldx, w, nullptr, y, ldy, M, N, K, workspace, workspace_bytes, s, true, nullptr, 0, nullptr, false, act, batch, x_batch, y_batch, gate, gate_ld);
     case 64: return gemm::launch<64>(x, ldx, w, nullptr, y, ldy, M, N, K, workspace, workspace_bytes, s, true, nullptr, 0, nullptr, false, act, batch, x_batch, y_batch, gate, gate_ld);
@@ -875,7 +899,7 @@ int b200_gemm_bf16_static_scratch(const void* x, int64_t ldx, const void* w, con
   if (!x || !w || !y || M <= 0 || N <= 0 || K <= 0) return B200_ERR_INVALID_ARGUMENT;
   if (K % 8 != 0 || ldx % 8 != 0 || ldx < K || ldy < N) return B200_ERR_ALIGNMENT;
   if (!aligned16(x) || !aligned16(w)) return B200_ERR_ALIGNMENT;
-  const size_t need = b200_gemm_bf16_workspace_bytes(M, N, K);
+  const size_t need = gemm::splitk_scratch_bytes(M, N, K);
   if (need > gemm::kStaticScratchBytes) return B200_ERR_SCRATCH_LIMIT;
   void* scratch = gemm::static_scratch_address();
   if (scratch == nullptr) return B200_ERR_LAUNCH;

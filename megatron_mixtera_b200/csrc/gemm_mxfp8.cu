@@ -39,6 +39,11 @@ struct Fp8Config {
                                    : kTmemNeeded <= 256 ? 256 : 512;
 };
 
+namespace pair {  // many tokens (gemm_pair.cu)
+static int launch_mxfp8(const void* xq, const void* x_sf, const void* wq, const void* w_sf, const void* bias, void* y, int64_t ldy, int M, int N, int K,
+                        cudaStream_t stream, float* partials, bool halves, void* q_out, void* sf_out);
+}  // namespace pair
+
 struct Fp8Operands {
   const uint8_t* w_sf;  // tile layout, [n tiles][K/128][512]
   const uint8_t* x_sf;  // tile layout, [ceil(M/128)][K/128][512]
@@ -491,6 +496,7 @@ size_t b200_mxfp8_scale_bytes(int rows, int K) {
 size_t b200_gemm_mxfp8_splitk_bytes(int M, int N, int K) {
   using namespace b200::gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (pair::preferred(M, N)) return static_cast<size_t>(M) * N * sizeof(float);
   const int bt = pick_bt(M);
   const int tiles = ((N + kTileN - 1) / kTileN) * ((M + bt - 1) / bt);
   return static_cast<size_t>(choose_splits(tiles, K / kFp8TileK)) * M * N * sizeof(float);
@@ -505,6 +511,11 @@ int b200_gemm_mxfp8_splitk(const void* xq, const void* x_sf, const void* wq, con
   if (!aligned16(xq) || !aligned16(wq) || !aligned16(x_sf) || !aligned16(w_sf) || !aligned16(partials))
     return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (gemm::pair::preferred(M, N)) {
+    if (partials_bytes < static_cast<size_t>(M) * N * sizeof(float)) return B200_ERR_WORKSPACE;
+    *num_splits = 1;
+    return gemm::pair::launch_mxfp8(xq, x_sf, wq, w_sf, nullptr, nullptr, N, M, N, K, s, partials, false, nullptr, nullptr);
+  }
   switch (gemm::pick_bt(M)) {
     case 32: return gemm::launch_mxfp8<32>(xq, x_sf, wq, w_sf, nullptr, nullptr, N, M, N, K, nullptr, 0, s, partials, partials_bytes, num_splits);
     case 64: return gemm::launch_mxfp8<64>(xq, x_sf, wq, w_sf, nullptr, nullptr, N, M, N, K, nullptr, 0, s, partials, partials_bytes, num_splits);
@@ -516,6 +527,7 @@ int b200_gemm_mxfp8_splitk(const void* xq, const void* x_sf, const void* wq, con
 size_t b200_gemm_mxfp8_workspace_bytes(int M, int N, int K) {
   using namespace b200::gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (pair::preferred(M, N)) return 0;
   const int bt = pick_bt(M);
   const int tiles = ((N + kTileN - 1) / kTileN) * ((M + bt - 1) / bt);
   const int splits = choose_splits(tiles, K / kFp8TileK);
@@ -530,6 +542,8 @@ int b200_gemm_mxfp8(const void* xq, const void* x_sf, const void* wq, const void
   if (K % 128 != 0 || ldy < N) return B200_ERR_ALIGNMENT;
   if (!aligned16(xq) || !aligned16(wq) || !aligned16(x_sf) || !aligned16(w_sf)) return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (gemm::pair::preferred(M, N))
+    return gemm::pair::launch_mxfp8(xq, x_sf, wq, w_sf, bias, y, ldy, M, N, K, s, nullptr, false, nullptr, nullptr);
   switch (gemm::pick_bt(M)) {
     case 32: return gemm::launch_mxfp8<32>(xq, x_sf, wq, w_sf, bias, y, ldy, M, N, K, workspace, workspace_bytes, s);
     case 64: return gemm::launch_mxfp8<64>(xq, x_sf, wq, w_sf, bias, y, ldy, M, N, K, workspace, workspace_bytes, s);
@@ -548,6 +562,8 @@ int b200_gemm_mxfp8_swiglu(const void* xq, const void* x_sf, const void* wq, con
       (sf_out && !aligned16(sf_out)) || (y_out && !aligned16(y_out)))
     return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (gemm::pair::preferred(M, 2 * F))
+    return gemm::pair::launch_mxfp8(xq, x_sf, wq, w_sf, nullptr, y_out, ldy, M, 2 * F, K, s, nullptr, true, q_out, sf_out);
   switch (gemm::pick_bt_pair(M)) {
     case 32: return gemm::launch_mxfp8_pair<32>(xq, x_sf, wq, w_sf, q_out, sf_out, y_out, ldy, M, F, K, s);
     case 64: return gemm::launch_mxfp8_pair<64>(xq, x_sf, wq, w_sf, q_out, sf_out, y_out, ldy, M, F, K, s);
