@@ -1312,6 +1312,13 @@ static int launch_attention(Params& p, cudaStream_t stream) {
   return rc;
 }
 
+// Long prompts: attention_prompt.cu.
+namespace prompt {
+static bool preferred(const Params& p, const int32_t* units, int num_units);
+template <int DK, int DV, int FORM>
+static int launch(const Params& p, const CUtensorMap* mk, const CUtensorMap* mv, const int32_t* units, int num_units, cudaStream_t stream);
+}  // namespace prompt
+
 template <int DK, int DV, int FORM>
 static int launch_prefill(Params& p, const int32_t* units, int num_units, cudaStream_t stream) {
   using C = Cfg<DK, DV>;
@@ -1321,8 +1328,10 @@ static int launch_prefill(Params& p, const int32_t* units, int num_units, cudaSt
   if (ensure_dynamic_smem(paged_prefill_kernel<DK, DV, FORM>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
   const int64_t ctas = static_cast<int64_t>(num_units) * p.nkv;
   if (ctas > 0x7fffffff) return B200_ERR_INVALID_ARGUMENT;
-  const int rc = launch_pdl(paged_prefill_kernel<DK, DV, FORM>, dim3(static_cast<unsigned>(ctas)), dim3(kThreads), C::kSmemBytes, stream,
-                            *mk, *mv, p, units);
+  const int rc = prompt::preferred(p, units, num_units)
+                     ? prompt::launch<DK, DV, FORM>(p, mk, mv, units, num_units, stream)
+                     : launch_pdl(paged_prefill_kernel<DK, DV, FORM>, dim3(static_cast<unsigned>(ctas)), dim3(kThreads), C::kSmemBytes, stream,
+                                  *mk, *mv, p, units);
   if (rc != B200_OK || !p.diff) return rc;
   return launch_diff_combine<__nv_bfloat16>(p, p.gate, p.out, DV, 1, stream);
 }

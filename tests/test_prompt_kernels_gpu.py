@@ -1,4 +1,7 @@
-"""Kernels for many tokens (prompts) at the edges of their tiles: GEMMs of CTA pairs."""
+"""Kernels for many tokens (prompts) at the edges of their tiles: GEMMs of CTA pairs, attention over blocks of 256 query rows."""
+import ctypes
+import math
+
 import pytest
 import torch
 
@@ -93,3 +96,124 @@ def test_pair_gemm_mxfp8_swiglu_equals_gemm_then_activation(ops, M, F, K):
     r, b = torch.arange(M)[:, None], torch.arange(F // 32)[None, :]
     at = ((r // 128) * (F // 128) * 512 + (b // 4) * 512 + (r % 32) * 16 + ((r % 128) // 32) * 4 + b % 4).reshape(-1).cuda()
     assert torch.equal(got.q, want.q) and torch.equal(got.sf[at], want.sf[at])
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+# Attention over prompts: units of several requests in one CTA, portions behind a past, short last units, every option of the separate layouts,
+# NaN in every pool row that no token wrote.  The output's bf16 rounding is 1.7e-3; the weights' hi + lo terms and fp32 sums add less than 1e-4.
+# ---------------------------------------------------------------------------------------------------------------------
+LENS, PAST = [700, 333, 1, 300, 900, 64], [0, 0, 300, 513, 64, 1]
+
+
+@pytest.mark.parametrize("form,heads,groups,dim,vdim,chunk,options", [
+    ("fused", 32, 8, 128, 128, 64, {}),
+    ("fused", 16, 16, 64, 64, 256, {}),
+    ("separate", 16, 8, 128, 128, 128, {"window": 200}),
+    ("separate", 24, 8, 64, 128, 64, {}),
+    ("separate", 16, 8, 128, 128, 64, {"window": 1}),
+    ("extra", 16, 8, 96, 72, 64, {"window": 150, "keep": 5, "sinks": True}),
+    ("extra", 16, 8, 128, 128, 256, {"window": 300, "cap": 5.0, "gates": "head"}),
+    ("extra", 16, 8, 128, 128, 64, {"window": 300, "keep": 70, "bias": 100, "cap": 7.0, "sinks": True}),
+    ("extra", 48, 8, 64, 64, 64, {"bias": 40}),
+    ("extra", 16, 16, 128, 128, 64, {"sinks": True, "gates": "value"}),
+    ("maps", 16, 8, 64, 128, 64, {}),
+])
+def test_prompt_attention_matches_the_plain_one(ops, form, heads, groups, dim, vdim, chunk, options):
+    from megatron_mixtera_b200 import _lib
+
+    o = {"window": 0, "keep": 0, "sinks": False, "cap": 0.0, "bias": 0, "gates": None, **options}
+    maps, dev = 2 if form == "maps" else 1, "cuda"
+    group, T, kv = heads // groups, sum(LENS), [n + p for n, p in zip(LENS, PAST)]
+    blocks = [-(-n // chunk) for n in kv]
+    order = torch.randperm(sum(blocks), generator=torch.Generator().manual_seed(1)).tolist()
+    table = torch.zeros(len(kv), max(blocks), dtype=torch.int32)
+    key_width = groups * maps * dim
+    width = key_width + groups * vdim
+    pool = torch.full((sum(blocks) + 1, chunk, width), float("nan"), dtype=BF16, device=dev)
+    keys, values = [], []
+    for r, n in enumerate(kv):
+        k, v = randn(n, key_width, seed=100 + r), randn(n, groups * vdim, seed=200 + r)
+        keys.append(k.view(n, groups, maps, dim)), values.append(v.view(n, groups, vdim))
+        rows = torch.cat([k, v], dim=1)
+        for b in range(blocks[r]):
+            table[r, b] = order.pop()
+            part = rows[b * chunk: (b + 1) * chunk]
+            pool[int(table[r, b]), : len(part)] = part
+    q = randn(T, groups, group, maps, dim, seed=3)
+    lengths = torch.cat([torch.arange(p + 1, p + n + 1) for n, p in zip(LENS, PAST)]).int().to(dev)
+    unit, units, t = 64 // group, [], 0
+    for r, n in enumerate(LENS):
+        units += [(r, t + a, min(unit, n - a), 0) for a in range(0, n, unit)]
+        t += n
+    units += [(0, 0, 0, 0)] * 3  # padding entries
+    units, table = torch.tensor(units, dtype=torch.int32, device=dev), table.to(dev)
+    assert -(-len(units) // 4) * groups * maps * 2 >= 148  # (fewer take the kernel for few units)
+    out = torch.full((T, heads * vdim), float("nan"), dtype=BF16, device=dev)
+
+    a = _lib.AttentionArgs()
+    if form == "fused":
+        qkv = torch.zeros(T, groups, group + 2, dim, dtype=BF16, device=dev)
+        qkv[:, :, :group] = q[:, :, :, 0]
+        pools = [pool[..., :key_width].contiguous(), pool[..., key_width:].contiguous()]
+        a.qkv, a.k_cache, a.v_cache = qkv.data_ptr(), pools[0].data_ptr(), pools[1].data_ptr()
+    else:
+        a.qkv, a.k_cache, a.v_cache = q.data_ptr(), pool.data_ptr(), pool.data_ptr() + 2 * key_width
+        a.separate, a.value_dim, a.pool_row_elems, a.window = (1 if form == "separate" else 2), vdim, width, o["window"]
+    sinks = torch.randn(heads, generator=torch.Generator().manual_seed(4)).to(dev)
+    bias = torch.randn(heads, max(o["bias"], 1), generator=torch.Generator().manual_seed(5)).to(dev)
+    gates = randn(T, heads * (vdim if o["gates"] != "head" else 1), seed=6)
+    work = torch.empty(T * 2 * heads * 129, device=dev)
+    if a.separate == 2:
+        a.out_scale, a.keep_first, a.softcap = 0.75, o["keep"], o["cap"]
+        if o["sinks"]:
+            a.sinks = sinks.data_ptr()
+        if o["bias"]:
+            a.distance_bias, a.bias_len = bias.data_ptr(), o["bias"]
+        if o["gates"] or maps == 2:
+            a.gate, a.gate_ld, a.value_gates = gates.data_ptr(), gates.shape[1], int(o["gates"] == "value")
+    if maps == 2:
+        a.maps, a.diff_scale, a.eps, a.workspace, a.workspace_bytes = 2, 0.7, 1e-5, work.data_ptr(), work.numel() * 4
+        a.lambda_ = 0.4
+    a.block_table, a.kv_seq_lengths, a.out = table.data_ptr(), lengths.data_ptr(), out.data_ptr()
+    a.num_tokens, a.num_q_heads, a.num_kv_heads, a.head_dim, a.chunk_size = T, heads, groups, dim, chunk
+    a.num_chunks, a.max_chunks_per_row, a.num_splits = pool.shape[0], table.shape[1], 1
+    rc = _lib.load().b200_paged_prefill_attention(ctypes.byref(a), units.data_ptr(), len(units), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert rc == 0 and ops.device_status() == 0
+
+    def plain(qs, ks, vs, past, n):  # [n, heads, dim], [keys, groups, dim], [keys, groups, vdim]
+        ks, vs = (x.double().repeat_interleave(group, 1) for x in (ks, vs))
+        s = torch.einsum("qhd,khd->hqk", qs.double(), ks) * dim ** -0.5
+        age = torch.arange(past, past + n, device=dev)[:, None] - torch.arange(past + n, device=dev)[None]
+        seen = age >= 0
+        if o["window"]:
+            seen &= (age < o["window"]) | (torch.arange(past + n, device=dev) < o["keep"])
+        if o["cap"]:
+            s = o["cap"] * torch.tanh(s / o["cap"])
+        if o["bias"]:
+            s = s + bias.double()[:, age.clamp(0, o["bias"] - 1)]
+        s = s.masked_fill(~seen, -math.inf)
+        if o["sinks"]:
+            s = torch.cat([s, sinks.double()[:, None, None].expand(-1, n, 1)], dim=-1)
+        return torch.einsum("hqk,khv->qhv", torch.softmax(s, dim=-1)[..., : past + n], vs)
+
+    want, t = [], 0
+    for r, (n, p) in enumerate(zip(LENS, PAST)):
+        qs = q[t: t + n].reshape(n, heads, maps, dim)
+        y = [plain(qs[:, :, m], keys[r][:, :, m], values[r], p, n) for m in range(maps)]
+        y = y[0] if maps == 1 else y[0] - 0.4 * y[1]
+        if maps == 2:
+            y = y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5) * 0.7
+        g = torch.sigmoid(gates[t: t + n].double())
+        if maps == 2 or o["gates"] == "value":
+            y = y * g.view(n, heads, vdim)
+        elif o["gates"] == "head":
+            y = y * g[:, :, None]
+        want.append(y * (0.75 if a.separate == 2 else 1.0))
+        t += n
+    want = torch.cat(want).reshape(T, -1)
+    assert not torch.isnan(out.float()).any()
+    assert rel(out, want) < (4e-3 if maps == 2 else 2.5e-3)
+    # one bf16 rounding is at most 2^-9 of a value; what the weights and sums add is small beside the outputs' scale
+    off = (out.double() - want).abs() - 2 ** -8 * want.abs()
+    assert float(off.max() / want.square().mean().sqrt()) < 1e-2
