@@ -9,6 +9,7 @@ the C ABI directly through ctypes.  Nothing here computes on the CPU or through 
 from __future__ import annotations
 
 import ctypes
+import weakref
 from typing import Optional, Tuple
 
 import torch
@@ -114,9 +115,15 @@ def _launch(name: str, *args):
 
 
 def _blob(struct) -> torch.Tensor:
-    """The bytes of a ctypes argument struct as a CPU uint8 tensor sharing its memory.  (Not kept on the struct: the tensor's storage holds the
-    struct, a cycle that no collector sees, and with it whatever else hangs on the struct - a key/value pool, expanded keys.)"""
-    return torch.frombuffer(struct, dtype=torch.uint8)
+    """The bytes of a ctypes argument struct as a CPU uint8 tensor sharing its memory, the same one for as long as a caller holds it.  (The struct
+    refers to it weakly: the tensor's storage holds the struct, so a strong reference would close a cycle that no collector sees, and keep whatever
+    else hangs on the struct - a key/value pool, expanded keys.)"""
+    kept = getattr(struct, "_blob_kept", None)
+    blob = None if kept is None else kept()
+    if blob is None:
+        blob = torch.frombuffer(struct, dtype=torch.uint8)
+        struct._blob_kept = weakref.ref(blob)
+    return blob
 
 
 def set_wait_limit_ns(limit_ns: int) -> None:
