@@ -1311,6 +1311,11 @@ static int launch_umma(const b200_latent_args& a, cudaStream_t s) {
   return launch_pdl(latent_combine_kernel, dim3(a.num_tokens * a.heads), dim3(128), 0, s, a);
 }
 
+namespace prompt {  // long prompts (latent_prompt.cu)
+static bool applicable(const b200_latent_args& a);
+static int launch_by_size(const b200_latent_args& a, cudaStream_t s);
+}  // namespace prompt
+
 template <int STEPS, int MAXV>
 static int launch_prompt(const b200_latent_args& a, cudaStream_t s) {
   static std::atomic<uint64_t> done{0};
@@ -1444,6 +1449,7 @@ int b200_latent_prompt_attention(const b200_latent_args* a, b200_stream_t stream
   if (a->value_gates && (a->gate_offset < 0 || a->gate_offset % 2 != 0 || a->gate_offset + a->heads * a->vdim > a->proj_ld))
     return B200_ERR_INVALID_ARGUMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (prompt::applicable(*a)) return prompt::launch_by_size(*a, s);
   const int steps = (a->dim + 15) / 16 + (a->rot_dim + 15) / 16;
   return steps <= 8 && a->vdim <= 64 ? launch_prompt<8, 64>(*a, s) : launch_prompt<kPrSteps, kPrMaxV>(*a, s);
 }

@@ -217,3 +217,66 @@ def test_prompt_attention_matches_the_plain_one(ops, form, heads, groups, dim, v
     # one bf16 rounding is at most 2^-9 of a value; what the weights and sums add is small beside the outputs' scale
     off = (out.double() - want).abs() - 2 ** -8 * want.abs()
     assert float(off.max() / want.square().mean().sqrt()) < 1e-2
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+# Latent attention of prompts on expanded keys: rows that start and that continue, windows, value and head gates, key sizes of one to three tiles of 64.
+# ---------------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("dim,rot,vdim,window,gates,sinks", [
+    (128, 64, 128, None, "head", False), (24, 16, 40, 33, "head", False), (64, 32, 64, 1, "head", True), (112, 8, 72, 150, "value", True),
+    (72, 0, 128, None, "value", True), (128, 64, 128, 257, "head", False)])
+def test_latent_prompts_match_the_plain_attention(ops, dim, rot, vdim, window, gates, sinks):
+    from megatron_mixtera_b200 import _lib
+
+    heads, lens, past, dev = 40, [300, 1, 700, 257], [0, 40, 65, 0], "cuda"
+    T, rows = sum(lens), len(lens)
+    first = [0 if window is None else max(0, p - window + 1) for p in past]
+    count = [n + p - f for n, p, f in zip(lens, past, first)]
+    E, kv_pad = sum(count), 48
+    width = -(-(kv_pad + rot) // 32) * 32
+    kv = randn(E, heads * (dim + vdim), seed=1)
+    key_rows = randn(E, width, seed=2)
+    key_rows[:, kv_pad + rot:] = 0
+    q, gate = randn(T, heads, dim + rot, seed=3), randn(T, heads * (vdim if gates == "value" else 1), seed=4)
+    gate_at = heads * (dim + rot)
+    proj = torch.zeros(T, gate_at + -(-gate.shape[1] // 8) * 8, dtype=BF16, device=dev)
+    proj[:, :gate_at], proj[:, gate_at: gate_at + gate.shape[1]] = q.reshape(T, -1), gate
+    q_rot = torch.zeros(T, heads, max(width - kv_pad, 8), dtype=BF16, device=dev)
+    q_rot[..., :rot] = q[..., dim:]
+    sink = torch.randn(heads, generator=torch.Generator().manual_seed(5)).to(dev)
+    out = torch.full((T, heads * vdim), float("nan"), dtype=BF16, device=dev)
+
+    def running(xs):
+        return torch.tensor([0] + xs).cumsum(0).int().to(dev)
+
+    cu_tokens, cu_keys, key_start = running(lens), running(count), torch.tensor(first, dtype=torch.int32, device=dev)
+    a = _lib.LatentArgs()
+    a.proj, a.proj_ld, a.gate_offset, a.value_gates = proj.data_ptr(), proj.shape[1], gate_at, int(gates == "value")
+    a.q_full, a.q_stride, a.q_rot_at, a.out = q_rot.data_ptr(), q_rot.shape[2], 0, out.data_ptr()
+    a.num_tokens, a.heads, a.dim, a.rot_dim, a.rot_dims, a.vdim = T, heads, dim, rot, rot, vdim
+    a.kv_rank, a.kv_pad, a.row_width, a.window, a.scale = kv_pad, kv_pad, width, window or 0, (dim + rot) ** -0.5
+    a.dtype, a.max_positions, a.num_splits, a.chunk_size, a.num_chunks, a.pool = ops.dtype_code(BF16), 1, 1, 64, 1, key_rows.data_ptr()
+    if sinks:
+        a.sinks = sink.data_ptr()
+    a.cu_tokens, a.cu_keys, a.key_start, a.key_rows, a.key_values = (t.data_ptr() for t in (cu_tokens, cu_keys, key_start, key_rows, kv))
+    a.num_rows, a.num_keys, a.max_row_tokens = rows, E, max(lens)
+    assert -(-max(lens) // 256) * rows * heads * 2 >= 148  # (fewer take the kernel of 64 queries)
+    ops.latent_prompt_attention(a, kv)
+    torch.cuda.synchronize()
+    t = e = 0
+    want = torch.empty(T, heads, vdim, dtype=torch.float64, device=dev)
+    for n, p, f, c in zip(lens, past, first, count):
+        k = torch.cat([kv[e: e + c, : heads * dim].view(c, heads, dim), key_rows[e: e + c, None, kv_pad: kv_pad + rot].expand(-1, heads, -1)], dim=-1).double()
+        v = kv[e: e + c, heads * dim:].view(c, heads, vdim).double()
+        s = torch.einsum("qhd,khd->hqk", q[t: t + n].double(), k) * a.scale
+        age = torch.arange(p, p + n, device=dev)[:, None] - torch.arange(f, f + c, device=dev)[None]
+        s = s.masked_fill((age < 0) | (age >= (window or 1 << 30)), -math.inf)
+        if sinks:
+            s = torch.cat([s, sink.double()[:, None, None].expand(-1, n, 1)], dim=-1)
+        want[t: t + n] = torch.einsum("hqk,khv->qhv", torch.softmax(s, dim=-1)[..., :c], v)
+        t, e = t + n, e + c
+    want *= torch.sigmoid(gate.double()).view(T, heads, -1)
+    want = want.reshape(T, -1)
+    assert not torch.isnan(out.float()).any() and rel(out, want) < 2.5e-3
+    off = (out.double() - want).abs() - 2 ** -8 * want.abs()
+    assert float(off.max() / want.square().mean().sqrt()) < 1e-2
