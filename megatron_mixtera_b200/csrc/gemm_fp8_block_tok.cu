@@ -1,19 +1,22 @@
-// Block-scaled FP8 GEMM (fp32 scales: 128 x 128 weight blocks, 1 x 128 token blocks) for token blocks of 128 and 256:
-// the 70B configuration's batch.  Same arithmetic as gemm_fp8_block.cu, other orientation.
+// Block-scaled FP8 GEMM (fp32 scales: 128 x 128 weight blocks, 1 x 128 token blocks) for more than 64 tokens: the 70B configuration's batch, and
+// prompts.  Same arithmetic as gemm_fp8_block.cu, other orientation.
 //
-// Here the TOKENS are the UMMA "M" side (one TMEM lane per token, 128 per MMA, two MMAs for 256 tokens) and the 128
-// weight rows of the CTA's tile are the "N" side (one TMEM column per output feature).  What that buys:
+// Here the TOKENS are the UMMA "M" side (one TMEM lane per token, 128 per CTA) and the weight rows of the CTA's one or two tiles are the "N" side (one
+// TMEM column per output feature).  What that buys:
 //   * a promoter thread owns ONE token, so the token scale of a K block is one scalar per thread and the promotion is
 //     one FFMA per accumulator element (the weight-major form needs a multiply and a shared-memory read per element
 //     on top, and was 5 x off the weight-streaming time at 256 tokens);
 //   * a thread ends up with 128 consecutive output features of its token: the epilogue stores 16-byte vectors
-//     straight from registers, no tensor-memory write-back, no transposition;
-//   * 256 tokens share every weight tile: each weight byte crosses from HBM once per 256 tokens.
+//     straight from registers, no tensor-memory write-back, no transposition.
+// Two weight tiles per CTA (more than 128 tokens) make products of N = 256, which read 12 KB of shared memory in 128 clocks; 256 tokens x one tile
+// made two of N = 128 at the 128 bytes per clock that shared memory delivers, beside the copies into it.  11000 tokens: 10240 x 8192 1171 -> 1020 us
+// (1810 TFLOP/s), 57344 x 8192 6.80 -> 6.25 ms, 8192 x 28672 3.16 -> 2.94 ms; 256 tokens: 230 -> 209, 107 -> 100 us.  What bounds it now is the chain products ->
+// commit -> promotion -> release over the two accumulators that tensor memory holds: without any copies it runs at the same rate.
 //
-//   warps 0 .. 4H-1 : promoters (H = 1 or 2 halves of 128 tokens; warp w: lane quadrant w % 4 of half w / 4)
-//   warp 4H, lane 0 : producer - per stage (= one K block) the token tile [H * 128 x 128 B], the weight tile
-//                     [128 x 128 B, tile-major] (TMA, 128-byte swizzle) and the tokens' scales (bulk copy)
-//   warp 4H+1, lane 0 : UMMA   - 4 x tcgen05.mma kind::f8f6f4 per half into one of two accumulator buffers
+//   warps 0 .. 4H-1 : promoters (H = 1 or 2 weight tiles; warp w: lane quadrant w % 4 of tile w / 4)
+//   warp 4H, lane 0 : producer - per stage (= one K block) the token tile [128 x 128 B], the weight tiles
+//                     [128 x 128 B each, tile-major] (TMA, 128-byte swizzle) and the tokens' scales (bulk copy)
+//   warp 4H+1, lane 0 : UMMA   - 4 x tcgen05.mma kind::f8f6f4 into one of two accumulator buffers
 #include "common.cuh"
 
 namespace b200 {
@@ -29,20 +32,20 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
       : "memory");
 }
 
-constexpr int kGroupM = 8;
+constexpr int kGroupM = 16;  // token blocks of a group of tiles
 
 template <int H>
 struct TokConfig {
-  static constexpr int kTokens = H * 128;
+  static constexpr int kTokens = 128;
   static constexpr int kPromoterWarps = 4 * H;
   static constexpr int kThreads = (kPromoterWarps + 2) * 32;
   static constexpr int kStageBytesX = kTokens * 128;
   static constexpr int kOffW = kStageBytesX;
-  static constexpr int kOffScale = kOffW + kTileN * 128;
+  static constexpr int kOffScale = kOffW + H * kTileN * 128;
   static constexpr int kStageBytes = (kOffScale + kTokens * 4 + 1023) / 1024 * 1024;
   static constexpr int kStages = 4;
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
-  static constexpr int kTmemCols = 2 * H * 128;  // two buffers of H accumulators, 128 feature columns each
+  static constexpr int kTmemCols = 2 * H * 128;  // two buffers of H x 128 feature columns
 };
 
 template <int H>
@@ -63,13 +66,12 @@ gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   const int warp = tid >> 5;
   const int lane = tid & 31;
   // Tiles in groups of kGroupM token blocks, token blocks innermost: the CTAs that run at a time share both operands in L2.  (With the weight tiles
-  // innermost every wave read other weights, all of them from HBM once per 256 tokens: 11000 x 57344 x 8192 7.8 ms, now 7.1 ms.)
+  // innermost every wave read other weights, all of them from HBM once per 256 tokens: 11000 x 57344 x 8192 7.8 ms, then 7.1 ms.)
   const int split = blockIdx.y;
   const int per_group = kGroupM * q.n_tiles, group = static_cast<int>(blockIdx.x) / per_group, in_group = static_cast<int>(blockIdx.x) - group * per_group;
   const int rows = min(kGroupM, q.m_blocks - group * kGroupM);
   const int n_tile = in_group / rows;
   const int m_block = group * kGroupM + (in_group - n_tile * rows);
-  const int n0 = n_tile * kTileN;
   const int m0 = m_block * C::kTokens;
   const int kb_begin = split * p.k_blocks_per_split;
   const int kb_end = min(p.num_k_blocks, kb_begin + p.k_blocks_per_split);
@@ -106,8 +108,11 @@ gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   if (warp == kProducerWarp) {
     if (lane == 0) {
       // ---------------- producer ----------------
-      auto load_w = [&](int i, int s) {  // weights are tile-major: tile (n_tile, k block) is 128 consecutive rows
-        tma_load_2d(smem + s * C::kStageBytes + C::kOffW, &map_w, &full_bar[s], 0, (n_tile * q.k_tiles + kb_begin + i) * kTileN);
+      auto load_w = [&](int i, int s) {  // weights are tile-major: a (tile, k block) is 128 consecutive rows
+#pragma unroll
+        for (int h = 0; h < H; ++h)  // (a second tile past the last one is filled with zeros)
+          tma_load_2d(smem + s * C::kStageBytes + C::kOffW + h * kTileN * 128, &map_w, &full_bar[s], 0,
+                      ((n_tile * H + h) * q.k_tiles + kb_begin + i) * kTileN);
       };
       auto load_x = [&](int i, int s) {
         uint8_t* stage = smem + s * C::kStageBytes;
@@ -134,7 +139,7 @@ gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   } else if (warp == kMmaWarp) {
     if (lane == 0) {
       // ---------------- UMMA issuer: D[token, feature] = X[token, k] * W[feature, k]^T ----------------
-      constexpr uint32_t idesc = umma_idesc_f8(128, kTileN);
+      constexpr uint32_t idesc = umma_idesc_f8(128, H * kTileN);
       for (int i = 0; i < num_kb; ++i) {
         const int s = i % C::kStages;
         const int b = i & 1;
@@ -143,13 +148,9 @@ gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
         tcgen05_fence_after_sync();
         const uint32_t stage_addr = smem_u32(smem + s * C::kStageBytes);
         const uint64_t w_desc = umma_desc_k_major_sw128(stage_addr + C::kOffW);
+        const uint64_t x_desc = umma_desc_k_major_sw128(stage_addr);
 #pragma unroll
-        for (int h = 0; h < H; ++h) {
-          const uint64_t x_desc = umma_desc_k_major_sw128(stage_addr + h * 128 * 128);
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_f8(tmem_base + (b * H + h) * 128, x_desc + 2 * k, w_desc + 2 * k, idesc, k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < 4; ++k) umma_f8(tmem_base + b * (H * 128), x_desc + 2 * k, w_desc + 2 * k, idesc, k > 0 ? 1u : 0u);
         umma_commit(&empty_bar[s]);
         umma_commit(&acc_full[b]);
       }
@@ -158,12 +159,14 @@ gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     // ---------------- promoters: one token per thread, 128 feature totals in registers ----------------
     pdl_wait();
     const int half = warp >> 2;
-    const int tok = half * 128 + (warp & 3) * 32 + lane;  // token of this thread inside the CTA's block
+    const int tok = (warp & 3) * 32 + lane;          // token of this thread inside the CTA's block
+    const int tile = n_tile * H + half;              // its weight tile
+    const int n0 = tile * kTileN;
     float total[kTileN];
 #pragma unroll
     for (int j = 0; j < kTileN; ++j) total[j] = 0.f;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + half * 128;
-    const float* w_scale = q.w_scale + static_cast<int64_t>(n_tile) * q.k_tiles + kb_begin;
+    const float* w_scale = q.w_scale + static_cast<int64_t>(min(tile, (p.N - 1) / kTileN)) * q.k_tiles + kb_begin;
     float sw_next = num_kb > 0 ? __ldg(w_scale) : 0.f;
     for (int i = 0; i < num_kb; ++i) {
       const int s = i % C::kStages;
@@ -196,7 +199,7 @@ gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
 
     // ---------------- epilogue: the thread's token row, 128 consecutive features, straight from registers ----------------
     const int m = m0 + tok;
-    if (m < p.M) {
+    if (m < p.M && n0 < p.N) {
       const bool full_tile = n0 + kTileN <= p.N;
       if (p.num_splits == 1 && !p.keep_partials) {
         __nv_bfloat16* dst = p.y + static_cast<int64_t>(m) * p.ldy + n0;
@@ -259,9 +262,9 @@ static int launch_fp8_block_tok(const void* xq, const float* x_scale, int m_pad,
   const CUtensorMap* mx_ = get_tensor_map(xq, 2, xd, xs, xb, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                           CU_TENSOR_MAP_DATA_TYPE_UINT8);
   if (!mw || !mx_) return B200_ERR_DRIVER;
-  const int m_blocks = (M + C::kTokens - 1) / C::kTokens;
+  const int m_blocks = (M + C::kTokens - 1) / C::kTokens, n_blocks = (n_tiles + H - 1) / H;
   const int num_kb = K / 128;
-  const int splits = choose_splits(n_tiles * m_blocks, num_kb, 1);  // 200 KiB of stages / 512 TMEM columns: one CTA per SM
+  const int splits = choose_splits(n_tiles * ((M + H * 128 - 1) / (H * 128)), num_kb, 1);  // 200 KiB of stages / 512 TMEM columns: one CTA per SM
   Params p;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.y = static_cast<__nv_bfloat16*>(y);
@@ -291,10 +294,10 @@ static int launch_fp8_block_tok(const void* xq, const float* x_scale, int m_pad,
   q.m_pad = m_pad;
   static std::atomic<uint64_t> smem_attr_done{0};
   if (ensure_dynamic_smem(gemm_fp8_block_tok_kernel<H>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
-  q.n_tiles = n_tiles;
+  q.n_tiles = n_blocks;
   q.m_blocks = m_blocks;
-  if (static_cast<int64_t>(n_tiles) * m_blocks > 0x7fffffff) return B200_ERR_INVALID_ARGUMENT;
-  dim3 grid(static_cast<unsigned>(n_tiles * m_blocks), splits);
+  if (static_cast<int64_t>(n_blocks) * m_blocks > 0x7fffffff) return B200_ERR_INVALID_ARGUMENT;
+  dim3 grid(static_cast<unsigned>(n_blocks * m_blocks), splits);
   const int rc = launch_pdl(gemm_fp8_block_tok_kernel<H>, grid, dim3(C::kThreads), C::kSmemBytes, stream, *mw, *mx_, p, q);
   if (rc != B200_OK || splits == 1 || p.keep_partials) return rc;
   return launch_splitk_reduce(p, stream);

@@ -280,3 +280,21 @@ def test_latent_prompts_match_the_plain_attention(ops, dim, rot, vdim, window, g
     assert not torch.isnan(out.float()).any() and rel(out, want) < 2.5e-3
     off = (out.double() - want).abs() - 2 ** -8 * want.abs()
     assert float(off.max() / want.square().mean().sqrt()) < 1e-2
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+# Blockwise FP8 over pairs of weight tiles (more than 128 tokens): an odd tile at the end, tokens inside the last block, K split or not.
+# ---------------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("M,N,K", [(129, 384, 512), (200, 2560, 4096), (257, 640, 128), (1000, 4224, 384), (4097, 1024, 512)])
+def test_blockwise_gemm_over_pairs_of_weight_tiles(ops, M, N, K):
+    from oracle import decode_oracle as O
+
+    x, w, b = randn(M, K, seed=1), randn(N, K, seed=2, scale=K ** -0.5), randn(N, seed=3)
+    xd, wd = O.dequantize_fp8_rowblock(*O.quantize_fp8_rowblock(x.cpu())), O.dequantize_fp8_block_weight(*O.quantize_fp8_block_weight(w.cpu()))
+    ref = (xd.double() @ wd.double().T).cuda()
+    xq, wq = ops.quantize_fp8_rowblock(x), ops.quantize_fp8_weight_block128(w)
+    assert rel(ops.gemm_fp8_block(xq, wq), ref) < 3e-3
+    assert rel(ops.gemm_fp8_block(xq, wq, b), ref.to(BF16).double() + b.double()) < 3e-3
+    parts = ops.gemm_splitk(xq, wq)
+    got = parts.buf.view(torch.float32)[: parts.num_splits * M * N].view(parts.num_splits, M, N).sum(0)
+    assert rel(got, ref) < 1e-5
