@@ -66,7 +66,8 @@ constexpr int kGatedSilu = 1, kGatedClamped = 2, kGatedPlain = 3;  // Params::ga
 
 // Many tokens: CTA pairs (gemm_pair.cu).
 namespace pair {
-static bool preferred(int M, int N);
+constexpr int kFewestRows = 256;
+static bool preferred(int M, int N, int fewest = kFewestRows);
 static int launch_bf16(const void* x, int64_t ldx, const void* w, const void* bias, void* y, int64_t ldy, int M, int N, int K, cudaStream_t stream,
                        float* partials, bool gated, int act);
 }  // namespace pair

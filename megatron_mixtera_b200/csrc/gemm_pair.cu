@@ -14,6 +14,8 @@
 // 1220 -> 1370; MXFP8, 13000 tokens, 28672 x 4096 with SwiGLU and quantisation: 1430 -> 2110, 4096 x 14336: 1410 -> 2100.  What bounds them now: power with
 // bf16 (cuBLAS reaches 1590 in the same run); with scales the copies of ~34 KB per K block and the read-out of the one accumulator.
 //
+// Experts' products (moe.cu) are the same kernel over a device-built list of (expert, first row, rows <= 256) entries, the shared expert's tiles in front.
+//
 // bf16 accumulators are double-buffered (2 x 256 columns = all of tensor memory); with scales there is one accumulator beside the scale slots, and
 // the eight epilogue warps read it out before they compute.  Tiles are walked in groups of kGroupM token blocks, features outermost within a group, so
 // that what the pairs work on at a time stays in L2.
@@ -29,7 +31,8 @@ constexpr int kThreadsPair = (kEpilogueWarps + 2) * 32;
 constexpr int kTile = 256;      // tokens, and features, of a pair's tile
 constexpr int kGroupM = 8;
 
-enum Form { kPlain, kGated64, kGatedHalves };  // features as they are; [64 gate | 64 up] rows; rank 0 holds gate rows, rank 1 the matching up rows
+// Features as they are; [64 gate | 64 up] rows; [16 gate | 16 up] rows (experts); rank 0 holds gate rows, rank 1 the matching up rows.
+enum Form { kPlain, kGated64, kGated16, kGatedHalves };
 
 template <bool MX>
 struct Config {
@@ -47,11 +50,24 @@ struct Config {
 };
 
 struct Args {
-  Params p;
+  Params p;         // experts: sizes of one expert's problem (N: weight rows per expert)
   uint8_t* q_out;   // kGatedHalves: E4M3 [M][F] and its scales instead of y
   uint8_t* sf_out;
   int k_tiles;      // K / 128 (scaled operands)
   int m_tiles, n_tiles, tiles;
+  // Experts: tokens sorted by expert, a device-built list of (expert, first row, rows <= 256) entries instead of m_tiles.  A second problem (a shared
+  // expert: all tokens, weights and sizes of its own) may come in front of it.
+  Params shared;
+  const int4* list;
+  const int32_t* list_length;
+  int list_capacity, experts, shared_n_tiles, shared_tiles;
+};
+
+// One 256 x 256 tile of work.
+struct Unit {
+  const Params* p;
+  int m0, m_end, nt, w_row;  // first token row and the end of the rows it may write, feature block, first weight row
+  bool shared;
 };
 
 __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
@@ -80,13 +96,6 @@ __device__ __forceinline__ void tmem_cp_32x128b_warpx4_pair(uint32_t taddr, uint
   asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(smem_desc) : "memory");
 }
 
-// Arrives on the barrier at this offset in BOTH CTAs once the pair's MMAs issued so far have completed.  (Two single commits per stage instead cost
-// 3-7 % of the rate at K = 4096 and 14336.)
-__device__ __forceinline__ void umma_commit_both(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "h"(static_cast<uint16_t>(3))
-               : "memory");
-}
 // 16 consecutive bf16 outputs (32 bytes, one sector) of a token.
 __device__ __forceinline__ void store16(__nv_bfloat16* dst, const float* v, int count, bool vec) {
   if (vec) {
@@ -108,7 +117,7 @@ __device__ __forceinline__ float swiglu_rounded(uint32_t g_bits, uint32_t u_bits
   return bf16_round(bf16_round(g / (1.f + expf(-g))) * u);
 }
 
-template <bool MX, int FORM>
+template <bool MX, int FORM, bool EXPERTS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsPair, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                  const __grid_constant__ CUtensorMap map_sfw, const __grid_constant__ CUtensorMap map_sfx, const __grid_constant__ Args a) {
@@ -123,11 +132,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const Params& p = a.p;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_cta_rank();  // 0 = leader
   const int first = blockIdx.x >> 1, stride = gridDim.x >> 1;
-  const int num_kb = p.num_k_blocks;
   constexpr int kProducerWarp = kEpilogueWarps, kMmaWarp = kEpilogueWarps + 1;
 
   if (tid == 0) {
@@ -155,28 +162,54 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   const uint32_t tmem_base = *tmem_slot;
   pdl_launch_dependents();
 
-  // tile number -> (token block, feature block)
-  auto place = [&](int tile, int& mt, int& nt) {
-    const int per_group = kGroupM * a.n_tiles;
-    const int group = tile / per_group, in = tile - group * per_group;
-    const int rows = min(kGroupM, a.m_tiles - group * kGroupM);
-    nt = in / rows;
-    mt = group * kGroupM + (in - nt * rows);
+  pdl_wait();  // operands (and the list of experts' tiles) are earlier kernels' output, and y may still be read by them
+  const int tiles = EXPERTS ? a.shared_tiles + min(*a.list_length, a.list_capacity) * a.n_tiles : a.tiles;
+  // tile number -> unit; false for an entry that no kernel of ours writes (every role leaves it out)
+  auto unit_of = [&](int tile, Unit& u) {
+    u.p = &a.p;
+    u.shared = false;
+    if constexpr (EXPERTS) {
+      if (tile < a.shared_tiles) {
+        u.p = &a.shared;
+        u.shared = true;
+        u.m0 = tile / a.shared_n_tiles * kTile;
+        u.nt = tile % a.shared_n_tiles;
+        u.m_end = a.shared.M;
+        u.w_row = u.nt * kTile;
+        return true;
+      }
+      const int4 e = a.list[(tile - a.shared_tiles) / a.n_tiles];
+      u.nt = (tile - a.shared_tiles) % a.n_tiles;
+      u.m0 = e.y;
+      u.m_end = min(e.y + min(e.z, kTile), a.p.M);
+      u.w_row = e.x * a.p.N + u.nt * kTile;
+      return static_cast<unsigned>(e.x) < static_cast<unsigned>(a.experts) && e.y >= 0 && e.z > 0;
+    } else {
+      const int per_group = kGroupM * a.n_tiles;
+      const int group = tile / per_group, in = tile - group * per_group;
+      const int rows = min(kGroupM, a.m_tiles - group * kGroupM);
+      u.nt = in / rows;
+      u.m0 = (group * kGroupM + (in - u.nt * rows)) * kTile;
+      u.m_end = a.p.M;
+      u.w_row = u.nt * kTile;
+      return true;
+    }
   };
 
   if (warp == kProducerWarp) {
     if (lane == 0) {
       const uint32_t leader_full0 = cluster_addr_of(&full_bar[0], 0);  // (barriers are 8 bytes apart)
-      pdl_wait();
       int it = 0;
-      for (int tile = first; tile < a.tiles; tile += stride) {
-        int mt, nt;
-        place(tile, mt, nt);
-        const int m0 = mt * kTile + static_cast<int>(rank) * 128;
-        // this CTA's weight tile (128 rows), and the two whose scales both CTAs need
-        const int tile0 = FORM == kGatedHalves ? nt : 2 * nt;
-        const int tile1 = FORM == kGatedHalves ? nt + a.n_tiles : 2 * nt + 1;
+      for (int tile = first; tile < tiles; tile += stride) {
+        Unit u;
+        if (!unit_of(tile, u)) continue;
+        const int m0 = u.m0 + static_cast<int>(rank) * 128, num_kb = u.p->num_k_blocks;
+        // scaled operands: this CTA's weight tile (128 rows), and the two whose scales both CTAs need
+        const int tile0 = FORM == kGatedHalves ? u.nt : 2 * u.nt;
+        const int tile1 = FORM == kGatedHalves ? u.nt + a.n_tiles : 2 * u.nt + 1;
         const int w_tile = rank == 0 ? tile0 : tile1;
+        const CUtensorMap* mx_ = EXPERTS && u.shared ? &map_sfx : &map_x;  // (without scales those maps are the second problem's)
+        const CUtensorMap* mw = EXPERTS && u.shared ? &map_sfw : &map_w;
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % C::kStages;
           mbar_wait_bounded(&empty_bar[s], ((it / C::kStages) & 1) ^ 1, abort_flag, kStatusGemmTimeout);
@@ -190,8 +223,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             tma_load_2d_pair(stage + C::kOffSfW, &map_sfw, full, 0, tile0 * a.k_tiles + kb);
             tma_load_2d_pair(stage + C::kOffSfW + 512, &map_sfw, full, 0, tile1 * a.k_tiles + kb);
           } else {
-            tma_load_2d_pair(stage, &map_x, full, kb * 64, m0);
-            tma_load_2d_pair(stage + C::kStageX, &map_w, full, kb * 64, w_tile * 128);
+            tma_load_2d_pair(stage, mx_, full, kb * 64, m0);
+            tma_load_2d_pair(stage + C::kStageX, mw, full, kb * 64, u.w_row + static_cast<int>(rank) * 128);
           }
         }
       }
@@ -200,7 +233,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     if (lane == 0 && rank == 0) {
       // ------- UMMA issuer (leader): D[token, feature] = X[token, k] * W[feature, k]^T, 256 x 256 per pair -------
       int it = 0, n = 0;
-      for (int tile = first; tile < a.tiles; tile += stride, ++n) {
+      for (int tile = first; tile < tiles; tile += stride) {
+        Unit u;
+        if (!unit_of(tile, u)) continue;
+        const int num_kb = u.p->num_k_blocks;
         const int b = n % C::kBuffers;
         mbar_wait_bounded(&acc_empty[b], ((n / C::kBuffers) & 1) ^ 1, abort_flag, kStatusGemmTimeout);
         const uint32_t acc = tmem_base + b * kTile;
@@ -227,21 +263,24 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           umma_commit_both(&empty_bar[s]);
         }
         umma_commit_both(&acc_full[b]);
+        ++n;
       }
     }
   } else {
     // ---------------- epilogue: lane quadrant = warp % 4, 128 of the 256 columns per warp ----------------
-    pdl_wait();  // the outputs may still be read by the previous kernel until here
     const int quad = warp & 3, half = warp >> 2;
     const uint32_t leader_acc_empty0 = cluster_addr_of(&acc_empty[0], 0);
     int n = 0;
-    for (int tile = first; tile < a.tiles; tile += stride, ++n) {
-      int mt, nt;
-      place(tile, mt, nt);
+    for (int tile = first; tile < tiles; tile += stride) {
+      Unit u;
+      if (!unit_of(tile, u)) continue;
+      const Params& p = *u.p;
+      const int nt = u.nt;
       const int b = n % C::kBuffers;
-      const int m = mt * kTile + static_cast<int>(rank) * 128 + quad * 32 + lane;  // this thread's token
-      const bool m_ok = m < p.M;
+      const int m = u.m0 + static_cast<int>(rank) * 128 + quad * 32 + lane;  // this thread's token
+      const bool m_ok = m < u.m_end;
       mbar_wait_bounded(&acc_full[b], (n / C::kBuffers) & 1, abort_flag, kStatusGemmTimeout);
+      ++n;
       tcgen05_fence_after_sync();
       const uint32_t acc = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + b * kTile;
       auto release = [&] {
@@ -294,6 +333,28 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             }
             if (left > 0) store16(dst + j, v, left, vec && left >= 16);
           }
+        }
+      } else if constexpr (FORM == kGated16) {
+        // columns [16 gate | 16 up] in turn: this warp's 128 columns give 64 outputs
+        const int o0 = nt * 128 + half * 64;
+        const uint32_t from = acc + half * 128;
+        const bool vec = (p.ldy & 7) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
+        const float scale = p.row_scale != nullptr && m_ok ? p.row_scale[m] : 1.f;
+#pragma unroll 1
+        for (int c0 = 0; c0 < 128; c0 += 32) {
+          uint32_t r[32];
+          __syncwarp();
+          tmem_ld_32x32b_x32(from + c0, r);
+          tmem_ld_wait();
+          if (c0 == 96) release();
+          if (!m_ok || o0 + c0 / 2 >= (p.N >> 1)) continue;
+          float v[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            const float gt = __uint_as_float(r[k]) * scale, up = __uint_as_float(r[16 + k]) * scale;
+            v[k] = p.gated == kGatedPlain ? __fdividef(gt, 1.f + __expf(-gt)) * up : clamped_glu_fast(gt, up, p.glu_limit, p.glu_alpha);
+          }
+          store16(p.y + static_cast<int64_t>(m) * p.ldy + o0 + c0 / 2, v, 16, vec);
         }
       } else if constexpr (FORM == kGated64) {
         // columns [64 gate | 64 up] twice: this warp's 128 columns give 64 outputs
@@ -374,23 +435,25 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   if (warp == kProducerWarp) tmem_dealloc_pair(tmem_base, C::kTmemCols);
 }
 
-// Whether the pairs' tiles are the better split: at least one for every pair of SMs.  (64 tiles, 1024 tokens x 4096 x 4096: 48.8 us here, 44.2 us with
-// K split over the streaming kernel's CTAs; 96 tiles, MXFP8 1024 x 6144 x 4096: 47.9 and 48.5 us.)
-static bool preferred(int M, int N) {
+// Whether the pairs' tiles are the better split: more rows than `fewest`, and at least one tile for every pair of SMs.  (64 tiles, 1024 tokens x 4096 x
+// 4096: 48.8 us here, 44.2 us with K split over the streaming kernel's CTAs; 96 tiles, MXFP8 1024 x 6144 x 4096: 47.9 and 48.5 us.)
+static bool preferred(int M, int N, int fewest) {
   const int64_t tiles = static_cast<int64_t>((M + kTile - 1) / kTile) * ((N + kTile - 1) / kTile);
-  return M > 256 && tiles >= sm_count() / 2;
+  return M > fewest && tiles >= sm_count() / 2;
 }
 
-template <bool MX, int FORM>
+template <bool MX, int FORM, bool EXPERTS = false>
 static int launch(Args& a, const CUtensorMap* mw, const CUtensorMap* mx_, const CUtensorMap* msw, const CUtensorMap* msx, cudaStream_t stream) {
   using C = Config<MX>;
-  a.m_tiles = (a.p.M + kTile - 1) / kTile;
   a.n_tiles = (a.p.N + kTile - 1) / kTile;
-  a.tiles = a.m_tiles * a.n_tiles;
+  if (!EXPERTS) {
+    a.m_tiles = (a.p.M + kTile - 1) / kTile;
+    a.tiles = a.m_tiles * a.n_tiles;
+  }
   static std::atomic<uint64_t> smem_attr_done{0};
-  if (ensure_dynamic_smem(gemm_pair_kernel<MX, FORM>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
+  if (ensure_dynamic_smem(gemm_pair_kernel<MX, FORM, EXPERTS>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
   const int pairs = min(sm_count() / 2, a.tiles);
-  return launch_pdl(gemm_pair_kernel<MX, FORM>, dim3(2 * pairs), dim3(kThreadsPair), C::kSmemBytes, stream, *mw, *mx_, *msw, *msx, a);
+  return launch_pdl(gemm_pair_kernel<MX, FORM, EXPERTS>, dim3(2 * pairs), dim3(kThreadsPair), C::kSmemBytes, stream, *mw, *mx_, *msw, *msx, a);
 }
 
 static Params params(void* y, int64_t ldy, const void* bias, int M, int N, int K, int k_block, int act, float* partials) {
@@ -447,6 +510,45 @@ static int launch_mxfp8(const void* xq, const void* x_sf, const void* wq, const 
   a.q_out = static_cast<uint8_t*>(q_out);
   a.sf_out = static_cast<uint8_t*>(sf_out);
   return halves ? launch<true, kGatedHalves>(a, mw, mx_, msw, msx, stream) : launch<true, kPlain>(a, mw, mx_, msw, msx, stream);
+}
+
+// Experts' products (and the shared expert's, where there is one) over a list of 256-row entries.
+static int launch_experts(const GroupedProblem& routed, const GroupedProblem& shared, const GroupedParams& gp, cudaStream_t stream) {
+  auto maps = [&](const GroupedProblem& g, const Params& p, const CUtensorMap*& mw, const CUtensorMap*& mx_) {
+    const uint64_t wd[2] = {static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.N) * g.experts}, xd[2] = {static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.M)};
+    const uint64_t ws[1] = {static_cast<uint64_t>(p.K) * 2}, xs[1] = {static_cast<uint64_t>(g.ldx) * 2};
+    const uint32_t box[2] = {64, 128};
+    mw = get_tensor_map(g.w, 2, wd, ws, box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    mx_ = get_tensor_map(g.x, 2, xd, xs, box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    return mw && mx_;
+  };
+  const CUtensorMap *mw, *mx_;
+  if (!maps(routed, gp.routed, mw, mx_)) return B200_ERR_DRIVER;
+  const CUtensorMap *mws = mw, *mxs = mx_;
+  Args a = {};
+  a.p = gp.routed;
+  a.shared_n_tiles = 1;
+  if (shared.x != nullptr) {
+    if (!maps(shared, gp.shared, mws, mxs)) return B200_ERR_DRIVER;
+    a.shared = gp.shared;
+    a.shared_n_tiles = (gp.shared.N + kTile - 1) / kTile;
+    a.shared_tiles = a.shared_n_tiles * ((gp.shared.M + kTile - 1) / kTile);
+  }
+  for (Params* p : {&a.p, &a.shared}) {
+    p->num_k_blocks = (p->K + 63) / 64;
+    p->num_splits = 1;
+    p->keep_partials = 0;
+    p->partials = nullptr;
+    p->bias = nullptr;
+  }
+  a.list = gp.tiles;
+  a.list_length = gp.num_tiles;
+  a.list_capacity = gp.max_tiles;
+  a.experts = gp.experts;
+  const int64_t most = a.shared_tiles + static_cast<int64_t>(gp.max_tiles) * ((gp.routed.N + kTile - 1) / kTile);
+  if (most > 0x7fffffff) return B200_ERR_INVALID_ARGUMENT;
+  a.tiles = static_cast<int>(most);
+  return gp.routed.gated != 0 ? launch<false, kGated16, true>(a, mw, mx_, mws, mxs, stream) : launch<false, kPlain, true>(a, mw, mx_, mws, mxs, stream);
 }
 
 }  // namespace pair

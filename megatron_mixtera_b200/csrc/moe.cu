@@ -393,7 +393,7 @@ static int grouped(const b200_moe_args& a, bool up, cudaStream_t s) {
     case 32: return gemm::launch_grouped<32>(routed, shared, gp, s);
     case 64: return gemm::launch_grouped<64>(routed, shared, gp, s);
     case 128: return gemm::launch_grouped<128>(routed, shared, gp, s);
-    case 256: return gemm::launch_grouped<256>(routed, shared, gp, s);
+    case 256: return gemm::pair::launch_experts(routed, shared, gp, s);
     default: return B200_ERR_INVALID_ARGUMENT;
   }
 }

@@ -34,9 +34,9 @@ def rel(a, b):
 # ---------------------------------------------------------------------------------------------------------------------
 SHAPES = [
     (257, 14336, 128),   # one token in the second token block
-    (1000, 4100, 72),    # K of one block and a bit, N 4 past a tile
-    (4097, 1000, 512),   # N inside the last tile's first half
-    (2048, 2048, 1000),  # K no multiple of a block
+    (1000, 4868, 72),    # K of one block and a bit, N 4 past a tile
+    (4097, 1128, 512),   # N inside the last tile's first half
+    (2048, 2560, 1000),  # K no multiple of a block
     (5000, 1160, 64),    # a single K block
     (300, 16384, 192),
 ]
@@ -58,7 +58,7 @@ def test_pair_gemm_matches_the_fp32_product(ops, M, N, K):
     assert torch.equal(wide[:, :N], ops.gemm(x, w)) and not wide[:, N:].any()
 
 
-@pytest.mark.parametrize("M,F,K", [(257, 7168, 256), (2048, 1024, 512), (1500, 3200, 72)])
+@pytest.mark.parametrize("M,F,K", [(257, 7168, 256), (2048, 1280, 512), (1500, 3200, 72)])
 def test_pair_gemm_swiglu_equals_gemm_then_activation(ops, M, F, K):
     x, w = randn(M, K, seed=4), randn(2 * F, K, seed=5, scale=K ** -0.5)
     assert ops.gemm_swiglu_supported(M, 2 * F, K)
@@ -66,7 +66,7 @@ def test_pair_gemm_swiglu_equals_gemm_then_activation(ops, M, F, K):
     assert torch.equal(got, ops.activation(ops.gemm(x, w), "swiglu"))
 
 
-@pytest.mark.parametrize("M,N,K", [(257, 14336, 128), (1000, 4224, 384), (4097, 1024, 512), (2048, 2048 + 40, 1024)])
+@pytest.mark.parametrize("M,N,K", [(257, 14336, 128), (1000, 4864, 384), (4097, 1152, 512), (2048, 2560 + 40, 1024)])
 def test_pair_gemm_mxfp8_matches_the_dequantised_product(ops, M, N, K):
     from oracle import decode_oracle as O
 
@@ -87,7 +87,7 @@ def test_pair_gemm_mxfp8_matches_the_dequantised_product(ops, M, N, K):
     assert rel(ops.gemm_mxfp8(xq, wq, b), ref.to(BF16).double() + b.double()) < 3e-3
 
 
-@pytest.mark.parametrize("M,F,K", [(257, 7168, 256), (1500, 2176, 384), (2048, 1024, 1024)])
+@pytest.mark.parametrize("M,F,K", [(257, 7168, 256), (1500, 2176, 384), (2048, 1280, 1024)])
 def test_pair_gemm_mxfp8_swiglu_equals_gemm_then_activation(ops, M, F, K):
     x, w = ops.quantize_mxfp8(randn(M, K, seed=9)), ops.quantize_mxfp8_weight(randn(2 * F, K, seed=10, scale=K ** -0.5))
     y = ops.gemm_mxfp8(x, w)
