@@ -12,8 +12,10 @@
 //                        head - share W_w2's rows in shared memory.  The product with W_w2, the decay, the unit key, the head
 //                        norm and the output gate are part of it.
 //   delta_scan_kernel    rows of any length: one CTA per (row, head, block of columns) walks the row's tokens.  Compute warps
-//                        hold a column per thread (the vectors are then one shared-memory broadcast per four key channels);
-//                        as many other warps prepare the next 16 tokens (decay, unit key, removal vector) meanwhile.
+//                        hold two columns on four lanes (a vector is read from shared memory once for both); as many other
+//                        warps prepare the next 16 tokens (decay, unit key, removal vector) meanwhile.  Bound by the chain of a
+//                        token - dot product, lane sum, update, dot product - on one warp per scheduler; four tokens are
+//                        unrolled so that the next one's vectors are read under it.
 //   delta_finish_kernel  head norm + weight + output gate behind the scan (a head's columns may be spread over CTAs there).
 #include "common.cuh"
 
@@ -339,10 +341,24 @@ delta_decode_kernel(b200_delta_args a, int w2_stride) {
 // ---------------------------------------------------------------------------------------------------------------
 // Scan
 // ---------------------------------------------------------------------------------------------------------------
-template <int DIM, int COLS, int N>
-struct ScanShape {  // COLS columns per CTA, N of them per thread
-  static constexpr int I = DIM <= 128 ? DIM / 2 : 128;
-  static constexpr int NI = DIM / I;  // lanes of a column: half a warp apart, so that a quarter warp reads one address
+// The k-th longest row.  A row's tokens are one chain, so the longest rows end last: their CTAs start first and get an SM of their own, the shortest
+// rows share what is left.  (Warp-collective; more than 32 rows are taken as they come.)
+__device__ __forceinline__ int longest_first(const int32_t* cu_tokens, int rows, int k) {
+  if (rows > 32) return k;
+  const int lane = threadIdx.x & 31, len = lane < rows ? cu_tokens[lane + 1] - cu_tokens[lane] : -1;
+  int rank = 0;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    const int other = __shfl_sync(0xffffffffu, len, j);
+    rank += other > len || (other == len && j < lane);
+  }
+  return __ffs(__ballot_sync(0xffffffffu, rank == k)) - 1;
+}
+
+template <int DIM, int COLS, int N, int LANES>
+struct ScanShape {  // COLS columns per CTA, N of them per thread, LANES lanes per column
+  static constexpr int I = DIM / LANES;
+  static constexpr int NI = LANES;  // 32 / NI apart: neighbouring lanes read one address
   static constexpr int kStride = 32 / NI;
   static constexpr int kComputeThreads = COLS / N * NI;
   static constexpr int kComputeWarps = kComputeThreads / 32;
@@ -357,17 +373,17 @@ struct ScanShape {  // COLS columns per CTA, N of them per thread
   static constexpr int kSmemBytes = 2 * kBufFloats * 4;
 };
 
-template <typename T, int DIM, int COLS, int N>
-__global__ void __launch_bounds__(ScanShape<DIM, COLS, N>::kThreads)
+template <typename T, int DIM, int COLS, int N, int LANES>
+__global__ void __launch_bounds__(ScanShape<DIM, COLS, N, LANES>::kThreads)
 delta_scan_kernel(b200_delta_args a) {
-  using Sh = ScanShape<DIM, COLS, N>;
+  using Sh = ScanShape<DIM, COLS, N, LANES>;
   constexpr int NI = Sh::NI, I = Sh::I, EL = Sh::kElems, VL = (COLS + 31) / 32;
   extern __shared__ __align__(16) float smem[];
   const int tid = threadIdx.x, lane = tid & 31;
   const int dim = a.dim;
   const int col_blocks = (dim + COLS - 1) / COLS;
   const int head = blockIdx.x / col_blocks, cb = blockIdx.x - head * col_blocks;
-  const int row = blockIdx.y;
+  const int row = longest_first(a.cu_tokens, a.num_rows, blockIdx.y);
   pdl_launch_dependents();
   const int t_begin = a.cu_tokens[row], n_tok = min(a.cu_tokens[row + 1], a.num_tokens) - t_begin;
   pdl_wait();
@@ -464,7 +480,7 @@ delta_scan_kernel(b200_delta_args a) {
     const float* buf = smem + (c & 1) * Sh::kBufFloats;
     const float* values = buf + kScanTokens * 5 * DIM + group;
     const int cnt = min(kScanTokens, n_tok - c * kScanTokens);
-#pragma unroll 1
+#pragma unroll 4
     for (int tt = 0; tt < cnt; ++tt) {
       const float* v0 = buf + tt * 5 * DIM;
       const TokenVectors tv{v0, v0 + DIM, v0 + 2 * DIM, v0 + 3 * DIM, v0 + 4 * DIM};
@@ -593,25 +609,25 @@ static int decode_by_dim(const b200_delta_args& a, cudaStream_t s) {
   if (a.dim <= 128) return launch_decode<T, 128>(a, s);
   return launch_decode<T, 256>(a, s);
 }
-template <typename T, int DIM, int COLS, int N>
+template <typename T, int DIM, int COLS, int N, int LANES>
 static int launch_scan(const b200_delta_args& a, cudaStream_t s) {
-  using Sh = ScanShape<DIM, COLS, N>;
+  using Sh = ScanShape<DIM, COLS, N, LANES>;
   static std::atomic<uint64_t> done{0};
-  if (ensure_dynamic_smem(delta_scan_kernel<T, DIM, COLS, N>, Sh::kSmemBytes, done) != B200_OK) return B200_ERR_LAUNCH;
+  if (ensure_dynamic_smem(delta_scan_kernel<T, DIM, COLS, N, LANES>, Sh::kSmemBytes, done) != B200_OK) return B200_ERR_LAUNCH;
   const int col_blocks = (a.dim + COLS - 1) / COLS;
   // Not a programmatic launch: CTAs that arrive while the previous kernel still holds most SMs would pile up on the others,
   // and a CTA stays where it is for the length of a prompt.
-  delta_scan_kernel<T, DIM, COLS, N><<<dim3(a.heads * col_blocks, a.num_rows), Sh::kThreads, Sh::kSmemBytes, s>>>(a);
+  delta_scan_kernel<T, DIM, COLS, N, LANES><<<dim3(a.heads * col_blocks, a.num_rows), Sh::kThreads, Sh::kSmemBytes, s>>>(a);
   return launch_status();
 }
 template <typename T>
 static int scan_by_dim(const b200_delta_args& a, cudaStream_t s) {
-  if (a.dim <= 32) return launch_scan<T, 32, 32, 1>(a, s);
-  // With enough rows to fill the GPU, two columns per thread halve the shared-memory reads per product.
-  if (a.dim <= 64)
-    return static_cast<int64_t>(a.heads) * a.num_rows >= 8 * sm_count() ? launch_scan<T, 64, 64, 2>(a, s) : launch_scan<T, 64, 64, 1>(a, s);
-  if (a.dim <= 128) return launch_scan<T, 128, 64, 1>(a, s);
-  return launch_scan<T, 256, 32, 1>(a, s);
+  // Two columns on four lanes: 1024 tokens x 64 heads of 64 304 -> 251 us, 6208 tokens in 5 rows x 32 heads 886 -> 746 us (one column on two lanes before);
+  // with the longest rows first on top, which alone is 886 -> 700.  One column on four or eight lanes: 270, 304 us.
+  if (a.dim <= 32) return launch_scan<T, 32, 32, 1, 2>(a, s);
+  if (a.dim <= 64) return launch_scan<T, 64, 64, 2, 4>(a, s);
+  if (a.dim <= 128) return launch_scan<T, 128, 64, 2, 4>(a, s);
+  return launch_scan<T, 256, 32, 1, 2>(a, s);
 }
 
 }  // namespace delta

@@ -298,3 +298,36 @@ def test_blockwise_gemm_over_pairs_of_weight_tiles(ops, M, N, K):
     parts = ops.gemm_splitk(xq, wq)
     got = parts.buf.view(torch.float32)[: parts.num_splits * M * N].view(parts.num_splits, M, N).sum(0)
     assert rel(got, ref) < 1e-5
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+# Scans start their longest rows first (up to 32 rows): the bits of every row are those of the row alone, whatever its place.
+# ---------------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("heads,dim,rows", [(2, 64, 32), (2, 64, 33), (1, 128, 5), (1, 48, 1)])
+def test_scanned_rows_do_not_depend_on_the_others(ops, heads, dim, rows):
+    from test_zinurax_kernels_gpu import DeltaCase
+
+    rank, lens = 16, [(7 * i + 3) % 41 for i in range(rows)]  # ties, and a row of no token from 6 rows on
+    T = sum(lens)
+    c = DeltaCase(heads, dim, rank, T, torch.bfloat16, seed=50)
+    at = torch.tensor([0] + lens).cumsum(0).int()
+    slots = torch.arange(rows, dtype=torch.int32)
+    z = None
+    results = []
+    for alone in (False, True):
+        state = torch.randn(rows, heads, dim, dim, generator=torch.Generator().manual_seed(51)).cuda()
+        o, out = torch.zeros(T, c.n, device="cuda"), torch.empty(T, c.n, dtype=BF16, device="cuda")
+        lora = torch.empty(T, rank, dtype=BF16, device="cuda")
+        for group in ([[r] for r in range(rows)] if alone else [list(range(rows))]):
+            rd = slots[group[0]: group[-1] + 1].cuda()
+            cu = at[group[0]: group[-1] + 2].cuda()
+            a = c.args(state, rd, rd, out)
+            a.num_rows, a.cu_tokens, a.o_f32, a.lora = len(group), cu.data_ptr(), o.data_ptr(), lora.data_ptr()
+            if z is None:
+                ops.delta_lora(a, state)
+                z = ops.linear(lora, c.dev[1])
+            a.z = z.data_ptr()
+            ops.delta_scan(a, state)
+            torch.cuda.synchronize()
+        results.append((o, state))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
