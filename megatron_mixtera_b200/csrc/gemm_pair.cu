@@ -435,8 +435,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   if (warp == kProducerWarp) tmem_dealloc_pair(tmem_base, C::kTmemCols);
 }
 
-// Whether the pairs' tiles are the better split: more rows than `fewest`, and at least one tile for every pair of SMs.  (64 tiles, 1024 tokens x 4096 x
-// 4096: 48.8 us here, 44.2 us with K split over the streaming kernel's CTAs; 96 tiles, MXFP8 1024 x 6144 x 4096: 47.9 and 48.5 us.)
+// Whether the pairs' tiles are the better split: more rows than `fewest`, and at least one tile for every pair of SMs.  bf16 above 128 rows (256 x 128256 x
+// 8192: 489 us on the streaming kernel, 417 here); with scales above 256 (up to there the streaming kernel reads a weight once as well).  64 tiles, 1024
+// tokens x 4096 x 4096: 48.8 us here, 44.2 us with K split over the streaming kernel's CTAs; 96 tiles, MXFP8 1024 x 6144 x 4096: 47.9 and 48.5 us.
 static bool preferred(int M, int N, int fewest) {
   const int64_t tiles = static_cast<int64_t>((M + kTile - 1) / kTile) * ((N + kTile - 1) / kTile);
   return M > fewest && tiles >= sm_count() / 2;

@@ -39,6 +39,7 @@ SHAPES = [
     (2048, 2560, 1000),  # K no multiple of a block
     (5000, 1160, 64),    # a single K block
     (300, 16384, 192),
+    (129, 18828, 136),   # one token block, half of it used
 ]
 
 
