@@ -343,7 +343,65 @@ __device__ __forceinline__ void epilogue(const Params& p, uint32_t tmem_base, ui
   }
 }
 
-template <int BT, bool GATE>
+// The K splits of an output tile are the CTAs of a cluster: each leaves its partial tile in shared memory, then all of them sum a share of it over the
+// others' shared memory, in split order - the bits of partial sums through global memory and splitk_reduce_kernel - and store bf16.  N a multiple of 4.
+// Up to 32 tokens and four splits: 1 x 10304 x 2048 10.8 -> 9.8 us, 4 x 2560 x 512 5.3 -> 4.4, MXFP8 5 x 1024 x 1024 5.3 -> 4.3 us, the reduction's launch.
+// Clusters of more CTAs leave SMs of a GPC idle (64 x 6144 x 4096, 48 tiles in six splits: 13.4 -> 23.1 us), and larger tiles take longer through the
+// cluster than through L2 (a decode step of 64 tokens with its 64-token tiles in clusters 599 us, without 588).
+constexpr int kMaxClusterSplits = 4, kMaxClusterTokens = 32;
+template <int BT>
+__device__ __forceinline__ void epilogue_cluster(const Params& p, uint32_t tmem_base, uint8_t* stage_smem, int n_tile, int split, int m0, int m_end) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+  float* tile = reinterpret_cast<float*>(stage_smem);  // [BT tokens][128 features] (every UMMA has completed)
+  const int rows = min(BT, m_end - m0);
+#pragma unroll 1
+  for (int c0 = 0; c0 < rows; c0 += 32) {
+    uint32_t r[32];
+    tmem_ld_32x32b_x32(lane_addr + c0, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 32; ++j) tile[(c0 + j) * kTileN + warp * 32 + lane] = __uint_as_float(r[j]);
+  }
+  cluster_barrier();
+  const int S = p.num_splits;
+  const uint32_t own = smem_u32(tile);
+  for (int u = split * kThreads + tid; u < rows * (kTileN / 4); u += S * kThreads) {
+    const int m = m0 + (u >> 5), n = n_tile * kTileN + (u & 31) * 4;
+    if (n >= p.N) continue;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int s = 0; s < S; ++s) {
+      uint32_t from;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(from) : "r"(own + u * 16), "r"(s));
+      const float4 v = ld_cluster_f4(from);
+      acc.x += v.x;
+      acc.y += v.y;
+      acc.z += v.z;
+      acc.w += v.w;
+    }
+    float v[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (p.bias != nullptr) v[k] = bf16_round(v[k]) + __bfloat162float(p.bias[n + k]);  // bias is added to the bf16-rounded product
+      v[k] = apply_act(v[k], p.act);
+    }
+    __nv_bfloat16* dst = p.y + static_cast<int64_t>(m) * p.ldy + n;
+    if ((p.ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0) {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) dst[k] = __float2bfloat16_rn(v[k]);
+    }
+  }
+  cluster_barrier();  // nobody leaves while its tile is read
+}
+// Whether the K splits of a call that wants bf16 form clusters.
+static bool splits_in_clusters(int splits, int bt, int N) {
+  return splits > 1 && splits <= kMaxClusterSplits && bt <= kMaxClusterTokens && N % 4 == 0;
+}
+
+template <int BT, bool GATE, bool CLUSTER>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, Params p) {
   using C = Config<BT>;
@@ -446,7 +504,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   mbar_wait_bounded(accum_bar, 0, abort_flag, kStatusGemmTimeout);
   tcgen05_fence_after_sync();
 
-  epilogue<BT, GATE>(p, tmem_base, smem, n_tile, split, m0, p.M, p.y + batch * p.y_batch, batch * p.y_batch);
+  if constexpr (CLUSTER)
+    epilogue_cluster<BT>(p, tmem_base, smem, n_tile, split, m0, p.M);
+  else
+    epilogue<BT, GATE>(p, tmem_base, smem, n_tile, split, m0, p.M, p.y + batch * p.y_batch, batch * p.y_batch);
 
   tcgen05_fence_before_sync();
   __syncthreads();
@@ -682,6 +743,7 @@ static int launch(const void* x, int64_t ldx, const void* w, const void* bias, v
   const int m_blocks = (M + BT - 1) / BT;
   const int num_kb = (K + kTileK - 1) / kTileK;
   const int splits = batch > 1 || gate != nullptr ? 1 : choose_splits(n_tiles * m_blocks, num_kb);
+  const bool clusters = partials_out == nullptr && splits_in_clusters(splits, BT, N);
   Params p;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.y = static_cast<__nv_bfloat16*>(y);
@@ -707,7 +769,7 @@ static int launch(const void* x, int64_t ldx, const void* w, const void* bias, v
     if (partials_bytes < static_cast<size_t>(splits) * M * N * sizeof(float)) return B200_ERR_WORKSPACE;
     p.partials = partials_out;
     *splits_out = splits;
-  } else if (splits > 1) {
+  } else if (splits > 1 && !clusters) {
     const size_t need = static_cast<size_t>(splits) * M * N * sizeof(float);
     if (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)) return B200_ERR_WORKSPACE;
     p.partials = static_cast<float*>(workspace);
@@ -716,11 +778,18 @@ static int launch(const void* x, int64_t ldx, const void* w, const void* bias, v
   dim3 grid(n_tiles, splits, m_blocks * batch);
   int rc;
   if (gate != nullptr) {
-    if (ensure_dynamic_smem(gemm_bf16_kernel<BT, true>, C::kSmemBytes, smem_attr_done_gate) != B200_OK) return B200_ERR_LAUNCH;
-    rc = launch_pdl(gemm_bf16_kernel<BT, true>, grid, dim3(kThreads), C::kSmemBytes, stream, *mw, *mx, p);
+    if (ensure_dynamic_smem(gemm_bf16_kernel<BT, true, false>, C::kSmemBytes, smem_attr_done_gate) != B200_OK) return B200_ERR_LAUNCH;
+    rc = launch_pdl(gemm_bf16_kernel<BT, true, false>, grid, dim3(kThreads), C::kSmemBytes, stream, *mw, *mx, p);
+  } else if (clusters) {
+    if constexpr (BT <= kMaxClusterTokens) {
+      static std::atomic<uint64_t> smem_attr_done_cluster{0};
+      if (ensure_dynamic_smem(gemm_bf16_kernel<BT, false, true>, C::kSmemBytes, smem_attr_done_cluster) != B200_OK) return B200_ERR_LAUNCH;
+      return launch_pdl_clusters(gemm_bf16_kernel<BT, false, true>, grid, splits, dim3(kThreads), C::kSmemBytes, stream, *mw, *mx, p);
+    }
+    return B200_ERR_INVALID_ARGUMENT;
   } else {
-    if (ensure_dynamic_smem(gemm_bf16_kernel<BT, false>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
-    rc = launch_pdl(gemm_bf16_kernel<BT, false>, grid, dim3(kThreads), C::kSmemBytes, stream, *mw, *mx, p);
+    if (ensure_dynamic_smem(gemm_bf16_kernel<BT, false, false>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
+    rc = launch_pdl(gemm_bf16_kernel<BT, false, false>, grid, dim3(kThreads), C::kSmemBytes, stream, *mw, *mx, p);
   }
   if (rc != B200_OK || splits == 1 || p.keep_partials) return rc;
   return launch_splitk_reduce(p, stream);
@@ -809,7 +878,8 @@ size_t b200_gemm_bf16_workspace_bytes(int M, int N, int K) {
   using namespace b200::gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (pair::preferred(M, N, pair::kFewestRowsBf16)) return 0;
-  return splitk_scratch_bytes(M, N, K);
+  const size_t bytes = splitk_scratch_bytes(M, N, K);
+  return splits_in_clusters(static_cast<int>(bytes / (static_cast<size_t>(M) * N * sizeof(float))), pick_bt(M), N) ? 0 : bytes;
 }
 
 int b200_gemm_bf16(const void* x, int64_t ldx, const void* w, const void* bias, void* y, int64_t ldy, int M, int N,

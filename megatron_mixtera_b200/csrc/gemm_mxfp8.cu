@@ -50,7 +50,7 @@ struct Fp8Operands {
   int k_tiles;          // K / 128
 };
 
-template <int BT>
+template <int BT, bool CLUSTER>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, Params p,
                   Fp8Operands q) {
@@ -172,7 +172,10 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   pdl_wait();
   mbar_wait_bounded(accum_bar, 0, abort_flag, kStatusGemmTimeout);
   tcgen05_fence_after_sync();
-  epilogue<BT>(p, tmem_base, smem, n_tile, split, m_block * BT, p.M, p.y);
+  if constexpr (CLUSTER)
+    epilogue_cluster<BT>(p, tmem_base, smem, n_tile, split, m_block * BT, p.M);
+  else
+    epilogue<BT>(p, tmem_base, smem, n_tile, split, m_block * BT, p.M, p.y);
 
   tcgen05_fence_before_sync();
   __syncthreads();
@@ -200,6 +203,7 @@ static int launch_mxfp8(const void* xq, const void* x_sf, const void* wq, const 
   const int m_blocks = (M + BT - 1) / BT;
   const int num_kb = K / kFp8TileK;
   const int splits = choose_splits(n_tiles * m_blocks, num_kb);
+  const bool clusters = partials_out == nullptr && splits_in_clusters(splits, BT, N);
   Params p;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.y = static_cast<__nv_bfloat16*>(y);
@@ -217,7 +221,7 @@ static int launch_mxfp8(const void* xq, const void* x_sf, const void* wq, const 
     if (partials_bytes < static_cast<size_t>(splits) * M * N * sizeof(float)) return B200_ERR_WORKSPACE;
     p.partials = partials_out;
     *splits_out = splits;
-  } else if (splits > 1) {
+  } else if (splits > 1 && !clusters) {
     const size_t need = static_cast<size_t>(splits) * M * N * sizeof(float);
     if (workspace == nullptr || workspace_bytes < need || !aligned16(workspace)) return B200_ERR_WORKSPACE;
     p.partials = static_cast<float*>(workspace);
@@ -226,10 +230,18 @@ static int launch_mxfp8(const void* xq, const void* x_sf, const void* wq, const 
   q.w_sf = static_cast<const uint8_t*>(w_sf);
   q.x_sf = static_cast<const uint8_t*>(x_sf);
   q.k_tiles = num_kb;
-  static std::atomic<uint64_t> smem_attr_done{0};
-  if (ensure_dynamic_smem(gemm_mxfp8_kernel<BT>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
   dim3 grid(n_tiles, splits, m_blocks);
-  const int rc = launch_pdl(gemm_mxfp8_kernel<BT>, grid, dim3(kThreads), C::kSmemBytes, stream, *mw, *mx, p, q);
+  if (clusters) {
+    if constexpr (BT <= kMaxClusterTokens) {
+      static std::atomic<uint64_t> smem_attr_done_cluster{0};
+      if (ensure_dynamic_smem(gemm_mxfp8_kernel<BT, true>, C::kSmemBytes, smem_attr_done_cluster) != B200_OK) return B200_ERR_LAUNCH;
+      return launch_pdl_clusters(gemm_mxfp8_kernel<BT, true>, grid, splits, dim3(kThreads), C::kSmemBytes, stream, *mw, *mx, p, q);
+    }
+    return B200_ERR_INVALID_ARGUMENT;
+  }
+  static std::atomic<uint64_t> smem_attr_done{0};
+  if (ensure_dynamic_smem(gemm_mxfp8_kernel<BT, false>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
+  const int rc = launch_pdl(gemm_mxfp8_kernel<BT, false>, grid, dim3(kThreads), C::kSmemBytes, stream, *mw, *mx, p, q);
   if (rc != B200_OK || splits == 1 || p.keep_partials) return rc;
   return launch_splitk_reduce(p, stream);
 }
@@ -531,7 +543,7 @@ size_t b200_gemm_mxfp8_workspace_bytes(int M, int N, int K) {
   const int bt = pick_bt(M);
   const int tiles = ((N + kTileN - 1) / kTileN) * ((M + bt - 1) / bt);
   const int splits = choose_splits(tiles, K / kFp8TileK);
-  if (splits == 1) return 0;
+  if (splits == 1 || splits_in_clusters(splits, bt, N)) return 0;
   return static_cast<size_t>(splits) * static_cast<size_t>(M) * N * sizeof(float);
 }
 

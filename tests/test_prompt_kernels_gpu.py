@@ -332,3 +332,32 @@ def test_scanned_rows_do_not_depend_on_the_others(ops, heads, dim, rows):
             torch.cuda.synchronize()
         results.append((o, state))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+# K splits as clusters: bf16 out of the sums of partial tiles, against the same sums through `gemm_splitk` (same splits, same order: same bits).
+# ---------------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("M,N,K", [(1, 10304, 2048), (4, 2560, 512), (33, 384, 1024), (64, 6144, 4096), (100, 6144, 4096), (128, 132, 4096), (17, 1000, 640)])
+def test_splits_in_clusters_give_the_bits_of_the_summed_partials(ops, M, N, K):
+    x, w, b = randn(M, K, seed=1), randn(N, K, seed=2, scale=K ** -0.5), randn(N, seed=3)
+    parts = ops.gemm_splitk(x, w)
+    assert parts.num_splits > 1
+    p = parts.buf.view(torch.float32)[: parts.num_splits * M * N].view(parts.num_splits, M, N).clone()
+    total = p[0].clone()
+    for s in range(1, parts.num_splits):
+        total += p[s]
+    y = ops.gemm(x, w)
+    assert torch.equal(y, total.to(BF16))
+    assert torch.equal(ops.gemm(x, w, b), (total.to(BF16).float() + b.float()).to(BF16))
+    assert torch.equal(ops.linear(x, w, act="relu2"), torch.relu(total).square().to(BF16))
+    wide = torch.zeros(M, N + 3, dtype=BF16, device="cuda")
+    ops.linear(x, w, out=wide[:, :N])
+    assert torch.equal(wide[:, :N], y) and not wide[:, N:].any()
+    if K % 128 == 0:
+        xq, wq = ops.quantize_mxfp8(x), ops.quantize_mxfp8_weight(w)
+        parts = ops.gemm_splitk(xq, wq)
+        p = parts.buf.view(torch.float32)[: parts.num_splits * M * N].view(parts.num_splits, M, N).clone()
+        total = p[0].clone()
+        for s in range(1, parts.num_splits):
+            total += p[s]
+        assert torch.equal(ops.gemm_mxfp8(xq, wq), total.to(BF16))
