@@ -121,6 +121,8 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 int64_t split_stride, PeerSrc ps) {
   __shared__ float red[32];
   pdl_launch_dependents();
+  if (gamma != nullptr)  // a weight: on its way while the kernel before ends
+    for (int i = threadIdx.x * 8; i < hidden / 8; i += blockDim.x * 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(gamma + i * 8));
   pdl_wait();
   if constexpr (kSrc == 2) {
     peer_row_handshake(ps, blockIdx.x);
@@ -227,6 +229,9 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     finish();
     return;
   }
+  const Vec8* gv = reinterpret_cast<const Vec8*>(gamma);
+  Vec8 weights;  // one vector per thread: read here; behind the block's sums it would be one more trip to L2 (with more vectors it would cost CTAs)
+  if (kMaxVec == 1 && threadIdx.x < nvec) weights = gv[threadIdx.x];
   float mean = 0.f, rstd;
   if (beta != nullptr) {  // LayerNorm: two-pass variance on the cached values
     mean = block_sum(sum, red) / hidden;
@@ -246,7 +251,6 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
   } else {
     rstd = rsqrtf(block_sum(sumsq, red) / hidden + eps);
   }
-  const Vec8* gv = reinterpret_cast<const Vec8*>(gamma);
   const Vec8* betav = beta ? reinterpret_cast<const Vec8*>(beta) : nullptr;
 #pragma unroll
   for (int it = 0; it < kMaxVec; ++it) {
@@ -254,7 +258,7 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     const bool valid = i < nvec;
     float y[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (valid) {
-      const Vec8 g = gv[i];
+      const Vec8 g = kMaxVec == 1 ? weights : gv[i];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         y[2 * k] = (vals[it][2 * k] - mean) * rstd * bf16_lo(g.w[k]);

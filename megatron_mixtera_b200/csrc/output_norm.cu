@@ -9,9 +9,9 @@ namespace outnorm {
 
 constexpr int kThreads = 256;
 constexpr int kMaxWidth = 16384;  // the row is kept in shared memory
-// Rows of up to kVec * kThreads * 4 elements stay in registers (the multiple-of-4 widths that real models have).
-constexpr int kVec = 8;
+constexpr int kMaxVecWidth = 8192;  // multiples of 4 up to here stay in registers (the widths that real models have)
 
+template <int THREADS = kThreads>
 __device__ __forceinline__ float block_sum(float v, float* red) {
   v = warp_sum(v);
   __syncthreads();  // `red` may still be read from the previous call
@@ -19,7 +19,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   __syncthreads();
   float s = 0.f;
 #pragma unroll
-  for (int i = 0; i < kThreads / 32; ++i) s += red[i];
+  for (int i = 0; i < THREADS / 32; ++i) s += red[i];
   return s;
 }
 
@@ -49,27 +49,47 @@ __device__ __forceinline__ bool source_row(const b200_out_norm_args& a, int row,
   return src >= 0 && src < a.source_rows;
 }
 
-// width % 4 == 0 and width <= kVec * 1024: the row lives in registers.
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
+// width % 4 == 0 and width <= SLOTS * THREADS * 4: the row lives in registers.  Bound by latency with few rows, by bytes in flight with many.  What the sums do
+// not need is read before them, the weight before the kernel in front has ended, the residual row together with the sublayer's: behind two block sums
+// each was one more trip to memory.  One row of 2048 and eight splits 3.6 -> 2.3 us, 64 of 4096 6.3 -> 3.9, 6208 of 2048 58.9 -> 37.0 us (floor 26.8).
+template <typename T, int SLOTS, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 out_norm_vec_kernel(b200_out_norm_args a) {
-  __shared__ float red[kThreads / 32];
+  __shared__ float red[THREADS / 32];
   pdl_launch_dependents();
   const int tid = threadIdx.x;
   const int row = blockIdx.x;
   const int W = a.width;
   const T* gamma = static_cast<const T*>(a.gamma);
+  constexpr bool kEarly = SLOTS <= 2;  // (more would cost CTAs: 8192 rows of 8192 240 -> 390 us)
+  constexpr int kEarlySlots = kEarly ? SLOTS : 1;
+  float4 v[SLOTS], early_g[kEarlySlots], early_h[kEarlySlots];
+  if constexpr (kEarly) {
+#pragma unroll
+    for (int i = 0; i < SLOTS; ++i) {
+      const int c = (i * THREADS + tid) * 4;
+      if (c < W) early_g[i] = load4(gamma + c);
+    }
+  }
   pdl_wait();
-  float4 v[kVec];
+  float* hidden = a.hidden + static_cast<int64_t>(row) * W;
+  if constexpr (kEarly) {
+#pragma unroll
+    for (int i = 0; i < SLOTS; ++i) {
+      const int c = (i * THREADS + tid) * 4;
+      if (a.accumulate && c < W) early_h[i] = *reinterpret_cast<const float4*>(hidden + c);
+    }
+  }
   float sum = 0.f;
   if (a.partials != nullptr) {
     const float* base = a.partials + static_cast<int64_t>(row) * W;
     const int64_t stride = static_cast<int64_t>(a.rows) * W;
 #pragma unroll
-    for (int i = 0; i < kVec; ++i) {
-      const int c = (i * kThreads + tid) * 4;
+    for (int i = 0; i < SLOTS; ++i) {
+      const int c = (i * THREADS + tid) * 4;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       if (c < W) {
+#pragma unroll 4
         for (int s = 0; s < a.num_splits; ++s) {
           const float4 t = __ldcg(reinterpret_cast<const float4*>(base + s * stride + c));
           acc.x += t.x;
@@ -84,20 +104,20 @@ out_norm_vec_kernel(b200_out_norm_args a) {
     int64_t src;
     const bool ok = source_row(a, row, src);
 #pragma unroll
-    for (int i = 0; i < kVec; ++i) {
-      const int c = (i * kThreads + tid) * 4;
+    for (int i = 0; i < SLOTS; ++i) {
+      const int c = (i * THREADS + tid) * 4;
       v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (c < W && ok)
         v[i] = a.table ? load4(static_cast<const T*>(a.table) + src * W + c) : load4(a.rows_in + src * W + c);
     }
   }
 #pragma unroll
-  for (int i = 0; i < kVec; ++i) sum += v[i].x + v[i].y + v[i].z + v[i].w;
-  const float mean = block_sum(sum, red) / W;
+  for (int i = 0; i < SLOTS; ++i) sum += v[i].x + v[i].y + v[i].z + v[i].w;
+  const float mean = block_sum<THREADS>(sum, red) / W;
   float sq = 0.f;
 #pragma unroll
-  for (int i = 0; i < kVec; ++i) {
-    const int c = (i * kThreads + tid) * 4;
+  for (int i = 0; i < SLOTS; ++i) {
+    const int c = (i * THREADS + tid) * 4;
     if (c < W) {
       v[i].x -= mean;
       v[i].y -= mean;
@@ -106,20 +126,19 @@ out_norm_vec_kernel(b200_out_norm_args a) {
       sq += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
     }
   }
-  const float inv = 1.f / sqrtf(block_sum(sq, red) / W + a.eps);
+  const float inv = 1.f / sqrtf(block_sum<THREADS>(sq, red) / W + a.eps);
 #pragma unroll
-  for (int i = 0; i < kVec; ++i) {
-    const int c = (i * kThreads + tid) * 4;
+  for (int i = 0; i < SLOTS; ++i) {
+    const int c = (i * THREADS + tid) * 4;
     if (c < W) {
-      const float4 g = load4(gamma + c);
+      const float4 g = kEarly ? early_g[i % kEarlySlots] : load4(gamma + c);
       float4 o = make_float4(v[i].x * inv * g.x, v[i].y * inv * g.y, v[i].z * inv * g.z, v[i].w * inv * g.w);
       if (a.hidden != nullptr) {
-        float* h = a.hidden + static_cast<int64_t>(row) * W + c;
         if (a.accumulate) {
-          const float4 p = *reinterpret_cast<const float4*>(h);
+          const float4 p = kEarly ? early_h[i % kEarlySlots] : *reinterpret_cast<const float4*>(hidden + c);
           o = make_float4(p.x + o.x, p.y + o.y, p.z + o.z, p.w + o.w);
         }
-        store4(h, o);
+        store4(hidden + c, o);
       }
       if (a.y != nullptr) store4(static_cast<T*>(a.y) + static_cast<int64_t>(row) * W + c, o);
     }
@@ -171,9 +190,20 @@ out_norm_any_kernel(b200_out_norm_args a) {
 
 template <typename T>
 static int launch(const b200_out_norm_args& a, cudaStream_t s) {
-  const bool aligned = a.width % 4 == 0 && a.width <= kVec * kThreads * 4 && aligned16(a.partials) && aligned16(a.table) &&
-                       aligned16(a.rows_in) && aligned16(a.gamma) && aligned16(a.hidden) && aligned16(a.y);
-  if (aligned) return launch_pdl(out_norm_vec_kernel<T>, dim3(a.rows), dim3(kThreads), 0, s, a);
+  const bool aligned = a.width % 4 == 0 && a.width <= kMaxVecWidth && aligned16(a.partials) && aligned16(a.table) && aligned16(a.rows_in) &&
+                       aligned16(a.gamma) && aligned16(a.hidden) && aligned16(a.y);
+  const dim3 grid(a.rows);
+  if (aligned && a.rows <= 2 * sm_count()) {  // few rows: more threads for each
+    if (a.width > 4096) return launch_pdl(out_norm_vec_kernel<T, 2, 1024>, grid, dim3(1024), 0, s, a);
+    if (a.width > 2048) return launch_pdl(out_norm_vec_kernel<T, 1, 1024>, grid, dim3(1024), 0, s, a);
+    if (a.width > 1024) return launch_pdl(out_norm_vec_kernel<T, 1, 512>, grid, dim3(512), 0, s, a);
+  }
+  if (aligned) {
+    if (a.width <= 1024) return launch_pdl(out_norm_vec_kernel<T, 1, kThreads>, grid, dim3(kThreads), 0, s, a);
+    if (a.width <= 2048) return launch_pdl(out_norm_vec_kernel<T, 2, kThreads>, grid, dim3(kThreads), 0, s, a);
+    if (a.width <= 4096) return launch_pdl(out_norm_vec_kernel<T, 2, 512>, grid, dim3(512), 0, s, a);
+    return launch_pdl(out_norm_vec_kernel<T, 8, kThreads>, grid, dim3(kThreads), 0, s, a);
+  }
   static std::atomic<uint64_t> done{0};
   if (ensure_dynamic_smem(out_norm_any_kernel<T>, kMaxWidth * 4, done) != B200_OK) return B200_ERR_LAUNCH;
   return launch_pdl(out_norm_any_kernel<T>, dim3(a.rows), dim3(kThreads), static_cast<size_t>(a.width) * 4, s, a);

@@ -53,6 +53,17 @@ residual_norm_kernel(b200_residual_norm_args a) {
         for (int i = blockIdx.x * kThreads + tid; i < pieces; i += gridDim.x * kThreads)
           asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(a.filter[n]) + i * 128));
   }
+  constexpr bool kEarly = SLOTS * VEC <= 4;  // the norms' weights in registers before the wait; in longer rows they would cost CTAs
+  float early[2][kEarly ? SLOTS : 1][VEC];
+  if constexpr (kEarly) {
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int i = 0; i < SLOTS; ++i) {
+        const int c = (i * kThreads + tid) * VEC;
+        if (a.y[n] != nullptr && a.taps == 0 && c < W) load<T, VEC>(static_cast<const T*>(a.gamma[n]) + c, early[n][i]);
+      }
+  }
   pdl_wait();
   const int64_t row = a.row_index ? a.row_index[blockIdx.x] : blockIdx.x;
   const bool ok = row >= 0 && row < a.source_rows;
@@ -195,7 +206,12 @@ residual_norm_kernel(b200_residual_norm_args a) {
       const int c = (i * kThreads + tid) * VEC;
       if (c >= W) continue;
       float g[VEC], o[VEC];
-      load<T, VEC>(gamma + c, g);
+      if constexpr (kEarly) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) g[e] = early[n][i][e];
+      } else {
+        load<T, VEC>(gamma + c, g);
+      }
 #pragma unroll
       for (int e = 0; e < VEC; ++e) o[e] = v[i][e] * inv * (a.gain + g[e]);
       store<T, VEC>(y + c, o);

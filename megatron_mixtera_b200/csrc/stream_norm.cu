@@ -16,23 +16,34 @@ __device__ __forceinline__ void zero(float (&v)[N]) {
   for (int e = 0; e < N; ++e) v[e] = 0.f;
 }
 
-// SLOTS * VEC * kThreads >= width: the blended row lives in registers.  S >= streams.
-template <typename T, int VEC, int SLOTS, int S>
-__global__ void __launch_bounds__(kThreads)
+// SLOTS * VEC * THREADS >= width: the blended row lives in registers.  S >= streams.
+template <typename T, int VEC, int SLOTS, int S, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 stream_norm_kernel(b200_stream_norm_args a) {
-  __shared__ float red[kThreads / 32];
+  __shared__ float red[THREADS / 32];
   __shared__ int64_t expert_row[kMaxTop];
   __shared__ float expert_weight[kMaxTop];
   __shared__ float mix_s[S * S], out_s[S], in_s[S];
   pdl_launch_dependents();
   const int tid = threadIdx.x, W = a.width, n = a.streams;
-  for (int i = tid; i < S * S; i += kThreads) {  // weights: no kernel writes them
+  for (int i = tid; i < S * S; i += THREADS) {  // weights: no kernel writes them
     const int s = i / S, t = i - s * S;
     mix_s[i] = s < n && t < n ? (a.mix != nullptr ? a.mix[s * n + t] : s == t ? 1.f : 0.f) : 0.f;
   }
   if (tid < S) {
     out_s[tid] = tid < n && a.mix != nullptr ? a.out[tid] : 0.f;
     in_s[tid] = tid < n ? (a.in != nullptr ? a.in[tid] : 1.f) : 0.f;
+  }
+  constexpr bool kEarly = SLOTS * VEC <= 4;  // the norm's weights in registers before the wait; in longer rows they would cost CTAs
+  float early_g[kEarly ? SLOTS : 1][VEC], early_b[kEarly ? SLOTS : 1][VEC];
+  if constexpr (kEarly) {
+#pragma unroll
+    for (int i = 0; i < SLOTS; ++i) {
+      const int c = (i * THREADS + tid) * VEC;
+      if (a.y == nullptr || c >= W) continue;
+      conv::load<T, VEC>(static_cast<const T*>(a.gamma) + c, early_g[i]);
+      conv::load<T, VEC>(static_cast<const T*>(a.beta) + c, early_b[i]);
+    }
   }
   pdl_wait();
   const int64_t row = a.row_index ? a.row_index[blockIdx.x] : blockIdx.x;
@@ -64,7 +75,7 @@ stream_norm_kernel(b200_stream_norm_args a) {
   float sum = 0.f;
 #pragma unroll
   for (int i = 0; i < SLOTS; ++i) {
-    const int c = (i * kThreads + tid) * VEC;
+    const int c = (i * THREADS + tid) * VEC;
     zero(v[i]);
     if (c >= W || !ok) continue;
     float xs[S][VEC], add[VEC], x[VEC];
@@ -146,40 +157,46 @@ stream_norm_kernel(b200_stream_norm_args a) {
     for (int e = 0; e < VEC; ++e) sum += v[i][e];
   }
   if (a.y == nullptr) return;
-  const float mean = outnorm::block_sum(sum, red) / W;
+  const float mean = outnorm::block_sum<THREADS>(sum, red) / W;
   float sq = 0.f;
 #pragma unroll
   for (int i = 0; i < SLOTS; ++i)
-    if ((i * kThreads + tid) * VEC < W)
+    if ((i * THREADS + tid) * VEC < W)
 #pragma unroll
       for (int e = 0; e < VEC; ++e) {
         v[i][e] -= mean;
         sq = fmaf(v[i][e], v[i][e], sq);
       }
-  const float inv = 1.f / sqrtf(outnorm::block_sum(sq, red) / W + a.eps);
+  const float inv = 1.f / sqrtf(outnorm::block_sum<THREADS>(sq, red) / W + a.eps);
   const T* gamma = static_cast<const T*>(a.gamma);
   const T* beta = static_cast<const T*>(a.beta);
   T* y = static_cast<T*>(a.y) + static_cast<int64_t>(blockIdx.x) * W;
 #pragma unroll
   for (int i = 0; i < SLOTS; ++i) {
-    const int c = (i * kThreads + tid) * VEC;
+    const int c = (i * THREADS + tid) * VEC;
     if (c >= W) continue;
     float g[VEC], b[VEC], o[VEC];
-    conv::load<T, VEC>(gamma + c, g);
-    conv::load<T, VEC>(beta + c, b);
+    if constexpr (!kEarly) {
+      conv::load<T, VEC>(gamma + c, g);
+      conv::load<T, VEC>(beta + c, b);
+    }
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) o[e] = fmaf(v[i][e] * inv, g[e], b[e]);
+    for (int e = 0; e < VEC; ++e)
+      if constexpr (kEarly)
+        o[e] = fmaf(v[i][e] * inv, early_g[i][e], early_b[i][e]);
+      else
+        o[e] = fmaf(v[i][e] * inv, g[e], b[e]);
     conv::store<T, VEC>(y + c, o);
   }
 }
 
-template <typename T, int VEC, int SLOTS>
+template <typename T, int VEC, int SLOTS, int THREADS = kThreads>
 static int by_streams(const b200_stream_norm_args& a, cudaStream_t s) {
-  const dim3 grid(a.rows), block(kThreads);
-  if (a.streams <= 2) return launch_pdl(stream_norm_kernel<T, VEC, SLOTS, 2>, grid, block, 0, s, a);
-  if (a.streams <= 4) return launch_pdl(stream_norm_kernel<T, VEC, SLOTS, 4>, grid, block, 0, s, a);
-  if (a.streams <= 8) return launch_pdl(stream_norm_kernel<T, VEC, SLOTS, 8>, grid, block, 0, s, a);
-  return launch_pdl(stream_norm_kernel<T, VEC, SLOTS, kMaxStreams>, grid, block, 0, s, a);
+  const dim3 grid(a.rows), block(THREADS);
+  if (a.streams <= 2) return launch_pdl(stream_norm_kernel<T, VEC, SLOTS, 2, THREADS>, grid, block, 0, s, a);
+  if (a.streams <= 4) return launch_pdl(stream_norm_kernel<T, VEC, SLOTS, 4, THREADS>, grid, block, 0, s, a);
+  if (a.streams <= 8) return launch_pdl(stream_norm_kernel<T, VEC, SLOTS, 8, THREADS>, grid, block, 0, s, a);
+  return launch_pdl(stream_norm_kernel<T, VEC, SLOTS, kMaxStreams, THREADS>, grid, block, 0, s, a);
 }
 
 template <typename T>
@@ -188,6 +205,10 @@ static int launch(const b200_stream_norm_args& a, cudaStream_t s) {
   for (const void* p : {a.table, static_cast<const void*>(a.partials), a.branch_bias, a.expert_rows, a.expert_input,
                         static_cast<const void*>(a.hidden), a.gamma, a.beta, static_cast<const void*>(a.y)})
     aligned = aligned && aligned16(p);
+  if (aligned && a.rows <= 2 * sm_count()) {  // few rows: more threads for each
+    if (a.width > 1024 && a.width <= 2048) return by_streams<T, 4, 1, 512>(a, s);
+    if (a.width > 2048 && a.width <= 4096) return by_streams<T, 4, 2, 512>(a, s);
+  }
   if (aligned) {
     if (a.width <= 1024) return by_streams<T, 4, 1>(a, s);
     if (a.width <= 2048) return by_streams<T, 4, 2>(a, s);

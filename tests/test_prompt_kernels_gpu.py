@@ -361,3 +361,21 @@ def test_splits_in_clusters_give_the_bits_of_the_summed_partials(ops, M, N, K):
         for s in range(1, parts.num_splits):
             total += p[s]
         assert torch.equal(ops.gemm_mxfp8(xq, wq), total.to(BF16))
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+# Output norm: few rows and many, one to eight vectors per thread, widths that end inside a thread's vectors.  fp32 sums of up to 8192 terms: 1e-5.
+# ---------------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("accumulate", [0, 1])
+@pytest.mark.parametrize("rows,width,splits", [(1, 2048, 8), (5, 1000, 3), (3, 1028, 1), (296, 4096, 2), (7, 8192, 5), (2, 4100, 1), (297, 2048, 1), (300, 96, 2),
+                                               (400, 2052, 1), (310, 4096, 2), (298, 8188, 1), (3, 8200, 2)])
+def test_output_norm_by_rows_and_width(ops, rows, width, splits, accumulate):
+    p = torch.randn(splits, rows, width, generator=torch.Generator().manual_seed(1)).cuda()
+    gamma, before = randn(width, seed=2), torch.randn(rows, width, generator=torch.Generator().manual_seed(3)).cuda()
+    hidden = before.clone()
+    y = ops.out_norm(ops.GemmPartials(p, splits, (rows, width)), gamma, eps=1e-5, hidden=hidden, accumulate=bool(accumulate))
+    x = p.double().sum(0)
+    x = x - x.mean(-1, keepdim=True)
+    want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * gamma.double() + accumulate * before.double()
+    assert float((hidden.double() - want).abs().max()) < 1e-5 * float(want.abs().max())
+    assert torch.equal(y, hidden.to(BF16))
