@@ -111,6 +111,9 @@ __device__ __forceinline__ void peer_row_handshake(const PeerSrc& ps, int row) {
 // vector per thread and up to 1024 threads, so that all partial loads of a row are in flight at once.
 // kSrc 2 ("peers"): x = bf16(sum over the tensor-parallel ranks, in rank order, of their bf16 rows), after the
 // row handshake above; every rank computes the same bits.
+// Bound by bytes with many rows, and close behind them by conversions: pairs are rounded with one instruction, whose result is also what is stored.
+// 13000 rows of 4096 with a residual 79.6 -> 72.3 us (floor 64), with MXFP8 87.3 -> 81.1; 11000 of 8192 to blockwise FP8 192 -> 156; 64 of 4096 2.9 -> 2.5 us.
+// (Rows of 4096 without a residual, one norm of a model, 31.1 -> 33.8 us.)
 template <int kMaxVec, int kSrc>
 __global__ void __launch_bounds__(kSrc != 0 ? 1024 : 256)
 add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ bias,
@@ -153,6 +156,7 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     const int i = threadIdx.x + it * blockDim.x;
     if (i < nvec) {
       float f[8];
+      Vec8 h;  // the row so far, bf16 pairs: rounded by one conversion a pair, which is also what gets stored
       if constexpr (kSrc == 2) {
         // all peers' vectors are requested before any is used: one NVLink round trip, not `world` of them
         uint4 u[8];
@@ -173,7 +177,7 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
           }
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) f[k] = bf16_round(f[k]);
+        for (int k = 0; k < 4; ++k) h.w[k] = pack_bf16x2(f[2 * k], f[2 * k + 1]);
       } else if constexpr (kSrc == 1) {
         const float4* src = reinterpret_cast<const float4*>(partials + off) + 2 * i;
         const int64_t stride4 = split_stride / 4;
@@ -185,37 +189,28 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
           a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
           b.x += w.x; b.y += w.y; b.z += w.z; b.w += w.w;
         }
-        f[0] = bf16_round(a.x); f[1] = bf16_round(a.y); f[2] = bf16_round(a.z); f[3] = bf16_round(a.w);
-        f[4] = bf16_round(b.x); f[5] = bf16_round(b.y); f[6] = bf16_round(b.z); f[7] = bf16_round(b.w);
+        h.w[0] = pack_bf16x2(a.x, a.y);
+        h.w[1] = pack_bf16x2(a.z, a.w);
+        h.w[2] = pack_bf16x2(b.x, b.y);
+        h.w[3] = pack_bf16x2(b.z, b.w);
       } else {
-        const Vec8 v = xv[i];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          f[2 * k] = bf16_lo(v.w[k]);
-          f[2 * k + 1] = bf16_hi(v.w[k]);
-        }
+        h = xv[i];
       }
       if (bv) {
         const Vec8 b = bv[i];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          f[2 * k] = bf16_round(f[2 * k] + bf16_lo(b.w[k]));
-          f[2 * k + 1] = bf16_round(f[2 * k + 1] + bf16_hi(b.w[k]));
-        }
+        for (int k = 0; k < 4; ++k) h.w[k] = pack_bf16x2(bf16_lo(h.w[k]) + bf16_lo(b.w[k]), bf16_hi(h.w[k]) + bf16_hi(b.w[k]));
       }
       if (rv) {
         const Vec8 r = rv[i];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          f[2 * k] = bf16_round(f[2 * k] + bf16_lo(r.w[k]));
-          f[2 * k + 1] = bf16_round(f[2 * k + 1] + bf16_hi(r.w[k]));
-        }
+        for (int k = 0; k < 4; ++k) h.w[k] = pack_bf16x2(bf16_lo(h.w[k]) + bf16_lo(r.w[k]), bf16_hi(h.w[k]) + bf16_hi(r.w[k]));
       }
-      if (hidden_out) {
-        Vec8 o;
+      if (hidden_out) reinterpret_cast<Vec8*>(hidden_out + off)[i] = h;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) o.w[k] = pack_bf16x2(f[2 * k], f[2 * k + 1]);
-        reinterpret_cast<Vec8*>(hidden_out + off)[i] = o;
+      for (int k = 0; k < 4; ++k) {
+        f[2 * k] = bf16_lo(h.w[k]);
+        f[2 * k + 1] = bf16_hi(h.w[k]);
       }
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
@@ -272,16 +267,17 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
           y[2 * k + 1] += bf16_hi(b.w[k]);
         }
       }
-      if (normed_out) {
-        Vec8 o;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) o.w[k] = pack_bf16x2(y[2 * k], y[2 * k + 1]);
-        reinterpret_cast<Vec8*>(normed_out + off)[i] = o;
-      }
     }
+    Vec8 o;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o.w[k] = pack_bf16x2(y[2 * k], y[2 * k + 1]);
+    if (valid && normed_out) reinterpret_cast<Vec8*>(normed_out + off)[i] = o;
     if (q_out) {  // quantise the bf16-rounded normalised row (what an unfused quantiser would read)
 #pragma unroll
-      for (int k = 0; k < 8; ++k) y[k] = bf16_round(y[k]);
+      for (int k = 0; k < 4; ++k) {
+        y[2 * k] = bf16_lo(o.w[k]);
+        y[2 * k + 1] = bf16_hi(o.w[k]);
+      }
       mx::quantize8_any(q_mode, y, valid, blockIdx.x, i * 8, q_out, hidden, sf_out, hidden / 128, m_pad);
     }
   }
@@ -341,9 +337,8 @@ __global__ void activation_kernel(const __nv_bfloat16* __restrict__ in, const __
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float a = bf16_round(silu_f(bf16_lo(g.w[k]))) * bf16_lo(u.w[k]);
-      const float b = bf16_round(silu_f(bf16_hi(g.w[k]))) * bf16_hi(u.w[k]);
-      o.w[k] = pack_bf16x2(a, b);
+      const uint32_t act = pack_bf16x2(silu_f(bf16_lo(g.w[k])), silu_f(bf16_hi(g.w[k])));
+      o.w[k] = pack_bf16x2(bf16_lo(act) * bf16_lo(u.w[k]), bf16_hi(act) * bf16_hi(u.w[k]));
     }
   } else {
     const Vec8 v = partials != nullptr ? sum_partials8(partials + static_cast<int64_t>(r) * F + i * 8, splits, split_stride)
