@@ -113,7 +113,6 @@ paged_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  pdl_launch_dependents();
   const int h = blockIdx.x % p.nkv;
   // the last units of a request see the most keys: they start first
   const int first_unit = ((num_units + kUnitsPerCta - 1) / kUnitsPerCta - 1 - static_cast<int>(blockIdx.x / p.nkv)) * kUnitsPerCta;
@@ -145,6 +144,7 @@ paged_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  pdl_launch_dependents();  // (behind the allocation: a successor's CTA must not hold tensor memory we wait for)
   pdl_wait();  // queries, pool and lengths are earlier kernels' output
 
   // this CTA's units; padding entries and malformed ones have no tokens

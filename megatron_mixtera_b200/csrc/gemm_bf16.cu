@@ -541,32 +541,12 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  pdl_launch_dependents();
   int unit = blockIdx.x;
   const bool is_shared = unit < gp.shared_units;
   const Params& p = is_shared ? gp.shared : gp.routed;
-  int n_tile, m0, m_end, w_row;
-  if (is_shared) {
-    n_tile = unit % gp.shared_n_tiles;
-    m0 = unit / gp.shared_n_tiles * BT;
-    m_end = p.M;
-    w_row = n_tile * kTileN;
-  } else {
-    unit -= gp.shared_units;
-    n_tile = unit % gp.routed_n_tiles;
-    const int tile = unit / gp.routed_n_tiles;
-    pdl_wait();  // the tile list is a kernel's output
-    if (tile >= min(*gp.num_tiles, gp.max_tiles)) return;
-    const int4 e = gp.tiles[tile];
-    if (static_cast<unsigned>(e.x) >= static_cast<unsigned>(gp.experts) || e.y < 0 || e.z <= 0) return;
-    m0 = e.y;
-    m_end = min(e.y + min(e.z, BT), p.M);
-    w_row = e.x * p.N + n_tile * kTileN;
-  }
   const CUtensorMap* mw = is_shared ? &map_ws : &map_w;
   const CUtensorMap* mx = is_shared ? &map_xs : &map_x;
   const int num_kb = p.num_k_blocks;
-
   if (tid == 0) {
     for (int s = 0; s < C::kStages; ++s) {
       mbar_init(&full_bar[s], 1);
@@ -586,6 +566,28 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();  // (behind the allocation: a successor's CTA must not hold tensor memory we wait for)
+
+  int n_tile, m0, m_end, w_row;
+  if (is_shared) {
+    n_tile = unit % gp.shared_n_tiles;
+    m0 = unit / gp.shared_n_tiles * BT;
+    m_end = p.M;
+    w_row = n_tile * kTileN;
+  } else {
+    unit -= gp.shared_units;
+    n_tile = unit % gp.routed_n_tiles;
+    const int tile = unit / gp.routed_n_tiles;
+    pdl_wait();  // the tile list is a kernel's output
+    const int4 e = tile < min(*gp.num_tiles, gp.max_tiles) ? gp.tiles[tile] : make_int4(-1, -1, 0, 0);
+    if (static_cast<unsigned>(e.x) >= static_cast<unsigned>(gp.experts) || e.y < 0 || e.z <= 0) {
+      if (warp == 0) tmem_dealloc(tmem_base, C::kTmemCols);
+      return;
+    }
+    m0 = e.y;
+    m_end = min(e.y + min(e.z, BT), p.M);
+    w_row = e.x * p.N + n_tile * kTileN;
+  }
 
   if (warp == 0) {
     if (lane == 0) {

@@ -324,7 +324,6 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     prefetch_tensormap(&map_x);
   }
 
-  pdl_launch_dependents();
   const uint8_t* sf_gate = p.w_sf + static_cast<int64_t>(pair) * p.k_tiles * kSfTileBytes;
   const uint8_t* sf_up = p.w_sf + static_cast<int64_t>(p.F / kTileN + pair) * p.k_tiles * kSfTileBytes;
   const uint8_t* sf_x = p.x_sf + static_cast<int64_t>(m0 / 128) * p.k_tiles * kSfTileBytes;
@@ -357,6 +356,7 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();  // (behind the allocation: a successor's CTA must not hold tensor memory we wait for)
 
   if (warp == 0 && lane == 0) {
     // ---------------- producer ----------------

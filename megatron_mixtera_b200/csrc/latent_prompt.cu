@@ -59,7 +59,6 @@ latent_prompt_umma_kernel(const __grid_constant__ CUtensorMap map_kv, const __gr
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row = blockIdx.y, head = blockIdx.z;
-  pdl_launch_dependents();
   const int t_begin = a.cu_tokens[row], n_tok = a.cu_tokens[row + 1] - t_begin;
   const int q0 = (gridDim.x - 1 - blockIdx.x) * kQueries;  // the blocks with the most keys start first
   const int e_begin = a.cu_keys[row], key_begin = a.key_start[row];
@@ -97,6 +96,7 @@ latent_prompt_umma_kernel(const __grid_constant__ CUtensorMap map_kv, const __gr
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  pdl_launch_dependents();  // (behind the allocation: a successor's CTA must not hold tensor memory we wait for)
   pdl_wait();
 
   if (warp == kSoftmaxWarps) {
