@@ -349,11 +349,12 @@ latent_prompt_umma_kernel(const __grid_constant__ CUtensorMap map_kv, const __gr
   if (warp == kSoftmaxWarps) tmem_dealloc(tmem, 512);
 }
 
-// Whether this kernel takes the call: 64-column tiles that hold a key and a value, and enough CTAs of 256 queries for the SMs.
+// Whether this kernel takes the call: 64-column tiles that hold a key and a value, and enough CTAs of 256 queries for the SMs.  It masks and takes maxima
+// in front of the scale, which therefore has to be positive: the other kernel has any.
 static bool applicable(const b200_latent_args& a) {
   const int key_tiles = (a.dim + 63) / 64 + (a.rot_dim + 63) / 64;
   const int64_t ctas = static_cast<int64_t>((a.max_row_tokens + kQueries - 1) / kQueries) * a.num_rows * a.heads;
-  return key_tiles <= 3 && a.vdim <= 128 && a.num_keys > 0 && a.row_width % 8 == 0 && a.kv_pad % 8 == 0 && a.num_tokens >= kQueries &&
+  return a.scale > 0.f && key_tiles <= 3 && a.vdim <= 128 && a.num_keys > 0 && a.row_width % 8 == 0 && a.kv_pad % 8 == 0 && a.num_tokens >= kQueries &&
          ctas * 2 >= sm_count() && aligned16(a.q_full);
 }
 

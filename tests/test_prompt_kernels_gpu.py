@@ -227,6 +227,16 @@ def test_prompt_attention_matches_the_plain_one(ops, form, heads, groups, dim, v
     (128, 64, 128, None, "head", False), (24, 16, 40, 33, "head", False), (64, 32, 64, 1, "head", True), (112, 8, 72, 150, "value", True),
     (72, 0, 128, None, "value", True), (128, 64, 128, 257, "head", False)])
 def test_latent_prompts_match_the_plain_attention(ops, dim, rot, vdim, window, gates, sinks):
+    latent_prompts(ops, dim, rot, vdim, window, gates, sinks, (dim + rot) ** -0.5)
+
+
+@pytest.mark.parametrize("scale", [-0.1, 0.0])
+@pytest.mark.parametrize("window", [None, 150])
+def test_latent_prompts_with_a_scale_that_is_not_positive(ops, window, scale):
+    latent_prompts(ops, 128, 64, 128, window, "head", False, scale)  # (scores would be masked with -inf in front of the scale)
+
+
+def latent_prompts(ops, dim, rot, vdim, window, gates, sinks, scale):
     from megatron_mixtera_b200 import _lib
 
     heads, lens, past, dev = 40, [300, 1, 700, 257], [0, 40, 65, 0], "cuda"
@@ -255,7 +265,7 @@ def test_latent_prompts_match_the_plain_attention(ops, dim, rot, vdim, window, g
     a.proj, a.proj_ld, a.gate_offset, a.value_gates = proj.data_ptr(), proj.shape[1], gate_at, int(gates == "value")
     a.q_full, a.q_stride, a.q_rot_at, a.out = q_rot.data_ptr(), q_rot.shape[2], 0, out.data_ptr()
     a.num_tokens, a.heads, a.dim, a.rot_dim, a.rot_dims, a.vdim = T, heads, dim, rot, rot, vdim
-    a.kv_rank, a.kv_pad, a.row_width, a.window, a.scale = kv_pad, kv_pad, width, window or 0, (dim + rot) ** -0.5
+    a.kv_rank, a.kv_pad, a.row_width, a.window, a.scale = kv_pad, kv_pad, width, window or 0, scale
     a.dtype, a.max_positions, a.num_splits, a.chunk_size, a.num_chunks, a.pool = ops.dtype_code(BF16), 1, 1, 64, 1, key_rows.data_ptr()
     if sinks:
         a.sinks = sink.data_ptr()
