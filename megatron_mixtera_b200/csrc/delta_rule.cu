@@ -371,6 +371,9 @@ struct ScanShape {  // COLS columns per CTA, N of them per thread, LANES lanes p
   static_assert(kComputeThreads % 32 == 0 && kScanTokens % kPrepWarps == 0 && kTokPerWarp % kBatch == 0 && DIM % 32 == 0, "");
   static constexpr int kBufFloats = kScanTokens * (5 * DIM + COLS);
   static constexpr int kSmemBytes = 2 * kBufFloats * 4;
+  // Tokens unrolled: 256 channels fill the registers (the next token's vectors would be spilled: 64 rows of 256 tokens x 8 heads of 256 9.0 ms with four,
+  // 7.6 with one; heads of 192 6.9 and 5.4).
+  static constexpr int kUnroll = DIM <= 128 ? 4 : 1;
 };
 
 template <typename T, int DIM, int COLS, int N, int LANES>
@@ -480,7 +483,7 @@ delta_scan_kernel(b200_delta_args a) {
     const float* buf = smem + (c & 1) * Sh::kBufFloats;
     const float* values = buf + kScanTokens * 5 * DIM + group;
     const int cnt = min(kScanTokens, n_tok - c * kScanTokens);
-#pragma unroll 4
+#pragma unroll Sh::kUnroll
     for (int tt = 0; tt < cnt; ++tt) {
       const float* v0 = buf + tt * 5 * DIM;
       const TokenVectors tv{v0, v0 + DIM, v0 + 2 * DIM, v0 + 3 * DIM, v0 + 4 * DIM};

@@ -530,6 +530,11 @@ struct ScanShape {  // COLS columns per CTA, N of them per thread, LANES lanes p
   static constexpr int kTokenFloats = Rule::kVecs * DIM + COLS + 4;
   static constexpr int kBufFloats = kScanTokens * kTokenFloats;
   static constexpr int kSmemBytes = 2 * kBufFloats * 4;
+  // Tokens unrolled: four where their vectors fit the registers beside the state, else one.  64 rows, 16384 tokens, four against one: 32 heads of 32: delta
+  // 303, 255 us, wkv 245, 222, memory 248, 230; of 64: memory 723, 528 (4 rows 455, 429), wkv 445, 512, delta 644, 586 (4 rows 398, 454); 16 heads of 128: wkv
+  // 866, 1086, delta 992, 1067, memory 799, 1005; 8 of 256: delta 4010, 3316 (a kilobyte spilled), wkv 3242, 4324, memory 2573, 2730.
+  static constexpr int kUnroll =
+      DIM <= 32 || (Rule::kKind == B200_RECURRENCE_MEMORY && DIM == 64) || (Rule::kKind == B200_RECURRENCE_DELTA && DIM == 256) ? 1 : 4;
   static_assert(kComputeThreads % 32 == 0 && kScanTokens % kPrepWarps == 0 && kTokPerWarp % kBatch == 0 && COLS % 4 == 0, "");
 };
 
@@ -727,7 +732,7 @@ scan_kernel(b200_recurrence_args a, bool vec_k) {
   for (int c = 0; c < chunks; ++c) {
     const float* buf = smem + (c & 1) * Sh::kBufFloats;
     const int cnt = min(kScanTokens, n_tok - c * kScanTokens);
-#pragma unroll 4
+#pragma unroll Sh::kUnroll
     for (int tt = 0; tt < cnt; ++tt) {
       const float* vec = buf + tt * Sh::kTokenFloats;
       const float* values = vec + Rule::kVecs * DIM;
@@ -967,7 +972,7 @@ static int launch_scan(const b200_recurrence_args& a, cudaStream_t s) {
 }
 template <typename T, typename Rule>
 static int scan_by_dim(const b200_recurrence_args& a, cudaStream_t s) {
-  // Two columns on four lanes, four tokens unrolled (6016 tokens in 4 rows): wkv, 32 heads of 64: 316 -> 288 us; delta, 16 heads of 128: 581 -> 530; memory, 16
+  // Two columns on four lanes (6016 tokens in 4 rows): wkv, 32 heads of 64: 316 -> 288 us; delta, 16 heads of 128: 581 -> 530; memory, 16
   // heads of 128: 498 -> 467.  Other splits (one column on 2, 4, 8 lanes, two on 8, four on 8): 2 to 40 % slower.
   if (a.dim <= 32) return launch_scan<T, Rule, 32, 32, 1, 2, 1>(a, s);
   if (a.dim <= 64) return launch_scan<T, Rule, 64, 64, 2, 4, 1>(a, s);
