@@ -169,6 +169,7 @@ class AttentionArgs(ctypes.Structure):
         ("keep_first", c_int32),
         ("maps", c_int32),
         ("value_gates", c_int32),
+        ("unit_mix", c_int32),
     ]
 
 

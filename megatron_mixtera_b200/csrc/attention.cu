@@ -600,21 +600,59 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 // CTA per token (the decode kernel used row-wise) a K/V tile is read once per 64 / G tokens instead of
 // once per token.  Keys and values are already in the pool (b200_rope_append ran before); the queries are
 // rotated here, in registers.  bf16 pool only.
+//
+// REST: attention_prompt.cu has taken the groups of units that are its own, and a CTA looks through its share of the (unit, KV head) pairs for the others.
 // ---------------------------------------------------------------------------------------------
+constexpr int kUnitsPerGroup = 4;
+constexpr int kAnyRequests = 0, kLongRequests = 1, kShortRequests = 2;  // b200_attention_args::unit_mix
+
+// A unit of the list; padding entries and malformed ones have no tokens.
+__device__ __forceinline__ int4 unit_entry(const Params& p, const int32_t* units, int num_units, int u) {
+  int4 e = make_int4(0, 0, 0, 0);
+  if (u < num_units) e = *reinterpret_cast<const int4*>(units + 4 * static_cast<int64_t>(u));
+  if (e.z > 64 / p.G || e.y < 0 || e.y + e.z > p.T) e.z = 0;
+  return e;
+}
+
+// Whether a group of four units is attention_prompt.cu's, of a list that mixes long and short requests.  That kernel takes a group's requests one after the
+// other, 4 us each beside the tiles, on an SM that holds two to four of the CTAs here: so one request, or two whose units see two tiles of 128 keys on
+// average (four, with 64 value columns: half as long here).  Both kernels ask, and each unit is taken by one of them.  32 heads of 128 in 8 groups, 16
+// requests of 2000 tokens with one more each beside prompts of 2048 and 1000: 284 us with the kernel here alone, 223 with the other, 171 with both; 250 of 500 beside
+// 2048: 355, 271, 217.  Prompts of 20 tokens, 64 of them: 26 here, 29 there, 28 with both - a caller that knows says so (unit_mix).
+template <int DV>
+__device__ __forceinline__ bool prompt_group(const Params& p, const int32_t* units, int num_units, int first) {
+  int4 e[kUnitsPerGroup];
+#pragma unroll
+  for (int u = 0; u < kUnitsPerGroup; ++u) e[u] = unit_entry(p, units, num_units, first + u);
+  int runs = 0;
+#pragma unroll
+  for (int u = 0; u < kUnitsPerGroup; ++u) {
+    bool seen = e[u].z <= 0;
+#pragma unroll
+    for (int v = 0; v < u; ++v) seen = seen || (e[v].z > 0 && e[v].x == e[u].x);
+    runs += !seen;
+  }
+  if (runs != 2) return runs == 1;
+  int tiles = 0;
+#pragma unroll
+  for (int u = 0; u < kUnitsPerGroup; ++u)
+    if (e[u].z > 0) {
+      const int kv = p.kv_len[e[u].y + e[u].z - 1];
+      tiles += ((p.window > 0 ? min(kv, p.window + p.keep_first) : kv) + 2 * kTile - 1) / (2 * kTile);
+    }
+  return tiles >= (DV == 64 ? 4 : 2) * kUnitsPerGroup;
+}
+
+// One unit and KV head.  first: the barriers are still to be set up; ring: tiles that went through the ring before.  Returns how many went through it here.
 template <int DK, int DV, int FORM>
-__global__ void __launch_bounds__(kThreads, 2)
-paged_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, Params p,
-                     const int32_t* __restrict__ units) {
+__device__ __forceinline__ int prefill_unit(const CUtensorMap& map_k, const CUtensorMap& map_v, const Params p, const int32_t* unit, int h, bool first,
+                                            int ring) {
   using C = Cfg<DK, DV>;
   constexpr bool SEPARATE = FORM != kFused, EXTRA = FORM == kExtra;
   constexpr int D = DK;  // fused layout: one width for queries, keys and values
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-
-  pdl_launch_dependents();
-  const int h = blockIdx.x % p.nkv;
-  const int32_t* unit = units + 4 * (blockIdx.x / p.nkv);
   const int row = unit[0];
   const int t0 = unit[1];
   const int n_tok = unit[2];
@@ -622,7 +660,7 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
   const int qb = 64 / G;  // tokens per unit
   if (n_tok <= 0 || n_tok > qb || t0 < 0 || t0 + n_tok > p.T) {  // padding entry (or a malformed one)
     pdl_wait();
-    return;
+    return 0;
   }
   int max_kv = 0, min_kv = 0x7fffffff;
   for (int j = 0; j < n_tok; ++j) {
@@ -640,7 +678,7 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
   uint64_t* empty_bar = full_bar + kStages;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty_bar + kStages);
 
-  if (tid == 0) {
+  if (first && tid == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], kConsumerWarps);
@@ -650,7 +688,7 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
     prefetch_tensormap(&map_k);
     prefetch_tensormap(&map_v);
   }
-  __syncthreads();
+  if (first) __syncthreads();
 
   if (warp == kConsumerWarps) {
     if (lane == 0) {
@@ -658,8 +696,8 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
       const int32_t* bt_row = p.block_table + static_cast<int64_t>(row) * p.max_chunks;
       int cur_c = -1, cur_id = 0;
       for (int i = 0; i < n_tiles; ++i) {
-        const int s = i % kStages;
-        const uint32_t phase = (i / kStages) & 1;
+        const int s = (ring + i) % kStages;
+        const uint32_t phase = ((ring + i) / kStages) & 1;
         const int tok0 = tile_key(i);
         const int c = tok0 / p.chunk;
         if (c != cur_c) {
@@ -677,7 +715,7 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         for (int sub = 0; sub < C::kSubV; ++sub) tma_load_3d(vdst + sub * C::kSubBytes, &map_v, &full_bar[s], sub * 64, EXTRA ? h >> p.kshift : h, tok_row);
       }
     }
-    return;
+    return n_tiles;
   }
 
   // --------------------------------- consumer warps ---------------------------------
@@ -777,13 +815,21 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
     for (int r = 0; r < 2; ++r) far_bias[r] = __ldg(bias_r[r] + p.bias_len - 1) * kLog2e;
 
   for (int i = 0; i < n_tiles; ++i) {
-    const int s = i % kStages;
-    const uint32_t phase = (i / kStages) & 1;
+    const int s = (ring + i) % kStages;
+    const uint32_t phase = ((ring + i) / kStages) & 1;
     const int tok0 = tile_key(i);
     mbar_wait_bounded(&full_bar[s], phase, abort_flag, kStatusAttnTimeout);
     uint8_t* ktile = smem + s * C::kStageBytes;
     uint8_t* vtile = ktile + C::kTileBytesK;
     if (tok0 < warp_kv && (!SEPARATE || tok0 + kTile > warp_first || (EXTRA && tok0 < p.keep_first))) {
+      if (tok0 + kTile > max_kv) {  // value rows behind the newest key hold anything, and a zero weight must not meet a NaN (every warp clears them for itself)
+#pragma unroll
+        for (int sub = 0; sub < C::kSubV; ++sub)
+          for (int v = (max_kv - tok0) * 8 + lane; v < kTile * 8; v += 32)
+            *reinterpret_cast<uint4*>(vtile + sub * C::kSubBytes + v * 16) = make_uint4(0, 0, 0, 0);
+        fence_proxy_async_smem();  // (a later tile's copy comes behind)
+        __syncwarp();
+      }
       // ---- S = Q K^T: 16 rows x 64 tokens ----
       float sacc[8][4];
 #pragma unroll
@@ -934,6 +980,34 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
       const int col = i2 * 8 + tig * 2;
       if (col < p.dv) *reinterpret_cast<uint32_t*>(o + col) = pack_bf16x2(oacc[i2][2 * r] * inv, oacc[i2][2 * r + 1] * inv);
     }
+  }
+  return n_tiles;
+}
+
+template <int DK, int DV, int FORM, bool REST>
+__global__ void __launch_bounds__(kThreads, 2)
+paged_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, Params p, const int32_t* __restrict__ units,
+                     int num_units) {
+  pdl_launch_dependents();
+  if constexpr (!REST) {
+    prefill_unit<DK, DV, FORM>(map_k, map_v, p, units + 4 * (blockIdx.x / p.nkv), blockIdx.x % p.nkv, true, 0);
+  } else {
+    const unsigned pairs = num_units * p.nkv, lane = threadIdx.x & 31;
+    bool first = true;
+    int ring = 0;
+    for (unsigned at = blockIdx.x; at < pairs; at += 32 * gridDim.x) {  // every warp finds the same ones, a pair per lane
+      const int u = (at + lane * gridDim.x) / p.nkv;  // (no entry behind the last one)
+      const int4 e = unit_entry(p, units, num_units, u);
+      unsigned todo = __ballot_sync(0xffffffffu, e.z > 0 && !prompt_group<DV>(p, units, num_units, u / kUnitsPerGroup * kUnitsPerGroup));
+      for (; todo != 0; todo &= todo - 1) {
+        const int l = __ffs(todo) - 1;
+        const unsigned pair = at + l * gridDim.x;
+        ring += prefill_unit<DK, DV, FORM>(map_k, map_v, p, units + 4 * static_cast<int64_t>(pair / p.nkv), pair % p.nkv, first, ring);
+        first = false;
+        __syncwarp();
+      }
+    }
+    if (first && blockIdx.x == 0) pdl_wait();  // (a kernel never ends before its predecessor)
   }
 }
 
@@ -1314,24 +1388,34 @@ static int launch_attention(Params& p, cudaStream_t stream) {
 
 // Long prompts: attention_prompt.cu.
 namespace prompt {
-static bool preferred(const Params& p, const int32_t* units, int num_units);
+template <int DK, int DV>
+static bool preferred(const Params& p, const int32_t* units, int num_units, int mix);
 template <int DK, int DV, int FORM>
-static int launch(const Params& p, const CUtensorMap* mk, const CUtensorMap* mv, const int32_t* units, int num_units, cudaStream_t stream);
+static int launch(const Params& p, const CUtensorMap* mk, const CUtensorMap* mv, const int32_t* units, int num_units, bool all, cudaStream_t stream);
 }  // namespace prompt
 
-template <int DK, int DV, int FORM>
-static int launch_prefill(Params& p, const int32_t* units, int num_units, cudaStream_t stream) {
+// Units of this file's kernel: all of them, one (unit, KV head) pair per CTA, or (REST) those that the prompt kernel has left.
+template <int DK, int DV, int FORM, bool REST>
+static int launch_units(const Params& p, const CUtensorMap* mk, const CUtensorMap* mv, const int32_t* units, int num_units, cudaStream_t stream) {
   using C = Cfg<DK, DV>;
+  static std::atomic<uint64_t> smem_attr_done{0};
+  if (ensure_dynamic_smem(paged_prefill_kernel<DK, DV, FORM, REST>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
+  const int pairs = num_units * p.nkv, ctas = REST ? std::min(pairs, 8 * sm_count()) : pairs;
+  return launch_pdl(paged_prefill_kernel<DK, DV, FORM, REST>, dim3(ctas), dim3(kThreads), C::kSmemBytes, stream, *mk, *mv, p, units, num_units);
+}
+
+template <int DK, int DV, int FORM>
+static int launch_prefill(Params& p, const int32_t* units, int num_units, int mix, cudaStream_t stream) {
   const CUtensorMap *mk, *mv;
   if (!pool_maps(p, mk, mv)) return B200_ERR_DRIVER;
-  static std::atomic<uint64_t> smem_attr_done{0};
-  if (ensure_dynamic_smem(paged_prefill_kernel<DK, DV, FORM>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
-  const int64_t ctas = static_cast<int64_t>(num_units) * p.nkv;
-  if (ctas > 0x7fffffff) return B200_ERR_INVALID_ARGUMENT;
-  const int rc = prompt::preferred(p, units, num_units)
-                     ? prompt::launch<DK, DV, FORM>(p, mk, mv, units, num_units, stream)
-                     : launch_pdl(paged_prefill_kernel<DK, DV, FORM>, dim3(static_cast<unsigned>(ctas)), dim3(kThreads), C::kSmemBytes, stream,
-                                  *mk, *mv, p, units);
+  if (static_cast<int64_t>(num_units) * p.nkv > 0x7fffffff) return B200_ERR_INVALID_ARGUMENT;
+  int rc;
+  if (!prompt::preferred<DK, DV>(p, units, num_units, mix)) {
+    rc = launch_units<DK, DV, FORM, false>(p, mk, mv, units, num_units, stream);
+  } else {
+    rc = prompt::launch<DK, DV, FORM>(p, mk, mv, units, num_units, mix == kLongRequests, stream);
+    if (rc == B200_OK && mix != kLongRequests) rc = launch_units<DK, DV, FORM, true>(p, mk, mv, units, num_units, stream);
+  }
   if (rc != B200_OK || !p.diff) return rc;
   return launch_diff_combine<__nv_bfloat16>(p, p.gate, p.out, DV, 1, stream);
 }
@@ -1377,7 +1461,8 @@ int b200_paged_prefill_attention(const b200_attention_args* a, const int32_t* un
   }
   if (64 % p.G != 0 && !p.separate) return B200_ERR_INVALID_ARGUMENT;  // group sizes 1, 2, 4, 8, 16
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  return attn::by_layout(p, [&](auto dk, auto dv, auto sep) { return attn::launch_prefill<dk, dv, sep>(p, units, num_units, s); });
+  if (a->unit_mix < 0 || a->unit_mix > 2) return B200_ERR_INVALID_ARGUMENT;
+  return attn::by_layout(p, [&](auto dk, auto dv, auto sep) { return attn::launch_prefill<dk, dv, sep>(p, units, num_units, a->unit_mix, s); });
 }
 
 size_t b200_paged_attention_workspace_bytes(int num_tokens, int num_q_heads, int head_dim, int num_splits) {

@@ -28,7 +28,7 @@ namespace prompt {
 constexpr int kSoftmaxWarps = 8, kThreadsPrompt = (kSoftmaxWarps + 2) * 32;
 constexpr int kKeys = 128;         // keys per tile: two pool tiles of kTile
 constexpr int kRingStages = 2;
-constexpr int kUnitsPerCta = 4;
+constexpr int kUnitsPerCta = kUnitsPerGroup;
 constexpr float kLazy = 8.f;       // log2 of how far a maximum may grow before O is rescaled
 constexpr uint32_t kTransposeB = 1u << 16;  // instruction descriptor: B is MN-major
 
@@ -96,7 +96,7 @@ struct Run {
 template <int DK, int DV, int FORM>
 __global__ void __launch_bounds__(kThreadsPrompt, 1)
 paged_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const __grid_constant__ Params p,
-                    const int32_t* __restrict__ units, int num_units) {
+                    const int32_t* __restrict__ units, int num_units, int all) {
   using C = Config<DK, DV>;
   constexpr bool SEPARATE = FORM != kFused, EXTRA = FORM == kExtra;
   extern __shared__ uint8_t smem_raw[];
@@ -116,7 +116,11 @@ paged_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   const int h = blockIdx.x % p.nkv;
   // the last units of a request see the most keys: they start first
   const int first_unit = ((num_units + kUnitsPerCta - 1) / kUnitsPerCta - 1 - static_cast<int>(blockIdx.x / p.nkv)) * kUnitsPerCta;
-  const int G = p.G, qb = 64 / G;
+  if (!all && !prompt_group<DV>(p, units, num_units, first_unit)) {  // paged_prefill_kernel's, or padding
+    if (blockIdx.x == 0) pdl_wait();                                 // (a kernel never ends before its predecessor)
+    return;
+  }
+  const int G = p.G;
 
   if (tid == 0) {
     for (int s = 0; s < kRingStages; ++s) {
@@ -147,15 +151,9 @@ paged_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   pdl_launch_dependents();  // (behind the allocation: a successor's CTA must not hold tensor memory we wait for)
   pdl_wait();  // queries, pool and lengths are earlier kernels' output
 
-  // this CTA's units; padding entries and malformed ones have no tokens
-  int left = 0;
+  int left = 0;  // units to do
 #pragma unroll
-  for (int u = 0; u < kUnitsPerCta; ++u) {
-    if (first_unit + u < num_units) {
-      const int4 e = *reinterpret_cast<const int4*>(units + 4 * static_cast<int64_t>(first_unit + u));
-      if (e.z > 0 && e.z <= qb && e.y >= 0 && e.y + e.z <= p.T) left |= 1 << u;
-    }
-  }
+  for (int u = 0; u < kUnitsPerCta; ++u) left |= (unit_entry(p, units, num_units, first_unit + u).z > 0) << u;
   auto unit_at = [&](int u) { return *reinterpret_cast<const int4*>(units + 4 * static_cast<int64_t>(first_unit + u)); };
   // The next run (warp-collective; every warp finds the same ones).
   auto next_run = [&](Run& r) {
@@ -548,21 +546,27 @@ paged_prompt_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   if (warp == kSoftmaxWarps) tmem_dealloc(tmem, 512);
 }
 
-// Whether four units per CTA leave enough CTAs for the SMs: one for every second SM.  (A prompt of 300 tokens, 40 CTAs here and 152 there: 17.5 us with
-// either; 8 prompts of 300, 304 CTAs: 44 us here, 61 us with one unit per CTA.)
-static bool preferred(const Params& p, const int32_t* units, int num_units) {
-  return aligned16(units) && static_cast<int64_t>((num_units + kUnitsPerCta - 1) / kUnitsPerCta) * p.nkv * 2 >= sm_count();
+// Whether four units per CTA leave enough CTAs for the SMs: one for every second SM, of the units that the tokens fill.  (A prompt of 300 tokens, 40 CTAs
+// here and 152 there: 17.5 us with either; 8 prompts of 300, 304 CTAs: 44 us here, 60 us with one unit per CTA.)  With keys and values of 64 columns the
+// other kernel takes half as long: there only lists come here whose units are 97 % full, so few of them a request's last (8 prompts of 300 over 16 heads
+// 27 us here, 21 there; 4 of 2048 113 and 201).
+template <int DK, int DV>
+static bool preferred(const Params& p, const int32_t* units, int num_units, int mix) {
+  const int qb = 64 / p.G, filled = std::min(num_units, (p.T + qb - 1) / qb);
+  if (mix == kShortRequests || (DK == 64 && DV == 64 && (num_units - filled) * 32 > num_units)) return false;
+  return aligned16(units) && static_cast<int64_t>((filled + kUnitsPerCta - 1) / kUnitsPerCta) * p.nkv * 2 >= sm_count();
 }
 
 template <int DK, int DV, int FORM>
-static int launch(const Params& p, const CUtensorMap* mk, const CUtensorMap* mv, const int32_t* units, int num_units, cudaStream_t stream) {
+static int launch(const Params& p, const CUtensorMap* mk, const CUtensorMap* mv, const int32_t* units, int num_units, bool all,
+                  cudaStream_t stream) {
   using C = Config<DK, DV>;
   static std::atomic<uint64_t> smem_attr_done{0};
   if (ensure_dynamic_smem(paged_prompt_kernel<DK, DV, FORM>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
   const int64_t ctas = static_cast<int64_t>((num_units + kUnitsPerCta - 1) / kUnitsPerCta) * p.nkv;
   if (ctas > 0x7fffffff) return B200_ERR_INVALID_ARGUMENT;
   return launch_pdl(paged_prompt_kernel<DK, DV, FORM>, dim3(static_cast<unsigned>(ctas)), dim3(kThreadsPrompt), C::kSmemBytes, stream, *mk, *mv, p,
-                    units, num_units);
+                    units, num_units, all ? 1 : 0);
 }
 
 }  // namespace prompt

@@ -352,6 +352,7 @@ class DynamicInferenceContext(BaseInferenceContext):
         self.prefill_q_block = 0
         self.prefill_units = None
         self.prefill_unit_count = 0
+        self._unit_mix = {}  # block size -> what the step's list holds
         self._more_units = {}  # further block sizes (head groupings that differ between layers) -> [host, numpy, device, count]
         self._copy_event = torch.cuda.Event() if pin else None
         self._copies_pending = False
@@ -389,17 +390,40 @@ class DynamicInferenceContext(BaseInferenceContext):
         _, _, device, count = self._more_units[q_block]
         return device, count
 
-    def _build_prefill_units(self, ql: np.ndarray, n_rows: int, padded: int, graphs: bool) -> None:
-        self.prefill_unit_count = self._fill_units(self.prefill_q_block, self._h_units, self._h_units_np, self.prefill_units, ql, n_rows,
-                                                   padded, graphs)
-        for qb, entry in self._more_units.items():
-            entry[3] = self._fill_units(qb, *entry[:3], ql, n_rows, padded, graphs)
+    def prefill_unit_mix(self, q_block: int) -> int:
+        """What this step's work list for blocks of ``q_block`` tokens holds (``AttentionArgs.unit_mix``)."""
+        return self._unit_mix.get(q_block, 0)
 
-    def _fill_units(self, qb: int, host: Tensor, u: np.ndarray, device: Tensor, ql: np.ndarray, n_rows: int, padded: int, graphs: bool) -> int:
+    @staticmethod
+    def _mix_of(nb: np.ndarray, keys: np.ndarray) -> int:
+        """`AttentionArgs.unit_mix` of requests of ``nb`` units that see ``keys`` keys on average.  A list of both kinds counts as one of short requests
+        where the long ones are less than a fifth of the short ones' work: two kernels, one behind the other, would take longer (300 beside 250 requests
+        of 500, two maps of 64: 258 us with one, 296 with two; with 1024 more tokens beside 64 of 1000, 32 heads in 8 groups, 141 and 117)."""
+        some = nb > 0
+        nb, keys = nb[some], keys[some]
+        if not nb.size:
+            return 0
+        long = nb >= 8
+        if long.all() or not (nb % 4).any():
+            return 1
+        if not long.any():
+            return 2 if nb.max() == 1 or keys.max() < 768 else 0
+        work = nb * keys
+        return 0 if 5 * work[long].sum() >= work[~long].sum() else 2
+
+    def _build_prefill_units(self, ql: np.ndarray, kv: np.ndarray, n_rows: int, padded: int, graphs: bool) -> None:
+        self.prefill_unit_count = self._fill_units(self.prefill_q_block, self._h_units, self._h_units_np, self.prefill_units, ql, kv,
+                                                   n_rows, padded, graphs)
+        for qb, entry in self._more_units.items():
+            entry[3] = self._fill_units(qb, *entry[:3], ql, kv, n_rows, padded, graphs)
+
+    def _fill_units(self, qb: int, host: Tensor, u: np.ndarray, device: Tensor, ql: np.ndarray, kv: np.ndarray, n_rows: int, padded: int,
+                    graphs: bool) -> int:
         """Split every request's query tokens into blocks of ``qb`` (host side, vectorised); returns how many."""
         ql = ql.astype(np.int64)
         nb = -(-ql // qb)
         total = int(nb.sum())
+        self._unit_mix[qb] = 0 if graphs else self._mix_of(nb, kv - ql // 2)  # (a graph is replayed with other lists)
         # under a CUDA graph the launch size is fixed by the padded sizes; unused entries have 0 tokens
         bound = (-(-padded // qb) + n_rows) if graphs else max(total, 1)
         bound = min(max(bound, total), u.shape[0])
@@ -710,7 +734,7 @@ class DynamicInferenceContext(BaseInferenceContext):
                 t32[1, a:padded] = 0
             self._push_rows(self._d_tok32, self._h_tok32, 2, 0, padded)
             if self.prefill_q_block > 0:
-                self._build_prefill_units(ql, n_rows, padded, graphs)
+                self._build_prefill_units(ql, kv, n_rows, padded, graphs)
         if decode:
             # One CTA per (row, KV head) runs for a time proportional to the row's context: starting the long rows
             # first keeps the SMs evenly loaded to the end of the kernel.  Padding rows (length 0) come last.

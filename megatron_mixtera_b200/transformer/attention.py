@@ -108,6 +108,7 @@ class PagedFlashDecodeAttention(torch.nn.Module):
             ops.rope_append(args)
             if getattr(ctx, "prefill_q_block", 0) > 0 and ctx.prefill_q_block == ops.prefill_q_block(self.num_q_heads, self.num_kv_heads):
                 out.zero_()  # padding tokens belong to no unit
+                args.unit_mix = ctx.prefill_unit_mix(ctx.prefill_q_block)
                 ops.paged_prefill_attention(args, ctx.prefill_units, ctx.prefill_unit_count)
             else:
                 ops.paged_attention(args)

@@ -162,4 +162,5 @@ class GroupedAttention(torch.nn.Module):
             ops.separate_attention(a, proj.dtype, tensor_cores=tc)
         else:
             units, count = ctx.prefill_units_of(self.prefill_unit_tokens())
+            a.unit_mix = ctx.prefill_unit_mix(self.prefill_unit_tokens())
             ops.separate_attention(a, proj.dtype, units=units, num_units=count, tensor_cores=True)

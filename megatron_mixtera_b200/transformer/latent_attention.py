@@ -149,6 +149,7 @@ class LatentAttention(torch.nn.Module):
         a.gate, a.gate_ld = proj.data_ptr() + self.gate_offset * proj.element_size(), proj.stride(0)
         a.value_gates, a._anchor = int(m.gate == "value"), key_values
         units, count = ctx.prefill_units_of(self.BLOCK_TOKENS)
+        a.unit_mix = ctx.prefill_unit_mix(self.BLOCK_TOKENS)
         ops.separate_attention(a, queries.dtype, units=units, num_units=count, tensor_cores=True)
 
     def forward(self, x, ctx, rope=None, step=None):

@@ -108,6 +108,7 @@ class ShortConvAttention(torch.nn.Module):
         if tc:
             out.zero_()  # padding tokens belong to no unit
             units, count = ctx.prefill_units_of(self.prefill_unit_tokens())
+            a.unit_mix = ctx.prefill_unit_mix(self.prefill_unit_tokens())
             ops.separate_attention(a, queries.dtype, units=units, num_units=count, tensor_cores=True)
         else:
             ops.separate_attention(a, queries.dtype, tensor_cores=False)

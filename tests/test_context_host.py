@@ -540,3 +540,28 @@ def test_log_probs_match_the_reference_context():
         assert np.array_equal(np.array([v for x in only_last for v in x]), z[f"s{step}_last_log_probs"]), step
         ctx.update_requests(np.ones(n_req, dtype=np.uint8), new_tokens.numpy())
     assert z["s2_lengths"].tolist() == [1, 1, 6]  # the mixed step: two decoding requests and one prompt
+
+
+@pytest.mark.parametrize("lens,want", [([200, 130], (1, 1)), ([64, 128], (1, 1)), ([100, 33], (2, 0)), ([200, 1], (0, 0)), ([2, 1], (2, 2)),
+                                       ([112], (2, 1))])
+def test_what_a_prefill_work_list_holds(lens, want):
+    """1: only requests of eight units or whole groups of four; 2: only of fewer; 0: both.  Per block size, anew each step."""
+    c = make_ctx(max_requests_override=4, max_tokens_override=512)
+    c.set_prefill_q_block(16, 8)
+    assert c.prefill_unit_mix(16) == 0
+    c.schedule_tokens([(100, [1] * 300), (101, [1])])
+    c.initialize_attention_state()
+    assert c.prefill_unit_mix(16) == 0
+    c.complete_step([100, 101])
+    c.schedule_tokens([(r, [1] * n) for r, n in enumerate(lens)])
+    c.initialize_attention_state()
+    assert (c.prefill_unit_mix(16), c.prefill_unit_mix(8)) == want
+
+
+@pytest.mark.parametrize("units,keys,want", [
+    ([19, 1, 1], [150, 500, 500], 0),
+    ([19] + [1] * 250, [150] + [500] * 250, 2),   # (the long request is little of the work)
+    ([2] * 64, [1009] * 64, 0), ([1] * 64, [1009] * 64, 2), ([5] * 4, [150] * 4, 2),  # few units behind a long past: two kernels may share them
+    ([0, 4, 8], [0, 10, 10], 1), ([0, 0], [0, 0], 0)])
+def test_mix_of_units_and_keys(units, keys, want):
+    assert DynamicInferenceContext._mix_of(np.array(units), np.array(keys)) == want

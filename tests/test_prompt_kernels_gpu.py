@@ -120,11 +120,33 @@ LENS, PAST = [700, 333, 1, 300, 900, 64], [0, 0, 300, 513, 64, 1]
     ("maps", 16, 8, 64, 128, 64, {}),
 ])
 def test_prompt_attention_matches_the_plain_one(ops, form, heads, groups, dim, vdim, chunk, options):
+    prompt_attention(ops, form, heads, groups, dim, vdim, chunk, options, LENS, PAST, 1)
+
+
+# Lists of short and long requests: two kernels share them by groups of four units.  Groups of one, two and more requests, of two that see few or many
+# tiles, padding behind the list; every value of the hint, whatever the list holds.
+MIXED = [1] * 9 + [300, 5, 64, 64, 200, 700, 1, 33] + [16] * 5 + [2, 400, 1]
+MIXED_PAST = [40, 700, 0, 1, 63, 64, 65, 130, 7] + [0, 900, 0, 0, 513, 1, 64, 3] + [0] * 5 + [600, 0, 250]
+
+
+@pytest.mark.parametrize("mix", [0, 1, 2])
+@pytest.mark.parametrize("form,heads,groups,dim,vdim,chunk,options", [
+    ("fused", 32, 8, 128, 128, 64, {}),
+    ("fused", 64, 16, 64, 64, 64, {}),
+    ("separate", 16, 8, 128, 128, 128, {"window": 200}),
+    ("extra", 16, 16, 128, 128, 64, {"window": 300, "keep": 70, "bias": 100, "cap": 7.0, "sinks": True}),
+    ("maps", 16, 8, 64, 128, 64, {}),
+])
+def test_prompt_attention_of_mixed_lists(ops, form, heads, groups, dim, vdim, chunk, options, mix):
+    prompt_attention(ops, form, heads, groups, dim, vdim, chunk, options, MIXED, MIXED_PAST, mix)
+
+
+def prompt_attention(ops, form, heads, groups, dim, vdim, chunk, options, lens, past, mix):
     from megatron_mixtera_b200 import _lib
 
     o = {"window": 0, "keep": 0, "sinks": False, "cap": 0.0, "bias": 0, "gates": None, **options}
     maps, dev = 2 if form == "maps" else 1, "cuda"
-    group, T, kv = heads // groups, sum(LENS), [n + p for n, p in zip(LENS, PAST)]
+    group, T, kv = heads // groups, sum(lens), [n + p for n, p in zip(lens, past)]
     blocks = [-(-n // chunk) for n in kv]
     order = torch.randperm(sum(blocks), generator=torch.Generator().manual_seed(1)).tolist()
     table = torch.zeros(len(kv), max(blocks), dtype=torch.int32)
@@ -141,14 +163,14 @@ def test_prompt_attention_matches_the_plain_one(ops, form, heads, groups, dim, v
             part = rows[b * chunk: (b + 1) * chunk]
             pool[int(table[r, b]), : len(part)] = part
     q = randn(T, groups, group, maps, dim, seed=3)
-    lengths = torch.cat([torch.arange(p + 1, p + n + 1) for n, p in zip(LENS, PAST)]).int().to(dev)
+    lengths = torch.cat([torch.arange(p + 1, p + n + 1) for n, p in zip(lens, past)]).int().to(dev)
     unit, units, t = 64 // group, [], 0
-    for r, n in enumerate(LENS):
+    for r, n in enumerate(lens):
         units += [(r, t + a, min(unit, n - a), 0) for a in range(0, n, unit)]
         t += n
     units += [(0, 0, 0, 0)] * 3  # padding entries
     units, table = torch.tensor(units, dtype=torch.int32, device=dev), table.to(dev)
-    assert -(-len(units) // 4) * groups * maps * 2 >= 148  # (fewer take the kernel for few units)
+    assert -(-(-(-T // unit)) // 4) * groups * maps * 2 >= 148  # (fewer take the kernel for few units)
     out = torch.full((T, heads * vdim), float("nan"), dtype=BF16, device=dev)
 
     a = _lib.AttentionArgs()
@@ -175,6 +197,7 @@ def test_prompt_attention_matches_the_plain_one(ops, form, heads, groups, dim, v
     if maps == 2:
         a.maps, a.diff_scale, a.eps, a.workspace, a.workspace_bytes = 2, 0.7, 1e-5, work.data_ptr(), work.numel() * 4
         a.lambda_ = 0.4
+    a.unit_mix = mix
     a.block_table, a.kv_seq_lengths, a.out = table.data_ptr(), lengths.data_ptr(), out.data_ptr()
     a.num_tokens, a.num_q_heads, a.num_kv_heads, a.head_dim, a.chunk_size = T, heads, groups, dim, chunk
     a.num_chunks, a.max_chunks_per_row, a.num_splits = pool.shape[0], table.shape[1], 1
@@ -199,7 +222,7 @@ def test_prompt_attention_matches_the_plain_one(ops, form, heads, groups, dim, v
         return torch.einsum("hqk,khv->qhv", torch.softmax(s, dim=-1)[..., : past + n], vs)
 
     want, t = [], 0
-    for r, (n, p) in enumerate(zip(LENS, PAST)):
+    for r, (n, p) in enumerate(zip(lens, past)):
         qs = q[t: t + n].reshape(n, heads, maps, dim)
         y = [plain(qs[:, :, m], keys[r][:, :, m], values[r], p, n) for m in range(maps)]
         y = y[0] if maps == 1 else y[0] - 0.4 * y[1]
