@@ -351,7 +351,12 @@ latent_prompt_umma_kernel(const __grid_constant__ CUtensorMap map_kv, const __gr
 
 // Whether this kernel takes the call: 64-column tiles that hold a key and a value, and enough CTAs of 256 queries for the SMs.  It masks and takes maxima
 // in front of the scale, which therefore has to be positive: the other kernel has any.
+// Rows of up to 64 tokens are one CTA in either kernel, on an SM that holds one here and two or three there (16 heads, 64 rows of 64 tokens 82 us here, 47
+// there); from about 100 on a row saves CTAs here (64 of 100: 95 and 109).  A long row among short ones saves ~0.023 us a head for each 64 x 64 products,
+// a short row costs ~0.03 us a head (32 heads, 64 rows that continue with a token beside 4 of 300: 206 us here, 151 there; beside one of 2048: 361, 565).
 static bool applicable(const b200_latent_args& a) {
+  const int64_t longest = a.max_row_tokens;
+  if (longest <= 64 || (a.num_tokens < 64ll * a.num_rows && longest * longest < 12000ll * a.num_rows)) return false;
   const int key_tiles = (a.dim + 63) / 64 + (a.rot_dim + 63) / 64;
   const int64_t ctas = static_cast<int64_t>((a.max_row_tokens + kQueries - 1) / kQueries) * a.num_rows * a.heads;
   return a.scale > 0.f && key_tiles <= 3 && a.vdim <= 128 && a.num_keys > 0 && a.row_width % 8 == 0 && a.kv_pad % 8 == 0 && a.num_tokens >= kQueries &&
