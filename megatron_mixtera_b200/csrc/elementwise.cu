@@ -111,9 +111,11 @@ __device__ __forceinline__ void peer_row_handshake(const PeerSrc& ps, int row) {
 // vector per thread and up to 1024 threads, so that all partial loads of a row are in flight at once.
 // kSrc 2 ("peers"): x = bf16(sum over the tensor-parallel ranks, in rank order, of their bf16 rows), after the
 // row handshake above; every rank computes the same bits.
-// Bound by bytes with many rows, and close behind them by conversions: pairs are rounded with one instruction, whose result is also what is stored.
-// 13000 rows of 4096 with a residual 79.6 -> 72.3 us (floor 64), with MXFP8 87.3 -> 81.1; 11000 of 8192 to blockwise FP8 192 -> 156; 64 of 4096 2.9 -> 2.5 us.
-// (Rows of 4096 without a residual, one norm of a model, 31.1 -> 33.8 us.)
+// Bound by bytes with many rows, and close behind them by conversions: pairs are rounded with one instruction, whose result is also what is stored.  13000
+// rows of 4096 with a residual 65.6 us (floor 64 at the copy rate; pair by pair 77.5), with MXFP8 71 (82), 11000 of 8192 to blockwise FP8 150 (192); without a
+// residual 45.5 (45.7).  With two vectors a thread the normalised row is packed where it is stored only: 38 registers, six CTAs per SM, against 43 and five
+// (13000 rows of 4096 without a residual 50.7 us).  No prefetch of gamma in front of the wait: a request per CTA costs more than the trip it saves (8000
+// rows of 1024 16.1 us with it, 10.1 without).
 template <int kMaxVec, int kSrc>
 __global__ void __launch_bounds__(kSrc != 0 ? 1024 : 256)
 add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ bias,
@@ -124,8 +126,6 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
                 int64_t split_stride, PeerSrc ps) {
   __shared__ float red[32];
   pdl_launch_dependents();
-  if (gamma != nullptr)  // a weight: on its way while the kernel before ends
-    for (int i = threadIdx.x * 8; i < hidden / 8; i += blockDim.x * 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(gamma + i * 8));
   pdl_wait();
   if constexpr (kSrc == 2) {
     peer_row_handshake(ps, blockIdx.x);
@@ -225,8 +225,8 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     return;
   }
   const Vec8* gv = reinterpret_cast<const Vec8*>(gamma);
-  Vec8 weights;  // one vector per thread: read here; behind the block's sums it would be one more trip to L2 (with more vectors it would cost CTAs)
-  if (kMaxVec == 1 && threadIdx.x < nvec) weights = gv[threadIdx.x];
+  Vec8 weights;  // of one long row per CTA: read here; behind the block's sums it would be one more trip to L2 (with several CTAs per SM it would cost some)
+  if (kSrc != 0 && threadIdx.x < nvec) weights = gv[threadIdx.x];
   float mean = 0.f, rstd;
   if (beta != nullptr) {  // LayerNorm: two-pass variance on the cached values
     mean = block_sum(sum, red) / hidden;
@@ -253,7 +253,7 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     const bool valid = i < nvec;
     float y[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (valid) {
-      const Vec8 g = kMaxVec == 1 ? weights : gv[i];
+      const Vec8 g = kSrc != 0 ? weights : gv[i];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         y[2 * k] = (vals[it][2 * k] - mean) * rstd * bf16_lo(g.w[k]);
@@ -269,14 +269,17 @@ add_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
       }
     }
     Vec8 o;
+    const bool store = valid && normed_out != nullptr;
+    if (kMaxVec != 2 || store) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) o.w[k] = pack_bf16x2(y[2 * k], y[2 * k + 1]);
-    if (valid && normed_out) reinterpret_cast<Vec8*>(normed_out + off)[i] = o;
+      for (int k = 0; k < 4; ++k) o.w[k] = pack_bf16x2(y[2 * k], y[2 * k + 1]);
+    }
+    if (store) reinterpret_cast<Vec8*>(normed_out + off)[i] = o;
     if (q_out) {  // quantise the bf16-rounded normalised row (what an unfused quantiser would read)
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        y[2 * k] = bf16_lo(o.w[k]);
-        y[2 * k + 1] = bf16_hi(o.w[k]);
+        y[2 * k] = kMaxVec != 2 ? bf16_lo(o.w[k]) : bf16_round(y[2 * k]);
+        y[2 * k + 1] = kMaxVec != 2 ? bf16_hi(o.w[k]) : bf16_round(y[2 * k + 1]);
       }
       mx::quantize8_any(q_mode, y, valid, blockIdx.x, i * 8, q_out, hidden, sf_out, hidden / 128, m_pad);
     }
