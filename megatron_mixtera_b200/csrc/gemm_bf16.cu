@@ -345,10 +345,11 @@ __device__ __forceinline__ void epilogue(const Params& p, uint32_t tmem_base, ui
 
 // The K splits of an output tile are the CTAs of a cluster: each leaves its partial tile in shared memory, then all of them sum a share of it over the
 // others' shared memory, in split order - the bits of partial sums through global memory and splitk_reduce_kernel - and store bf16.  N a multiple of 4.
-// Up to 32 tokens and four splits: 1 x 10304 x 2048 10.8 -> 9.8 us, 4 x 2560 x 512 5.3 -> 4.4, MXFP8 5 x 1024 x 1024 5.3 -> 4.3 us, the reduction's launch.
+// Up to 24 tokens and four splits: 1 x 10304 x 2048 10.8 -> 9.8 us, 4 x 2560 x 512 5.3 -> 4.4, MXFP8 5 x 1024 x 1024 5.3 -> 4.3 us, the reduction's launch.
+// From 25 rows on the shares are a full tile's: 32 x 10304 x 2048 10.9 us through global memory, 11.2 here, MXFP8 8.0 and 8.6.
 // Clusters of more CTAs leave SMs of a GPC idle (64 x 6144 x 4096, 48 tiles in six splits: 13.4 -> 23.1 us), and larger tiles take longer through the
 // cluster than through L2 (a decode step of 64 tokens with its 64-token tiles in clusters 599 us, without 588).
-constexpr int kMaxClusterSplits = 4, kMaxClusterTokens = 32;
+constexpr int kMaxClusterSplits = 4, kMaxClusterTokens = 32, kMaxClusterRows = 24;
 template <int BT>
 __device__ __forceinline__ void epilogue_cluster(const Params& p, uint32_t tmem_base, uint8_t* stage_smem, int n_tile, int split, int m0, int m_end) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -397,8 +398,8 @@ __device__ __forceinline__ void epilogue_cluster(const Params& p, uint32_t tmem_
   cluster_barrier();  // nobody leaves while its tile is read
 }
 // Whether the K splits of a call that wants bf16 form clusters.
-static bool splits_in_clusters(int splits, int bt, int N) {
-  return splits > 1 && splits <= kMaxClusterSplits && bt <= kMaxClusterTokens && N % 4 == 0;
+static bool splits_in_clusters(int splits, int M, int N) {
+  return splits > 1 && splits <= kMaxClusterSplits && M <= kMaxClusterRows && N % 4 == 0;
 }
 
 template <int BT, bool GATE, bool CLUSTER>
@@ -745,7 +746,7 @@ static int launch(const void* x, int64_t ldx, const void* w, const void* bias, v
   const int m_blocks = (M + BT - 1) / BT;
   const int num_kb = (K + kTileK - 1) / kTileK;
   const int splits = batch > 1 || gate != nullptr ? 1 : choose_splits(n_tiles * m_blocks, num_kb);
-  const bool clusters = partials_out == nullptr && splits_in_clusters(splits, BT, N);
+  const bool clusters = partials_out == nullptr && splits_in_clusters(splits, M, N);
   Params p;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.y = static_cast<__nv_bfloat16*>(y);
@@ -881,7 +882,7 @@ size_t b200_gemm_bf16_workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (pair::preferred(M, N, pair::kFewestRowsBf16)) return 0;
   const size_t bytes = splitk_scratch_bytes(M, N, K);
-  return splits_in_clusters(static_cast<int>(bytes / (static_cast<size_t>(M) * N * sizeof(float))), pick_bt(M), N) ? 0 : bytes;
+  return splits_in_clusters(static_cast<int>(bytes / (static_cast<size_t>(M) * N * sizeof(float))), M, N) ? 0 : bytes;
 }
 
 int b200_gemm_bf16(const void* x, int64_t ldx, const void* w, const void* bias, void* y, int64_t ldy, int M, int N,

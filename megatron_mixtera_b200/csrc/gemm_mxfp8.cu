@@ -203,7 +203,7 @@ static int launch_mxfp8(const void* xq, const void* x_sf, const void* wq, const 
   const int m_blocks = (M + BT - 1) / BT;
   const int num_kb = K / kFp8TileK;
   const int splits = choose_splits(n_tiles * m_blocks, num_kb);
-  const bool clusters = partials_out == nullptr && splits_in_clusters(splits, BT, N);
+  const bool clusters = partials_out == nullptr && splits_in_clusters(splits, M, N);
   Params p;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.y = static_cast<__nv_bfloat16*>(y);
@@ -543,7 +543,7 @@ size_t b200_gemm_mxfp8_workspace_bytes(int M, int N, int K) {
   const int bt = pick_bt(M);
   const int tiles = ((N + kTileN - 1) / kTileN) * ((M + bt - 1) / bt);
   const int splits = choose_splits(tiles, K / kFp8TileK);
-  if (splits == 1 || splits_in_clusters(splits, bt, N)) return 0;
+  if (splits == 1 || splits_in_clusters(splits, M, N)) return 0;
   return static_cast<size_t>(splits) * static_cast<size_t>(M) * N * sizeof(float);
 }
 
