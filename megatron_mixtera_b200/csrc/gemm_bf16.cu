@@ -66,8 +66,10 @@ constexpr int kGatedSilu = 1, kGatedClamped = 2, kGatedPlain = 3;  // Params::ga
 
 // Many tokens: CTA pairs (gemm_pair.cu).
 namespace pair {
-constexpr int kFewestRows = 256, kFewestRowsBf16 = 128;
-static bool preferred(int M, int N, int fewest = kFewestRows);
+static bool preferred_bf16(int M, int N, int K);
+static bool preferred_swiglu(int M, int N);
+static bool preferred_mxfp8(int M, int N, int K);
+static bool preferred_mxfp8_swiglu(int M, int F, int K);
 static int launch_bf16(const void* x, int64_t ldx, const void* w, const void* bias, void* y, int64_t ldy, int M, int N, int K, cudaStream_t stream,
                        float* partials, bool gated, int act);
 }  // namespace pair
@@ -825,7 +827,7 @@ int b200_set_gemm_split_policy(int ctas_per_sm, int min_k_blocks_per_split, int 
 int b200_gemm_bf16_swiglu_supported(int M, int N, int K) {
   using namespace b200::gemm;
   if (M <= 0 || N <= 0 || K <= 0 || N % 128 != 0 || K % 8 != 0) return 0;
-  if (pair::preferred(M, N, pair::kFewestRowsBf16)) return 1;
+  if (pair::preferred_swiglu(M, N)) return 1;
   const int bt = pick_bt(M);
   const int tiles = (N / kTileN) * ((M + bt - 1) / bt);
   return choose_splits(tiles, (K + kTileK - 1) / kTileK) == 1 ? 1 : 0;
@@ -839,7 +841,7 @@ int b200_gemm_bf16_swiglu(const void* x, int64_t ldx, const void* w, void* y, in
   if (!aligned16(x) || !aligned16(w)) return B200_ERR_ALIGNMENT;
   if (!b200_gemm_bf16_swiglu_supported(M, N, K)) return B200_ERR_INVALID_ARGUMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (gemm::pair::preferred(M, N, gemm::pair::kFewestRowsBf16)) return gemm::pair::launch_bf16(x, ldx, w, nullptr, y, ldy, M, N, K, s, nullptr, true, B200_ACT_NONE);
+  if (gemm::pair::preferred_swiglu(M, N)) return gemm::pair::launch_bf16(x, ldx, w, nullptr, y, ldy, M, N, K, s, nullptr, true, B200_ACT_NONE);
   switch (gemm::pick_bt(M)) {
     case 32: return gemm::launch<32>(x, ldx, w, nullptr, y, ldy, M, N, K, nullptr, 0, s, true, nullptr, 0, nullptr, true);
     case 64: return gemm::launch<64>(x, ldx, w, nullptr, y, ldy, M, N, K, nullptr, 0, s, true, nullptr, 0, nullptr, true);
@@ -851,7 +853,7 @@ int b200_gemm_bf16_swiglu(const void* x, int64_t ldx, const void* w, void* y, in
 size_t b200_gemm_bf16_splitk_bytes(int M, int N, int K) {
   using namespace b200::gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (pair::preferred(M, N, pair::kFewestRowsBf16)) return static_cast<size_t>(M) * N * sizeof(float);
+  if (pair::preferred_bf16(M, N, K)) return static_cast<size_t>(M) * N * sizeof(float);
   const int bt = pick_bt(M);
   const int tiles = ((N + kTileN - 1) / kTileN) * ((M + bt - 1) / bt);
   return static_cast<size_t>(choose_splits(tiles, (K + kTileK - 1) / kTileK)) * M * N * sizeof(float);
@@ -864,7 +866,7 @@ int b200_gemm_bf16_splitk(const void* x, int64_t ldx, const void* w, int M, int 
   if (K % 8 != 0 || ldx % 8 != 0 || ldx < K) return B200_ERR_ALIGNMENT;
   if (!aligned16(x) || !aligned16(w) || !aligned16(partials)) return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (gemm::pair::preferred(M, N, gemm::pair::kFewestRowsBf16)) {
+  if (gemm::pair::preferred_bf16(M, N, K)) {
     if (partials_bytes < static_cast<size_t>(M) * N * sizeof(float)) return B200_ERR_WORKSPACE;
     *num_splits = 1;
     return gemm::pair::launch_bf16(x, ldx, w, nullptr, nullptr, N, M, N, K, s, partials, false, B200_ACT_NONE);
@@ -880,7 +882,7 @@ int b200_gemm_bf16_splitk(const void* x, int64_t ldx, const void* w, int M, int 
 size_t b200_gemm_bf16_workspace_bytes(int M, int N, int K) {
   using namespace b200::gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (pair::preferred(M, N, pair::kFewestRowsBf16)) return 0;
+  if (pair::preferred_bf16(M, N, K)) return 0;
   const size_t bytes = splitk_scratch_bytes(M, N, K);
   return splits_in_clusters(static_cast<int>(bytes / (static_cast<size_t>(M) * N * sizeof(float))), M, N) ? 0 : bytes;
 }
@@ -892,7 +894,7 @@ int b200_gemm_bf16(const void* x, int64_t ldx, const void* w, const void* bias, 
   if (K % 8 != 0 || ldx % 8 != 0 || ldx < K || ldy < N) return B200_ERR_ALIGNMENT;
   if (!aligned16(x) || !aligned16(w)) return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (gemm::pair::preferred(M, N, gemm::pair::kFewestRowsBf16)) return gemm::pair::launch_bf16(x, ldx, w, bias, y, ldy, M, N, K, s, nullptr, false, B200_ACT_NONE);
+  if (gemm::pair::preferred_bf16(M, N, K)) return gemm::pair::launch_bf16(x, ldx, w, bias, y, ldy, M, N, K, s, nullptr, false, B200_ACT_NONE);
   switch (gemm::pick_bt(M)) {
     case 32: return gemm::launch<32>(x, ldx, w, bias, y, ldy, M, N, K, workspace, workspace_bytes, s);
     case 64: return gemm::launch<64>(x, ldx, w, bias, y, ldy, M, N, K, workspace, workspace_bytes, s);
@@ -913,7 +915,7 @@ int b200_linear_bf16(const void* x, int64_t ldx, const void* w, void* y, int64_t
   if (gate && (gate_ld < (batch - 1) * y_batch + N || act != B200_ACT_NONE)) return B200_ERR_INVALID_ARGUMENT;
   if (!aligned16(x) || !aligned16(w)) return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (batch == 1 && gate == nullptr && gemm::pair::preferred(M, N, gemm::pair::kFewestRowsBf16))
+  if (batch == 1 && gate == nullptr && gemm::pair::preferred_bf16(M, N, K))
     return gemm::pair::launch_bf16(x, ldx, w, nullptr, y, ldy, M, N, K, s, nullptr, false, act);
   switch (gemm::pick_bt(M)) {
     case 32: return gemm::launch<32>(x, ldx, w, nullptr, y, ldy, M, N, K, workspace, workspace_bytes, s, true, nullptr, 0, nullptr, false, act, batch, x_batch, y_batch, gate, gate_ld);

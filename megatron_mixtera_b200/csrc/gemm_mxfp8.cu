@@ -508,7 +508,7 @@ size_t b200_mxfp8_scale_bytes(int rows, int K) {
 size_t b200_gemm_mxfp8_splitk_bytes(int M, int N, int K) {
   using namespace b200::gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (pair::preferred(M, N)) return static_cast<size_t>(M) * N * sizeof(float);
+  if (pair::preferred_mxfp8(M, N, K)) return static_cast<size_t>(M) * N * sizeof(float);
   const int bt = pick_bt(M);
   const int tiles = ((N + kTileN - 1) / kTileN) * ((M + bt - 1) / bt);
   return static_cast<size_t>(choose_splits(tiles, K / kFp8TileK)) * M * N * sizeof(float);
@@ -523,7 +523,7 @@ int b200_gemm_mxfp8_splitk(const void* xq, const void* x_sf, const void* wq, con
   if (!aligned16(xq) || !aligned16(wq) || !aligned16(x_sf) || !aligned16(w_sf) || !aligned16(partials))
     return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (gemm::pair::preferred(M, N)) {
+  if (gemm::pair::preferred_mxfp8(M, N, K)) {
     if (partials_bytes < static_cast<size_t>(M) * N * sizeof(float)) return B200_ERR_WORKSPACE;
     *num_splits = 1;
     return gemm::pair::launch_mxfp8(xq, x_sf, wq, w_sf, nullptr, nullptr, N, M, N, K, s, partials, false, nullptr, nullptr);
@@ -539,7 +539,7 @@ int b200_gemm_mxfp8_splitk(const void* xq, const void* x_sf, const void* wq, con
 size_t b200_gemm_mxfp8_workspace_bytes(int M, int N, int K) {
   using namespace b200::gemm;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (pair::preferred(M, N)) return 0;
+  if (pair::preferred_mxfp8(M, N, K)) return 0;
   const int bt = pick_bt(M);
   const int tiles = ((N + kTileN - 1) / kTileN) * ((M + bt - 1) / bt);
   const int splits = choose_splits(tiles, K / kFp8TileK);
@@ -554,7 +554,7 @@ int b200_gemm_mxfp8(const void* xq, const void* x_sf, const void* wq, const void
   if (K % 128 != 0 || ldy < N) return B200_ERR_ALIGNMENT;
   if (!aligned16(xq) || !aligned16(wq) || !aligned16(x_sf) || !aligned16(w_sf)) return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (gemm::pair::preferred(M, N))
+  if (gemm::pair::preferred_mxfp8(M, N, K))
     return gemm::pair::launch_mxfp8(xq, x_sf, wq, w_sf, bias, y, ldy, M, N, K, s, nullptr, false, nullptr, nullptr);
   switch (gemm::pick_bt(M)) {
     case 32: return gemm::launch_mxfp8<32>(xq, x_sf, wq, w_sf, bias, y, ldy, M, N, K, workspace, workspace_bytes, s);
@@ -574,7 +574,7 @@ int b200_gemm_mxfp8_swiglu(const void* xq, const void* x_sf, const void* wq, con
       (sf_out && !aligned16(sf_out)) || (y_out && !aligned16(y_out)))
     return B200_ERR_ALIGNMENT;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (gemm::pair::preferred(M, 2 * F))
+  if (gemm::pair::preferred_mxfp8_swiglu(M, F, K))
     return gemm::pair::launch_mxfp8(xq, x_sf, wq, w_sf, nullptr, y_out, ldy, M, 2 * F, K, s, nullptr, true, q_out, sf_out);
   switch (gemm::pick_bt_pair(M)) {
     case 32: return gemm::launch_mxfp8_pair<32>(xq, x_sf, wq, w_sf, q_out, sf_out, y_out, ldy, M, F, K, s);

@@ -435,12 +435,29 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   if (warp == kProducerWarp) tmem_dealloc_pair(tmem_base, C::kTmemCols);
 }
 
-// Whether the pairs' tiles are the better split: more rows than `fewest`, and at least one tile for every pair of SMs.  bf16 above 128 rows (256 x 128256 x
-// 8192: 489 us on the streaming kernel, 417 here); with scales above 256 (up to there the streaming kernel reads a weight once as well).  64 tiles, 1024
-// tokens x 4096 x 4096: 48.8 us here, 44.2 us with K split over the streaming kernel's CTAs; 96 tiles, MXFP8 1024 x 6144 x 4096: 47.9 and 48.5 us.
-static bool preferred(int M, int N, int fewest) {
-  const int64_t tiles = static_cast<int64_t>((M + kTile - 1) / kTile) * ((N + kTile - 1) / kTile);
-  return M > fewest && tiles >= sm_count() / 2;
+// Whether the pairs' tiles are the better split: at least one tile for every pair of SMs, of more rows than one block of the streaming kernels' tokens.  (64
+// tiles, 1024 tokens x 4096 x 4096: 48.8 us here, 44.2 us with K split over the streaming kernel's CTAs.)
+static int64_t tiles_of(int M, int N) { return static_cast<int64_t>((M + kTile - 1) / kTile) * ((N + kTile - 1) / kTile); }
+static bool enough(int M, int N, int fewest) { return M > fewest && tiles_of(M, N) >= sm_count() / 2; }
+
+// A pair's tile costs ~8 us more than its products do here (start, operands only behind the wait, the last epilogue), the streaming kernel's two CTAs for the
+// same outputs ~4.  Up to two waves of pairs (148 tiles) that is made up for by about 370 000 tiles x K: K 512 20 us against 13, 1024 23.5 and 18.4, 2048 31.5 and
+// 28.8, 4096 50.5 and 49-58 (75 tiles 47.8, 112 51.9), 8192 1.04-1.11 x as fast.  From three waves on by K 1280 (1.04-1.16 x; 1024: 0.87-1.03 x, 1.04-1.13 x from
+// 444 tiles on; 512: 0.70-0.86 x).  256 x 128256 x 8192: 489 us on the streaming kernel, 417 here.
+static bool preferred_bf16(int M, int N, int K) {
+  if (!enough(M, N, 128)) return false;
+  const int64_t tiles = tiles_of(M, N);
+  return tiles <= sm_count() ? tiles * K >= 368640 : K >= (tiles >= 3 * sm_count() ? 1024 : 1280);
+}
+// SwiGLU in the epilogue, which the streaming kernel does not overlap: 1.1-2.0 x as fast at any K.
+static bool preferred_swiglu(int M, int N) { return enough(M, N, 128); }
+// Scales double what a byte of operands is worth: up to 148 tiles from K 1024 on (1.03-1.6 x as fast; 512: 0.91-0.94 x), else from 512 on (0.98-1.17 x; 256: 0.88-0.99 x).
+// Up to 256 rows the streaming kernel reads a weight once as well.
+static bool preferred_mxfp8(int M, int N, int K) { return enough(M, N, 256) && K >= (tiles_of(M, N) <= sm_count() ? 1024 : 512); }
+// The streaming kernel's CTAs take 128 x 128 gate and up rows: one wave of them is faster than two of pairs (1100 x 4096 x 4096, 144 CTAs or 80 tiles: 27.5 and 39.6 us).
+static bool preferred_mxfp8_swiglu(int M, int F, int K) {
+  const bool one_wave = static_cast<int64_t>((M + 127) / 128) * (F / 128) <= sm_count() && tiles_of(M, 2 * F) > sm_count() / 2;
+  return preferred_mxfp8(M, 2 * F, K) && !one_wave;
 }
 
 template <bool MX, int FORM, bool EXPERTS = false>

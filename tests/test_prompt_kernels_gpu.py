@@ -40,6 +40,11 @@ SHAPES = [
     (5000, 1160, 64),    # a single K block
     (300, 16384, 192),
     (129, 18828, 136),   # one token block, half of it used
+    # (the pairs take these; of the ones above, which the streaming kernel takes, its SwiGLU only)
+    (257, 19204, 1352),  # one token in the second token block, N 4 past a tile, K of 21 blocks and a bit
+    (4097, 2312, 1280),  # N inside the last tile's first half
+    (129, 38532, 1288),  # one token block, half of it used
+    (700, 6400, 5000),   # two waves: long K only
 ]
 
 
@@ -59,7 +64,7 @@ def test_pair_gemm_matches_the_fp32_product(ops, M, N, K):
     assert torch.equal(wide[:, :N], ops.gemm(x, w)) and not wide[:, N:].any()
 
 
-@pytest.mark.parametrize("M,F,K", [(257, 7168, 256), (2048, 1280, 512), (1500, 3200, 72)])
+@pytest.mark.parametrize("M,F,K", [(257, 7168, 256), (2048, 1280, 512), (1500, 3200, 72), (300, 9664, 1352)])
 def test_pair_gemm_swiglu_equals_gemm_then_activation(ops, M, F, K):
     x, w = randn(M, K, seed=4), randn(2 * F, K, seed=5, scale=K ** -0.5)
     assert ops.gemm_swiglu_supported(M, 2 * F, K)
@@ -67,7 +72,8 @@ def test_pair_gemm_swiglu_equals_gemm_then_activation(ops, M, F, K):
     assert torch.equal(got, ops.activation(ops.gemm(x, w), "swiglu"))
 
 
-@pytest.mark.parametrize("M,N,K", [(257, 14336, 128), (1000, 4864, 384), (4097, 1152, 512), (2048, 2560 + 40, 1024)])
+@pytest.mark.parametrize("M,N,K", [(257, 14336, 128), (1000, 4864, 384), (4097, 1152, 512), (2048, 2560 + 40, 1024), (257, 14592, 1152), (4097, 1128, 1024),
+                                   (3000, 3328, 640)])  # (the pairs take the last four)
 def test_pair_gemm_mxfp8_matches_the_dequantised_product(ops, M, N, K):
     from oracle import decode_oracle as O
 
@@ -88,7 +94,7 @@ def test_pair_gemm_mxfp8_matches_the_dequantised_product(ops, M, N, K):
     assert rel(ops.gemm_mxfp8(xq, wq, b), ref.to(BF16).double() + b.double()) < 3e-3
 
 
-@pytest.mark.parametrize("M,F,K", [(257, 7168, 256), (1500, 2176, 384), (2048, 1280, 1024)])
+@pytest.mark.parametrize("M,F,K", [(257, 7168, 256), (1500, 2176, 384), (2048, 1280, 1024), (257, 7168, 1024), (1500, 2176, 1152), (1100, 2048, 1024)])
 def test_pair_gemm_mxfp8_swiglu_equals_gemm_then_activation(ops, M, F, K):
     x, w = ops.quantize_mxfp8(randn(M, K, seed=9)), ops.quantize_mxfp8_weight(randn(2 * F, K, seed=10, scale=K ** -0.5))
     y = ops.gemm_mxfp8(x, w)
