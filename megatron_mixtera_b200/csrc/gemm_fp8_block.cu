@@ -39,7 +39,7 @@ struct BlkOperands {
   const float* x_scale;  // [K/128][m_pad]
   int k_tiles;
   int m_pad;
-  int n_tiles = 0, m_blocks = 0;  // gemm_fp8_block_tok.cu: the grid
+  int n_tiles = 0, m_blocks = 0, m_rows = 0;  // gemm_fp8_block_tok.cu: the grid, tokens of a block
 };
 
 __device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32]) {

@@ -68,11 +68,14 @@ gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   // Tiles in groups of kGroupM token blocks, token blocks innermost: the CTAs that run at a time share both operands in L2.  (With the weight tiles
   // innermost every wave read other weights, all of them from HBM once per 256 tokens: 11000 x 57344 x 8192 7.8 ms, then 7.1 ms.)
   const int split = blockIdx.y;
-  const int per_group = kGroupM * q.n_tiles, group = static_cast<int>(blockIdx.x) / per_group, in_group = static_cast<int>(blockIdx.x) - group * per_group;
-  const int rows = min(kGroupM, q.m_blocks - group * kGroupM);
-  const int n_tile = in_group / rows;
-  const int m_block = group * kGroupM + (in_group - n_tile * rows);
-  const int m0 = m_block * C::kTokens;
+  int n_tile = blockIdx.x, m_block = 0;
+  if (q.m_blocks > 1) {
+    const int per_group = kGroupM * q.n_tiles, group = n_tile / per_group, in_group = n_tile - group * per_group;
+    const int rows = min(kGroupM, q.m_blocks - group * kGroupM);
+    n_tile = in_group / rows;
+    m_block = group * kGroupM + (in_group - n_tile * rows);
+  }
+  const int m0 = m_block * q.m_rows;
   const int kb_begin = split * p.k_blocks_per_split;
   const int kb_end = min(p.num_k_blocks, kb_begin + p.k_blocks_per_split);
   const int num_kb = kb_end - kb_begin;
@@ -199,7 +202,7 @@ gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
 
     // ---------------- epilogue: the thread's token row, 128 consecutive features, straight from registers ----------------
     const int m = m0 + tok;
-    if (m < p.M && n0 < p.N) {
+    if (tok < q.m_rows && m < p.M && n0 < p.N) {
       const bool full_tile = n0 + kTileN <= p.N;
       if (p.num_splits == 1 && !p.keep_partials) {
         __nv_bfloat16* dst = p.y + static_cast<int64_t>(m) * p.ldy + n0;
@@ -296,6 +299,9 @@ static int launch_fp8_block_tok(const void* xq, const float* x_scale, int m_pad,
   if (ensure_dynamic_smem(gemm_fp8_block_tok_kernel<H>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
   q.n_tiles = n_blocks;
   q.m_blocks = m_blocks;
+  // The blocks share the tokens evenly (scales are copied 4 at a time): with a last block of one token the others' stores would take as long as two
+  // full ones.  129 tokens, 2048 x 2048: 15.2 us with blocks of 128 and 1, 10.9 with 68 and 61; 6144 x 4096: 22.7 and 18.6.
+  q.m_rows = min(C::kTokens, ((M + m_blocks - 1) / m_blocks + 3) / 4 * 4);
   if (static_cast<int64_t>(n_blocks) * m_blocks > 0x7fffffff) return B200_ERR_INVALID_ARGUMENT;
   dim3 grid(static_cast<unsigned>(n_blocks * m_blocks), splits);
   const int rc = launch_pdl(gemm_fp8_block_tok_kernel<H>, grid, dim3(C::kThreads), C::kSmemBytes, stream, *mw, *mx_, p, q);
