@@ -19,9 +19,9 @@ from .hybrid_config import HybridConfig, LatentAttentionConfig
 def choose_latent_splits(num_rows: int, heads: int, window, max_sequence_length: int, blocks_per_row: int) -> int:
     """Key splits of a decode row, each of them ``blocks_per_row`` CTAs: a function of capture-time constants.  The fewest splits that
     fill the CTAs the GPU holds at once to 85 % (else the best there is): one below 256 keys, none below 64 keys at the longest visible range,
-    beyond 16 splits none below 256.  (A CTA walks its tiles of 32 keys one after the other, 3 us each: a step of one request with 700 tokens, 2 layers of
-    this kind, takes 412 us with splits of 384 keys and 390 with 128, one of 16 requests with 600 tokens 394 and 381.  With 100 tokens one split 378 and
-    two 380 us; with 8192 16 splits 411 and 64 splits 434 us: merging them takes longer.)"""
+    beyond 16 splits none below 256.  (A CTA walks its tiles of 32 keys one after the other: a step of one request with 700 tokens, 2 layers of this kind,
+    takes 412 us with splits of 384 keys and 390 with 128, eight tiles fewer in a layer, 1.4 us each; one of 16 requests with 600 tokens 394 and 381.  With
+    100 tokens one split 378 and two 380 us; with 8192 16 splits 411 and 64 splits 434 us: merging them takes longer.)"""
     slots = _sm_count() * (2 if heads <= 16 else 1)
     blocks = max(1, num_rows * blocks_per_row)
     keys = max_sequence_length if window is None else min(window, max_sequence_length)

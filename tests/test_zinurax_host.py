@@ -311,3 +311,31 @@ def test_scaling_factor_of_the_rotation():
     assert freq == pytest.approx([10000.0 ** (-2 * i / 8) for i in range(4)])  # everything turns often over such a context
     freq, _ = Z.rope_frequencies({"base": 10000.0, "dims": 8, "scaling": {"factor": 4.0, "original": 1.0, "fast": 2.0, "slow": 1.0}})
     assert freq[1:] == pytest.approx([10000.0 ** (-2 * i / 8) / 4.0 for i in range(1, 4)])
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+# Key splits of latent decode
+# ---------------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("window", [None, 33, 200, 256, 1000])
+@pytest.mark.parametrize("keys", [1, 100, 255, 256, 640, 1024, 4096, 8192, 131072])
+def test_latent_key_splits(monkeypatch, keys, window):
+    """One split below 256 keys; none shorter than 64 keys, nor, beyond 16 splits, than 256; 64 at most; the fewest that fill the GPU."""
+    from megatron_mixtera_b200.transformer import latent_attention as L
+
+    monkeypatch.setattr(L, "_sm_count", lambda: 148)
+    seen = keys if window is None else min(keys, window)
+    for heads in (16, 32):
+        slots = 148 * (2 if heads == 16 else 1)
+        for rows in (1, 3, 16, 64, 200):
+            for blocks in (1, 2):
+                s = L.choose_latent_splits(rows, heads, window, keys, blocks)
+                assert 1 <= s <= 64
+                if seen < 256:
+                    assert s == 1
+                else:
+                    assert s * 64 <= seen and (s <= 16 or s * 256 <= seen)
+                if rows * blocks >= 0.85 * slots and rows * blocks <= slots:
+                    assert s == 1
+    one = {255: 1, 256: 4, 640: 10, 1024: 16, 4096: 16, 8192: 32, 131072: 64}
+    if window is None and keys in one:  # one request: as many as the limits leave
+        assert L.choose_latent_splits(1, 16, None, keys, 1) == one[keys]
