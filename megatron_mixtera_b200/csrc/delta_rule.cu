@@ -342,10 +342,11 @@ delta_decode_kernel(b200_delta_args a, int w2_stride) {
 // Scan
 // ---------------------------------------------------------------------------------------------------------------
 // The k-th longest row.  A row's tokens are one chain, so the longest rows end last: their CTAs start first and get an SM of their own, the shortest
-// rows share what is left.  (Warp-collective; more than 32 rows are taken as they come.)
+// rows share what is left.  (Warp-collective; more than 32 rows are taken as they come.  A row whose tokens end before they start counts as an empty one:
+// any row is in front of the lanes that have none.)
 __device__ __forceinline__ int longest_first(const int32_t* cu_tokens, int rows, int k) {
   if (rows > 32) return k;
-  const int lane = threadIdx.x & 31, len = lane < rows ? cu_tokens[lane + 1] - cu_tokens[lane] : -1;
+  const int lane = threadIdx.x & 31, len = lane < rows ? max(cu_tokens[lane + 1] - cu_tokens[lane], 0) : -1;
   int rank = 0;
 #pragma unroll
   for (int j = 0; j < 32; ++j) {

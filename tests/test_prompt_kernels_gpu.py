@@ -373,6 +373,26 @@ def test_scanned_rows_do_not_depend_on_the_others(ops, heads, dim, rows):
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
 
 
+def test_a_row_that_ends_before_it_starts_is_left_out(ops):
+    from test_zinurax_kernels_gpu import DeltaCase
+
+    T = 40
+    c = DeltaCase(2, 64, 16, T, torch.bfloat16, seed=50)
+    before = torch.randn(3, 2, 64, 64, generator=torch.Generator().manual_seed(51)).cuda()
+    slots = torch.arange(3, dtype=torch.int32, device="cuda")
+    o, out, lora = torch.zeros(T, c.n, device="cuda"), torch.empty(T, c.n, dtype=BF16, device="cuda"), torch.empty(T, 16, dtype=BF16, device="cuda")
+    state = before.clone()
+    a = c.args(state, slots, slots, out)
+    whole, torn = (torch.tensor(at, dtype=torch.int32, device="cuda") for at in ([0, 20, 20, 40], [0, 20, 10, 40]))  # (rows 0 and 2 share tokens 10 to 19)
+    a.num_rows, a.cu_tokens, a.o_f32, a.lora = 3, whole.data_ptr(), o.data_ptr(), lora.data_ptr()
+    ops.delta_lora(a, state)
+    z = ops.linear(lora, c.dev[1])
+    a.z, a.cu_tokens = z.data_ptr(), torn.data_ptr()
+    ops.delta_scan(a, state)
+    torch.cuda.synchronize()
+    assert torch.equal(state[1], before[1]) and not torch.equal(state[0], before[0]) and not torch.equal(state[2], before[2])
+
+
 # ---------------------------------------------------------------------------------------------------------------------
 # K splits as clusters: bf16 out of the sums of partial tiles, against the same sums through `gemm_splitk` (same splits, same order: same bits).
 # ---------------------------------------------------------------------------------------------------------------------
