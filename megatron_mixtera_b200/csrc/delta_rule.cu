@@ -373,8 +373,8 @@ struct ScanShape {  // COLS columns per CTA, N of them per thread, LANES lanes p
   static constexpr int kBufFloats = kScanTokens * (5 * DIM + COLS);
   static constexpr int kSmemBytes = 2 * kBufFloats * 4;
   // Tokens unrolled: 256 channels fill the registers (the next token's vectors would be spilled: 64 rows of 256 tokens x 8 heads of 256 9.0 ms with four,
-  // 7.6 with one; heads of 192 6.9 and 5.4).
-  static constexpr int kUnroll = DIM <= 128 ? 4 : 1;
+  // 7.6 with one; heads of 192 6.9 and 5.4); 32 have nothing to hide, and cost registers (four heads of 32, 300 rows of 20 tokens 25.2 us, 22.1).
+  static constexpr int kUnroll = DIM > 32 && DIM <= 128 ? 4 : 1;
 };
 
 template <typename T, int DIM, int COLS, int N, int LANES>
