@@ -50,10 +50,11 @@ __device__ __forceinline__ bool source_row(const b200_out_norm_args& a, int row,
 }
 
 // width % 4 == 0 and width <= SLOTS * THREADS * 4: the row lives in registers.  Bound by latency with few rows, by bytes in flight with many.  What the sums do
-// not need is read before them, the weight before the kernel in front has ended, the residual row together with the sublayer's: behind two block sums
-// each was one more trip to memory.  One row of 2048 and eight splits 3.6 -> 2.3 us, 64 of 4096 6.3 -> 3.9, 6208 of 2048 58.9 -> 37.0 us (floor 26.8).
-template <typename T, int SLOTS, int THREADS>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
+// not need is read before them (kEarly), the weight before the kernel in front has ended, the residual row together with the sublayer's: behind two block sums
+// each was one more trip to memory.  One row of 2048 and eight splits 3.6 -> 2.3 us, 64 of 4096 6.3 -> 3.9, 6208 of 2048 58.9 -> 37.0 us (floor 26.8).  It costs
+// registers, so CTAs (8192 rows of 8192 240 -> 390 us): with several rows on an SM only short ones do it.
+template <typename T, int SLOTS, int THREADS, bool kEarly, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS)
 out_norm_vec_kernel(b200_out_norm_args a) {
   __shared__ float red[THREADS / 32];
   pdl_launch_dependents();
@@ -61,7 +62,6 @@ out_norm_vec_kernel(b200_out_norm_args a) {
   const int row = blockIdx.x;
   const int W = a.width;
   const T* gamma = static_cast<const T*>(a.gamma);
-  constexpr bool kEarly = SLOTS <= 2;  // (more would cost CTAs: 8192 rows of 8192 240 -> 390 us)
   constexpr int kEarlySlots = kEarly ? SLOTS : 1;
   float4 v[SLOTS], early_g[kEarlySlots], early_h[kEarlySlots];
   if constexpr (kEarly) {
@@ -188,21 +188,26 @@ out_norm_any_kernel(b200_out_norm_args a) {
   }
 }
 
+template <typename T, int SLOTS, int THREADS, bool kEarly, int CTAS>
+static int launch_vec(const b200_out_norm_args& a, cudaStream_t s) {
+  return launch_pdl(out_norm_vec_kernel<T, SLOTS, THREADS, kEarly, CTAS>, dim3(a.rows), dim3(THREADS), 0, s, a);
+}
 template <typename T>
 static int launch(const b200_out_norm_args& a, cudaStream_t s) {
   const bool aligned = a.width % 4 == 0 && a.width <= kMaxVecWidth && aligned16(a.partials) && aligned16(a.table) && aligned16(a.rows_in) &&
                        aligned16(a.gamma) && aligned16(a.hidden) && aligned16(a.y);
-  const dim3 grid(a.rows);
-  if (aligned && a.rows <= 2 * sm_count()) {  // few rows: more threads for each
-    if (a.width > 4096) return launch_pdl(out_norm_vec_kernel<T, 2, 1024>, grid, dim3(1024), 0, s, a);
-    if (a.width > 2048) return launch_pdl(out_norm_vec_kernel<T, 1, 1024>, grid, dim3(1024), 0, s, a);
-    if (a.width > 1024) return launch_pdl(out_norm_vec_kernel<T, 1, 512>, grid, dim3(512), 0, s, a);
-  }
   if (aligned) {
-    if (a.width <= 1024) return launch_pdl(out_norm_vec_kernel<T, 1, kThreads>, grid, dim3(kThreads), 0, s, a);
-    if (a.width <= 2048) return launch_pdl(out_norm_vec_kernel<T, 2, kThreads>, grid, dim3(kThreads), 0, s, a);
-    if (a.width <= 4096) return launch_pdl(out_norm_vec_kernel<T, 2, 512>, grid, dim3(512), 0, s, a);
-    return launch_pdl(out_norm_vec_kernel<T, 8, kThreads>, grid, dim3(kThreads), 0, s, a);
+    const int slots = (a.width + 2047) / 2048, sms = sm_count();
+    if (a.width <= 1024) return launch_vec<T, 1, 256, true, 4>(a, s);
+    if (slots == 1) return a.rows <= 2 * sms ? launch_vec<T, 1, 512, true, 2>(a, s) : launch_vec<T, 2, 256, true, 4>(a, s);
+    // Longer rows: one on each SM; up to 3072 columns (three vectors for each of 256 threads) four; else two, or three if there are more rows than that.
+    // One CTA of 1024 threads a row up to 296 rows, and 512 or 256 threads with more, had been slower there than 256 for every row (us with 1, 4 splits, that
+    // first / 1024 and so on / now): 200 rows of 3072 4.3, 4.9 / 5.1, 5.9 / 3.9, 4.3; 296 of 4096 5.3, 6.1 / 5.9, 6.9 / 3.5, 4.6; 600 of 8192 13.3, 28.3 / 13.7, 32.3 /
+    // 11.5, 25.3; 1200 of 4096 11.9, 22.8 / 11.9, 25.8 / 9.7, 20.6.
+    if (a.rows <= sms) return slots == 2 ? launch_vec<T, 2, 512, true, 1>(a, s) : slots == 3 ? launch_vec<T, 3, 512, true, 1>(a, s) : launch_vec<T, 4, 512, true, 1>(a, s);
+    if (a.width <= 3072) return launch_vec<T, 3, 256, false, 4>(a, s);
+    if (a.rows <= 2 * sms) return slots == 2 ? launch_vec<T, 2, 512, true, 2>(a, s) : slots == 3 ? launch_vec<T, 3, 512, false, 2>(a, s) : launch_vec<T, 4, 512, false, 2>(a, s);
+    return slots == 2 ? launch_vec<T, 2, 512, false, 3>(a, s) : slots == 3 ? launch_vec<T, 3, 512, false, 3>(a, s) : launch_vec<T, 4, 512, false, 3>(a, s);
   }
   static std::atomic<uint64_t> done{0};
   if (ensure_dynamic_smem(out_norm_any_kernel<T>, kMaxWidth * 4, done) != B200_OK) return B200_ERR_LAUNCH;

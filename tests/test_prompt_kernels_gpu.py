@@ -438,3 +438,11 @@ def test_output_norm_by_rows_and_width(ops, rows, width, splits, accumulate):
     want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * gamma.double() + accumulate * before.double()
     assert float((hidden.double() - want).abs().max()) < 1e-5 * float(want.abs().max())
     assert torch.equal(y, hidden.to(BF16))
+
+
+# One row more than SMs, and than twice as many, with two, three and four vectors a thread; three on 256 threads.
+@pytest.mark.parametrize("accumulate", [0, 1])
+@pytest.mark.parametrize("rows,width,splits", [(148, 2052, 1), (148, 6144, 3), (148, 8192, 2), (149, 2052, 2), (149, 3076, 1), (149, 4100, 1), (149, 8188, 3),
+                                               (296, 6144, 2), (297, 3072, 1), (297, 3076, 2), (297, 6144, 1), (297, 6148, 3)])
+def test_output_norm_by_rows_on_an_sm(ops, rows, width, splits, accumulate):
+    test_output_norm_by_rows_and_width(ops, rows, width, splits, accumulate)
