@@ -249,6 +249,33 @@ def test_expert_tiles(tile, monkeypatch):
         assert H.rel(got[pick], F.mixture(x[pick].double(), w, "l0.mlp", mlp)) < LIMIT[torch.bfloat16] / 4
 
 
+def test_expert_pairs_over_several_units_each():
+    """More than two 256 x 256 tiles for each of the 74 pairs of SMs: tiles of the shared expert (four blocks of features, K 328 up and 456 down), then the
+    experts' (two blocks, the last one partly filled, K 328 and 200), so that ring stages and accumulators are carried from one problem's tiles into the
+    other's; one expert takes part in most choices, one in none, and the last tile of each holds a remainder."""
+    experts, top, ff, shared_ff, width, tokens = 12, 3, 200, 456, 328, 7000
+    mlp = H.experts(experts, top, ff, 1.0, shared_ff)
+    cfg, w0, _, model, _ = one_layer(H.wkv(mlp=mlp), torch.bfloat16, width=width)
+    w0["l0.mlp.router"][0, 0], w0["l0.mlp.router"][3, 0] = 0.5, -30.0
+    model.load_checkpoint(w0)
+    w = {k: v.double() for k, v in w0.items()}
+    x = rows(tokens, width, 4)
+    x[:, 0] = 6.0
+    moe = model.layers[0].moe
+    assert moe.tile_tokens(tokens * top, experts, False) == 256
+    shared_tiles, least = -(-tokens // 256), tokens * top // 256  # (tiles of 256 rows; experts' remainders come on top)
+    assert min(-(-2 * shared_ff // 256) * shared_tiles + 2 * least, -(-width // 256) * shared_tiles + 2 * least) > 2 * 74
+    got = add_up(model, 0, x, torch.zeros(tokens, width))
+    score = torch.sigmoid(x.double() @ w["l0.mlp.router"].T)
+    chosen, order = torch.topk(score, top).indices, score.sort(-1, descending=True).values
+    counts = chosen.flatten().bincount(minlength=experts)
+    assert counts[3] == 0 and counts[0] > 2 * counts.double().mean()
+    pick = torch.cat([(chosen == e).any(-1).nonzero()[-9:, 0] for e in range(experts)] + [torch.arange(0, tokens, 97)]).unique()  # (each expert's last tile)
+    pick = [t for t in pick.tolist() if order[t, top - 1] - order[t, top] > 1e-6]
+    assert H.rel(got[pick], F.mixture(x[pick].double(), w, "l0.mlp", mlp)) < LIMIT[torch.bfloat16] / 4
+    assert not torch.isnan(got).any()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("width", [32, 100, 101, 160, 1028, 2056, 4100, 8200])
 def test_residual_stream_and_norms(width, dtype):

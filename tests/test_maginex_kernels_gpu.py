@@ -444,6 +444,34 @@ def test_expert_tiles(tile, monkeypatch):
         assert H.rel(got[pick], M.experts(x[pick].double(), w, "l0.mlp.", mlp)) < LIMIT[torch.bfloat16] / 3
 
 
+def test_expert_pairs_over_several_units_each():
+    """More than two 256 x 256 tiles for each of the 74 pairs of SMs, without gates: the shared expert's (K 328 up and 712 down) in front of the experts' (K 328
+    and 392, features that end inside a tile), so that ring stages and accumulators are carried from one problem's tiles into the other's; one expert takes
+    part in most choices, one in none."""
+    from megatron_mixtera_b200.transformer.moe import MixtureOfExperts
+
+    experts, top, ff, shared_ff, width, tokens = 12, 3, 392, 712, 328, 7000
+    mlp = H.experts(experts, top, ff, shared_ff)
+
+    def edit(w):
+        w["l0.mlp.router.b"] = torch.tensor([2.0, 0.0, 0.0, -100.0] + [0.0] * 8).to(torch.bfloat16)
+
+    cfg, w0, model, _ = model_of(H.mingru(8, mlp=mlp), torch.bfloat16, width=width, edit=edit)
+    w = {k: v.double() for k, v in w0.items()}
+    x = rows(tokens, width, 4)
+    assert MixtureOfExperts.tile_tokens(tokens * top, experts, False) == 256
+    shared_tiles, least = -(-tokens // 256), tokens * top // 256  # (tiles of 256 rows; experts' remainders come on top)
+    assert min(-(-shared_ff // 256) * shared_tiles + 2 * least, 2 * shared_tiles + 2 * least) > 2 * 74
+    got = add_up(model, x, torch.zeros(tokens, width))
+    chosen, _ = M.choose(x.double() @ w["l0.mlp.router"].T + w["l0.mlp.router.b"], top)
+    counts = chosen.flatten().bincount(minlength=experts)
+    assert counts[3] == 0 and counts[0] > 2 * counts.double().mean()
+    pick = torch.cat([(chosen == e).any(-1).nonzero()[-9:, 0] for e in range(experts)] + [torch.arange(0, tokens, 97)]).unique().tolist()
+    pick = [pick[i] for i in sure_of(x[pick], w, top)]
+    assert H.rel(got[pick], M.experts(x[pick].double(), w, "l0.mlp.", mlp)) < LIMIT[torch.bfloat16] / 3
+    assert not torch.isnan(got).any()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("M_,N,K,batch", [(1, 64, 64, 1), (33, 128, 48, 3), (64, 40, 128, 5), (130, 24, 16, 2), (300, 256, 64, 1), (5, 13, 21, 3)])
 def test_gated_linear(M_, N, K, batch, dtype):

@@ -422,6 +422,31 @@ def test_splits_in_clusters_give_the_bits_of_the_summed_partials(ops, M, N, K):
         assert torch.equal(ops.gemm_mxfp8(xq, wq), total.to(BF16))
 
 
+# Both sides of the limits of clusters: four splits, 24 rows, N a multiple of 4 (of the shapes above, those of 33 rows and more do not form any).  K splits of
+# bf16 and MXFP8, and whether they form clusters, which need no scratch.
+@pytest.mark.parametrize("M,N,K,bf16,mxfp8", [
+    (24, 4700, 1024, (4, True), (2, True)),    # the most rows and splits; N 92 past a tile
+    (25, 4700, 1024, (4, False), (2, False)),  # one row more
+    (31, 388, 768, (3, False), None),
+    (32, 4700, 2048, (8, False), (4, False)),  # a full tile
+    (8, 384, 1280, (5, False), (2, True)),     # one split more
+    (12, 388, 768, (3, True), None),
+    (3, 390, 1024, (4, False), (2, False)),    # N even only
+    (24, 4700, 2048, (8, False), (4, True)),
+    (7, 132, 1536, (6, False), (3, True)),
+    (1, 4, 1024, (4, True), (2, True)),        # the smallest N
+    (2, 128, 2560, (10, False), (5, False)),
+])
+def test_splits_on_both_sides_of_the_cluster_limits(ops, M, N, K, bf16, mxfp8):
+    from megatron_mixtera_b200 import _lib
+
+    lib = _lib.load()
+    for recipe, scratch, expected in ((None, lib.b200_gemm_bf16_workspace_bytes, bf16), ("mxfp8", lib.b200_gemm_mxfp8_workspace_bytes, mxfp8)):
+        if expected is not None:
+            assert (ops.gemm_num_splits(recipe, M, N, K), scratch(M, N, K) == 0) == expected
+    test_splits_in_clusters_give_the_bits_of_the_summed_partials(ops, M, N, K)
+
+
 # ---------------------------------------------------------------------------------------------------------------------
 # Output norm: few rows and many, one to eight vectors per thread, widths that end inside a thread's vectors.  fp32 sums of up to 8192 terms: 1e-5.
 # ---------------------------------------------------------------------------------------------------------------------
