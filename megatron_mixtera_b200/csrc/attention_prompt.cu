@@ -18,7 +18,9 @@
 //
 // Three products of 128 x 128 x 128 per tile and block (one for S, two for P's terms) take 1536 clocks, a block's softmax about as many.  O is rescaled only
 // when a row's maximum has grown by more than 2^8 since the last time: P and the row sums stay relative to the maximum in use, in fp32 until the
-// split, so the result is the same within rounding.  Units of several requests in one CTA are taken request by request (a "run"), the other rows idle.
+// split, so the result is the same within rounding.  (Two blocks in turn and the lazy maximum are steps of a published method, FlashAttention-4; the maximum in
+// use moves for all rows of a warp when one of them grows, so a row's last bits may depend on its neighbours'.)  Units of several requests in one CTA are taken
+// request by request (a "run"), the other rows idle.
 #include "common.cuh"
 
 namespace b200 {

@@ -11,8 +11,8 @@
 //   warp 9, lane 0      leader only: the pair's MMAs; commits go to both CTAs' barriers
 //
 // Measured, before -> after (burst; the power cap takes 10 % off both in long runs): bf16, 7700 tokens, 28672 x 4096: 1145 -> 1400 TFLOP/s, 4096 x 14336:
-// 1220 -> 1370; MXFP8, 13000 tokens, 28672 x 4096 with SwiGLU and quantisation: 1430 -> 2110, 4096 x 14336: 1410 -> 2100.  What bounds them now: power with
-// bf16 (cuBLAS reaches 1590 in the same run); with scales the copies of ~34 KB per K block and the read-out of the one accumulator.
+// 1220 -> 1370; MXFP8, 13000 tokens, 28672 x 4096 with SwiGLU and quantisation: 1430 -> 2110, 4096 x 14336: 1410 -> 2100.  What bounds them now: with scales the
+// copies of ~34 KB per K block and the read-out of the one accumulator; bf16 stops short of the power cap (cuBLAS reaches 1590 in the same burst).
 //
 // Experts' products (moe.cu) are the same kernel over a device-built list of (expert, first row, rows <= 256) entries, the shared expert's tiles in front.
 //

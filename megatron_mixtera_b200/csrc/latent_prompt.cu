@@ -4,7 +4,7 @@
 // tiles of 64 columns, of the two arrays by a tensor map each.
 //
 // The queries of a 192-column key take 96 KB of shared memory and two key tiles as much; values then have one stage (32 KB) instead of two.  The mma.sync
-// kernel it stands beside (latent_prompt_kernel) takes 64 queries per CTA; it keeps the steps whose CTAs of 256 would leave most SMs idle.
+// kernel it stands beside (latent_prompt_kernel) takes 64 queries per CTA; it keeps the steps whose CTAs of 256 would leave most SMs idle, and short rows.
 //
 // Measured, 128 + 64 entries per key, 128 per value: 6208 tokens in 5 rows x 16 heads 489 -> 188 us, 2048 tokens of one row 262 -> 75 us, 3264 in 3 rows x 32
 // heads 413 -> 157 us; 896 tokens in 8 rows (128 CTAs) 25.5 -> 22.7 us, the line below which the other kernel stays.
