@@ -439,7 +439,7 @@ typedef struct {
   int32_t bias_len, keep_first, maps;
   int32_t value_gates; /* != 0 (b200_paged_prefill_attention, maps < 2): the gates are num_q_heads * value_dim columns, one per value channel */
   int32_t unit_mix; /* b200_paged_prefill_attention, what the caller knows of its work list (for the choice of kernels; any value is right for any list): 0
-                       nothing, 1 only requests of many units (eight, or whole groups of four), 2 only requests of fewer */
+                       nothing, 1 only requests of many units (eight, or whole groups of four) or next to nothing else, 2 only requests of fewer */
 } b200_attention_args;
 
 size_t b200_paged_attention_workspace_bytes(int num_tokens, int num_q_heads, int head_dim, int num_splits);

@@ -398,7 +398,10 @@ class DynamicInferenceContext(BaseInferenceContext):
     def _mix_of(nb: np.ndarray, keys: np.ndarray) -> int:
         """`AttentionArgs.unit_mix` of requests of ``nb`` units that see ``keys`` keys on average.  A list of both kinds counts as one of short requests
         where the long ones are less than a fifth of the short ones' work: two kernels, one behind the other, would take longer (300 beside 250 requests
-        of 500, two maps of 64: 258 us with one, 296 with two; with 1024 more tokens beside 64 of 1000, 32 heads in 8 groups, 141 and 117)."""
+        of 500, two maps of 64: 258 us with one, 296 with two; with 1024 more tokens beside 64 of 1000, 32 heads in 8 groups, 141 and 117).  It counts as one of
+        long requests where the short ones are less than a tenth of the work, and four of them, which may share a CTA, see no more keys than a long one: they
+        fit beside it, and the second kernel would be 25 us (7 prompts of 100 to 800 tokens, two maps of 64 and 128 wide heads: 83 and 85 us with one kernel,
+        103 and 110 with two)."""
         some = nb > 0
         nb, keys = nb[some], keys[some]
         if not nb.size:
@@ -409,6 +412,8 @@ class DynamicInferenceContext(BaseInferenceContext):
         if not long.any():
             return 2 if nb.max() == 1 or keys.max() < 768 else 0
         work = nb * keys
+        if 10 * work[~long].sum() <= work[long].sum() and np.sort(keys[~long])[-4:].sum() <= keys[long].max():
+            return 1
         return 0 if 5 * work[long].sum() >= work[~long].sum() else 2
 
     def _build_prefill_units(self, ql: np.ndarray, kv: np.ndarray, n_rows: int, padded: int, graphs: bool) -> None:
