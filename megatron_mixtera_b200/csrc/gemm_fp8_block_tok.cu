@@ -48,7 +48,8 @@ struct TokConfig {
   static constexpr int kTmemCols = 2 * H * 128;  // two buffers of H x 128 feature columns
 };
 
-template <int H>
+// EVEN: blocks of m_rows tokens instead of 128, a form of its own because many tokens took 1 to 3 % longer with it (8192 x 57344 x 8192 4.77 -> 4.85 ms).
+template <int H, bool EVEN>
 __global__ void __launch_bounds__(TokConfig<H>::kThreads, 1)
 gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, Params p,
                           BlkOperands q) {
@@ -69,13 +70,13 @@ gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   // innermost every wave read other weights, all of them from HBM once per 256 tokens: 11000 x 57344 x 8192 7.8 ms, then 7.1 ms.)
   const int split = blockIdx.y;
   int n_tile = blockIdx.x, m_block = 0;
-  if (q.m_blocks > 1) {
+  if (H == 2 || q.m_blocks > 1) {
     const int per_group = kGroupM * q.n_tiles, group = n_tile / per_group, in_group = n_tile - group * per_group;
     const int rows = min(kGroupM, q.m_blocks - group * kGroupM);
     n_tile = in_group / rows;
     m_block = group * kGroupM + (in_group - n_tile * rows);
   }
-  const int m0 = m_block * q.m_rows;
+  const int m0 = m_block * (EVEN ? q.m_rows : C::kTokens);
   const int kb_begin = split * p.k_blocks_per_split;
   const int kb_end = min(p.num_k_blocks, kb_begin + p.k_blocks_per_split);
   const int num_kb = kb_end - kb_begin;
@@ -202,7 +203,7 @@ gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
 
     // ---------------- epilogue: the thread's token row, 128 consecutive features, straight from registers ----------------
     const int m = m0 + tok;
-    if (tok < q.m_rows && m < p.M && n0 < p.N) {
+    if ((!EVEN || tok < q.m_rows) && m < p.M && n0 < p.N) {
       const bool full_tile = n0 + kTileN <= p.N;
       if (p.num_splits == 1 && !p.keep_partials) {
         __nv_bfloat16* dst = p.y + static_cast<int64_t>(m) * p.ldy + n0;
@@ -295,16 +296,20 @@ static int launch_fp8_block_tok(const void* xq, const float* x_scale, int m_pad,
   q.x_scale = x_scale;
   q.k_tiles = num_kb;
   q.m_pad = m_pad;
-  static std::atomic<uint64_t> smem_attr_done{0};
-  if (ensure_dynamic_smem(gemm_fp8_block_tok_kernel<H>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
   q.n_tiles = n_blocks;
   q.m_blocks = m_blocks;
-  // The blocks share the tokens evenly (scales are copied 4 at a time): with a last block of one token the others' stores would take as long as two
-  // full ones.  129 tokens, 2048 x 2048: 15.2 us with blocks of 128 and 1, 10.9 with 68 and 61; 6144 x 4096: 22.7 and 18.6.
+  // Few blocks share the tokens evenly (scales are copied 4 at a time) where that leaves out an eighth of each: with a last block of one token the others'
+  // stores would take as long as two full ones.  129 tokens, 2048 x 2048: 15.2 us with blocks of 128 and 1, 10.9 with 68 and 61; 6144 x 4096: 22.7 and 18.6.
   q.m_rows = min(C::kTokens, ((M + m_blocks - 1) / m_blocks + 3) / 4 * 4);
   if (static_cast<int64_t>(n_blocks) * m_blocks > 0x7fffffff) return B200_ERR_INVALID_ARGUMENT;
   dim3 grid(static_cast<unsigned>(n_blocks * m_blocks), splits);
-  const int rc = launch_pdl(gemm_fp8_block_tok_kernel<H>, grid, dim3(C::kThreads), C::kSmemBytes, stream, *mw, *mx_, p, q);
+  auto run = [&](auto even) {
+    constexpr bool EVEN = decltype(even)::value;
+    static std::atomic<uint64_t> smem_attr_done{0};
+    if (ensure_dynamic_smem(gemm_fp8_block_tok_kernel<H, EVEN>, C::kSmemBytes, smem_attr_done) != B200_OK) return static_cast<int>(B200_ERR_LAUNCH);
+    return launch_pdl(gemm_fp8_block_tok_kernel<H, EVEN>, grid, dim3(C::kThreads), C::kSmemBytes, stream, *mw, *mx_, p, q);
+  };
+  const int rc = H == 2 && q.m_rows <= C::kTokens / 8 * 7 ? run(std::bool_constant<H == 2>{}) : run(std::false_type{});
   if (rc != B200_OK || splits == 1 || p.keep_partials) return rc;
   return launch_splitk_reduce(p, stream);
 }
