@@ -399,22 +399,24 @@ class DynamicInferenceContext(BaseInferenceContext):
         """`AttentionArgs.unit_mix` of requests of ``nb`` units that see ``keys`` keys on average.  A list of both kinds counts as one of short requests
         where the long ones are less than a fifth of the short ones' work: two kernels, one behind the other, would take longer (300 beside 250 requests
         of 500, two maps of 64: 258 us with one, 296 with two; with 1024 more tokens beside 64 of 1000, 32 heads in 8 groups, 141 and 117).  It counts as one of
-        long requests where the short ones are less than a tenth of the work, and four of them, which may share a CTA, see no more keys than a long one: they
-        fit beside it, and the second kernel would be 25 us (7 prompts of 100 to 800 tokens, two maps of 64 and 128 wide heads: 83 and 85 us with one kernel,
-        103 and 110 with two)."""
-        some = nb > 0
-        nb, keys = nb[some], keys[some]
-        if not nb.size:
+        long requests where the short ones are less than a quarter of the work, and four of them, which may share a CTA, see at most twice the keys of a long
+        one: they fit beside it (two layers, 7 prompts of 164 to 800 tokens, two maps of 64 and 128 wide heads: 161 and 172 us with one kernel, 206 and 225 with
+        two; 7 prompts of 36 to 167, 32 heads: 55 and 76).  (Plain numbers: a dozen array operations on a few rows would take 20 us.)"""
+        units = nb.tolist()
+        if min(units, default=0) >= 8:
+            return 1
+        rows = [(n, k) for n, k in zip(units, keys.tolist()) if n > 0]
+        short = [(n, k) for n, k in rows if n < 8]
+        if not rows:
             return 0
-        long = nb >= 8
-        if long.all() or not (nb % 4).any():
+        if not short or not any(n % 4 for n, _ in rows):
             return 1
-        if not long.any():
-            return 2 if nb.max() == 1 or keys.max() < 768 else 0
-        work = nb * keys
-        if 10 * work[~long].sum() <= work[long].sum() and np.sort(keys[~long])[-4:].sum() <= keys[long].max():
+        if len(short) == len(rows):
+            return 2 if max(units) == 1 or max(k for _, k in rows) < 768 else 0
+        long_work, short_work = sum(n * k for n, k in rows if n >= 8), sum(n * k for n, k in short)
+        if 4 * short_work <= long_work and sum(sorted(k for _, k in short)[-4:]) <= 2 * max(k for n, k in rows if n >= 8):
             return 1
-        return 0 if 5 * work[long].sum() >= work[~long].sum() else 2
+        return 0 if 5 * long_work >= short_work else 2
 
     def _build_prefill_units(self, ql: np.ndarray, kv: np.ndarray, n_rows: int, padded: int, graphs: bool) -> None:
         self.prefill_unit_count = self._fill_units(self.prefill_q_block, self._h_units, self._h_units_np, self.prefill_units, ql, kv,

@@ -542,14 +542,14 @@ def test_log_probs_match_the_reference_context():
     assert z["s2_lengths"].tolist() == [1, 1, 6]  # the mixed step: two decoding requests and one prompt
 
 
-@pytest.mark.parametrize("lens,want", [([200, 130], (1, 1)), ([64, 128], (1, 1)), ([100, 33], (2, 0)), ([200, 1], (1, 1)), ([2, 1], (2, 2)),
+@pytest.mark.parametrize("lens,want", [([200, 130], (1, 1)), ([64, 128], (1, 1)), ([100, 33], (2, 1)), ([200, 1], (1, 1)), ([2, 1], (2, 2)),
                                        ([112], (2, 1))])
 def test_what_a_prefill_work_list_holds(lens, want):
     """1: only requests of eight units or whole groups of four, or next to nothing else; 2: only of fewer; 0: both.  Per block size, anew each step."""
     c = make_ctx(max_requests_override=4, max_tokens_override=512)
     c.set_prefill_q_block(16, 8)
     assert c.prefill_unit_mix(16) == 0
-    c.schedule_tokens([(100, [1] * 300), (101, [1] * 100)])
+    c.schedule_tokens([(100, [1] * 130), (101, [1] * 100)])
     c.initialize_attention_state()
     assert c.prefill_unit_mix(16) == 0
     c.complete_step([100, 101])
@@ -560,7 +560,8 @@ def test_what_a_prefill_work_list_holds(lens, want):
 
 @pytest.mark.parametrize("units,keys,want", [
     ([19, 1, 1], [150, 500, 500], 0),
-    ([19, 1, 1], [150, 30, 30], 1), ([19] + [1] * 5, [150] + [40] * 5, 0), ([40, 7], [300, 171], 1), ([40, 7], [300, 172], 0),  # (short ones fit beside it, or not)
+    # (short ones fit beside it, or not)
+    ([40, 7], [300, 428], 1), ([40, 7], [300, 429], 0), ([40, 1, 1, 1, 1, 1], [300] + [150] * 5, 1), ([40, 1, 1, 1, 1], [300] + [151] * 4, 0),
     ([19] + [1] * 250, [150] + [500] * 250, 2),   # (the long request is little of the work)
     ([2] * 64, [1009] * 64, 0), ([1] * 64, [1009] * 64, 2), ([5] * 4, [150] * 4, 2),  # few units behind a long past: two kernels may share them
     ([0, 4, 8], [0, 10, 10], 1), ([0, 0], [0, 0], 0)])
