@@ -11,11 +11,10 @@
 //                        two columns per lane group at a time with the next two on their way; the CTA's warps - rows of one
 //                        head - share W_w2's rows in shared memory.  The product with W_w2, the decay, the unit key, the head
 //                        norm and the output gate are part of it.
-//   delta_scan_kernel    rows of any length: one CTA per (row, head, block of columns) walks the row's tokens.  Compute warps
-//                        hold two columns on four lanes (a vector is read from shared memory once for both); as many other
-//                        warps prepare the next 16 tokens (decay, unit key, removal vector) meanwhile.  Bound by the chain of a
-//                        token - dot product, lane sum, update, dot product - on one warp per scheduler; four tokens are
-//                        unrolled so that the next one's vectors are read under it.
+//   delta_block_scan_kernel  rows of any length, heads of 33 to 128: one CTA per (row, head, 64 columns) walks the row's tokens four at a time.  Compute warps
+//                        hold two columns on four lanes (a vector is read from shared memory once for both); other warps prepare blocks of
+//                        four tokens (decays, unit key, removal vector, their products with one another) meanwhile.
+//   delta_scan_kernel    the same a token at a time, for the other sizes
 //   delta_finish_kernel  head norm + weight + output gate behind the scan (a head's columns may be spread over CTAs there).
 #include "common.cuh"
 
@@ -25,6 +24,13 @@ namespace delta {
 constexpr int kScanTokens = 16;  // tokens prepared at a time
 
 __device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
+
+// The same without a branch, so that several are under way together: the fast reciprocal and one Newton-Raphson step, r (2 - y r), which is as close as the
+// division (6e-8).  Below e^-80 it stays there.
+__device__ __forceinline__ float sigmoid_in_line(float x) {
+  const float y = 1.f + expf(-x > 80.f ? 80.f : -x), r = __fdividef(1.f, y);
+  return fmaf(r, fmaf(-y, r, 1.f), r);
+}
 
 // For output gates: fp32 arithmetic with the fast exponential and division (about 1e-6 relative).
 __device__ __forceinline__ float gate_sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
@@ -372,9 +378,6 @@ struct ScanShape {  // COLS columns per CTA, N of them per thread, LANES lanes p
   static_assert(kComputeThreads % 32 == 0 && kScanTokens % kPrepWarps == 0 && kTokPerWarp % kBatch == 0 && DIM % 32 == 0, "");
   static constexpr int kBufFloats = kScanTokens * (5 * DIM + COLS);
   static constexpr int kSmemBytes = 2 * kBufFloats * 4;
-  // Tokens unrolled: 256 channels fill the registers (the next token's vectors would be spilled: 64 rows of 256 tokens x 8 heads of 256 9.0 ms with four,
-  // 7.6 with one; heads of 192 6.9 and 5.4); 32 have nothing to hide, and cost registers (four heads of 32, 300 rows of 20 tokens 25.2 us, 22.1).
-  static constexpr int kUnroll = DIM > 32 && DIM <= 128 ? 4 : 1;
 };
 
 template <typename T, int DIM, int COLS, int N, int LANES>
@@ -484,7 +487,7 @@ delta_scan_kernel(b200_delta_args a) {
     const float* buf = smem + (c & 1) * Sh::kBufFloats;
     const float* values = buf + kScanTokens * 5 * DIM + group;
     const int cnt = min(kScanTokens, n_tok - c * kScanTokens);
-#pragma unroll Sh::kUnroll
+#pragma unroll 1  // (256 channels fill the registers, 32 have nothing to hide)
     for (int tt = 0; tt < cnt; ++tt) {
       const float* v0 = buf + tt * 5 * DIM;
       const TokenVectors tv{v0, v0 + DIM, v0 + 2 * DIM, v0 + 3 * DIM, v0 + 4 * DIM};
@@ -498,6 +501,332 @@ delta_scan_kernel(b200_delta_args a) {
         if (ni == 0 && cb * COLS + n * Sh::kGroups + group < dim) o_dst[n * Sh::kGroups] = sum;
       }
       o_dst += hd;
+    }
+    __syncthreads();  // chunk c has been read, chunk c + 1 is ready
+  }
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int j = cb * COLS + n * Sh::kGroups + group;
+    if (static_cast<unsigned>(out) < static_cast<unsigned>(a.state_slots) && j < dim)
+      store_column<NI, I>(a.state + (static_cast<int64_t>(out) * a.heads + head) * head_elems + static_cast<int64_t>(j) * dim, dim, ni, full, s[n]);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Scan, four tokens at a time
+// ---------------------------------------------------------------------------------------------------------------
+// With S the state in front of four tokens and w[a..b] the product of their decays, what token j removes and reads is
+//
+//   d_j = (u_j w[0..j-1]) . S + sum_(s<j)  (u_j . k_s w[s+1..j-1]) v_s - (u_j . a_s u_s w[s+1..j-1]) d_s
+//   o_j = (r_j w[0..j]) . S   + sum_(s<=j) (r_j . k_s w[s+1..j]) v_s   - (r_j . a_s u_s w[s+1..j]) d_s
+//   S  <- w[0..3] S + sum_s (k_s w[s+1..3]) v_s - (a_s u_s w[s+1..3]) d_s
+//
+// so one pass over a column's registers gives all eight dot products with S and one more all four updates: one lane sum in the chain for four tokens instead
+// of four.  Decays are only ever multiplied, never divided by, so nothing grows however small they are.
+// A row is a chain of tokens; what bounds one is what its SM can do for a token.  2048 tokens, 32 heads of 64: 506 us a token at a time, 372 now; the compute
+// warps alone take 297 (84 16-byte reads of shared memory and 272 packed multiply-adds for each block and warp), the preparing ones 250 (mostly the exponentials;
+// with a branch in the sigmoids' divisions 338).  Products of 16 tokens on mma.sync in three bf16 terms need as many instructions to prepare: 388 to 403 us.
+constexpr int kBlockTokens = 4;
+// Of a block, in floats: u w[0..j-1], r w[0..j], k w[s+1..3], a u w[s+1..3] of its tokens and w[0..3], each [DIM]; the values [4][COLS]; the products of the
+// tokens with one another, four matrices [4][4] (j, s): u.k, u.au (zero where s >= j), r.k, r.au (zero where s > j).
+template <int DIM, int COLS, int BLOCKS>
+struct BlockShape {
+  static constexpr int kU = 0, kR = 4 * DIM, kK = 8 * DIM, kB = 12 * DIM, kW = 16 * DIM, kV = 17 * DIM, kPairs = kV + 4 * COLS;
+  static constexpr int kFloats = kPairs + 64;
+  static constexpr int NI = 4, N = 2, I = DIM / NI, kStride = 32 / NI;
+  static constexpr int kGroups = COLS / N, kComputeThreads = kGroups * NI, kComputeWarps = kComputeThreads / 32;
+  static constexpr int kTokens = BLOCKS * kBlockTokens, kBlocks = BLOCKS, kPrepWarps = kBlocks, kThreads = kComputeThreads + kPrepWarps * 32;
+  static constexpr int kElems = DIM / 32, kValues = COLS / 32;
+  static constexpr int kSmemBytes = 2 * kBlocks * kFloats * 4;
+  static_assert(COLS % 32 == 0 && DIM % 32 == 0 && kFloats % 4 == 0, "");
+};
+
+// Sum of value i over the warp, in lane i.
+__device__ __forceinline__ float transposed_sum(float (&v)[32], int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const bool high = lane & o;
+      const float give = high ? v[i] : v[i + o], keep = high ? v[i + o] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  return v[0];
+}
+
+template <typename T, int DIM, int COLS, int BLOCKS>
+__global__ void __launch_bounds__(BlockShape<DIM, COLS, BLOCKS>::kThreads)
+delta_block_scan_kernel(b200_delta_args a) {
+  using Sh = BlockShape<DIM, COLS, BLOCKS>;
+  constexpr int NI = Sh::NI, I = Sh::I, N = Sh::N, EL = Sh::kElems, VL = Sh::kValues, J = kBlockTokens;
+  extern __shared__ __align__(16) float smem[];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int dim = a.dim;
+  const int col_blocks = (dim + COLS - 1) / COLS;
+  const int head = blockIdx.x / col_blocks, cb = blockIdx.x - head * col_blocks;
+  const int row = longest_first(a.cu_tokens, a.num_rows, blockIdx.y);
+  pdl_launch_dependents();
+  const int t_begin = a.cu_tokens[row], n_tok = min(a.cu_tokens[row + 1], a.num_tokens) - t_begin;
+  pdl_wait();
+  if (n_tok <= 0) return;
+  const int64_t hd = static_cast<int64_t>(a.heads) * dim;
+  const int chunks = (n_tok + Sh::kTokens - 1) / Sh::kTokens;
+
+  if (tid >= Sh::kComputeThreads) {
+    // ------------------------------- preparing warps: a block each -------------------------------
+    const int warp = (tid - Sh::kComputeThreads) >> 5;
+    const T* proj = static_cast<const T*>(a.proj) + head * dim;
+    const T* zin = static_cast<const T*>(a.z) + head * dim;
+    float bias_w[EL], bias_a[EL];
+    int at[EL], col[VL];  // clamped, so that the loads need no branches and are all in flight together
+#pragma unroll
+    for (int e = 0; e < EL; ++e) {
+      at[e] = min(lane + e * 32, dim - 1);
+      bias_w[e] = simt::to_f32(static_cast<const T*>(a.decay_bias)[head * dim + at[e]]);
+      bias_a[e] = simt::to_f32(static_cast<const T*>(a.removal_bias)[head * dim + at[e]]);
+    }
+#pragma unroll
+    for (int e = 0; e < VL; ++e) col[e] = min(cb * COLS + lane + e * 32, dim - 1);
+    // Where this lane's product of two tokens goes: (j, s) of s < j first u.k, then u.au, of s <= j then r.k, then r.au.
+    int place = 0;
+    {
+      int i = 0;
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+#pragma unroll
+          for (int s = 0; s < J; ++s)
+            if (m < 2 ? s < j : s <= j) {
+              if (i == lane) place = (m * J + j) * J + s;
+              ++i;
+            }
+    }
+    for (int i = lane; i < 2 * 64; i += 32) smem[((i / 64) * Sh::kBlocks + warp) * Sh::kFloats + Sh::kPairs + i % 64] = 0.f;
+    __syncwarp();
+    T xr[J][EL], xk[J][EL], xa[J][EL], xz[J][EL], xv[J][VL];
+    auto fetch = [&](int c) {
+#pragma unroll
+      for (int q = 0; q < J; ++q) {
+        const int64_t t = t_begin + min(c * Sh::kTokens + warp * J + q, n_tok - 1);
+        const T* p = proj + t * a.proj_ld;
+        const T* z = zin + t * hd;
+#pragma unroll
+        for (int e = 0; e < EL; ++e) {
+          xr[q][e] = p[a.off_r + at[e]];
+          xk[q][e] = p[a.off_k + at[e]];
+          xa[q][e] = p[a.off_a + at[e]];
+          xz[q][e] = z[at[e]];
+        }
+#pragma unroll
+        for (int e = 0; e < VL; ++e) xv[q][e] = p[a.off_v + col[e]];
+      }
+    };
+    fetch(0);
+    for (int c = 0; c < chunks; ++c) {
+      float* buf = smem + ((c & 1) * Sh::kBlocks + warp) * Sh::kFloats + lane;
+      float r[J][EL], w[J][EL], k[J][EL], u[J][EL], au[J][EL], sums[J];
+#pragma unroll
+      for (int q = 0; q < J; ++q) {
+        const bool live = c * Sh::kTokens + warp * J + q < n_tok;  // (past the end: nothing is written, nothing decays)
+        float ksq = 0.f;
+#pragma unroll
+        for (int e = 0; e < EL; ++e) {
+          const bool ok = live && lane + e * 32 < dim;
+          k[q][e] = ok ? simt::to_f32(xk[q][e]) : 0.f;
+          r[q][e] = ok ? simt::to_f32(xr[q][e]) : 0.f;
+          ksq += k[q][e] * k[q][e];
+        }
+        sums[q] = warp_sum(ksq);
+#pragma unroll
+        for (int e = 0; e < EL; ++e) {
+          w[q][e] = live ? expf(-a.decay_scale * sigmoid_in_line(simt::to_f32(xz[q][e]) + bias_w[e])) : 1.f;
+          au[q][e] = sigmoid_in_line(simt::to_f32(xa[q][e]) + bias_a[e]);
+        }
+#pragma unroll
+        for (int e = 0; e < VL; ++e) buf[Sh::kV + q * COLS + e * 32] = live ? simt::to_f32(xv[q][e]) : 0.f;
+      }
+      if (c + 1 < chunks) fetch(c + 1);
+      // One root and one division for the four tokens, a lane each.
+      const float root = 1.f / sqrtf((lane & 2 ? lane & 1 ? sums[3] : sums[2] : lane & 1 ? sums[1] : sums[0]) + a.unit_eps);
+#pragma unroll
+      for (int q = 0; q < J; ++q) {
+        const float unit = __shfl_sync(0xffffffffu, root, q);
+#pragma unroll
+        for (int e = 0; e < EL; ++e) {
+          u[q][e] = k[q][e] * unit;
+          au[q][e] *= u[q][e];
+        }
+      }
+      float pairs[32];
+      {
+        // k and a u of token s on their way through the decays behind it
+        float kk[J][EL], bb[J][EL];
+#pragma unroll
+        for (int s = 0; s < J; ++s)
+#pragma unroll
+          for (int e = 0; e < EL; ++e) {
+            kk[s][e] = k[s][e];
+            bb[s][e] = au[s][e];
+          }
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+#pragma unroll
+          for (int s = 0; s <= j; ++s) {
+            float uk = 0.f, ub = 0.f, rk = 0.f, rb = 0.f;
+#pragma unroll
+            for (int e = 0; e < EL; ++e) {
+              if (s < j) {
+                uk = fmaf(u[j][e], kk[s][e], uk);
+                ub = fmaf(u[j][e], bb[s][e], ub);
+                kk[s][e] *= w[j][e];
+                bb[s][e] *= w[j][e];
+              }
+              rk = fmaf(r[j][e], kk[s][e], rk);
+              rb = fmaf(r[j][e], bb[s][e], rb);
+            }
+            if (s < j) {
+              pairs[j * (j - 1) / 2 + s] = uk;
+              pairs[6 + j * (j - 1) / 2 + s] = ub;
+            }
+            pairs[12 + j * (j + 1) / 2 + s] = rk;
+            pairs[22 + j * (j + 1) / 2 + s] = rb;
+          }
+#pragma unroll
+        for (int s = 0; s < J; ++s)
+#pragma unroll
+          for (int e = 0; e < EL; ++e) {
+            buf[Sh::kK + s * DIM + e * 32] = kk[s][e];
+            buf[Sh::kB + s * DIM + e * 32] = bb[s][e];
+          }
+      }
+#pragma unroll
+      for (int e = 0; e < EL; ++e) {
+        float p = w[0][e];
+        buf[Sh::kU + e * 32] = u[0][e];
+        buf[Sh::kR + e * 32] = r[0][e] * p;
+#pragma unroll
+        for (int j = 1; j < J; ++j) {
+          buf[Sh::kU + j * DIM + e * 32] = u[j][e] * p;
+          p *= w[j][e];
+          buf[Sh::kR + j * DIM + e * 32] = r[j][e] * p;
+        }
+        buf[Sh::kW + e * 32] = p;
+      }
+      const float sum = transposed_sum(pairs, lane);
+      buf[Sh::kPairs - lane + place] = sum;
+      __syncthreads();  // chunk c is ready, chunk c - 1 has been read: its buffer is free
+    }
+    __syncthreads();
+    return;
+  }
+
+  // --------------------------------- compute warps ---------------------------------
+  const bool full = dim == DIM;
+  const int in = a.state_in[row], out = a.state_out[row];
+  const int64_t head_elems = static_cast<int64_t>(dim) * dim;
+  constexpr int ST = Sh::kStride;
+  const int ni = lane / ST, group = (tid >> 5) * ST + lane % ST;  // this thread's columns: cb * COLS + n * kGroups + group
+  f32x2 s[N][I / 2];
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int j = cb * COLS + n * Sh::kGroups + group;
+    if (static_cast<unsigned>(in) < static_cast<unsigned>(a.state_slots) && j < dim) {
+      load_column<NI, I>(a.state + (static_cast<int64_t>(in) * a.heads + head) * head_elems + static_cast<int64_t>(j) * dim, dim, ni, full, s[n]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < I / 2; ++e) s[n][e] = 0ull;
+    }
+  }
+  float* o_dst = a.o_f32 + (static_cast<int64_t>(t_begin) + ni) * hd + head * dim + cb * COLS + group;  // this lane's token of every block
+  __syncthreads();  // chunk 0 is ready
+  for (int c = 0; c < chunks; ++c) {
+    const int left = n_tok - c * Sh::kTokens, blocks = min(Sh::kBlocks, (left + J - 1) / J);
+#pragma unroll 2
+    for (int b = 0; b < blocks; ++b) {
+      const float* buf = smem + ((c & 1) * Sh::kBlocks + b) * Sh::kFloats;
+      f32x2 du[J][N], dr[J][N];
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int n = 0; n < N; ++n) du[j][n] = dr[j][n] = 0ull;
+#pragma unroll
+      for (int q = 0; q < I / 4; ++q) {
+        const int i = (q * NI + ni) * 4;
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          const ulonglong2 u = piece(buf + Sh::kU + j * DIM + i);
+#pragma unroll
+          for (int n = 0; n < N; ++n) du[j][n] = fma2(u.y, s[n][q * 2 + 1], fma2(u.x, s[n][q * 2], du[j][n]));
+        }
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          const ulonglong2 r = piece(buf + Sh::kR + j * DIM + i);
+#pragma unroll
+          for (int n = 0; n < N; ++n) dr[j][n] = fma2(r.y, s[n][q * 2 + 1], fma2(r.x, s[n][q * 2], dr[j][n]));
+        }
+      }
+      float v[J][N], d[J][N];
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          v[j][n] = buf[Sh::kV + j * COLS + n * Sh::kGroups + group];
+          d[j][n] = lane_sum<NI, ST>(sum2(du[j][n]));
+        }
+      const float* pairs = buf + Sh::kPairs;
+#pragma unroll
+      for (int j = 1; j < J; ++j) {
+        const float4 uk = *reinterpret_cast<const float4*>(pairs + j * J), ub = *reinterpret_cast<const float4*>(pairs + 16 + j * J);
+        const float k[3] = {uk.x, uk.y, uk.z}, g[3] = {ub.x, ub.y, ub.z};
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+          for (int t = 0; t < j; ++t) d[j][n] = fmaf(-g[t], d[t][n], fmaf(k[t], v[t][n], d[j][n]));
+      }
+      f32x2 vv[J][N], nd[J][N];
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          vv[j][n] = pack2(v[j][n], v[j][n]);
+          nd[j][n] = pack2(-d[j][n], -d[j][n]);
+        }
+#pragma unroll
+      for (int q = 0; q < I / 4; ++q) {
+        const int i = (q * NI + ni) * 4;
+        const ulonglong2 w = piece(buf + Sh::kW + i);
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          s[n][q * 2] = mul2(w.x, s[n][q * 2]);
+          s[n][q * 2 + 1] = mul2(w.y, s[n][q * 2 + 1]);
+        }
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          const ulonglong2 k = piece(buf + Sh::kK + j * DIM + i), g = piece(buf + Sh::kB + j * DIM + i);
+#pragma unroll
+          for (int n = 0; n < N; ++n) {
+            s[n][q * 2] = fma2(g.x, nd[j][n], fma2(k.x, vv[j][n], s[n][q * 2]));
+            s[n][q * 2 + 1] = fma2(g.y, nd[j][n], fma2(k.y, vv[j][n], s[n][q * 2 + 1]));
+          }
+        }
+      }
+      // Token ni's output: its four partial sums from the lanes of the column, and what the block's tokens up to it wrote.
+      const float4 rk = *reinterpret_cast<const float4*>(pairs + 32 + ni * J), rb = *reinterpret_cast<const float4*>(pairs + 48 + ni * J);
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        float p[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) p[j] = sum2(dr[j][n]);
+        const bool high = ni & 2, odd = ni & 1;
+        const float a0 = (high ? p[2] : p[0]) + __shfl_xor_sync(0xffffffffu, high ? p[0] : p[2], 2 * ST);
+        const float a1 = (high ? p[3] : p[1]) + __shfl_xor_sync(0xffffffffu, high ? p[1] : p[3], 2 * ST);
+        float o = (odd ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, ST);
+        o = fmaf(rk.x, v[0][n], fmaf(rk.y, v[1][n], fmaf(rk.z, v[2][n], fmaf(rk.w, v[3][n], o))));
+        o = fmaf(-rb.x, d[0][n], fmaf(-rb.y, d[1][n], fmaf(-rb.z, d[2][n], fmaf(-rb.w, d[3][n], o))));
+        if (b * J + ni < left && cb * COLS + n * Sh::kGroups + group < dim) o_dst[n * Sh::kGroups] = o;
+      }
+      o_dst += J * hd;
     }
     __syncthreads();  // chunk c has been read, chunk c + 1 is ready
   }
@@ -624,13 +953,31 @@ static int launch_scan(const b200_delta_args& a, cudaStream_t s) {
   delta_scan_kernel<T, DIM, COLS, N, LANES><<<dim3(a.heads * col_blocks, a.num_rows), Sh::kThreads, Sh::kSmemBytes, s>>>(a);
   return launch_status();
 }
+template <typename T, int DIM, int COLS, int BLOCKS>
+static int launch_block_scan(const b200_delta_args& a, cudaStream_t s) {
+  using Sh = BlockShape<DIM, COLS, BLOCKS>;
+  static std::atomic<uint64_t> done{0};
+  if (ensure_dynamic_smem(delta_block_scan_kernel<T, DIM, COLS, BLOCKS>, Sh::kSmemBytes, done) != B200_OK) return B200_ERR_LAUNCH;
+  const int col_blocks = (a.dim + COLS - 1) / COLS;
+  delta_block_scan_kernel<T, DIM, COLS, BLOCKS><<<dim3(a.heads * col_blocks, a.num_rows), Sh::kThreads, Sh::kSmemBytes, s>>>(a);  // (not programmatic: see launch_scan)
+  return launch_status();
+}
+template <typename T, int DIM>
+static int block_scan_by_size(const b200_delta_args& a, cudaStream_t s) {
+  // Eight preparing warps, and one CTA on an SM, while a CTA's own pace counts: rows of 128 tokens and more on average and, with heads of up to 64, CTAs for
+  // little more than two rounds of the SMs.  Else four, and two CTAs of up to 64.  us, eight / four: heads of 64, 160 CTAs 378 / 481, 256 of 400 tokens and less
+  // 102 / 110, 320 583 / 615, 384 682 / 647, 512 841 / 764; rows of 64 tokens 33.8 / 29.8.  Heads of 128: 256 CTAs 791 / 961, 2048 1340 / 1497; rows of 16 40 / 34.
+  const int64_t ctas = static_cast<int64_t>(a.num_rows) * a.heads;
+  if (a.num_tokens / 128 >= a.num_rows && (DIM > 64 || 4 * ctas <= 9 * sm_count())) return launch_block_scan<T, DIM, 64, 8>(a, s);
+  return launch_block_scan<T, DIM, 64, 4>(a, s);
+}
 template <typename T>
 static int scan_by_dim(const b200_delta_args& a, cudaStream_t s) {
-  // Two columns on four lanes: 1024 tokens x 64 heads of 64 304 -> 251 us, 6208 tokens in 5 rows x 32 heads 886 -> 746 us (one column on two lanes before);
-  // with the longest rows first on top, which alone is 886 -> 700.  One column on four or eight lanes: 270, 304 us.
+  // Blocks of four tokens against one token at a time: 6208 tokens in 5 rows x 32 heads of 64 378 us, 581; 8 rows x 64 heads 764, 872; 16 heads of 128, 5448
+  // tokens in 4 rows 711, 918; 64 rows x 32 heads of one token 42, 42.  256 channels do not fit the registers four times, 32 are not worth the preparation.
   if (a.dim <= 32) return launch_scan<T, 32, 32, 1, 2>(a, s);
-  if (a.dim <= 64) return launch_scan<T, 64, 64, 2, 4>(a, s);
-  if (a.dim <= 128) return launch_scan<T, 128, 64, 2, 4>(a, s);
+  if (a.dim <= 64) return block_scan_by_size<T, 64>(a, s);
+  if (a.dim <= 128) return block_scan_by_size<T, 128>(a, s);
   return launch_scan<T, 256, 32, 1, 2>(a, s);
 }
 

@@ -453,6 +453,39 @@ def test_delta_scan(dtype, heads, dim, rank):
         at += n
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,dim", [(2, 64), (1, 40), (1, 128), (2, 68)])
+def test_delta_scan_of_long_rows(dtype, heads, dim):
+    """Rows of 128 tokens and more on average are prepared 32 tokens at a time: rows that end one token before, at and behind a block of four and a group of
+    32, one that is empty, padding tokens behind them that nothing is written for.  Tolerances as in test_delta_scan."""
+    from megatron_mixtera_b200 import ops
+
+    lens, rank = [257, 3, 0, 320, 189, 130], 8
+    T, pad = sum(lens), 4
+    c = DeltaCase(heads, dim, rank, T + pad, dtype, seed=50)
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    state = rand(12, heads, dim, dim, seed=51)
+    rd = torch.tensor([0, 2, -1, -1, 6, 7], dtype=torch.int32)
+    wr = torch.tensor([1, 3, -1, 5, 6, 9], dtype=torch.int32)
+    d_state, d_rd, d_wr = state.to(DEV), rd.to(DEV), wr.to(DEV)
+    o_f32 = torch.full((T + pad, c.n), 7.0, device=DEV)
+    z = ops.linear(torch.tanh(c.dev[0][:, 5 * c.n:]).contiguous(), c.dev[1])
+    a = c.args(d_state, d_rd, d_wr, o_f32)
+    a.num_rows, a.cu_tokens, a.o_f32, a.z = len(lens), cu.data_ptr(), o_f32.data_ptr(), z.data_ptr()
+    ops.delta_scan(a, d_state)
+    new, at = d_state.cpu(), 0
+    tol = 1e-4 if dtype == torch.float32 else 2e-2
+    for row, n in enumerate(lens):
+        if n == 0:
+            continue
+        S0 = state[rd[row]].double().transpose(1, 2) if rd[row] >= 0 else None
+        o, S = Z.delta_scan(*c.inputs(at, at + n), state=S0)
+        assert (new[wr[row]].double().transpose(1, 2) - S).abs().max() < tol * S.abs().max()
+        assert (o_f32[at: at + n].cpu().double() - o.reshape(n, -1)).abs().max() < tol * o.abs().max()
+        at += n
+    assert bool((o_f32[T:] == 7.0).all())
+
+
 def test_delta_state_survives_long_rows():
     """A value written at the first token with decay close to one is still there 600 tokens later, and only there."""
     from megatron_mixtera_b200 import ops
