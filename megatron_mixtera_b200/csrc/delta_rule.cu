@@ -541,16 +541,19 @@ struct BlockShape {
   static_assert(COLS % 32 == 0 && DIM % 32 == 0 && kFloats % 4 == 0, "");
 };
 
-// Sum of value i over the warp, in lane i.
-__device__ __forceinline__ float transposed_sum(float (&v)[32], int lane) {
+// Sums of N values over the warp, that of value i in lane i (and N, 2 N, ... further on).
+template <int N>
+__device__ __forceinline__ float transposed_sum(float (&v)[N], int lane) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
+  for (int o = N / 2; o > 0; o >>= 1)
 #pragma unroll
     for (int i = 0; i < o; ++i) {
       const bool high = lane & o;
       const float give = high ? v[i] : v[i + o], keep = high ? v[i + o] : v[i];
       v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
     }
+#pragma unroll
+  for (int o = N; o < 32; o <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
   return v[0];
 }
 
@@ -713,7 +716,7 @@ delta_block_scan_kernel(b200_delta_args a) {
         }
         buf[Sh::kW + e * 32] = p;
       }
-      const float sum = transposed_sum(pairs, lane);
+      const float sum = transposed_sum<32>(pairs, lane);
       buf[Sh::kPairs - lane + place] = sum;
       __syncthreads();  // chunk c is ready, chunk c - 1 has been read: its buffer is free
     }

@@ -11,6 +11,7 @@
 //
 //   decode_kernel  one token per row, a warp per (row, head), everything from the projections to the gated output
 //   scan_kernel    rows of any length, one CTA per (row, head, block of columns); other warps prepare the next 16 tokens
+//   wkv_block_scan_kernel  the same for Wkv with heads of 33 to 128, four tokens at a time
 //   finish_kernel  head norm, weight and gate behind the scan
 //   gates_kernel   Memory: the running maximum and the factors of every token of a step, a CTA per (row, head)
 //
@@ -531,8 +532,8 @@ struct ScanShape {  // COLS columns per CTA, N of them per thread, LANES lanes p
   static constexpr int kBufFloats = kScanTokens * kTokenFloats;
   static constexpr int kSmemBytes = 2 * kBufFloats * 4;
   // Tokens unrolled: four where their vectors fit the registers beside the state, else one.  64 rows, 16384 tokens, four against one: 32 heads of 32: delta
-  // 303, 255 us, wkv 245, 222, memory 248, 230; of 64: memory 723, 528 (4 rows 455, 429), wkv 445, 512, delta 644, 586 (4 rows 398, 454); 16 heads of 128: wkv
-  // 866, 1086, delta 992, 1067, memory 799, 1005; 8 of 256: delta 4010, 3316 (a kilobyte spilled), wkv 3242, 4324, memory 2573, 2730.
+  // 303, 255 us, wkv 245, 222, memory 248, 230; of 64: memory 723, 528 (4 rows 455, 429), delta 644, 586 (4 rows 398, 454); 16 heads of 128:
+  // delta 992, 1067, memory 799, 1005; 8 of 256: delta 4010, 3316 (a kilobyte spilled), wkv 3242, 4324, memory 2573, 2730.
   static constexpr int kUnroll =
       DIM <= 32 || (Rule::kKind == B200_RECURRENCE_MEMORY && DIM == 64) || (Rule::kKind == B200_RECURRENCE_DELTA && DIM == 256) ? 1 : 4;
   static_assert(kComputeThreads % 32 == 0 && kScanTokens % kPrepWarps == 0 && kTokPerWarp % kBatch == 0 && COLS % 4 == 0, "");
@@ -755,6 +756,267 @@ scan_kernel(b200_recurrence_args a, bool vec_k) {
   }
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// Scan of Wkv, four tokens at a time (as in delta_rule.cu)
+// ---------------------------------------------------------------------------------------------------------------
+// With S the state in front of four tokens and w[a..b] the product of their decays:
+//
+//   o_j = (r_j w[0..j-1]) . S + sum_(s<j) (r_j . k_s w[s+1..j-1]) v_s + (r_j . b k_j) v_j,   S <- w[0..3] S + sum_s (k_s w[s+1..3]) v_s
+//
+// nine passes over a column's registers and a vector each, where four tokens one after another take twelve, and one lane sum for four tokens.  Bound by the reads
+// of shared memory and the multiply-adds of the compute warps.  6016 tokens in 4 rows x 32 heads of 64 340 -> 218 us, 16 heads of 128 504 -> 343.  Decays are
+// only multiplied, so none can be too small.  (Delta in the same form, two dot products for each token, 16 heads of 128: 532 -> 527 us with four lanes for a
+// column, 464 with eight, and 8 % more rounding error: it stays with a token at a time.)
+constexpr int kBlockTokens = 4;
+// Of a block, in floats: r w[0..j-1] and k w[s+1..3] of its tokens and w[0..3], each [DIM]; the values [4][COLS]; the products of the tokens with one another
+// [4][4] (j, s; zero where s > j).
+template <int DIM, int COLS, int LANES, int BLOCKS>
+struct BlockShape {
+  static constexpr int kR = 0, kK = 4 * DIM, kW = 8 * DIM, kV = 9 * DIM, kPairs = kV + 4 * COLS, kFloats = kPairs + 16;
+  static constexpr int NI = LANES, N = LANES / 2, I = DIM / NI, kStride = 32 / NI;  // N columns on NI lanes
+  static constexpr int kComputeThreads = COLS / N * NI;
+  static constexpr int kBlocks = BLOCKS, kTokens = BLOCKS * kBlockTokens, kThreads = kComputeThreads + BLOCKS * 32;
+  static constexpr int kElems = DIM / 32, kValues = COLS / 32;
+  static constexpr int kSmemBytes = 2 * kBlocks * kFloats * 4;
+  static_assert(COLS % 32 == 0 && kFloats % 4 == 0 && (LANES == 4 || LANES == 8), "");
+};
+
+template <typename T, int DIM, int COLS, int LANES, int BLOCKS>
+__global__ void __launch_bounds__(BlockShape<DIM, COLS, LANES, BLOCKS>::kThreads)
+wkv_block_scan_kernel(b200_recurrence_args a, bool vec_k) {
+  using Sh = BlockShape<DIM, COLS, LANES, BLOCKS>;
+  constexpr int NI = Sh::NI, I = Sh::I, N = Sh::N, EL = Sh::kElems, VL = Sh::kValues, J = kBlockTokens;
+  extern __shared__ __align__(16) float smem[];
+  const int tid = threadIdx.x, lane = tid & 31, dim = a.dim, vdim = a.vdim;
+  const int col_blocks = (vdim + COLS - 1) / COLS;
+  const int head = blockIdx.x / col_blocks, cb = blockIdx.x - head * col_blocks, row = delta::longest_first(a.cu_tokens, a.num_rows, blockIdx.y);
+  pdl_launch_dependents();
+  const int t_begin = a.cu_tokens[row], n_tok = min(a.cu_tokens[row + 1], a.num_tokens) - t_begin;
+  pdl_wait();
+  if (n_tok <= 0) return;
+  const int chunks = (n_tok + Sh::kTokens - 1) / Sh::kTokens;
+
+  if (tid >= Sh::kComputeThreads) {
+    // ------------------------------- preparing warps: a block each -------------------------------
+    const int warp = (tid - Sh::kComputeThreads) >> 5;
+    const T* proj = static_cast<const T*>(a.proj);
+    const int64_t hd = static_cast<int64_t>(a.heads) * dim;
+    float bias[EL], bonus[EL];
+#pragma unroll
+    for (int e = 0; e < EL; ++e) {
+      const int i = head * dim + min(lane * EL + e, dim - 1);
+      bias[e] = simt::to_f32(static_cast<const T*>(a.decay_bias)[i]);
+      bonus[e] = simt::to_f32(static_cast<const T*>(a.bonus)[i]);
+    }
+    int place = -1;  // where the product of two tokens that this lane sums goes
+    {
+      int i = 0;
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int s = 0; s <= j; ++s, ++i)
+          if (i == lane) place = j * J + s;
+    }
+    smem[((lane / 16) * Sh::kBlocks + warp) * Sh::kFloats + Sh::kPairs + lane % 16] = 0.f;  // (in both buffers)
+    __syncwarp();
+    T xv[J][VL];
+    float xr[J][EL], xk[J][EL], xz[J][EL];
+    auto fetch = [&](auto vec_c, int c) {  // no branches between the loads: all in flight together
+      constexpr bool V = decltype(vec_c)::value;
+      const int first = c * Sh::kTokens + warp * J;
+#pragma unroll
+      for (int q = 0; q < J; ++q) {
+        const int64_t t = t_begin + min(first + q, n_tok - 1);
+        const T* p = proj + t * a.proj_ld;
+        const T* v = p + a.off_v + head * vdim;
+        load_channels<V, T, EL>(p + a.off_r + head * dim, lane, dim, xr[q]);
+        load_channels<V, T, EL>(p + a.off_k + head * dim, lane, dim, xk[q]);
+        load_channels<V, float, EL>(a.z + t * hd + head * dim, lane, dim, xz[q]);
+#pragma unroll
+        for (int e = 0; e < VL; ++e) xv[q][e] = v[min(cb * COLS + lane + e * 32, vdim - 1)];
+      }
+      for (int s = 1; s < a.z_splits; ++s)
+#pragma unroll
+        for (int q = 0; q < J; ++q) {
+          const int64_t t = t_begin + min(first + q, n_tok - 1);
+          float more[EL];
+          load_channels<V, float, EL>(a.z + (static_cast<int64_t>(s) * a.num_tokens + t) * hd + head * dim, lane, dim, more);
+#pragma unroll
+          for (int e = 0; e < EL; ++e) xz[q][e] += more[e];
+        }
+    };
+    auto fetch_any = [&](int c) {
+      if (vec_k)
+        fetch(std::true_type{}, c);
+      else
+        fetch(std::false_type{}, c);
+    };
+    fetch_any(0);
+    for (int c = 0; c < chunks; ++c) {
+      float* buf = smem + ((c & 1) * Sh::kBlocks + warp) * Sh::kFloats;
+      const int left = n_tok - c * Sh::kTokens - warp * J;  // (past the end: nothing is written, nothing decays)
+      float r[J][EL], k[J][EL], w[J][EL];
+#pragma unroll
+      for (int q = 0; q < J; ++q) {
+#pragma unroll
+        for (int e = 0; e < EL; ++e) {
+          const bool ok = q < left && lane * EL + e < dim;
+          r[q][e] = ok ? xr[q][e] : 0.f;
+          k[q][e] = ok ? xk[q][e] : 0.f;
+          w[q][e] = q < left ? expf(-expf(xz[q][e] + bias[e])) : 1.f;
+        }
+#pragma unroll
+        for (int e = 0; e < VL; ++e) buf[Sh::kV + q * COLS + lane + e * 32] = q < left ? simt::to_f32(xv[q][e]) : 0.f;
+      }
+      if (c + 1 < chunks) fetch_any(c + 1);
+      float sums[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) sums[i] = 0.f;
+#pragma unroll
+      for (int e = 0; e < EL; ++e) {
+        float kk[J], p = 1.f;  // keys on their way through the decays behind them; the decays so far
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+#pragma unroll
+          for (int s = 0; s < j; ++s) {
+            sums[j * (j + 1) / 2 + s] = fmaf(r[j][e], kk[s], sums[j * (j + 1) / 2 + s]);
+            kk[s] *= w[j][e];
+          }
+          sums[j * (j + 1) / 2 + j] = fmaf(r[j][e] * bonus[e], k[j][e], sums[j * (j + 1) / 2 + j]);
+          kk[j] = k[j][e];
+          buf[Sh::kR + j * DIM + lane * EL + e] = r[j][e] * p;
+          p *= w[j][e];
+        }
+#pragma unroll
+        for (int s = 0; s < J; ++s) buf[Sh::kK + s * DIM + lane * EL + e] = kk[s];
+        buf[Sh::kW + lane * EL + e] = lane * EL + e < dim ? p : 0.f;
+      }
+      const float mine = delta::transposed_sum<16>(sums, lane);
+      if (place >= 0) buf[Sh::kPairs + place] = mine;
+      __syncthreads();  // chunk c is ready, chunk c - 1 has been read: its buffer is free
+    }
+    __syncthreads();
+    return;
+  }
+
+  // --------------------------------- compute warps ---------------------------------
+  const bool full = dim == DIM;
+  const int in = a.state_in[row], out = a.state_out[row];
+  const int64_t head_elems = static_cast<int64_t>(dim) * vdim;
+  constexpr int ST = Sh::kStride;
+  const int ni = lane / ST, group = (tid >> 5) * ST + lane % ST;  // this thread's columns: first + n
+  const int first = cb * COLS + group * N;
+  f32x2 s[N][I / 2];
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int j = first + n;
+    if (static_cast<unsigned>(in) < static_cast<unsigned>(a.state_slots) && j < vdim) {
+      delta::load_column<NI, I>(a.state + (static_cast<int64_t>(in) * a.heads + head) * head_elems + static_cast<int64_t>(j) * dim, dim, ni, full, s[n]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < I / 2; ++e) s[n][e] = 0ull;
+    }
+  }
+  const int64_t hv = static_cast<int64_t>(a.heads) * vdim;
+  constexpr int M = NI == 8 ? N / 2 : N;  // columns of a token's output on a lane: with eight lanes the upper four have the second half
+  const int mine = ni % J, half = ni / J * M;
+  float* o_dst = a.o_f32 + (static_cast<int64_t>(t_begin) + mine) * hv + head * vdim + first + half;  // this lane's token of every block
+  __syncthreads();  // chunk 0 is ready
+  for (int c = 0; c < chunks; ++c) {
+    const int left = n_tok - c * Sh::kTokens, blocks = min(Sh::kBlocks, (left + J - 1) / J);
+#pragma unroll 2
+    for (int b = 0; b < blocks; ++b) {
+      const float* buf = smem + ((c & 1) * Sh::kBlocks + b) * Sh::kFloats;
+      f32x2 dr[J][N];
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int n = 0; n < N; ++n) dr[j][n] = 0ull;
+#pragma unroll
+      for (int q = 0; q < I / 4; ++q) {
+        const int i = (q * NI + ni) * 4;
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          const ulonglong2 r = piece(buf + Sh::kR + j * DIM + i);
+#pragma unroll
+          for (int n = 0; n < N; ++n) dr[j][n] = fma2(r.y, s[n][q * 2 + 1], fma2(r.x, s[n][q * 2], dr[j][n]));
+        }
+      }
+      float v[J][N];
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const float* at = buf + Sh::kV + j * COLS + group * N;
+        if constexpr (N == 4) {
+          const float4 x = *reinterpret_cast<const float4*>(at);
+          v[j][0] = x.x;
+          v[j][1] = x.y;
+          v[j][2] = x.z;
+          v[j][3] = x.w;
+        } else {
+          const float2 x = *reinterpret_cast<const float2*>(at);
+          v[j][0] = x.x;
+          v[j][1] = x.y;
+        }
+      }
+      f32x2 write[J][N];
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int n = 0; n < N; ++n) write[j][n] = pack2(v[j][n], v[j][n]);
+#pragma unroll
+      for (int q = 0; q < I / 4; ++q) {
+        const ulonglong2 w = piece(buf + Sh::kW + (q * NI + ni) * 4);
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          s[n][q * 2] = mul2(w.x, s[n][q * 2]);
+          s[n][q * 2 + 1] = mul2(w.y, s[n][q * 2 + 1]);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < I / 4; ++q)
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          const ulonglong2 k = piece(buf + Sh::kK + j * DIM + (q * NI + ni) * 4);
+#pragma unroll
+          for (int n = 0; n < N; ++n) {
+            s[n][q * 2] = fma2(k.x, write[j][n], s[n][q * 2]);
+            s[n][q * 2 + 1] = fma2(k.y, write[j][n], s[n][q * 2 + 1]);
+          }
+        }
+      // Token `mine`'s output: its partial sums from the lanes of the column, and what the block's tokens up to it wrote.
+      const float4 rk = *reinterpret_cast<const float4*>(buf + Sh::kPairs + mine * J);
+      const bool upper = ni & 4, high = ni & 2, odd = ni & 1;
+#pragma unroll
+      for (int n = 0; n < M; ++n) {
+        float p[J], wrote[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+          p[j] = sum2(dr[j][n]);
+          wrote[j] = v[j][n];
+          if constexpr (NI == 8) {
+            const float other = sum2(dr[j][n + M]);
+            p[j] = (upper ? other : p[j]) + __shfl_xor_sync(0xffffffffu, upper ? p[j] : other, 4 * ST);
+            wrote[j] = upper ? v[j][n + M] : wrote[j];
+          }
+        }
+        const float a0 = (high ? p[2] : p[0]) + __shfl_xor_sync(0xffffffffu, high ? p[0] : p[2], 2 * ST);
+        const float a1 = (high ? p[3] : p[1]) + __shfl_xor_sync(0xffffffffu, high ? p[1] : p[3], 2 * ST);
+        float o = (odd ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, ST);
+        o = fmaf(rk.x, wrote[0], fmaf(rk.y, wrote[1], fmaf(rk.z, wrote[2], fmaf(rk.w, wrote[3], o))));
+        if (b * J + mine < left && first + half + n < vdim) o_dst[n] = o;
+      }
+      o_dst += J * hv;
+    }
+    __syncthreads();  // chunk c has been read, chunk c + 1 is ready
+  }
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int j = first + n;
+    if (static_cast<unsigned>(out) < static_cast<unsigned>(a.state_slots) && j < vdim)
+      delta::store_column<NI, I>(a.state + (static_cast<int64_t>(out) * a.heads + head) * head_elems + static_cast<int64_t>(j) * dim, dim, ni, full, s[n]);
+  }
+}
+
 // LPH lanes of 4 channels per (token, head), kFinishUnits units in turn with all their loads in flight (LPH == 0: a warp, any size).
 constexpr int kFinishUnits = 4;
 // MEMORY: outputs are still to be divided, the gate is a plain sigmoid.
@@ -956,27 +1218,53 @@ static int decode_by_dim(const b200_recurrence_args& a, cudaStream_t s) {
   if (a.dim <= 128) return launch_decode<T, Rule, 128>(a, s);
   return launch_decode<T, Rule, 256>(a, s);
 }
+// Whether a lane's EL channels of a token can be one vector.
+template <typename Rule, int EL>
+static bool channels_in_vectors(const b200_recurrence_args& a) {
+  bool vec_k = a.dim % EL == 0 && a.proj_ld % 8 == 0 && aligned16(a.proj) && a.off_r % 8 == 0 && a.off_k % 8 == 0 && aligned16(a.conv) && aligned16(a.z);
+  if (Rule::kKind == B200_RECURRENCE_DELTA) vec_k = vec_k && (2 * a.kv_heads * a.dim + a.heads * a.vdim) % EL == 0;
+  return vec_k;
+}
 template <typename T, typename Rule, int DIM, int COLS, int N, int LANES, int CTAS>
 static int launch_scan(const b200_recurrence_args& a, cudaStream_t s) {
   using Sh = ScanShape<Rule, DIM, COLS, N, LANES>;
   static std::atomic<uint64_t> done{0};
   if (ensure_dynamic_smem(scan_kernel<T, Rule, DIM, COLS, N, LANES, CTAS>, Sh::kSmemBytes, done) != B200_OK) return B200_ERR_LAUNCH;
   const int col_blocks = (a.vdim + COLS - 1) / COLS;
-  constexpr int EL = Sh::kElems;
-  bool vec_k = a.dim % EL == 0 && a.proj_ld % 8 == 0 && aligned16(a.proj) && a.off_r % 8 == 0 && a.off_k % 8 == 0 && aligned16(a.conv) && aligned16(a.z);
-  if (Rule::kKind == B200_RECURRENCE_DELTA) vec_k = vec_k && (2 * a.kv_heads * a.dim + a.heads * a.vdim) % EL == 0;
   // Not a programmatic launch: CTAs that arrive while the previous kernel still holds most SMs would pile up on the others,
   // and a CTA stays where it is for the length of a prompt.
-  scan_kernel<T, Rule, DIM, COLS, N, LANES, CTAS><<<dim3(a.heads * col_blocks, a.num_rows), Sh::kThreads, Sh::kSmemBytes, s>>>(a, vec_k);
+  scan_kernel<T, Rule, DIM, COLS, N, LANES, CTAS><<<dim3(a.heads * col_blocks, a.num_rows), Sh::kThreads, Sh::kSmemBytes, s>>>(a, channels_in_vectors<Rule, Sh::kElems>(a));
   return launch_status();
+}
+template <typename T, int DIM, int LANES, int BLOCKS>
+static int launch_block_scan(const b200_recurrence_args& a, cudaStream_t s) {
+  using Sh = BlockShape<DIM, 64, LANES, BLOCKS>;
+  static std::atomic<uint64_t> done{0};
+  if (ensure_dynamic_smem(wkv_block_scan_kernel<T, DIM, 64, LANES, BLOCKS>, Sh::kSmemBytes, done) != B200_OK) return B200_ERR_LAUNCH;
+  wkv_block_scan_kernel<T, DIM, 64, LANES, BLOCKS>  // (not programmatic: see launch_scan)
+      <<<dim3(a.heads * ((a.vdim + 63) / 64), a.num_rows), Sh::kThreads, Sh::kSmemBytes, s>>>(a, channels_in_vectors<Wkv, Sh::kElems>(a));
+  return launch_status();
+}
+template <typename T, int DIM>
+static int block_scan_by_size(const b200_recurrence_args& a, cudaStream_t s) {
+  // Eight preparing warps and two columns on four lanes for rows of 64 tokens and more on average; else four, with four columns on eight lanes, and more CTAs on
+  // an SM.  us, the former / the latter / a token at a time: 32 heads of 64, rows of 64 tokens 13.6 / 15.0 / 15.5, 60 rows of 20 71 / 51 / 58, 64 rows of one
+  // 50 / 28 / 35; 64 rows of 256 tokens x 16 heads of 128 659 / 920 / 935.
+  if (a.num_tokens / 64 >= a.num_rows) return launch_block_scan<T, DIM, 4, 8>(a, s);
+  return launch_block_scan<T, DIM, 8, 4>(a, s);
 }
 template <typename T, typename Rule>
 static int scan_by_dim(const b200_recurrence_args& a, cudaStream_t s) {
-  // Two columns on four lanes (6016 tokens in 4 rows): wkv, 32 heads of 64: 316 -> 288 us; delta, 16 heads of 128: 581 -> 530; memory, 16
-  // heads of 128: 498 -> 467.  Other splits (one column on 2, 4, 8 lanes, two on 8, four on 8): 2 to 40 % slower.
+  // Two columns on four lanes (6016 tokens in 4 rows): delta, 16 heads of 128: 581 -> 530 us; memory, 16 heads of 128: 498 -> 467.  Other splits (one column on
+  // 2, 4, 8 lanes, two on 8, four on 8): 2 to 40 % slower.
   if (a.dim <= 32) return launch_scan<T, Rule, 32, 32, 1, 2, 1>(a, s);
-  if (a.dim <= 64) return launch_scan<T, Rule, 64, 64, 2, 4, 1>(a, s);
-  if (a.dim <= 128) return launch_scan<T, Rule, 128, 64, 2, 4, 1>(a, s);
+  if constexpr (Rule::kKind == B200_RECURRENCE_WKV) {
+    if (a.dim <= 64) return block_scan_by_size<T, 64>(a, s);
+    if (a.dim <= 128) return block_scan_by_size<T, 128>(a, s);
+  } else {
+    if (a.dim <= 64) return launch_scan<T, Rule, 64, 64, 2, 4, 1>(a, s);
+    if (a.dim <= 128) return launch_scan<T, Rule, 128, 64, 2, 4, 1>(a, s);
+  }
   return launch_scan<T, Rule, 256, 32, 1, 2, 1>(a, s);
 }
 template <typename T>

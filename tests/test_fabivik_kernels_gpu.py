@@ -68,6 +68,20 @@ def test_recurrent_mixers(kind, which, dtype):
     assert len(ctx._free_state_slots) == ctx.num_state_slots
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,dim", [(2, 64), (3, 36), (1, 128)])
+def test_wkv_rows_that_end_inside_a_block(heads, dim, dtype):
+    """Blocks of four tokens, prepared 32 tokens at a time for long rows and 16 for short ones: rows that end before, at and behind both, in one step and
+    continued in another one."""
+    layer = H.wkv(heads=heads, dim=dim, rank=8, mlp=None)
+    _, _, w, model, ctx = one_layer(layer, dtype)
+    hs = [rows(n, 96, 15 + i) for i, n in enumerate((193, 66, 131, 4))]
+    want = [F.wkv(h.double(), w, "l0.mix", layer["mixer"], 1e-5) for h in hs]
+    for schedule in ([[(0, 193), (1, 66), (2, 131)], [(3, 4)]], [[(0, 17), (1, 1), (2, 3), (3, 4)], [(0, 176), (1, 65), (2, 128)]]):
+        got = H.run_mixer(model, ctx, 0, hs, schedule)
+        assert all(close(g, x, dtype) for g, x in zip(got, want)), schedule
+
+
 @pytest.mark.parametrize("kind", list(MIXERS))
 def test_recurrent_state_after_a_portion(kind):
     """The state itself, and that a padding row or another request's slot is left alone."""
@@ -274,6 +288,51 @@ def test_expert_pairs_over_several_units_each():
     pick = [t for t in pick.tolist() if order[t, top - 1] - order[t, top] > 1e-6]
     assert H.rel(got[pick], F.mixture(x[pick].double(), w, "l0.mlp", mlp)) < LIMIT[torch.bfloat16] / 4
     assert not torch.isnan(got).any()
+
+
+@pytest.mark.parametrize("width,top,splits", [(520, 3, 2), (1024, 4, 1), (1032, 1, 3), (2048, 5, 0), (4096, 8, 1), (4104, 2, 1), (8192, 4, 1)])
+def test_residual_norm_of_many_rows(width, top, splits):
+    """More rows than two for every SM: sums of the branch, expert rows (some missing), a gated shared expert's and the stream; two norms.  32-bit sums of bf16
+    values in the stream (1e-5 of its scale), one rounding to bf16 in the norms (2^-8 of a value)."""
+    from megatron_mixtera_b200 import _lib, ops
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    T, E = 2 * torch.cuda.get_device_properties(0).multi_processor_count + 5, 7
+
+    def r(*shape):
+        return torch.randn(*shape, generator=g, device="cuda")
+
+    hidden, part, rows_, shared, gate = r(T, width), r(max(splits, 1), T, width), r(T * top, width).bfloat16(), r(T, width).bfloat16(), torch.rand(T, generator=g, device="cuda")
+    expert = torch.randint(0, E, (T * top,), generator=g, device="cuda")
+    counts = torch.bincount(expert, minlength=E)
+    offsets = torch.cat([counts.new_zeros(1), counts.cumsum(0)])
+    rank = torch.empty_like(expert)
+    order = torch.argsort(expert, stable=True)
+    rank[order] = torch.arange(T * top, device="cuda") - offsets[expert[order]]
+    at = (offsets[expert] + rank).view(T, top)
+    weight = torch.rand(T, top, generator=g, device="cuda")
+    lost = torch.zeros(T * top, dtype=torch.bool, device="cuda")
+    lost[::11] = True  # an expert that does not exist
+    pairs = torch.stack([torch.where(lost, E + 3, expert), rank], dim=1).int().contiguous()
+    gammas = [(0.3 * r(width)).bfloat16() for _ in range(2)]
+    out = [torch.empty(T, width, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    want = hidden.double() + (part.double().sum(0) if splits else 0.0) + gate.double()[:, None] * shared.double()
+    for j in range(top):
+        want += (weight[:, j].double() * ~lost.view(T, top)[:, j])[:, None] * rows_[at[:, j]].double()
+    a = _lib.ResidualNormArgs()
+    a.hidden, a.rows, a.source_rows, a.width, a.eps, a.gain, a.out_scale, a.dtype = hidden.data_ptr(), T, T, width, 1e-3, 1.0, 0.5, ops.dtype_code(torch.bfloat16)
+    if splits:
+        a.partials, a.num_splits = part.data_ptr(), splits
+    a.expert_rows, a.expert_row_count, a.pairs, a.offsets, offsets32 = rows_.data_ptr(), T * top, pairs.data_ptr(), 0, offsets.int()
+    a.offsets, a.top, a.experts, a.pair_weight = offsets32.data_ptr(), top, E, weight.data_ptr()
+    a.shared_rows, a.shared_gate = shared.data_ptr(), gate.data_ptr()
+    for i in range(2):
+        a.gamma[i], a.y[i] = gammas[i].data_ptr(), out[i].data_ptr()
+    ops.struct_kernel("residual_norm", a, hidden)
+    assert float((hidden.double() - want).abs().max()) < 1e-5 * float(want.abs().max())
+    for o, gamma in zip(out, gammas):
+        y = 0.5 * want / torch.sqrt((want * want).mean(-1, keepdim=True) + 1e-3) * (1.0 + gamma.double())
+        assert bool(((o.double() - y).abs() <= 2.0 ** -8 * y.abs() + 1e-5).all())
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
