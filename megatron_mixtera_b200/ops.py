@@ -895,6 +895,14 @@ def partials_of(p: GemmPartials):
     return p.buf.data_ptr(), p.num_splits
 
 
+def clear_padding_rows(rows, ctx) -> None:
+    """Zeros for the rows of the step's padding tokens, which no work unit and no request's scan writes.  They lie behind the active tokens' rows; a graph is
+    replayed with other numbers of those, so its steps clear every row."""
+    first = 0 if ctx.using_cuda_graph_this_step() else ctx.active_token_count
+    if first < rows.shape[0]:
+        rows[first:].zero_()
+
+
 def separate_attention(args: AttentionArgs, dtype, *, units=None, num_units: int = 0, tensor_cores: bool) -> None:
     """Attention of finished queries over a [keys | values] pool (``AttentionArgs.separate``); ``units``: a prefill step's work list."""
     global launch_count

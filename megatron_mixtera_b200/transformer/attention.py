@@ -107,7 +107,7 @@ class PagedFlashDecodeAttention(torch.nn.Module):
                                            num_splits=1, fuse_rope_append=False, **common)
             ops.rope_append(args)
             if getattr(ctx, "prefill_q_block", 0) > 0 and ctx.prefill_q_block == ops.prefill_q_block(self.num_q_heads, self.num_kv_heads):
-                out.zero_()  # padding tokens belong to no unit
+                ops.clear_padding_rows(out, ctx)
                 args.unit_mix = ctx.prefill_unit_mix(ctx.prefill_q_block)
                 ops.paged_prefill_attention(args, ctx.prefill_units, ctx.prefill_unit_count)
             else:

@@ -69,8 +69,7 @@ class GatedDelta(torch.nn.Module):
             c = short_conv_args(ctx, proj=proj, filter_=self.conv_filter, state=conv_state, channels=m.conv_channels, taps=m.conv, out=conv)
             ops.struct_kernel("conv_silu", c, state)
             a.conv, a.o_f32 = conv.data_ptr(), o.data_ptr()
-            if ctx.padded_active_token_count != ctx.active_token_count:
-                o.zero_()  # padding tokens belong to no row
+            ops.clear_padding_rows(o, ctx)
             ops.struct_kernel("recurrence_scan", a, state)
             ops.struct_kernel("recurrence_finish", a, state)
         return self.linear_proj(out, defer_reduction=True)[0]

@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import torch
 
+from .. import ops
 from ..tensor_parallel.layers import ColumnParallelLinear, RowParallelLinear, _device
 from .gated_scan import GatedScan
 from .grouped_attention import GroupedAttention
@@ -72,9 +73,10 @@ class JoinedMixer(torch.nn.Module):
         takes_partials = len(self.parts) == 1 and ctx.is_decode_only() and getattr(self.parts[0], "takes_partials", False)
         proj, _ = self.linear_in(x, defer_reduction=takes_partials)
         out = torch.empty((x.shape[0], self.linear_proj.weight.shape[1]), dtype=x.dtype, device=x.device)
-        if self.padded_outputs or not ctx.is_decode_only() and (
-                ctx.using_cuda_graph_this_step() or ctx.padded_active_token_count != ctx.active_token_count):
-            out.zero_()  # padding tokens belong to no row, padding columns to no part
+        if self.padded_outputs:
+            out.zero_()  # padding columns belong to no part
+        elif not ctx.is_decode_only():
+            ops.clear_padding_rows(out, ctx)
         for p, c, o, s, tables in zip(self.parts, self.columns, self.out_columns, self.scales, rope):
             p(x, proj, c, out, o, s, ctx, tables, step)
         return self.linear_proj(out, defer_reduction=True)[0]

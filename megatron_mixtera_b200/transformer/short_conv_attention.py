@@ -106,7 +106,7 @@ class ShortConvAttention(torch.nn.Module):
             return out
         a.kv_seq_lengths, a.row_of_token = ctx.token_kv_lengths.data_ptr(), ctx.token_to_block_table_row.data_ptr()
         if tc:
-            out.zero_()  # padding tokens belong to no unit
+            ops.clear_padding_rows(out, ctx)
             units, count = ctx.prefill_units_of(self.prefill_unit_tokens())
             a.unit_mix = ctx.prefill_unit_mix(self.prefill_unit_tokens())
             ops.separate_attention(a, queries.dtype, units=units, num_units=count, tensor_cores=True)

@@ -83,8 +83,7 @@ class Wkv(torch.nn.Module):
             o = torch.empty((T, n), dtype=torch.float32, device=dev)
             a.o_f32 = o.data_ptr()
             a.z, a.z_splits = ops.partials_of(ops.linear_partials(lora, self.decay_up))
-            if ctx.padded_active_token_count != ctx.active_token_count:
-                o.zero_()  # padding tokens belong to no row
+            ops.clear_padding_rows(o, ctx)
             ops.struct_kernel("recurrence_scan", a, state)
             ops.struct_kernel("recurrence_finish", a, state)
         return self.linear_proj(out, defer_reduction=True)[0]

@@ -567,3 +567,17 @@ def test_what_a_prefill_work_list_holds(lens, want):
     ([0, 4, 8], [0, 10, 10], 1), ([0, 0], [0, 0], 0)])
 def test_mix_of_units_and_keys(units, keys, want):
     assert DynamicInferenceContext._mix_of(np.array(units), np.array(keys)) == want
+
+
+def test_padding_rows_are_cleared_and_no_others():
+    """The rows behind the active tokens; all of them in a step that a graph is made of or replayed for, whose tokens change."""
+    import types
+
+    import torch
+
+    from megatron_mixtera_b200 import ops
+
+    for active, graph, cleared in ((0, False, 6), (4, False, 2), (6, False, 0), (6, True, 6), (3, True, 6)):
+        rows = torch.full((6, 3), float("nan"))
+        ops.clear_padding_rows(rows, types.SimpleNamespace(active_token_count=active, using_cuda_graph_this_step=lambda graph=graph: graph))
+        assert bool((rows[6 - cleared:] == 0).all()) and bool(rows[: 6 - cleared].isnan().all())
