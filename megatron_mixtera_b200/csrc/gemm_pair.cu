@@ -17,8 +17,8 @@
 // Experts' products (moe.cu) are the same kernel over a device-built list of (expert, first row, rows <= 256) entries, the shared expert's tiles in front.
 //
 // bf16 accumulators are double-buffered (2 x 256 columns = all of tensor memory); with scales there is one accumulator beside the scale slots, and
-// the eight epilogue warps read it out before they compute.  Tiles are walked in groups of kGroupM token blocks, features outermost within a group, so
-// that what the pairs work on at a time stays in L2.
+// the eight epilogue warps read it out before they compute.  Tiles are walked in groups of token blocks, features outermost within a group and backwards in
+// every other one, so that what the pairs work on at a time stays in L2.
 #include "common.cuh"
 #include "quant.cuh"
 
@@ -29,7 +29,6 @@ namespace pair {
 constexpr int kEpilogueWarps = 8;
 constexpr int kThreadsPair = (kEpilogueWarps + 2) * 32;
 constexpr int kTile = 256;      // tokens, and features, of a pair's tile
-constexpr int kGroupM = 8;
 
 // Features as they are; [64 gate | 64 up] rows; [16 gate | 16 up] rows (experts); rank 0 holds gate rows, rank 1 the matching up rows.
 enum Form { kPlain, kGated64, kGated16, kGatedHalves };
@@ -55,6 +54,7 @@ struct Args {
   uint8_t* sf_out;
   int k_tiles;      // K / 128 (scaled operands)
   int m_tiles, n_tiles, tiles;
+  int group_m;      // token blocks of a group of tiles
   // Experts: tokens sorted by expert, a device-built list of (expert, first row, rows <= 256) entries instead of m_tiles.  A second problem (a shared
   // expert: all tokens, weights and sizes of its own) may come in front of it.
   Params shared;
@@ -185,11 +185,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       u.w_row = e.x * a.p.N + u.nt * kTile;
       return static_cast<unsigned>(e.x) < static_cast<unsigned>(a.experts) && e.y >= 0 && e.z > 0;
     } else {
-      const int per_group = kGroupM * a.n_tiles;
+      const int per_group = a.group_m * a.n_tiles;
       const int group = tile / per_group, in = tile - group * per_group;
-      const int rows = min(kGroupM, a.m_tiles - group * kGroupM);
+      const int rows = min(a.group_m, a.m_tiles - group * a.group_m);
       u.nt = in / rows;
-      u.m0 = (group * kGroupM + (in - u.nt * rows)) * kTile;
+      u.m0 = (group * a.group_m + (in - u.nt * rows)) * kTile;
+      if (group & 1) u.nt = a.n_tiles - 1 - u.nt;
       u.m_end = a.p.M;
       u.w_row = u.nt * kTile;
       return true;
@@ -467,6 +468,10 @@ static int launch(Args& a, const CUtensorMap* mw, const CUtensorMap* mx_, const 
   if (!EXPERTS) {
     a.m_tiles = (a.p.M + kTile - 1) / kTile;
     a.tiles = a.m_tiles * a.n_tiles;
+    // The weights are read once for each group, so long groups, while their tokens stay in L2 beside the weights in use: 16 blocks of up to 8 KB a token.  In
+    // long runs at the power cap, us with 8 and 16 blocks, features always forwards: 7700 x 28672 x 4096 1420, 1397, x 14336 -> 4096 722, 732; MXFP8 15500 x 28672 x
+    // 4096 1830, 1804, x 14336 -> 4096 893, 902.  Every other group backwards: 0 to 1.2 % less.
+    a.group_m = static_cast<int64_t>(a.p.K) * (MX ? 1 : 2) <= 8192 ? 16 : 8;
   }
   static std::atomic<uint64_t> smem_attr_done{0};
   if (ensure_dynamic_smem(gemm_pair_kernel<MX, FORM, EXPERTS>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
