@@ -4,14 +4,15 @@
 // Here the TOKENS are the UMMA "M" side (one TMEM lane per token, 128 per CTA) and the weight rows of the CTA's one or two tiles are the "N" side (one
 // TMEM column per output feature).  What that buys:
 //   * a promoter thread owns ONE token, so the token scale of a K block is one scalar per thread and the promotion is
-//     one FFMA per accumulator element (the weight-major form needs a multiply and a shared-memory read per element
-//     on top, and was 5 x off the weight-streaming time at 256 tokens);
+//     half a packed multiply-add per accumulator element (the weight-major form needs a multiply and a shared-memory read
+//     per element on top, and was 5 x off the weight-streaming time at 256 tokens);
 //   * a thread ends up with 128 consecutive output features of its token: the epilogue stores 16-byte vectors
 //     straight from registers, no tensor-memory write-back, no transposition.
 // Two weight tiles per CTA (more than 128 tokens) make products of N = 256, which read 12 KB of shared memory in 128 clocks; 256 tokens x one tile
 // made two of N = 128 at the 128 bytes per clock that shared memory delivers, beside the copies into it.  11000 tokens: 10240 x 8192 1171 -> 1020 us
 // (1810 TFLOP/s), 57344 x 8192 6.80 -> 6.25 ms, 8192 x 28672 3.16 -> 2.94 ms; 256 tokens: 230 -> 209, 107 -> 100 us.  What bounds it now is the chain products ->
-// commit -> promotion -> release over the two accumulators that tensor memory holds: without any copies it runs at the same rate.
+// commit -> promotion -> release over the two accumulators that tensor memory holds, and the power cap: in long runs 10000 x 57344 x 8192 takes 5.91 ms (6.02 with a
+// multiply-add for every element; 5.17 without copies, 4.90 without the multiply-adds, 4.26 without both).  Sixteen promoter warps of 64 columns spill.
 //
 //   warps 0 .. 4H-1 : promoters (H = 1 or 2 weight tiles; warp w: lane quadrant w % 4 of tile w / 4)
 //   warp 4H, lane 0 : producer - per stage (= one K block) the token tile [128 x 128 B], the weight tiles
@@ -30,6 +31,17 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
+}
+
+// total += accumulator * factor for two elements with one packed multiply-add (the same roundings).  (Totals that are held as 64-bit pairs throughout took 5 %
+// longer than two multiply-adds.)
+__device__ __forceinline__ void promote2(float& t0, float& t1, uint32_t a0, uint32_t a1, float factor) {
+  unsigned long long t, a, f;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(t) : "f"(t0), "f"(t1));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "r"(a0), "r"(a1));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(f) : "f"(factor));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(t) : "l"(a), "l"(f));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(t));
 }
 
 constexpr int kGroupM = 16;  // token blocks of a group of tiles
@@ -191,7 +203,7 @@ gemm_fp8_block_tok_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
         tmem_ld_wait();
         if (c0 + 32 < kTileN) tmem_ld_32x32b_x32(acc_addr + c0 + 32, r[((c0 >> 5) & 1) ^ 1]);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) total[c0 + j] = fmaf(__uint_as_float(r[(c0 >> 5) & 1][j]), sc, total[c0 + j]);
+        for (int j = 0; j < 32; j += 2) promote2(total[c0 + j], total[c0 + j + 1], r[(c0 >> 5) & 1][j], r[(c0 >> 5) & 1][j + 1], sc);
       }
       tcgen05_fence_before_sync();
       __syncwarp();
