@@ -190,7 +190,10 @@ __device__ __forceinline__ void store_output(const Params& p, int t, int head, i
   }
 }
 
-template <int DK, int DV, int FORM>
+// STACK: at most eight query heads a KV head, so rows 8 to 15 of the products are free.  The second term of P takes them: one product with V where two were, one
+// row of scores on a thread instead of two.  (The kernel moves bytes at the HBM rate, but the step runs at the power cap, where what the SMs do sets their clock
+// and with it the rate.  Both terms' sums are added when the warps' parts are.)
+template <int DK, int DV, int FORM, bool STACK>
 __global__ void __launch_bounds__(kThreads, 2)
 paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, Params p) {
   using C = Cfg<DK, DV>;
@@ -384,10 +387,11 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int new_pos = kv_len - 1;  // position of this step's token (decode)
   const bool owns_new = !SEPARATE && p.fused && new_pos >= start && new_pos < end;
   const int r0 = warp * 16;        // this warp's token slice inside a tile
+  constexpr int kRows = STACK ? 1 : 2;  // rows of scores on a thread: gid, gid + 8
   const float* bias_r[2] = {nullptr, nullptr};
   if (EXTRA && p.bias != nullptr)
 #pragma unroll
-    for (int r = 0; r < 2; ++r) bias_r[r] = p.bias + static_cast<int64_t>(query_head<FORM>(p, h, min(gid + r * 8, G - 1))) * p.bias_len;
+    for (int r = 0; r < kRows; ++r) bias_r[r] = p.bias + static_cast<int64_t>(query_head<FORM>(p, h, min(gid + r * 8, G - 1))) * p.bias_len;
 
   for (int i = 0; i < n_tiles; ++i) {
     const int s = i % kStages;
@@ -460,7 +464,7 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < 2 * kRows; ++c) {
           const int tok = tok0 + r0 + nt * 8 + tig * 2 + (c & 1);
           float v = EXTRA ? extra_score(p, sacc[nt][c], bias_r[c >> 1], new_pos - tok) : sacc[nt][c] * scale_log2;
           if (tok >= end || (SEPARATE && tok < key_begin && !(EXTRA && tok < p.keep_first))) v = -INFINITY;
@@ -470,7 +474,7 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       }
       float alpha[2], m_use[2];
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
+      for (int r = 0; r < kRows; ++r) {
         mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
         mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
         const float m_new = fmaxf(m_run[r], mx[r]);
@@ -479,7 +483,8 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         m_run[r] = m_new;
         l_run[r] *= alpha[r];
       }
-      // P is fed to the tensor cores as hi + lo bf16 terms (two MMAs per V fragment): the bf16 rounding
+      if (STACK) alpha[1] = alpha[0];
+      // P is fed to the tensor cores as hi + lo bf16 terms (two MMAs per V fragment, or one with both): the bf16 rounding
       // of P alone would cost ~2e-3 relative accuracy per output; the pair keeps 16 bits (~2e-4 after the
       // output rounding).  A third term was measured: +5 us per launch for no visible gain downstream.
       uint32_t pf[4], pl[4];
@@ -488,27 +493,34 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < 2 * kRows; ++c) {
             pv[nt][c] = exp2f(sacc[nt][c] - m_use[c >> 1]);
             l_run[c >> 1] += pv[nt][c];
             pr[nt][c] = pv[nt][c] - bf16_round(pv[nt][c]);
           }
         }
         pf[0] = pack_bf16x2(pv[0][0], pv[0][1]);
-        pf[1] = pack_bf16x2(pv[0][2], pv[0][3]);
         pf[2] = pack_bf16x2(pv[1][0], pv[1][1]);
-        pf[3] = pack_bf16x2(pv[1][2], pv[1][3]);
-        pl[0] = pack_bf16x2(pr[0][0], pr[0][1]);
-        pl[1] = pack_bf16x2(pr[0][2], pr[0][3]);
-        pl[2] = pack_bf16x2(pr[1][0], pr[1][1]);
-        pl[3] = pack_bf16x2(pr[1][2], pr[1][3]);
+        if constexpr (STACK) {
+          pf[1] = pack_bf16x2(pr[0][0], pr[0][1]);
+          pf[3] = pack_bf16x2(pr[1][0], pr[1][1]);
+        } else {
+          pf[1] = pack_bf16x2(pv[0][2], pv[0][3]);
+          pf[3] = pack_bf16x2(pv[1][2], pv[1][3]);
+          pl[0] = pack_bf16x2(pr[0][0], pr[0][1]);
+          pl[1] = pack_bf16x2(pr[0][2], pr[0][3]);
+          pl[2] = pack_bf16x2(pr[1][0], pr[1][1]);
+          pl[3] = pack_bf16x2(pr[1][2], pr[1][3]);
+        }
       }
+      if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {  // (behind a request's first tokens the maximum seldom moves)
 #pragma unroll
-      for (int i2 = 0; i2 < DV / 8; ++i2) {
-        oacc[i2][0] *= alpha[0];
-        oacc[i2][1] *= alpha[0];
-        oacc[i2][2] *= alpha[1];
-        oacc[i2][3] *= alpha[1];
+        for (int i2 = 0; i2 < DV / 8; ++i2) {
+          oacc[i2][0] *= alpha[0];
+          oacc[i2][1] *= alpha[0];
+          oacc[i2][2] *= alpha[1];
+          oacc[i2][3] *= alpha[1];
+        }
       }
       // ---- O += P V ----
       const int v_row = r0 + (((lane >> 3) & 1) << 3) + (lane & 7);
@@ -521,9 +533,11 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         uint32_t b0, b1, b2, b3;
         ldmatrix_x4_trans(vbase + sub * C::kSubBytes + ((chunk16 ^ (v_row & 7)) << 4), b0, b1, b2, b3);
         mma_bf16_16816(oacc[dn * 2], pf, b0, b1);
-        mma_bf16_16816(oacc[dn * 2], pl, b0, b1);
         mma_bf16_16816(oacc[dn * 2 + 1], pf, b2, b3);
-        mma_bf16_16816(oacc[dn * 2 + 1], pl, b2, b3);
+        if constexpr (!STACK) {
+          mma_bf16_16816(oacc[dn * 2], pl, b0, b1);
+          mma_bf16_16816(oacc[dn * 2 + 1], pl, b2, b3);
+        }
       }
     }
     __syncwarp();
@@ -532,7 +546,7 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 
   // ------------------------------ merge the four warps ------------------------------
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
+  for (int r = 0; r < kRows; ++r) {
     l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 1);
     l_run[r] += __shfl_xor_sync(0xffffffffu, l_run[r], 2);
   }
@@ -544,17 +558,23 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   for (int i2 = 0; i2 < DV / 8; ++i2) {
     const int col = i2 * 8 + tig * 2;
     float* o0 = mo + (warp * 16 + gid) * DV + col;
-    float* o1 = mo + (warp * 16 + gid + 8) * DV + col;
-    o0[0] = oacc[i2][0];
-    o0[1] = oacc[i2][1];
-    o1[0] = oacc[i2][2];
-    o1[1] = oacc[i2][3];
+    if constexpr (STACK) {
+      o0[0] = oacc[i2][0] + oacc[i2][2];
+      o0[1] = oacc[i2][1] + oacc[i2][3];
+    } else {
+      float* o1 = mo + (warp * 16 + gid + 8) * DV + col;
+      o0[0] = oacc[i2][0];
+      o0[1] = oacc[i2][1];
+      o1[0] = oacc[i2][2];
+      o1[1] = oacc[i2][3];
+    }
   }
   if (tig == 0) {
-    mm[warp * 16 + gid] = m_run[0];
-    mm[warp * 16 + gid + 8] = m_run[1];
-    ml[warp * 16 + gid] = l_run[0];
-    ml[warp * 16 + gid + 8] = l_run[1];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      mm[warp * 16 + gid + r * 8] = m_run[r];
+      ml[warp * 16 + gid + r * 8] = l_run[r];
+    }
   }
   consumer_barrier();
   for (int i = tid; i < G * DV; i += kConsumerThreads) {
@@ -1369,17 +1389,22 @@ static bool pool_maps(const Params& p, const CUtensorMap*& mk, const CUtensorMap
   return mk && mv;
 }
 
+template <int DK, int DV, int FORM, bool STACK>
+static int launch_rows(const Params& p, const CUtensorMap* mk, const CUtensorMap* mv, unsigned units, cudaStream_t stream) {
+  using C = Cfg<DK, DV>;
+  static std::atomic<uint64_t> smem_attr_done{0};
+  if (ensure_dynamic_smem(paged_attention_kernel<DK, DV, FORM, STACK>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
+  return launch_pdl(paged_attention_kernel<DK, DV, FORM, STACK>, dim3(units), dim3(kThreads), C::kSmemBytes, stream, *mk, *mv, p);
+}
+
 template <int DK, int DV, int FORM>
 static int launch_attention(Params& p, cudaStream_t stream) {
-  using C = Cfg<DK, DV>;
   const CUtensorMap *mk, *mv;
   if (!pool_maps(p, mk, mv)) return B200_ERR_DRIVER;
-  static std::atomic<uint64_t> smem_attr_done{0};
-  if (ensure_dynamic_smem(paged_attention_kernel<DK, DV, FORM>, C::kSmemBytes, smem_attr_done) != B200_OK) return B200_ERR_LAUNCH;
   const int64_t units = static_cast<int64_t>(p.T) * p.nkv * p.num_splits;
   if (units > 0x7fffffff) return B200_ERR_INVALID_ARGUMENT;
-  int rc = launch_pdl(paged_attention_kernel<DK, DV, FORM>, dim3(static_cast<unsigned>(units)), dim3(kThreads), C::kSmemBytes,
-                      stream, *mk, *mv, p);
+  int rc = p.G <= 8 ? launch_rows<DK, DV, FORM, true>(p, mk, mv, static_cast<unsigned>(units), stream)
+                    : launch_rows<DK, DV, FORM, false>(p, mk, mv, static_cast<unsigned>(units), stream);
   if (rc != B200_OK) return rc;
   if (p.diff) return launch_diff_combine<__nv_bfloat16>(p, p.gate, p.out, DV, p.num_splits, stream);
   if (p.num_splits > 1) rc = launch_pdl(combine_kernel<DV>, dim3(p.T * p.nq), dim3(DV), 0, stream, p);
