@@ -190,6 +190,13 @@ __device__ __forceinline__ void store_output(const Params& p, int t, int head, i
   }
 }
 
+// 2^x; below the smallest normal number zero.
+__device__ __forceinline__ float exp2_fast(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // STACK: at most eight query heads a KV head, so rows 8 to 15 of the products are free.  The second term of P takes them: one product with V where two were, one
 // row of scores on a thread instead of two.  (The kernel moves bytes at the HBM rate, but the step runs at the power cap, where what the SMs do sets their clock
 // and with it the rate.  Both terms' sums are added when the warps' parts are.)
@@ -461,13 +468,14 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       }
       // ---- online softmax (log2 domain) ----
       float mx[2] = {-INFINITY, -INFINITY};
+      const bool edge = tok0 + r0 + 16 > end || (SEPARATE && tok0 + r0 < key_begin);  // of the keys that are seen
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt) {
 #pragma unroll
         for (int c = 0; c < 2 * kRows; ++c) {
           const int tok = tok0 + r0 + nt * 8 + tig * 2 + (c & 1);
           float v = EXTRA ? extra_score(p, sacc[nt][c], bias_r[c >> 1], new_pos - tok) : sacc[nt][c] * scale_log2;
-          if (tok >= end || (SEPARATE && tok < key_begin && !(EXTRA && tok < p.keep_first))) v = -INFINITY;
+          if (edge && (tok >= end || (SEPARATE && tok < key_begin && !(EXTRA && tok < p.keep_first)))) v = -INFINITY;
           sacc[nt][c] = v;
           mx[c >> 1] = fmaxf(mx[c >> 1], v);
         }
@@ -479,7 +487,7 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
         const float m_new = fmaxf(m_run[r], mx[r]);
         m_use[r] = (m_new == -INFINITY) ? 0.f : m_new;
-        alpha[r] = exp2f(m_run[r] - m_use[r]);
+        alpha[r] = exp2_fast(m_run[r] - m_use[r]);
         m_run[r] = m_new;
         l_run[r] *= alpha[r];
       }
@@ -494,7 +502,7 @@ paged_attention_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         for (int nt = 0; nt < 2; ++nt) {
 #pragma unroll
           for (int c = 0; c < 2 * kRows; ++c) {
-            pv[nt][c] = exp2f(sacc[nt][c] - m_use[c >> 1]);
+            pv[nt][c] = exp2_fast(sacc[nt][c] - m_use[c >> 1]);
             l_run[c >> 1] += pv[nt][c];
             pr[nt][c] = pv[nt][c] - bf16_round(pv[nt][c]);
           }

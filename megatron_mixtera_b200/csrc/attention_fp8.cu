@@ -36,7 +36,7 @@ constexpr int kQ8Bytes = 2 * 16 * kQ8Stride + 64;
 constexpr int kMergeBytes = kConsumerWarps * 16 * (D + 2) * 4;
 static_assert(kMergeBytes <= kStages * kStageBytes, "merge buffers reuse the tile ring");
 constexpr int kSmemBytes = kStages * kStageBytes + kQ16Bytes + 256 + kQ8Bytes + 1024;
-constexpr float kPScale = 256.f;            // P is multiplied by this before the E4M3 split
+constexpr float kPScaleLog2 = 8.f, kPScale = 256.f;  // P, and with it the sum of its row, is multiplied by this for the E4M3 split
 
 // Position inside a chunk at which token `tok`'s value bytes are stored (a permutation of every 32 tokens).
 // Slot 4t+e of a 16-token half holds token [2t, 2t+1, 8+2t, 9+2t][e]: what lane (., t) owns after S = Q K^T.
@@ -338,13 +338,14 @@ paged_attention_fp8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
       }
       // ---- online softmax (log2 domain) ----
       float mx[2] = {-INFINITY, -INFINITY};
+      const bool edge = tok0 + r0 + 32 > end;
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt) {
 #pragma unroll
         for (int c = 0; c < 2 * kRows; ++c) {
           const int tok = tok0 + r0 + nt * 8 + tig * 2 + (c & 1);
           float v = kStacked ? (sacc[nt][c] + sacc[nt][c + 2]) * row_scale[0] : sacc[nt][c] * row_scale[c >> 1];
-          if (tok >= end) v = -INFINITY;
+          if (edge && tok >= end) v = -INFINITY;
           sacc[nt][c] = v;
           mx[c >> 1] = fmaxf(mx[c >> 1], v);
         }
@@ -356,7 +357,8 @@ paged_attention_fp8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
         mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
         const float m_new = fmaxf(m_run[r], mx[r]);
         m_use[r] = (m_new == -INFINITY) ? 0.f : m_new;
-        alpha[r] = exp2f(m_run[r] - m_use[r]);
+        alpha[r] = attn::exp2_fast(m_run[r] - m_use[r]);
+        m_use[r] -= kPScaleLog2;
         m_run[r] = m_new;
         l_run[r] *= alpha[r];
       }
@@ -369,9 +371,8 @@ paged_attention_fp8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
         for (int nt = 0; nt < 4; ++nt) {
 #pragma unroll
           for (int c = 0; c < 2 * kRows; ++c) {
-            const float pv = exp2f(sacc[nt][c] - m_use[c >> 1]);
-            l_run[c >> 1] += pv;
-            const float ps = pv * kPScale;
+            const float ps = attn::exp2_fast(sacc[nt][c] - m_use[c >> 1]);
+            l_run[c >> 1] += ps;
             hi[nt][c] = round_to_e4m3_bits(ps);
             lo[nt][c] = ps - hi[nt][c];
           }
@@ -448,10 +449,10 @@ paged_attention_fp8_kernel(const __grid_constant__ CUtensorMap map_k, const __gr
   }
   if (tig == 0) {
     mm[warp * 16 + gid] = m_run[0];
-    ml[warp * 16 + gid] = l_run[0];
+    ml[warp * 16 + gid] = l_run[0] * (1.f / kPScale);
     if constexpr (kRows == 2) {
       mm[warp * 16 + gid + 8] = m_run[1];
-      ml[warp * 16 + gid + 8] = l_run[1];
+      ml[warp * 16 + gid + 8] = l_run[1] * (1.f / kPScale);
     }
   }
   consumer_barrier();
