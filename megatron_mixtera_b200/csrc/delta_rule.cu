@@ -7,7 +7,7 @@
 // [head][value channel][key channel].  Everything is fp32 from the loads on, two key channels per instruction (fma.f32x2); only
 // the linears' outputs (r, k, v, x_a, x_g, x_w1 / z) arrive in `dtype`.
 //
-//   delta_decode_kernel  one token per row; bound by reading and writing the state once.  A warp takes a (row, head) by itself,
+//   delta_decode_kernel  one token per row; bound by reading and writing the state once.  A warp takes a (row, head) by itself (few of them: two or four warps),
 //                        two columns per lane group at a time with the next two on their way; the CTA's warps - rows of one
 //                        head - share W_w2's rows in shared memory.  The product with W_w2, the decay, the unit key, the head
 //                        norm and the output gate are part of it.
@@ -190,14 +190,18 @@ __device__ __forceinline__ float dot16(const float* w, const float* l, float z) 
 }
 
 // Shared memory: per warp six vectors [DIM] and tanh(x_w1) [rank, rounded up]; then W_w2's rows of the head.
-template <typename T, int DIM>
+// PARTS warps share a (row, head): each takes every PARTS-th pass over the columns, and all prepare the token.
+template <typename T, int DIM, int PARTS>
 __global__ void __launch_bounds__(DecodeShape<DIM>::kWarps * 32, DIM <= 64 ? 1 : 2)
 delta_decode_kernel(b200_delta_args a, int w2_stride) {
   using D = DecodeShape<DIM>;
   constexpr int NI = D::NI, I = D::kI, N = D::kCols, EL = D::kElems, VEC = 16 / sizeof(T);
   extern __shared__ __align__(16) float dyn[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int head = blockIdx.x, dim = a.dim, row = blockIdx.y * D::kWarps + warp;
+  constexpr int kPasses = D::kPasses / PARTS;  // of a warp
+  static_assert(D::kPasses % PARTS == 0 && (kPasses == 1 || kPasses % 2 == 0), "");
+  const int head = blockIdx.x, dim = a.dim, row = blockIdx.y * (D::kWarps / PARTS) + warp / PARTS, part = warp % PARTS;
+  __shared__ float part_sq[D::kWarps];
   const bool full = dim == DIM;
   const int rank_pad = (a.rank + 3) / 4 * 4;
   float* vec = dyn + warp * (6 * DIM);  // r, w, k, u, a u, v (later o)
@@ -236,7 +240,7 @@ delta_decode_kernel(b200_delta_args a, int w2_stride) {
   };
   // The state was written by an earlier step (steps are separated by copies on the stream): fetch it before the wait.
   f32x2 cur[N][I / 2], ahead[N][I / 2];
-  fetch(cur, 0);
+  fetch(cur, part);
   float bias_w[EL], bias_a[EL], norm[EL];
 #pragma unroll
   for (int e = 0; e < EL; ++e) {
@@ -260,7 +264,7 @@ delta_decode_kernel(b200_delta_args a, int w2_stride) {
     xa[e] = p[a.off_a + i];
     xg[e] = p[a.off_g + i];
   }
-  fetch(ahead, 1);
+  if (kPasses > 1) fetch(ahead, part + PARTS);
 #pragma unroll
   for (int e = 0; e < 4; ++e)
     if (lane + e * 32 < a.rank) lora[lane + e * 32] = tanhf(simt::to_f32(xl[e]));
@@ -323,24 +327,34 @@ delta_decode_kernel(b200_delta_args a, int w2_stride) {
       }
     }
   };
-  if constexpr (D::kPasses == 1) {
-    run(cur, 0);
+  if constexpr (kPasses == 1) {
+    run(cur, part);
   } else {
 #pragma unroll 1
-    for (int pass = 0; pass < D::kPasses; pass += 2) {
-      run(cur, pass);
-      if (pass + 2 < D::kPasses) fetch(cur, pass + 2);
-      run(ahead, pass + 1);
-      if (pass + 3 < D::kPasses) fetch(ahead, pass + 3);
+    for (int k = 0; k < kPasses; k += 2) {
+      run(cur, part + k * PARTS);
+      if (k + 2 < kPasses) fetch(cur, part + (k + 2) * PARTS);
+      run(ahead, part + (k + 1) * PARTS);
+      if (k + 3 < kPasses) fetch(ahead, part + (k + 3) * PARTS);
     }
   }
-  const float inv = 1.f / sqrtf(warp_sum(osq) / dim + a.eps);
+  osq = warp_sum(osq);
+  if constexpr (PARTS > 1) {
+    if (lane == 0) part_sq[warp] = osq;
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / PARTS), "r"(32 * PARTS) : "memory");  // the warps of the row
+    osq = 0.f;
+#pragma unroll
+    for (int k = 0; k < PARTS; ++k) osq += part_sq[warp - part + k];
+  }
+  const float inv = 1.f / sqrtf(osq / dim + a.eps);
   __syncwarp();
   T* dst = static_cast<T*>(a.out) + row * hd + head * dim;
 #pragma unroll
   for (int e = 0; e < EL; ++e) {
     const int i = lane + e * 32;
-    if (i < dim) simt::store_as(dst + i, live ? vec[5 * DIM + i] * inv * norm[e] * gate_sigmoid(simt::to_f32(xg[e])) : 0.f);
+    if (e % PARTS != part) continue;
+    const int owner = i / (D::kGroups * N) % PARTS;  // the warp that had the column
+    if (i < dim) simt::store_as(dst + i, live ? vec[(owner - part) * 6 * DIM + 5 * DIM + i] * inv * norm[e] * gate_sigmoid(simt::to_f32(xg[e])) : 0.f);
   }
 }
 
@@ -932,11 +946,22 @@ static int launch_decode(const b200_delta_args& a, cudaStream_t s) {
     bytes += w2_bytes;
   else
     w2_stride = 0;  // read where it is used
-  static std::atomic<uint64_t> done{0};
   if (bytes > 200 * 1024) return B200_ERR_INVALID_ARGUMENT;
-  if (ensure_dynamic_smem(delta_decode_kernel<T, DIM>, 200 * 1024, done) != B200_OK) return B200_ERR_LAUNCH;
-  return launch_pdl(delta_decode_kernel<T, DIM>, dim3(a.heads, (a.num_rows + D::kWarps - 1) / D::kWarps), dim3(D::kWarps * 32), bytes,
-                    s, a, w2_stride);
+  auto go = [&](auto parts) {
+    constexpr int PARTS = decltype(parts)::value, kRows = D::kWarps / PARTS;
+    static std::atomic<uint64_t> done{0};
+    if (ensure_dynamic_smem(delta_decode_kernel<T, DIM, PARTS>, 200 * 1024, done) != B200_OK) return static_cast<int>(B200_ERR_LAUNCH);
+    return launch_pdl(delta_decode_kernel<T, DIM, PARTS>, dim3(a.heads, (a.num_rows + kRows - 1) / kRows), dim3(D::kWarps * 32), bytes, s, a, w2_stride);
+  };
+  if constexpr (D::kPasses >= 4) {
+    const int64_t tasks = static_cast<int64_t>(a.heads) * a.num_rows;
+    // Four warps for each of few tasks, two up to four tasks an SM; with more each of them has enough on its way, and the token would be prepared several times.
+    // us, one / two / four: 32 heads of 64, one row 4.8 / 3.7 / 3.3, 8 rows 7.2 / 4.8 / 4.2, 16 rows 7.3 / 5.1 / 8.1, 32 rows 9.3 / 12.3 / 18.5; 16 heads of 128, one row 12.3 /
+    // 7.8 / 5.9, 64 rows 27 / 30 / 37; two rows x 4 heads of 256 43.5 / 25.6 / 15.2.
+    if (tasks <= 2 * sm_count()) return go(std::integral_constant<int, 4>{});
+    if (tasks <= 4 * sm_count()) return go(std::integral_constant<int, 2>{});
+  }
+  return go(std::integral_constant<int, 1>{});
 }
 template <typename T>
 static int decode_by_dim(const b200_delta_args& a, cudaStream_t s) {

@@ -9,7 +9,7 @@
 // [head][value channel][key channel].  Delta's read-out after the write is rewritten over the state before it,
 // o = g S^T q + (q . k) u, so that both of its dot products run over the same registers in one pass.
 //
-//   decode_kernel  one token per row, a warp per (row, head), everything from the projections to the gated output
+//   decode_kernel  one token per row, one to four warps per (row, head), everything from the projections to the gated output
 //   scan_kernel    rows of any length, one CTA per (row, head, block of columns); other warps prepare the next 16 tokens
 //   wkv_block_scan_kernel  the same for Wkv with heads of 33 to 128, four tokens at a time
 //   finish_kernel  head norm, weight and gate behind the scan
@@ -284,17 +284,19 @@ struct ConvChannels {
 
 // Shared memory: per warp kVecs vectors [DIM], the values (later the outputs) [vpad], kScalars (8 floats); Wkv: lora [rank_pad] too,
 // then W_w2's rows of the head.
-template <typename T, typename Rule, int DIM, int TAPS>
+// PARTS warps share a (row, head): the first prepares the token, then each takes every PARTS-th pass over the columns.
+template <typename T, typename Rule, int DIM, int TAPS, int PARTS>
 __global__ void __launch_bounds__(DecodeShape<DIM>::kWarps * 32, DIM <= 64 ? 2 : DIM <= 128 ? 4 : 2)
 decode_kernel(b200_recurrence_args a, int vpad, int rank_pad, int w2_stride, bool vec_k, bool vec_v) {
   using D = DecodeShape<DIM>;
   constexpr int NI = D::NI, I = D::kI, N = D::kCols, EL = D::kElems, VEC = 16 / sizeof(T);
   extern __shared__ __align__(16) float dyn[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int head = blockIdx.x, dim = a.dim, vdim = a.vdim, row = blockIdx.y * D::kWarps + warp;
+  const int head = blockIdx.x, dim = a.dim, vdim = a.vdim, row = blockIdx.y * (D::kWarps / PARTS) + warp / PARTS, part = warp % PARTS;
+  __shared__ float part_sq[D::kWarps];
   const bool full = dim == DIM;
   const int per_warp = Rule::kVecs * DIM + vpad + 8 + rank_pad;
-  float* vec = dyn + warp * per_warp;
+  float* vec = dyn + warp / PARTS * per_warp;
   float* values = vec + Rule::kVecs * DIM;
   float* scalar = values + vpad;
   float* lora = scalar + 8;
@@ -337,7 +339,8 @@ decode_kernel(b200_recurrence_args a, int vpad, int rank_pad, int w2_stride, boo
   };
   // The state was written by an earlier step (steps are separated by copies on the stream): fetch it before the wait.
   f32x2 cur[N][I / 2], ahead[N][I / 2];
-  fetch(cur, 0);
+  fetch(cur, part);
+  float new_top = 0.f;  // (Memory)
   pdl_wait();
   const T* p = static_cast<const T*>(a.proj) + static_cast<int64_t>(min(row, a.num_rows - 1)) * a.proj_ld;
   if constexpr (Rule::kKind == B200_RECURRENCE_WKV) {
@@ -350,60 +353,66 @@ decode_kernel(b200_recurrence_args a, int vpad, int rank_pad, int w2_stride, boo
       load_channels<V, T, EL>(static_cast<const T*>(a.decay_bias) + head * dim, lane, dim, z);
       load_channels<V, T, EL>(static_cast<const T*>(a.bonus) + head * dim, lane, dim, bonus);
     };
-    if (vec_k)
-      fetch_token(std::true_type{});
-    else
-      fetch_token(std::false_type{});
-    clear_tail(r, lane, dim);
-    clear_tail(k, lane, dim);
-    for (int i = lane; i < a.rank; i += 32) lora[i] = simt::to_f32(lora_in[i]);
-    for (int i = lane; i < vdim; i += 32) values[i] = simt::to_f32(p[a.off_v + head * vdim + i]);
-    fetch(ahead, 1);
+    if (part == 0) {
+      if (vec_k)
+        fetch_token(std::true_type{});
+      else
+        fetch_token(std::false_type{});
+      clear_tail(r, lane, dim);
+      clear_tail(k, lane, dim);
+      for (int i = lane; i < a.rank; i += 32) lora[i] = simt::to_f32(lora_in[i]);
+      for (int i = lane; i < vdim; i += 32) values[i] = simt::to_f32(p[a.off_v + head * vdim + i]);
+    }
+    fetch(ahead, part + PARTS);
     if (w2_stride > 0) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();  // W_w2's rows (and, within the warp, lora)
-    if (w2_stride > 0) {
+    if (part == 0) {
+      if (w2_stride > 0) {
 #pragma unroll 2
-      for (int q = 0; q < a.rank; q += VEC)
+        for (int q = 0; q < a.rank; q += VEC)
 #pragma unroll
-        for (int e = 0; e < EL; ++e) z[e] = delta::dot16(w2_s + min(lane * EL + e, dim - 1) * w2_stride + q, lora + q, z[e]);
-    } else {
-      const T* w2 = static_cast<const T*>(a.w2) + static_cast<int64_t>(head) * dim * a.rank;
-      for (int q = 0; q < a.rank; ++q)
+          for (int e = 0; e < EL; ++e) z[e] = delta::dot16(w2_s + min(lane * EL + e, dim - 1) * w2_stride + q, lora + q, z[e]);
+      } else {
+        const T* w2 = static_cast<const T*>(a.w2) + static_cast<int64_t>(head) * dim * a.rank;
+        for (int q = 0; q < a.rank; ++q)
 #pragma unroll
-        for (int e = 0; e < EL; ++e)
-          z[e] = fmaf(simt::to_f32(w2[static_cast<int64_t>(min(lane * EL + e, dim - 1)) * a.rank + q]), lora[q], z[e]);
+          for (int e = 0; e < EL; ++e)
+            z[e] = fmaf(simt::to_f32(w2[static_cast<int64_t>(min(lane * EL + e, dim - 1)) * a.rank + q]), lora[q], z[e]);
+      }
+      put_wkv<DIM, EL>(vec, scalar, r, k, z, bonus, lane, dim);
     }
-    put_wkv<DIM, EL>(vec, scalar, r, k, z, bonus, lane, dim);
   } else if constexpr (Rule::kKind == B200_RECURRENCE_MEMORY) {
-    const int64_t t = min(row, a.num_rows - 1);
-    float q[EL], k[EL];
-    if (vec_k) {
-      load_channels<true, T, EL>(p + a.off_r + head * dim, lane, dim, q);
-      load_channels<true, T, EL>(p + a.off_k + head * dim, lane, dim, k);
-    } else {
-      load_channels<false, T, EL>(p + a.off_r + head * dim, lane, dim, q);
-      load_channels<false, T, EL>(p + a.off_k + head * dim, lane, dim, k);
-    }
-    clear_tail(q, lane, dim);
-    clear_tail(k, lane, dim);
-    for (int i = lane; i < vdim; i += 32) values[i] = simt::to_f32(p[a.off_v + head * vdim + i]);
-    const LogGates g = log_gates<T>(a, t, head);
-    const float before = in >= 0 ? a.top[static_cast<int64_t>(in) * a.heads + head] : 0.f, top = fmaxf(g.f + before, g.i);
-    const float write = expf(g.i - top), unit = 1.f / sqrtf(static_cast<float>(dim));
+    if (part == 0) {
+      const int64_t t = min(row, a.num_rows - 1);
+      float q[EL], k[EL];
+      if (vec_k) {
+        load_channels<true, T, EL>(p + a.off_r + head * dim, lane, dim, q);
+        load_channels<true, T, EL>(p + a.off_k + head * dim, lane, dim, k);
+      } else {
+        load_channels<false, T, EL>(p + a.off_r + head * dim, lane, dim, q);
+        load_channels<false, T, EL>(p + a.off_k + head * dim, lane, dim, k);
+      }
+      clear_tail(q, lane, dim);
+      clear_tail(k, lane, dim);
+      for (int i = lane; i < vdim; i += 32) values[i] = simt::to_f32(p[a.off_v + head * vdim + i]);
+      const LogGates g = log_gates<T>(a, t, head);
+      const float before = in >= 0 ? a.top[static_cast<int64_t>(in) * a.heads + head] : 0.f, top = fmaxf(g.f + before, g.i);
+      const float write = expf(g.i - top), unit = 1.f / sqrtf(static_cast<float>(dim));
 #pragma unroll
-    for (int e = 0; e < EL; ++e) {
-      vec[lane * EL + e] = q[e] * unit;
-      vec[DIM + lane * EL + e] = k[e] * write;
+      for (int e = 0; e < EL; ++e) {
+        vec[lane * EL + e] = q[e] * unit;
+        vec[DIM + lane * EL + e] = k[e] * write;
+      }
+      if (lane == 0) {
+        values[vdim] = 1.f;
+        scalar[0] = expf(g.f + before - top);
+        scalar[1] = expf(-top);
+      }
+      new_top = top;
     }
-    if (lane == 0) {
-      values[vdim] = 1.f;
-      scalar[0] = expf(g.f + before - top);
-      scalar[1] = expf(-top);
-      if (live) a.top[static_cast<int64_t>(out) * a.heads + head] = top;
-    }
-    fetch(ahead, 1);
+    fetch(ahead, part + PARTS);
   } else {
-    if (row < a.num_rows) {
+    if (row < a.num_rows && part == 0) {
       const int ratio = a.heads / a.kv_heads, kvh = head / ratio;
       const bool keep = head == kvh * ratio;  // one head of a group moves the group's query and key state on
       b200_conv_args c{};
@@ -465,9 +474,15 @@ decode_kernel(b200_recurrence_args a, int vpad, int rank_pad, int w2_stride, boo
       put_delta<DIM, EL, 1>(vec, 0, static_cast<int>(scalar - vec), q1, k1, lane, dim, a.unit_eps,
                             simt::to_f32(static_cast<const T*>(a.decay_rate)[head]), x_a, x_b);
     }
-    fetch(ahead, 1);
+    fetch(ahead, part + PARTS);
   }
-  __syncwarp();
+  auto row_sync = [&] {  // the warps of the row
+    if constexpr (PARTS == 1)
+      __syncwarp();
+    else
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / PARTS), "r"(32 * PARTS) : "memory");
+  };
+  row_sync();
   if (row >= a.num_rows) return;
   float osq = 0.f;
   auto run = [&](f32x2 (&s)[N][I / 2], int pass) {
@@ -492,22 +507,30 @@ decode_kernel(b200_recurrence_args a, int vpad, int rank_pad, int w2_stride, boo
   };
   const int passes = (cols + D::kGroups * N - 1) / (D::kGroups * N);
 #pragma unroll 1
-  for (int pass = 0; pass < passes; pass += 2) {
+  for (int pass = part; pass < passes; pass += 2 * PARTS) {
     run(cur, pass);
-    if (pass + 2 < passes) fetch(cur, pass + 2);
-    if (pass + 1 < passes) run(ahead, pass + 1);
-    if (pass + 3 < passes) fetch(ahead, pass + 3);
+    if (pass + 2 * PARTS < passes) fetch(cur, pass + 2 * PARTS);
+    if (pass + PARTS < passes) run(ahead, pass + PARTS);
+    if (pass + 3 * PARTS < passes) fetch(ahead, pass + 3 * PARTS);
   }
-  __syncwarp();
-  osq = warp_sum(osq) / vdim;
+  osq = warp_sum(osq);
+  if (PARTS > 1 && lane == 0) part_sq[warp] = osq;
+  row_sync();
+  if constexpr (PARTS > 1) {
+    osq = 0.f;
+#pragma unroll
+    for (int k = 0; k < PARTS; ++k) osq += part_sq[warp - part + k];
+  }
+  osq /= vdim;
   float inv = 1.f / sqrtf(osq + a.eps);
   if constexpr (Rule::kKind == B200_RECURRENCE_MEMORY) {
     const float unit = 1.f / memory_below(values[vdim], scalar[1]);
+    if (lane == 0 && part == 0 && live) a.top[static_cast<int64_t>(out) * a.heads + head] = new_top;
     inv = unit / sqrtf(osq * unit * unit + a.eps) * a.out_scale;
   }
   T* dst = static_cast<T*>(a.out) + (a.out_ld > 0 ? row * a.out_ld + head * vdim : (static_cast<int64_t>(row) * a.heads + head) * vdim);
   const T* weight = static_cast<const T*>(a.norm_weight) + (a.norm_per_head ? head * vdim : 0);
-  for (int i = lane; i < vdim; i += 32)
+  for (int i = part * 32 + lane; i < vdim; i += 32 * PARTS)
     simt::store_as(dst + i, live ? values[i] * inv * simt::to_f32(weight[i]) * output_gate<Rule>(simt::to_f32(p[a.off_g + head * vdim + i])) : 0.f);
 }
 
@@ -1200,16 +1223,31 @@ static int launch_decode(const b200_recurrence_args& a, cudaStream_t s) {
     vec_k = vec_k && aligned16(a.conv_filter) && aligned16(a.conv_state);
   const bool vec_v = vec_k && a.vdim % 4 == 0 && a.dim % 4 == 0;  // (then channels % 4 == 0)
   if (Rule::kKind == B200_RECURRENCE_DELTA) vec_k = vec_k && channels % EL == 0;
-  auto go = [&](auto taps) {
-    constexpr int TAPS = decltype(taps)::value;
+  auto go = [&](auto taps, auto parts) {
+    constexpr int TAPS = decltype(taps)::value, PARTS = decltype(parts)::value, kRows = D::kWarps / PARTS;
     static std::atomic<uint64_t> done{0};
-    if (ensure_dynamic_smem(decode_kernel<T, Rule, DIM, TAPS>, 200 * 1024, done) != B200_OK) return static_cast<int>(B200_ERR_LAUNCH);
-    return launch_pdl(decode_kernel<T, Rule, DIM, TAPS>, dim3(a.heads, (a.num_rows + D::kWarps - 1) / D::kWarps), dim3(D::kWarps * 32), bytes,
+    if (ensure_dynamic_smem(decode_kernel<T, Rule, DIM, TAPS, PARTS>, 200 * 1024, done) != B200_OK) return static_cast<int>(B200_ERR_LAUNCH);
+    return launch_pdl(decode_kernel<T, Rule, DIM, TAPS, PARTS>, dim3(a.heads, (a.num_rows + kRows - 1) / kRows), dim3(D::kWarps * 32), bytes,
                       s, a, vpad, rank_pad, w2_stride, vec_k, vec_v);
   };
+  const std::integral_constant<int, 1> one;
+  const std::integral_constant<int, 2> two;
+  const std::integral_constant<int, 4> four;
+  // A warp walks its columns a pass at a time, two passes' bytes on their way, so few (row, head) tasks are bound by that walk: four warps for each up to four tasks
+  // an SM, two up to eight and, with more than 64 channels, with any number.  us, one / two / four: memory, 16 heads of 128, one row 13.1 / 8.5 / 6.0, 32 rows 27.7 /
+  // 18.9 / 15.4, 64 rows 32.5 / 27.8 / 28.2, 200 rows 76.8 / 74.9 / 79.3; delta, 16 heads of 128, 8 rows 19.6 / 12.3 / 11.9, 64 rows 44.5 / 33.8 / 35.8; wkv, 32 heads of
+  // 64, 16 rows 10.7 / 7.2 / 5.9, 32 rows 15.0 / 10.2 / 14.2, 40 rows 16.2 / 17.7 / 21.0.  (32 channels are one pass.)
+  auto by_parts = [&](auto taps) {
+    if constexpr (DIM > 32) {
+      const int64_t tasks = static_cast<int64_t>(a.heads) * a.num_rows;
+      if (tasks <= 4 * sm_count()) return go(taps, four);
+      if (tasks <= 8 * sm_count() || DIM > 64) return go(taps, two);
+    }
+    return go(taps, one);
+  };
   if constexpr (Rule::kKind == B200_RECURRENCE_DELTA)
-    if (a.taps > 4) return go(std::integral_constant<int, 8>{});
-  return go(std::integral_constant<int, 4>{});
+    if (a.taps > 4) return by_parts(std::integral_constant<int, 8>{});
+  return by_parts(four);
 }
 template <typename T, typename Rule>
 static int decode_by_dim(const b200_recurrence_args& a, cudaStream_t s) {

@@ -82,6 +82,62 @@ def test_wkv_rows_that_end_inside_a_block(heads, dim, dtype):
         assert all(close(g, x, dtype) for g, x in zip(got, want)), schedule
 
 
+@pytest.mark.parametrize("kind", ["wkv", "delta", "memory"])
+@pytest.mark.parametrize("dim", [64, 48, 128])
+def test_recurrent_decode_shares_a_row_between_warps(kind, dim):
+    """One, two or four warps for a (row, head), by how many there are: the states are the same bits whichever takes a row, outputs up to the order of a head
+    norm's sum (bf16: one rounding apart)."""
+    from megatron_mixtera_b200 import _lib, ops
+
+    heads, most, rank, splits = 16, 90, 24, 3
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(11)
+
+    def r(*shape, scale=1.0):
+        return torch.randn(*shape, generator=g, device="cuda") * scale
+
+    def b(*shape, scale=1.0):
+        return r(*shape, scale=scale).bfloat16()
+
+    n, kv = heads * dim, heads // 2
+    channels = 2 * kv * dim + n
+    width = {"wkv": 4 * n, "memory": 4 * n, "delta": channels + n + 2 * heads}[kind]
+    x = dict(proj=b(most, width), norm=b(n), state0=r(2 * most, heads, dim + (kind == "memory"), dim, scale=0.3), top0=r(2 * most, heads), bias=b(max(n, 2 * heads)),
+             z=r(splits, most, 2 * heads), lora=b(most, rank), w2=b(n, rank, scale=rank ** -0.5), bonus=b(n), rate=b(heads), filter=b(4, channels, scale=0.4),
+             conv0=b(2 * most, 3, channels))
+    found = {}
+    for rows_ in (most, max(2, 5 * sms // heads), 3):
+        state, top, conv = x["state0"].clone(), x["top0"].clone(), x["conv0"].clone()
+        at = torch.arange(rows_, dtype=torch.int32, device="cuda")
+        rd, wr = at, at + most
+        out = torch.zeros(rows_, n, dtype=torch.bfloat16, device="cuda")
+        z = x["z"][:, :rows_].contiguous()
+        a = _lib.RecurrenceArgs()
+        a.kind = {"wkv": 0, "delta": 1, "memory": 2}[kind]
+        a.heads, a.kv_heads, a.dim, a.vdim, a.num_tokens, a.num_rows, a.norm_per_head = heads, kv if kind == "delta" else heads, dim, dim, rows_, rows_, int(kind != "delta")
+        a.proj, a.proj_ld, a.decay_bias, a.norm_weight, a.out = x["proj"].data_ptr(), width, x["bias"].data_ptr(), x["norm"].data_ptr(), out.data_ptr()
+        a.off_r, a.off_k, a.off_v, a.off_g = 0, n, 2 * n, 3 * n
+        if kind == "wkv":
+            a.lora, a.rank, a.w2, a.bonus = x["lora"].data_ptr(), rank, x["w2"].data_ptr(), x["bonus"].data_ptr()
+        elif kind == "memory":
+            a.z, a.z_splits, a.z_ld, a.top, a.gate_cap, a.out_scale = z.data_ptr(), splits, 2 * heads, top.data_ptr(), 15.0, 1.0
+        else:
+            a.off_g, a.off_b, a.off_a = channels, channels + n, channels + n + heads
+            a.decay_rate, a.conv_filter, a.conv_state, a.taps = x["rate"].data_ptr(), x["filter"].data_ptr(), conv.data_ptr(), 4
+        a.state, a.state_in, a.state_out, a.state_slots = state.data_ptr(), rd.data_ptr(), wr.data_ptr(), 2 * most
+        a.dtype, a.unit_eps, a.eps = ops.dtype_code(torch.bfloat16), 1e-6, 1e-5
+        ops.struct_kernel("recurrence_decode", a, state)
+        found[rows_] = (out, state[most: most + rows_], top[most: most + rows_], conv[most: most + rows_])
+        assert torch.equal(state[:most], x["state0"][:most]) and torch.equal(state[most + rows_:], x["state0"][most + rows_:])
+        assert bool(out.float().isfinite().all()) and float(out.float().abs().max()) > 0
+    sizes = sorted(found)
+    for few, many in zip(sizes, sizes[1:]):
+        a, b_ = found[few], found[many]
+        assert all(torch.equal(u, v[:few]) for u, v in zip(a[1:], b_[1:]))
+        d = (a[0].float() - b_[0][:few].float()).abs()
+        assert bool((d <= 2.0 ** -7 * a[0].float().abs() + 1e-6).all())
+
+
 @pytest.mark.parametrize("kind", list(MIXERS))
 def test_recurrent_state_after_a_portion(kind):
     """The state itself, and that a padding row or another request's slot is left alone."""

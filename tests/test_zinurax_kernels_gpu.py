@@ -417,6 +417,34 @@ def test_delta_decode(dtype, heads, dim, rank):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dim", [64, 48, 128])
+def test_delta_decode_shares_a_row_between_warps(dtype, dim):
+    """One, two or four warps for a (row, head), by how many there are: the same states, outputs up to the order of the head norm's sum."""
+    from megatron_mixtera_b200 import ops
+
+    heads, most = 16, 60
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    c = DeltaCase(heads, dim, 8, most, dtype, seed=60)
+    state = rand(2 * most, heads, dim, dim, seed=61)
+    found = {}
+    for n in (most, 3 * sms // heads, 2):
+        d_state, at = state.to(DEV), torch.arange(n, dtype=torch.int32, device=DEV)
+        rd, wr = at, at + most
+        out = torch.empty(n, c.n, dtype=dtype, device=DEV)
+        a = c.args(d_state, rd, wr, out)
+        a.num_tokens = a.num_rows = n
+        ops.delta_decode(a, d_state)
+        found[n] = (out, d_state[most: most + n])
+        assert torch.equal(d_state[:most].cpu(), state[:most]) and torch.equal(d_state[most + n:].cpu(), state[most + n:])
+    sizes = sorted(found)
+    for few, many in zip(sizes, sizes[1:]):
+        (a, s), (b, t) = found[few], found[many]
+        assert torch.equal(s, t[:few])
+        step = 2.0 ** -7 if dtype == torch.bfloat16 else 1e-5
+        assert bool(((a.float() - b[:few].float()).abs() <= step * a.float().abs() + 1e-6).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,dim,rank", DELTA_SHAPES)
 def test_delta_scan(dtype, heads, dim, rank):
     """Rows of 1, 2, 16, 17 and 40 tokens and an empty one in one launch, some continuing from a state."""
