@@ -135,7 +135,8 @@ route_kernel(b200_moe_args a) {
 
 // Softmax over experts and identity experts, choice by score + correction inside the best groups.  CHOSEN: scores are the logits plus a
 // bias, and the weights the softmax over the chosen ones.
-// Shared memory: [kWarps][columns + groups] scores and the groups' best choice scores.
+// Shared memory: [kWarps][2 columns + groups] scores, what the choice goes by, and the best of each group.  (A chain of short steps for a token.  With the corrections
+// read from memory at each step and a group's best found by one lane: 5952 tokens, 64 columns 42 us, 34 now; 64 tokens, 34 columns in 2 groups 10.5, 9.9.)
 template <typename T, bool CHOSEN>
 __global__ void __launch_bounds__(kWarps * 32)
 route_softmax_kernel(b200_moe_args a) {
@@ -149,16 +150,20 @@ route_softmax_kernel(b200_moe_args a) {
   const int t = blockIdx.x * kWarps + warp;
   const T* correction = static_cast<const T*>(a.correction);
   if (t < a.num_tokens) {
-    float* score = score_s + warp * (C + a.groups);
-    float* group_best = score + C;
+    float* score = score_s + warp * (2 * C + a.groups);
+    float* pick = score + C;  // minus infinity: can no longer be chosen
+    float* group_best = pick + C;
     const int64_t stride = static_cast<int64_t>(a.num_tokens) * a.router_ld;
     const float* z = a.router + static_cast<int64_t>(t) * a.router_ld;
     float top = -INFINITY, sum = 0.f;
     for (int e = lane; e < C; e += 32) {
       float x = 0.f;
+      const float more = simt::to_f32(correction[e]);
+#pragma unroll 8
       for (int s = 0; s < a.router_splits; ++s) x += z[s * stride + e];
-      if (CHOSEN) x += simt::to_f32(correction[e]);
+      if (CHOSEN) x += more;
       score[e] = x;
+      pick[e] = CHOSEN ? x : more;
       top = fmaxf(top, x);
     }
     top = warp_max(top);
@@ -168,12 +173,11 @@ route_softmax_kernel(b200_moe_args a) {
         sum += score[e];
       }
       sum = warp_sum(sum);
-      for (int e = lane; e < C; e += 32) score[e] /= sum;
+      for (int e = lane; e < C; e += 32) {
+        score[e] /= sum;
+        pick[e] += score[e];
+      }
     }
-    auto choice = [&](int e) {
-      if (CHOSEN) return score[e];
-      return score[e] < 0.f ? -INFINITY : score[e] + simt::to_f32(correction[e]);  // (negative: marked)
-    };
     // The largest of f over [0, n), the smallest index among equals (n: nothing above minus infinity).
     auto best_of = [&](int n, auto f) {
       float best = -INFINITY;
@@ -199,10 +203,11 @@ route_softmax_kernel(b200_moe_args a) {
     __syncwarp();
     if (a.groups > 1) {
       const int size = C / a.groups;
-      for (int g = lane; g < a.groups; g += 32) {
+      for (int g = 0; g < a.groups; ++g) {
         float m = -INFINITY;
-        for (int e = g * size; e < (g + 1) * size; ++e) m = fmaxf(m, choice(e));
-        group_best[g] = m;
+        for (int e = g * size + lane; e < (g + 1) * size; e += 32) m = fmaxf(m, pick[e]);
+        m = warp_max(m);
+        if (lane == 0) group_best[g] = m;
       }
       __syncwarp();
       for (int k = 0; k < a.keep_groups; ++k) {
@@ -212,12 +217,15 @@ route_softmax_kernel(b200_moe_args a) {
         __syncwarp();
       }
       for (int e = lane; e < C; e += 32)
-        if (group_best[e / size] != INFINITY) score[e] = kTaken;
+        if (group_best[e / size] != INFINITY) {
+          score[e] = kTaken;
+          pick[e] = -INFINITY;
+        }
       __syncwarp();
     }
     float total = 0.f;
     for (int k = 0; k < a.top; ++k) {
-      int at = best_of(C, choice);
+      int at = best_of(C, [&](int i) { return pick[i]; });
       if (at >= C) at = k;  // no number left (NaN scores): any expert, its output is NaN too
       const float s = CHOSEN ? expf(score[at] - top) : score[at];
       __syncwarp();
@@ -225,6 +233,7 @@ route_softmax_kernel(b200_moe_args a) {
         chosen_s[warp][k] = at;
         weight_s[warp][k] = s;
         score[at] = kTaken;
+        pick[at] = -INFINITY;
       }
       total += s;
       __syncwarp();
@@ -413,12 +422,12 @@ int b200_moe_route(const b200_moe_args* a, b200_stream_t stream) {
     if (a->identity < 0 || columns > moe::kMaxExperts || a->router_ld < columns || !a->correction || a->shared_gate || groups < 1 ||
         columns % groups != 0 || a->keep_groups < 1 || a->keep_groups > groups || a->top > columns / groups * a->keep_groups)
       return B200_ERR_INVALID_ARGUMENT;
-    const size_t bytes = static_cast<size_t>(moe::kWarps) * (columns + groups) * 4;
+    const size_t bytes = static_cast<size_t>(moe::kWarps) * (2 * columns + groups) * 4;
     auto go = [&](auto zero, auto CHOSEN) {
       using T = decltype(zero);
       static std::atomic<uint64_t> done{0};
       auto kernel = moe::route_softmax_kernel<T, CHOSEN.value>;
-      if (ensure_dynamic_smem(kernel, moe::kWarps * 2 * moe::kMaxExperts * 4, done) != B200_OK) return static_cast<int>(B200_ERR_LAUNCH);
+      if (ensure_dynamic_smem(kernel, moe::kWarps * 3 * moe::kMaxExperts * 4, done) != B200_OK) return static_cast<int>(B200_ERR_LAUNCH);
       return launch_pdl(kernel, dim3(blocks), dim3(moe::kWarps * 32), bytes, reinterpret_cast<cudaStream_t>(stream), *a);
     };
     if (a->plain == 2) return a->dtype == B200_DTYPE_F32 ? go(0.f, std::true_type{}) : go(__nv_bfloat16{}, std::true_type{});
