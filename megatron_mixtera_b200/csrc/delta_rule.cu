@@ -855,49 +855,48 @@ delta_block_scan_kernel(b200_delta_args a) {
   }
 }
 
-// A warp per (token, head), four of them in turn with all their loads in flight.
+// kFinishUnits (token, head) units in turn with all their loads in flight: LPH lanes of four channels each, in vectors, or (LPH == 0) a warp and any size.  Bound by
+// the bytes in flight: 6208 tokens x 32 heads of 64 55 us with a warp and single channels for each, 20 in vectors (floor 15).
 constexpr int kFinishUnits = 4;
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <typename T, int LPH>
+__global__ void __launch_bounds__(256, LPH > 0 ? 4 : 1)
 delta_finish_kernel(b200_delta_args a) {
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31, dim = a.dim;
+  const int dim = a.dim;
   const uint32_t total = static_cast<uint32_t>(a.num_tokens) * a.heads, heads = a.heads;  // (the launch checks that it fits)
-  const uint32_t first = (blockIdx.x * 8 + (threadIdx.x >> 5)) * kFinishUnits;
   const T* proj = static_cast<const T*>(a.proj);
   const T* weight = static_cast<const T*>(a.norm_weight);
   T* out = static_cast<T*>(a.out);
-  if (dim <= 128) {  // heads in registers
-    float v[kFinishUnits][4], w[kFinishUnits][4];
-    T g[kFinishUnits][4];
+  if constexpr (LPH > 0) {
+    constexpr int kGroups = 256 / LPH;
+    const int lane = threadIdx.x % LPH, i = min(lane * 4, dim - 4);
+    const uint32_t first = blockIdx.x * kGroups * kFinishUnits + threadIdx.x / LPH;  // then kGroups apart
+    float v[kFinishUnits][4], g[kFinishUnits][4], w[kFinishUnits][4];
 #pragma unroll
     for (int k = 0; k < kFinishUnits; ++k) {
-      const uint32_t unit = min(first + k, total - 1), t = unit / heads;
+      const uint32_t unit = min(first + k * kGroups, total - 1), t = unit / heads;
       const int at = static_cast<int>(unit - t * heads) * dim;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (e * 32 >= dim) break;
-        const int i = min(lane + e * 32, dim - 1);
-        v[k][e] = a.o_f32[static_cast<int64_t>(unit) * dim + i];
-        g[k][e] = proj[t * a.proj_ld + a.off_g + at + i];
-        w[k][e] = simt::to_f32(weight[at + i]);
-      }
+      conv::load<float, 4>(a.o_f32 + static_cast<int64_t>(unit) * dim + i, v[k]);
+      conv::load<T, 4>(proj + t * a.proj_ld + a.off_g + at + i, g[k]);
+      conv::load<T, 4>(weight + at + i, w[k]);
     }
 #pragma unroll
     for (int k = 0; k < kFinishUnits; ++k) {
-      float sq = 0.f;
+      float sq = lane * 4 < dim ? v[k][0] * v[k][0] + v[k][1] * v[k][1] + v[k][2] * v[k][2] + v[k][3] * v[k][3] : 0.f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) sq += lane + e * 32 < dim ? v[k][e] * v[k][e] : 0.f;
-      const float inv = 1.f / sqrtf(warp_sum(sq) / dim + a.eps);
+      for (int o = LPH / 2; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      const uint32_t unit = first + k * kGroups;
+      const float inv = 1.f / sqrtf(sq / dim + a.eps);
+      float y[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (lane + e * 32 < dim && first + k < total)
-          simt::store_as(out + static_cast<int64_t>(first + k) * dim + lane + e * 32,
-                         v[k][e] * inv * w[k][e] * gate_sigmoid(simt::to_f32(g[k][e])));
+      for (int e = 0; e < 4; ++e) y[e] = v[k][e] * inv * w[k][e] * gate_sigmoid(g[k][e]);
+      if (lane * 4 < dim && unit < total) conv::store<T, 4>(out + static_cast<int64_t>(unit) * dim + i, y);
     }
     return;
   }
+  const int lane = threadIdx.x & 31;
+  const uint32_t first = (blockIdx.x * 8 + (threadIdx.x >> 5)) * kFinishUnits;
   for (int k = 0; k < kFinishUnits; ++k) {
     const int64_t unit = first + k;
     if (unit >= total) return;
@@ -1045,10 +1044,18 @@ int b200_delta_finish(const b200_delta_args* a, b200_stream_t stream) {
   using namespace b200;
   if (!delta::valid_common(a) || !a->o_f32 || !a->norm_weight || !a->out || static_cast<int64_t>(a->num_tokens) * a->heads > (1u << 30))
     return B200_ERR_INVALID_ARGUMENT;
-  const unsigned blocks = static_cast<unsigned>((static_cast<int64_t>(a->num_tokens) * a->heads + 8 * delta::kFinishUnits - 1) / (8 * delta::kFinishUnits));
+  const bool vec = a->dim % 4 == 0 && a->dim <= 128 && a->proj_ld % 4 == 0 && a->off_g % 4 == 0 && aligned16(a->proj) && aligned16(a->o_f32) && aligned16(a->norm_weight) &&
+                   aligned16(a->out);
+  const int lanes = !vec ? 0 : a->dim <= 64 ? 16 : 32, per_block = (lanes ? 256 / lanes : 8) * delta::kFinishUnits;
+  const dim3 grid(static_cast<unsigned>((static_cast<int64_t>(a->num_tokens) * a->heads + per_block - 1) / per_block));
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (a->dtype == B200_DTYPE_F32) return launch_pdl(delta::delta_finish_kernel<float>, dim3(blocks), dim3(256), 0, s, *a);
-  return launch_pdl(delta::delta_finish_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, s, *a);
+  auto go = [&](auto zero) {
+    using T = decltype(zero);
+    if (lanes == 16) return launch_pdl(delta::delta_finish_kernel<T, 16>, grid, dim3(256), 0, s, *a);
+    if (lanes == 32) return launch_pdl(delta::delta_finish_kernel<T, 32>, grid, dim3(256), 0, s, *a);
+    return launch_pdl(delta::delta_finish_kernel<T, 0>, grid, dim3(256), 0, s, *a);
+  };
+  return a->dtype == B200_DTYPE_F32 ? go(0.f) : go(__nv_bfloat16{});
 }
 
 }  // extern "C"
