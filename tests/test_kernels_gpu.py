@@ -665,6 +665,37 @@ def test_paged_attention_fp8_pool(ops, nkv, G, chunk, kv_lens, splits, fused, si
     assert rel_l2(o, ref) < (6e-2 if single_term else 6e-3), rel_l2(o, ref)
 
 
+@pytest.mark.parametrize("nkv,G,D", [(2, 8, 128), (4, 4, 64), (6, 3, 64)])
+@pytest.mark.parametrize("recipe", [None, "mxfp8", "blockwise"])
+def test_splits_of_many_rows_merge_as_those_of_few(ops, nkv, G, D, recipe):
+    # many heads share a CTA's merge in fours (18 heads do not): the same sums in the same order, so the same bits as a part of the rows alone
+    if recipe == "blockwise" and D != 128:
+        pytest.skip("the 128-block recipe takes one scale per head of 128 dims")
+    lens = [0, 1, 64, 65, 200, 257, 320, 385]  # 0 to 6 splits of 64 tokens and more
+    T = 3 * 1024 // (nkv * G) // 8 * 8
+    c = make_paged_case(T=T, nkv=nkv, G=G, D=D, chunk=64, kv_lens=[lens[r * 5 % 8] for r in range(T)], seed=7)
+    cos, sin = (f(c["freqs"][:, : D // 2]).to(BF16).cuda() for f in (torch.cos, torch.sin))
+
+    def run(n):
+        kc, vc = c["k_cache"].cuda(), c["v_cache"].cuda()
+        d = {k: c[k][:n].contiguous().cuda() for k in ("qkv", "block_table", "kv_lens", "pos", "chunk_idx", "local")}
+        out = torch.zeros((n, c["nq"] * D), dtype=BF16, device="cuda")
+        quantised = None if recipe is None else ops.quantized_like(recipe, n, c["nq"] * D, "cuda")
+        ops.paged_attention(ops.make_attention_args(
+            qkv=d["qkv"], k_cache=kc, v_cache=vc, block_table=d["block_table"], kv_seq_lengths=d["kv_lens"], out=out, num_q_heads=c["nq"],
+            num_kv_heads=nkv, head_dim=D, chunk_size=c["chunk"], token_to_pos_ids=d["pos"], token_to_pos_in_request=d["pos"],
+            token_to_chunk_idx=d["chunk_idx"], token_to_local_pos=d["local"], rope_cos=cos, rope_sin=sin, num_splits=6, fuse_rope_append=True,
+            out_quantized=quantised))
+        torch.cuda.synchronize()
+        if quantised is None:
+            return [out.cpu()]
+        return [quantised.q[:n].view(torch.uint8).cpu()] + ([quantised.scale[:, :n].t().cpu()] if recipe == "blockwise" else [])
+
+    for many, few in zip(run(T), run(16)):
+        assert torch.equal(many[:16], few[:16]) and not torch.isnan(many.float()).any()
+    assert recipe is not None or bool((run(T)[0][0] == 0).all())
+
+
 @pytest.mark.parametrize("shards,vocab", [(2, 1000), (8, 128256), (4, 4096)])
 def test_shardwise_argmax_equals_argmax_of_the_gathered_rows(ops, shards, vocab):
     rows = 37
