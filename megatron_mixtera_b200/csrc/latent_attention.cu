@@ -924,12 +924,14 @@ latent_umma_kernel(const __grid_constant__ CUtensorMap map, b200_latent_args a, 
   if (warp == 0) tmem_dealloc(tmem, tmem_cols);
 }
 
-// One CTA per (token, head): merge the splits' normalised partial outputs by their log-sum-exp.
+// One CTA per (token, head): merge the splits' normalised partial outputs by their log-sum-exp.  A lane has two splits' weights, and the values of four splits (VEC
+// columns of them a thread) are on their way while those are found: bound by latency, one request of 700 tokens with 16 heads 6.0 -> 2.6 us.
+template <int VEC>
 __global__ void __launch_bounds__(128)
 latent_combine_kernel(b200_latent_args a) {
   pdl_launch_dependents();
   const int64_t pair = blockIdx.x;
-  const int t = static_cast<int>(pair / a.heads);
+  const int t = static_cast<int>(pair / a.heads), head = static_cast<int>(pair - static_cast<int64_t>(t) * a.heads), lane = threadIdx.x & 31;
   const int kv_len = a.kv_seq_lengths[t];
   pdl_wait();
   if (kv_len <= 0) return;
@@ -937,18 +939,43 @@ latent_combine_kernel(b200_latent_args a) {
   const int len = split_length(keys, a.num_splits);
   const int used = min(a.num_splits, (keys + len - 1) / len);
   const float* lse = a.workspace + static_cast<int64_t>(a.num_tokens) * a.heads * a.num_splits * a.kv_rank + pair * a.num_splits;
-  float m = -INFINITY, total = 0.f;
-  for (int s = 0; s < used; ++s) m = fmaxf(m, lse[s]);
-  for (int s = 0; s < used; ++s) total += exp2f(lse[s] - m);
-  const int head = static_cast<int>(pair % a.heads);
-  const float g = gate_of<__nv_bfloat16>(a, t, head) / (total + sink_weight(a, head, m));
   const float* part = a.workspace + pair * a.num_splits * a.kv_rank;
   __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.out) + pair * a.kv_rank;
-  for (int c = threadIdx.x; c < a.kv_rank; c += blockDim.x) {
-    float acc = 0.f;
-    for (int s = 0; s < used; ++s) acc += exp2f(lse[s] - m) * part[static_cast<int64_t>(s) * a.kv_rank + c];
-    dst[c] = __float2bfloat16_rn(acc * g);
+  constexpr int kAtOnce = 4;
+  float v[kAtOnce][VEC];
+  auto fetch = [&](int s0, int c) {
+#pragma unroll
+    for (int j = 0; j < kAtOnce; ++j)
+      if (s0 + j < used && c < a.kv_rank) conv::load<float, VEC>(part + static_cast<int64_t>(s0 + j) * a.kv_rank + c, v[j]);
+  };
+  fetch(0, threadIdx.x * VEC);
+  const float l0 = lane < used ? lse[lane] : -INFINITY, l1 = lane + 32 < used ? lse[lane + 32] : -INFINITY;
+  const float gate = gate_of<__nv_bfloat16>(a, t, head), m = warp_max(fmaxf(l0, l1));
+  const float w0 = lane < used ? exp2f(l0 - m) : 0.f, w1 = lane + 32 < used ? exp2f(l1 - m) : 0.f;
+  const float g = gate / (warp_sum(w0 + w1) + sink_weight(a, head, m));
+  for (int first = 0; first < a.kv_rank; first += 128 * VEC) {  // the same turns for a whole warp
+    const int c = first + threadIdx.x * VEC;
+    float acc[VEC] = {};
+    for (int s0 = 0; s0 < used; s0 += kAtOnce) {
+      if (first > 0 || s0 > 0) fetch(s0, c);
+#pragma unroll
+      for (int j = 0; j < kAtOnce; ++j) {
+        const int s = s0 + j;
+        const float w = __shfl_sync(0xffffffffu, s < 32 ? w0 : w1, s & 31);
+        if (s < used)
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) acc[e] = fmaf(w, v[j][e], acc[e]);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) acc[e] *= g;
+    if (c < a.kv_rank) conv::store<__nv_bfloat16, VEC>(dst + c, acc);
   }
+}
+static int launch_combine(const b200_latent_args& a, cudaStream_t s) {
+  const bool vec = a.kv_rank % 4 == 0 && aligned16(a.workspace) && aligned16(a.out);
+  return vec ? launch_pdl(latent_combine_kernel<4>, dim3(a.num_tokens * a.heads), dim3(128), 0, s, a)
+             : launch_pdl(latent_combine_kernel<1>, dim3(a.num_tokens * a.heads), dim3(128), 0, s, a);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -1308,7 +1335,7 @@ static int launch_umma(const b200_latent_args& a, cudaStream_t s) {
   const int rc = launch_pdl(latent_umma_kernel<N>, grid, dim3(UmmaShape<N>::kThreads), UmmaShape<N>::bytes(a.row_width, a.kv_pad, stages), s, *map,
                             a, stages, cols);
   if (rc != B200_OK || a.num_splits == 1) return rc;
-  return launch_pdl(latent_combine_kernel, dim3(a.num_tokens * a.heads), dim3(128), 0, s, a);
+  return launch_combine(a, s);
 }
 
 namespace prompt {  // long prompts (latent_prompt.cu)
@@ -1342,7 +1369,7 @@ static int launch_decode(const b200_latent_args& a, cudaStream_t s) {
   const int rc = launch_pdl(latent_decode_kernel<KVT>, dim3(a.num_tokens, 1, a.num_splits), dim3(kThreads),
                             D::fixed_bytes() + stages * D::stage_bytes(rs), s, a, stages);
   if (rc != B200_OK || a.num_splits == 1) return rc;
-  return launch_pdl(latent_combine_kernel, dim3(a.num_tokens * a.heads), dim3(128), 0, s, a);
+  return launch_combine(a, s);
 }
 
 }  // namespace latent

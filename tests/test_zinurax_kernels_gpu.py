@@ -205,6 +205,28 @@ def test_latent_decode_attention(dtype, shape):
         compare(out[:-1], want, dtype)
 
 
+@pytest.mark.parametrize("kv_rank,rot,heads", [(512, 64, 16), (640, 64, 4), (72, 24, 40)])
+def test_latent_decode_merges_more_splits_than_a_warp_has_lanes(kv_rank, rot, heads):
+    from megatron_mixtera_b200 import ops
+
+    lengths = [2624, 70, 2049, 1]  # 41, 2, 33 splits and one
+    pg = Paged(lengths, kv_rank, rot, heads, None, torch.bfloat16, seed=4)
+    T = len(lengths)
+    q = rand(T, heads, kv_rank + rot, seed=19, dtype=torch.bfloat16) * 0.1
+    for i, n in enumerate(lengths):
+        for h, key in enumerate([n - 1, 0, 2048, 31 * 64]):  # the last split, the first, the 33rd, the 32nd
+            if key < n:
+                stand_out(pg, q[i], i, n - 1, key, h)
+    gates = rand(T, heads, seed=20, dtype=torch.bfloat16)
+    want = torch.stack([pg.want(q[i], i, n - 1) for i, n in enumerate(lengths)]) * torch.sigmoid(gates.double())[:, :, None]
+    pool, qf, g, kv_len = pg.pool(), pg.padded(q).to(DEV), gates.to(DEV), torch.tensor(lengths, dtype=torch.int32, device=DEV)
+    out = torch.empty(T, heads, kv_rank, dtype=torch.bfloat16, device=DEV)
+    a = pg.args(T, qf, pool, g, out)
+    a.kv_seq_lengths, a.num_splits = kv_len.data_ptr(), 41
+    ops.latent_attention(a, pool)
+    compare(out, want, torch.bfloat16)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape", SHAPES)
 def test_latent_prompt_attention(dtype, shape):
