@@ -668,11 +668,12 @@ delta_block_scan_kernel(b200_delta_args a) {
       const float root = 1.f / sqrtf((lane & 2 ? lane & 1 ? sums[3] : sums[2] : lane & 1 ? sums[1] : sums[0]) + a.unit_eps);
 #pragma unroll
       for (int q = 0; q < J; ++q) {
+        const bool live = c * Sh::kTokens + warp * J + q < n_tok;  // (past the end: zeros whatever the root of unit_eps is)
         const float unit = __shfl_sync(0xffffffffu, root, q);
 #pragma unroll
         for (int e = 0; e < EL; ++e) {
-          u[q][e] = k[q][e] * unit;
-          au[q][e] *= u[q][e];
+          u[q][e] = live ? k[q][e] * unit : 0.f;
+          au[q][e] = live ? au[q][e] * u[q][e] : 0.f;
         }
       }
       float pairs[32];

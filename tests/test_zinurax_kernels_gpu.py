@@ -536,6 +536,37 @@ def test_delta_scan_of_long_rows(dtype, heads, dim):
     assert bool((o_f32[T:] == 7.0).all())
 
 
+def run_delta_scan(c, lens, state, rd, wr, unit_eps=1e-6):
+    """The scan alone over rows of ``lens`` tokens: (o [tokens][heads * dim] in 32 bits, the states)."""
+    from megatron_mixtera_b200 import ops
+
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    d_state, (d_rd, d_wr) = state.to(DEV), (torch.tensor(x, dtype=torch.int32, device=DEV) for x in (rd, wr))
+    o = torch.zeros(c.T, c.n, device=DEV)
+    z = ops.linear(torch.tanh(c.dev[0][:, 5 * c.n:]).contiguous(), c.dev[1])
+    a = c.args(d_state, d_rd, d_wr, o)
+    a.num_rows, a.cu_tokens, a.o_f32, a.z, a.unit_eps = len(lens), cu.data_ptr(), o.data_ptr(), z.data_ptr(), unit_eps
+    ops.delta_scan(a, d_state)
+    return o.cpu(), d_state.cpu()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,dim", [(2, 64), (1, 40), (1, 128), (2, 20)])
+@pytest.mark.parametrize("lens", [[133, 255, 130, 1, 4], [5, 1, 2, 3, 4]])
+def test_delta_scan_of_keys_without_an_epsilon(dtype, heads, dim, lens):
+    """Keys are never zero, so unit keys need no epsilon: rows of 4 n + 1 to 4 n + 4 tokens.  Tolerances as in test_delta_scan (1e-6 of a key's square sum,
+    which is above 1, changes nothing there)."""
+    c = DeltaCase(heads, dim, 8, sum(lens), dtype, seed=70)
+    state = rand(10, heads, dim, dim, seed=71)
+    o, new = run_delta_scan(c, lens, state, [0, -1, 2, 3, 4], [5, 6, 7, 8, 9], unit_eps=0.0)
+    tol, at = 1e-4 if dtype == torch.float32 else 2e-2, 0
+    for row, n in enumerate(lens):
+        want, S = Z.delta_scan(*c.inputs(at, at + n), state=None if row == 1 else state[row].double().transpose(1, 2))
+        assert (new[5 + row].double().transpose(1, 2) - S).abs().max() < tol * S.abs().max()
+        assert (o[at: at + n].double() - want.reshape(n, -1)).abs().max() < tol * want.abs().max()
+        at += n
+
+
 def test_delta_state_survives_long_rows():
     """A value written at the first token with decay close to one is still there 600 tokens later, and only there."""
     from megatron_mixtera_b200 import ops
