@@ -571,6 +571,11 @@ __device__ __forceinline__ float transposed_sum(float (&v)[N], int lane) {
   return v[0];
 }
 
+// o += a b where `p`, one predicated multiply-add.  (Selected operands make a block 2 % longer, 2048 tokens x 32 heads of 64 371 -> 381 us; branches 25 %.)
+__device__ __forceinline__ void add_if(bool p, float& o, float a, float b) {
+  asm("{ .reg .pred p; setp.ne.s32 p, %3, 0; @p fma.rn.f32 %0, %1, %2, %0; }" : "+f"(o) : "f"(a), "f"(b), "r"(static_cast<int>(p)));
+}
+
 template <typename T, int DIM, int COLS, int BLOCKS>
 __global__ void __launch_bounds__(BlockShape<DIM, COLS, BLOCKS>::kThreads)
 delta_block_scan_kernel(b200_delta_args a) {
@@ -840,8 +845,15 @@ delta_block_scan_kernel(b200_delta_args a) {
         const float a0 = (high ? p[2] : p[0]) + __shfl_xor_sync(0xffffffffu, high ? p[0] : p[2], 2 * ST);
         const float a1 = (high ? p[3] : p[1]) + __shfl_xor_sync(0xffffffffu, high ? p[1] : p[3], 2 * ST);
         float o = (odd ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, ST);
-        o = fmaf(rk.x, v[0][n], fmaf(rk.y, v[1][n], fmaf(rk.z, v[2][n], fmaf(rk.w, v[3][n], o))));
-        o = fmaf(-rb.x, d[0][n], fmaf(-rb.y, d[1][n], fmaf(-rb.z, d[2][n], fmaf(-rb.w, d[3][n], o))));
+        // (Later tokens' coefficients are zeros, but their values need not be numbers: they are left out.)
+        add_if(ni >= 3, o, rk.w, v[3][n]);
+        add_if(ni >= 2, o, rk.z, v[2][n]);
+        add_if(ni >= 1, o, rk.y, v[1][n]);
+        o = fmaf(rk.x, v[0][n], o);
+        add_if(ni >= 3, o, -rb.w, d[3][n]);
+        add_if(ni >= 2, o, -rb.z, d[2][n]);
+        add_if(ni >= 1, o, -rb.y, d[1][n]);
+        o = fmaf(-rb.x, d[0][n], o);
         if (b * J + ni < left && cb * COLS + n * Sh::kGroups + group < dim) o_dst[n * Sh::kGroups] = o;
       }
       o_dst += J * hd;
@@ -993,7 +1005,7 @@ static int launch_block_scan(const b200_delta_args& a, cudaStream_t s) {
 template <typename T, int DIM>
 static int block_scan_by_size(const b200_delta_args& a, cudaStream_t s) {
   // Eight preparing warps, and one CTA on an SM, while a CTA's own pace counts: rows of 128 tokens and more on average and, with heads of up to 64, CTAs for
-  // little more than two rounds of the SMs.  Else four, and two CTAs of up to 64.  us, eight / four: heads of 64, 160 CTAs 378 / 481, 256 of 400 tokens and less
+  // little more than two rounds of the SMs.  Else four, and two CTAs of up to 64 (which takes 128 registers a thread: with 130 rows of one token 41 -> 57).  us, eight / four: heads of 64, 160 CTAs 378 / 481, 256 of 400 tokens and less
   // 102 / 110, 320 583 / 615, 384 682 / 647, 512 841 / 764; rows of 64 tokens 33.8 / 29.8.  Heads of 128: 256 CTAs 791 / 961, 2048 1340 / 1497; rows of 16 40 / 34.
   const int64_t ctas = static_cast<int64_t>(a.num_rows) * a.heads;
   if (a.num_tokens / 128 >= a.num_rows && (DIM > 64 || 4 * ctas <= 9 * sm_count())) return launch_block_scan<T, DIM, 64, 8>(a, s);

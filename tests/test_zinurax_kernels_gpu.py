@@ -567,6 +567,23 @@ def test_delta_scan_of_keys_without_an_epsilon(dtype, heads, dim, lens):
         at += n
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,dim", [(2, 64), (1, 128), (2, 20)])
+@pytest.mark.parametrize("at", [3, 38, 129, 0])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_delta_scan_looks_at_no_later_token(dtype, heads, dim, at, value):
+    """A token that is no number (the fourth, third and second of a block, and the first) changes no bit of the tokens before it, nor of other rows."""
+    lens = [131, 150, 3]
+    c = DeltaCase(heads, dim, 8, sum(lens), dtype, seed=80)
+    state, rd, wr = rand(6, heads, dim, dim, seed=81), [0, -1, 2], [3, 4, 5]
+    o, new = run_delta_scan(c, lens, state, rd, wr)
+    t = lens[0] + at
+    c.dev[0][t] = value
+    o2, new2 = run_delta_scan(c, lens, state, rd, wr)
+    assert torch.equal(o2[:t], o[:t]) and torch.equal(o2[lens[0] + lens[1]:], o[lens[0] + lens[1]:]) and bool(o2[t].isnan().any())
+    assert all(torch.equal(new2[i], new[i]) for i in (3, 5))
+
+
 def test_delta_state_survives_long_rows():
     """A value written at the first token with decay close to one is still there 600 tokens later, and only there."""
     from megatron_mixtera_b200 import ops
