@@ -1025,7 +1025,10 @@ wkv_block_scan_kernel(b200_recurrence_args a, bool vec_k) {
         const float a0 = (high ? p[2] : p[0]) + __shfl_xor_sync(0xffffffffu, high ? p[0] : p[2], 2 * ST);
         const float a1 = (high ? p[3] : p[1]) + __shfl_xor_sync(0xffffffffu, high ? p[1] : p[3], 2 * ST);
         float o = (odd ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, ST);
-        o = fmaf(rk.x, wrote[0], fmaf(rk.y, wrote[1], fmaf(rk.z, wrote[2], fmaf(rk.w, wrote[3], o))));
+        delta::add_if(mine >= 3, o, rk.w, wrote[3]);  // (later tokens' coefficients are zeros, but their values need not be numbers)
+        delta::add_if(mine >= 2, o, rk.z, wrote[2]);
+        delta::add_if(mine >= 1, o, rk.y, wrote[1]);
+        o = fmaf(rk.x, wrote[0], o);
         if (b * J + mine < left && first + half + n < vdim) o_dst[n] = o;
       }
       o_dst += J * hv;

@@ -82,6 +82,56 @@ def test_wkv_rows_that_end_inside_a_block(heads, dim, dtype):
         assert all(close(g, x, dtype) for g, x in zip(got, want)), schedule
 
 
+class WkvCase:
+    """Inputs of the wkv scan alone, with a state in front of every row (slots 0 to ``most`` - 1; row i writes slot ``most`` + i)."""
+
+    def __init__(self, heads, dim, tokens, most, dtype, seed):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+
+        def r(*shape):
+            return torch.randn(*shape, generator=g, device="cuda")
+
+        n = heads * dim
+        self.heads, self.dim, self.n, self.most, self.dtype = heads, dim, n, most, dtype
+        self.proj, self.z, self.state0 = r(tokens, 3 * n).to(dtype), r(1, tokens, n), r(2 * most, heads, dim, dim)
+        self.bias, self.bonus, self.norm = (r(n).to(dtype) for _ in range(3))
+
+    def scan(self, lens):
+        """Rows of ``lens`` tokens from the first token on: (o [tokens][n] in 32 bits, the rows' states)."""
+        from megatron_mixtera_b200 import _lib, ops
+
+        T, rows_, state = sum(lens), len(lens), self.state0.clone()
+        cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+        rd = torch.arange(rows_, dtype=torch.int32, device="cuda")
+        wr, o, z = rd + self.most, torch.zeros(T, self.n, device="cuda"), self.z[:, :T].contiguous()
+        a = _lib.RecurrenceArgs()
+        a.kind, a.heads, a.kv_heads, a.dim, a.vdim, a.num_tokens, a.num_rows, a.norm_per_head = 0, self.heads, self.heads, self.dim, self.dim, T, rows_, 1
+        a.proj, a.proj_ld, a.off_r, a.off_k, a.off_v = self.proj.data_ptr(), 3 * self.n, 0, self.n, 2 * self.n
+        a.decay_bias, a.bonus, a.norm_weight, a.z, a.z_splits = self.bias.data_ptr(), self.bonus.data_ptr(), self.norm.data_ptr(), z.data_ptr(), 1
+        a.state, a.state_in, a.state_out, a.state_slots, a.cu_tokens = state.data_ptr(), rd.data_ptr(), wr.data_ptr(), 2 * self.most, cu.data_ptr()
+        a.o_f32, a.dtype, a.eps = o.data_ptr(), ops.dtype_code(self.dtype), 1e-5
+        ops.struct_kernel("recurrence_scan", a, state)
+        return o, state[self.most: self.most + rows_]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,dim", [(2, 64), (1, 128), (2, 20)])
+@pytest.mark.parametrize("at", [3, 38, 129, 0])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_wkv_scan_looks_at_no_later_token(dtype, heads, dim, at, value):
+    """A token that is no number (the fourth, third and second of a block, and the first) changes no bit of the tokens before it, nor of other rows: long rows
+    and short ones."""
+    for lens in ([131, 150, 3], [5] * 26 + [1] + [150] + [3] * 20):
+        c = WkvCase(heads, dim, sum(lens), len(lens), dtype, 20)
+        o, new = c.scan(lens)
+        row = lens.index(150)
+        t, end = sum(lens[:row]) + at, sum(lens[: row + 1])
+        c.proj[t] = value
+        o2, new2 = c.scan(lens)
+        assert torch.equal(o2[:t], o[:t]) and torch.equal(o2[end:], o[end:]) and bool(o2[t].isnan().any())
+        assert torch.equal(new2[:row], new[:row]) and torch.equal(new2[row + 1:], new[row + 1:])
+
+
 @pytest.mark.parametrize("kind", ["wkv", "delta", "memory"])
 @pytest.mark.parametrize("dim", [64, 48, 128])
 def test_recurrent_decode_shares_a_row_between_warps(kind, dim):
