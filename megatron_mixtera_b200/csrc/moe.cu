@@ -135,9 +135,8 @@ route_kernel(b200_moe_args a) {
 
 // Softmax over experts and identity experts, choice by score + correction inside the best groups.  CHOSEN: scores are the logits plus a
 // bias, and the weights the softmax over the chosen ones.
-// Shared memory: [kWarps][2 columns + groups] scores, what the choice goes by, and the best of each group.  (A chain of short steps for a token.  With the corrections
-// read from memory at each step and a group's best found by one lane: 64 tokens, 34 columns in 2 groups 10.7 us, 9.9 now; without groups as
-// before: 5952 tokens, 64 columns 32.)
+// Shared memory: [kWarps][2 columns + groups] scores, what the choice goes by (CHOSEN: the scores themselves), and the best of each group.  (A chain of short steps
+// for a token.  With the corrections read from memory at each step and a group's best found by one lane: 64 tokens, 34 columns in 2 groups 10.7 us, 9.9 now.)
 template <typename T, bool CHOSEN>
 __global__ void __launch_bounds__(kWarps * 32)
 route_softmax_kernel(b200_moe_args a) {
@@ -151,8 +150,8 @@ route_softmax_kernel(b200_moe_args a) {
   const int t = blockIdx.x * kWarps + warp;
   const T* correction = static_cast<const T*>(a.correction);
   if (t < a.num_tokens) {
-    float* score = score_s + warp * (2 * C + a.groups);
-    float* pick = score + C;  // minus infinity: can no longer be chosen
+    float* score = score_s + warp * ((CHOSEN ? 1 : 2) * C + a.groups);
+    float* pick = CHOSEN ? score : score + C;  // minus infinity: can no longer be chosen
     float* group_best = pick + C;
     const int64_t stride = static_cast<int64_t>(a.num_tokens) * a.router_ld;
     const float* z = a.router + static_cast<int64_t>(t) * a.router_ld;
@@ -164,7 +163,7 @@ route_softmax_kernel(b200_moe_args a) {
       for (int s = 0; s < a.router_splits; ++s) x += z[s * stride + e];
       if (CHOSEN) x += more;
       score[e] = x;
-      pick[e] = CHOSEN ? x : more;
+      if (!CHOSEN) pick[e] = more;
       top = fmaxf(top, x);
     }
     top = warp_max(top);
@@ -204,11 +203,17 @@ route_softmax_kernel(b200_moe_args a) {
     __syncwarp();
     if (a.groups > 1) {
       const int size = C / a.groups;
-      for (int g = 0; g < a.groups; ++g) {
+      // 2^shift lanes for each group: as many as find all groups' best at once.  (6000 tokens, us with these / a warp for one group after the other: 256 columns in 128
+      // groups 34.5 / 114, in 8 31.5 / 37.3, in 2 29.0 / 30.2; 64 in 8 22.2 / 24.6.)
+      int shift = 5;
+      while (shift > 0 && (32 >> shift) < a.groups) --shift;
+      const int lanes = 1 << shift, sub = lane & (lanes - 1);
+      for (int g = lane >> shift; g - (lane >> shift) < a.groups; g += 32 >> shift) {  // (the same turns for all lanes)
         float m = -INFINITY;
-        for (int e = g * size + lane; e < (g + 1) * size; e += 32) m = fmaxf(m, pick[e]);
-        m = warp_max(m);
-        if (lane == 0) group_best[g] = m;
+        if (g < a.groups)
+          for (int e = sub; e < size; e += lanes) m = fmaxf(m, pick[g * size + e]);
+        for (int o = lanes / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (g < a.groups && sub == 0) group_best[g] = m;
       }
       __syncwarp();
       for (int k = 0; k < a.keep_groups; ++k) {
@@ -423,7 +428,7 @@ int b200_moe_route(const b200_moe_args* a, b200_stream_t stream) {
     if (a->identity < 0 || columns > moe::kMaxExperts || a->router_ld < columns || !a->correction || a->shared_gate || groups < 1 ||
         columns % groups != 0 || a->keep_groups < 1 || a->keep_groups > groups || a->top > columns / groups * a->keep_groups)
       return B200_ERR_INVALID_ARGUMENT;
-    const size_t bytes = static_cast<size_t>(moe::kWarps) * (2 * columns + groups) * 4;
+    const size_t bytes = static_cast<size_t>(moe::kWarps) * ((a->plain == 2 ? 1 : 2) * columns + groups) * 4;
     auto go = [&](auto zero, auto CHOSEN) {
       using T = decltype(zero);
       static std::atomic<uint64_t> done{0};

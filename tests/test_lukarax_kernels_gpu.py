@@ -329,6 +329,40 @@ def sure_of(x, w, r):
     return keep
 
 
+@pytest.mark.parametrize("columns,groups,keep,top", [(34, 2, 1, 4), (34, 17, 5, 6), (48, 3, 2, 8), (40, 5, 5, 3), (64, 32, 7, 9), (256, 8, 4, 8), (256, 128, 9, 8), (1024, 256, 2, 8), (33, 1, 1, 33), (1024, 1, 1, 64),
+                                                     (70, 0, 1, 5), (1024, 0, 1, 64)])
+def test_choice_inside_groups(columns, groups, keep, top):
+    """Any number of groups of any size, and (0 groups) the softmax over the chosen ones: scores on a grid that rounding cannot reorder, weights within 32-bit roundings."""
+    from megatron_mixtera_b200 import _lib, ops
+
+    T, chosen_only = 21, groups == 0
+    groups = max(groups, 1)
+    g = torch.Generator().manual_seed(columns + groups)
+    z = torch.stack([torch.randperm(columns, generator=g) for _ in range(T)]).double() * (4.0 / columns)
+    plus = torch.randint(0, 2, (columns,), generator=g).double() * 2.0 ** -9
+    score = torch.softmax(z, -1)
+    pick = z + plus if chosen_only else score + plus
+    best = pick.view(T, groups, -1).max(-1).values.topk(keep, -1).indices
+    open_ = torch.zeros(T, groups, dtype=torch.bool).scatter_(1, best, True).repeat_interleave(columns // groups, 1)
+    want = pick.masked_fill(~open_, -math.inf).topk(top, -1).indices
+    weight = torch.softmax((z + plus).gather(1, want), -1) if chosen_only else score.gather(1, want) / score.gather(1, want).sum(-1, keepdim=True)
+    a = _lib.MoeArgs()
+    d_z, d_plus = z.float().cuda()[None].contiguous(), plus.float().cuda()
+    P = T * top
+    pairs, weights = torch.zeros(T, top, 2, dtype=torch.int32, device="cuda"), torch.zeros(T, top, device="cuda")
+    counts, offsets = (torch.zeros(columns + 1, dtype=torch.int32, device="cuda") for _ in range(2))
+    a.max_tiles = P // 32 + min(columns, P)
+    tiles, num_tiles = torch.zeros(a.max_tiles, 4, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    a.num_tokens, a.width, a.experts, a.top, a.ff, a.tile_tokens, a.dtype = T, 64, columns, top, 64, 32, ops.dtype_code(torch.float32)
+    a.plain, a.groups, a.keep_groups, a.weight_scale, a.correction = 2 if chosen_only else 1, groups, keep, 1.0, d_plus.data_ptr()
+    a.router, a.router_splits, a.router_ld = d_z.data_ptr(), 1, columns
+    a.counts, a.pairs, a.pair_weight, a.offsets, a.tiles, a.num_tiles = (t.data_ptr() for t in (counts, pairs, weights, offsets, tiles, num_tiles))
+    ops.struct_kernel("moe_route", a, d_z)
+    assert torch.equal(pairs[..., 0].cpu().long(), want)
+    assert torch.equal(offsets.cpu()[1:] - offsets.cpu()[:-1], torch.bincount(want.flatten(), minlength=columns).int())
+    assert float((weights.cpu().double() - weight).abs().max()) < 2e-6
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("tokens", [1, 7, 64, 300, 2000])
 @pytest.mark.parametrize("case", range(7))
