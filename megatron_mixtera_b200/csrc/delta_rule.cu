@@ -868,8 +868,9 @@ delta_block_scan_kernel(b200_delta_args a) {
   }
 }
 
-// kFinishUnits (token, head) units in turn with all their loads in flight: LPH lanes of four channels each, in vectors, or (LPH == 0) a warp and any size.  Bound by
-// the bytes in flight: 6208 tokens x 32 heads of 64 55 us with a warp and single channels for each, 20 in vectors (floor 15).
+// kFinishUnits (token, head) units in turn with all their loads in flight: LPH lanes of four channels each, in vectors, or (LPH == 0) a warp: channels 32 apart, up to
+// 128 of them in registers.  Bound by the bytes in flight: 6208 tokens x 32 heads of 64 55 us with a warp and single channels for each, 20 in vectors (floor 15);
+// 6000 x 32 heads of 66, which are no vectors, 63 us in registers, 87 in the loop.
 constexpr int kFinishUnits = 4;
 template <typename T, int LPH>
 __global__ void __launch_bounds__(256, LPH > 0 ? 4 : 1)
@@ -910,6 +911,36 @@ delta_finish_kernel(b200_delta_args a) {
   }
   const int lane = threadIdx.x & 31;
   const uint32_t first = (blockIdx.x * 8 + (threadIdx.x >> 5)) * kFinishUnits;
+  if (dim <= 128) {  // heads in registers
+    float v[kFinishUnits][4], w[kFinishUnits][4];
+    T g[kFinishUnits][4];
+#pragma unroll
+    for (int k = 0; k < kFinishUnits; ++k) {
+      const uint32_t unit = min(first + k, total - 1), t = unit / heads;
+      const int at = static_cast<int>(unit - t * heads) * dim;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (e * 32 >= dim) break;
+        const int i = min(lane + e * 32, dim - 1);
+        v[k][e] = a.o_f32[static_cast<int64_t>(unit) * dim + i];
+        g[k][e] = proj[t * a.proj_ld + a.off_g + at + i];
+        w[k][e] = simt::to_f32(weight[at + i]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kFinishUnits; ++k) {
+      float sq = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sq += lane + e * 32 < dim ? v[k][e] * v[k][e] : 0.f;
+      const float inv = 1.f / sqrtf(warp_sum(sq) / dim + a.eps);
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (lane + e * 32 < dim && first + k < total)
+          simt::store_as(out + static_cast<int64_t>(first + k) * dim + lane + e * 32,
+                         v[k][e] * inv * w[k][e] * gate_sigmoid(simt::to_f32(g[k][e])));
+    }
+    return;
+  }
   for (int k = 0; k < kFinishUnits; ++k) {
     const int64_t unit = first + k;
     if (unit >= total) return;

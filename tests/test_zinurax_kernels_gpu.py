@@ -504,6 +504,25 @@ def test_delta_scan(dtype, heads, dim, rank):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,dim", [(3, 1), (3, 34), (5, 66), (2, 127), (2, 130), (3, 4), (2, 132)])
+def test_delta_output_norm(dtype, heads, dim):
+    """Heads in vectors, 32 channels apart and in the loop; the last units of the last CTA.  One rounding to the type, 1e-6 of the gate's fast exponential."""
+    from megatron_mixtera_b200 import ops
+
+    T = 37
+    c = DeltaCase(heads, dim, 4, T, dtype, seed=90)
+    o, state = rand(T, c.n, seed=91), torch.zeros(1, heads, dim, dim, device=DEV)
+    at = torch.zeros(1, dtype=torch.int32, device=DEV)
+    d_o, out = o.to(DEV), torch.empty(T, c.n, dtype=dtype, device=DEV)
+    a = c.args(state, at, at, out)
+    a.num_rows, a.o_f32 = 1, d_o.data_ptr()
+    ops.delta_finish(a, state)
+    want = c.finish(o.double().view(T, heads, dim), 0, T, 1e-5)
+    step = 1e-5 if dtype == torch.float32 else 2.0 ** -8
+    assert bool(((out.cpu().double() - want).abs() <= step * want.abs() + 1e-6).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,dim", [(2, 64), (1, 40), (1, 128), (2, 68)])
 def test_delta_scan_of_long_rows(dtype, heads, dim):
     """Rows of 128 tokens and more on average are prepared 32 tokens at a time: rows that end one token before, at and behind a block of four and a group of
