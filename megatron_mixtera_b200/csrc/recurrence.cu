@@ -805,7 +805,7 @@ struct BlockShape {
 };
 
 template <typename T, int DIM, int COLS, int LANES, int BLOCKS>
-__global__ void __launch_bounds__(BlockShape<DIM, COLS, LANES, BLOCKS>::kThreads)
+__global__ void __launch_bounds__(BlockShape<DIM, COLS, LANES, BLOCKS>::kThreads, DIM <= 64 && BLOCKS == 4 ? 2 : 0)
 wkv_block_scan_kernel(b200_recurrence_args a, bool vec_k) {
   using Sh = BlockShape<DIM, COLS, LANES, BLOCKS>;
   constexpr int NI = Sh::NI, I = Sh::I, N = Sh::N, EL = Sh::kElems, VL = Sh::kValues, J = kBlockTokens;
@@ -1288,11 +1288,15 @@ static int launch_block_scan(const b200_recurrence_args& a, cudaStream_t s) {
 }
 template <typename T, int DIM>
 static int block_scan_by_size(const b200_recurrence_args& a, cudaStream_t s) {
-  // Eight preparing warps and two columns on four lanes for rows of 64 tokens and more on average; else four, with four columns on eight lanes, and more CTAs on
-  // an SM.  us, the former / the latter / a token at a time: 32 heads of 64, rows of 64 tokens 13.6 / 15.0 / 15.5, 60 rows of 20 71 / 51 / 58, 64 rows of one
-  // 50 / 28 / 35; 64 rows of 256 tokens x 16 heads of 128 659 / 920 / 935.
-  if (a.num_tokens / 64 >= a.num_rows) return launch_block_scan<T, DIM, 4, 8>(a, s);
-  return launch_block_scan<T, DIM, 8, 4>(a, s);
+  // Rows of 64 tokens and more on average: two columns on four lanes, with eight preparing warps while there are few CTAs or the state leaves one CTA an SM anyway, and
+  // with four, two CTAs an SM, from eight CTAs an SM on.  us, eight / four / a token at a time, 32 heads of 64: 4 rows of 2048 tokens and less 214 / 262 / 286, 80 rows of
+  // 70 200 / 148 / 174, 64 of 256 405 / 344 / 419; 64 heads: 24 rows of 64 115 / 86 / 101.  What a long row has beside it slows it then: one of 2000 tokens and 20 of three,
+  // 32 heads 203 / 229 / 266, 64 heads 206 / 265 / 284 (24 rows of 64, 32 heads, 58 / 47 / 56, stay with eight for that).
+  // Shorter rows: four columns on eight lanes.  us, four lanes and eight warps / eight lanes and four warps / a token at a time: 60 rows of 20 71 / 49 / 57, 64 rows of one
+  // 46 / 25 / 33; 64 rows of 256 tokens x 16 heads of 128 658 / 754 / 847.
+  if (a.num_tokens / 64 < a.num_rows) return launch_block_scan<T, DIM, 8, 4>(a, s);
+  if (DIM <= 64 && static_cast<int64_t>(a.num_rows) * a.heads * ((a.vdim + 63) / 64) > 8 * sm_count()) return launch_block_scan<T, DIM, 4, DIM <= 64 ? 4 : 8>(a, s);
+  return launch_block_scan<T, DIM, 4, 8>(a, s);
 }
 template <typename T, typename Rule>
 static int scan_by_dim(const b200_recurrence_args& a, cudaStream_t s) {

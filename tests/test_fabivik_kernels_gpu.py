@@ -132,6 +132,21 @@ def test_wkv_scan_looks_at_no_later_token(dtype, heads, dim, at, value):
         assert torch.equal(new2[:row], new[:row]) and torch.equal(new2[row + 1:], new[row + 1:])
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dim", [64, 40, 128])
+def test_wkv_scan_of_a_row_in_any_company(dim, dtype):
+    """A row alone, among enough rows of its length for two CTAs an SM, and beside many short rows.  Four lanes a column sum in one order, so the first two agree in
+    every bit; short rows' eight lanes split a head's channels further, so the third agrees within a few roundings of 32-bit sums.  States have one order."""
+    heads, n = 16, 67
+    many = 8 * torch.cuda.get_device_properties(0).multi_processor_count // heads + 3
+    c = WkvCase(heads, dim, many * n, many, dtype, 21)
+    found = [c.scan(lens) for lens in ([n], [n] * many, [n] + [2] * 40)]
+    (o, s), (o2, s2), (o3, s3) = ((o[:n], s[0]) for o, s in found)
+    assert torch.equal(o, o2) and torch.equal(s, s2) and torch.equal(s, s3)
+    assert float((o - o3).abs().max()) < 2.0 ** -24 * 16 * float(o.abs().max())
+    assert bool(found[1][0].isfinite().all()) and bool(found[1][0][-n:].abs().max() > 0)
+
+
 @pytest.mark.parametrize("kind", ["wkv", "delta", "memory"])
 @pytest.mark.parametrize("dim", [64, 48, 128])
 def test_recurrent_decode_shares_a_row_between_warps(kind, dim):
