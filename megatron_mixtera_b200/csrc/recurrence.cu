@@ -1237,14 +1237,23 @@ static int launch_decode(const b200_recurrence_args& a, cudaStream_t s) {
   const std::integral_constant<int, 2> two;
   const std::integral_constant<int, 4> four;
   // A warp walks its columns a pass at a time, two passes' bytes on their way, so few (row, head) tasks are bound by that walk: four warps for each up to four tasks
-  // an SM, two up to eight and, with more than 64 channels, with any number.  us, one / two / four: memory, 16 heads of 128, one row 13.1 / 8.5 / 6.0, 32 rows 27.7 /
+  // an SM, two up to eight and, with more than 64 channels, with more.  us, one / two / four: memory, 16 heads of 128, one row 13.1 / 8.5 / 6.0, 32 rows 27.7 /
   // 18.9 / 15.4, 64 rows 32.5 / 27.8 / 28.2, 200 rows 76.8 / 74.9 / 79.3; delta, 16 heads of 128, 8 rows 19.6 / 12.3 / 11.9, 64 rows 44.5 / 33.8 / 35.8; wkv, 32 heads of
   // 64, 16 rows 10.7 / 7.2 / 5.9, 32 rows 15.0 / 10.2 / 14.2, 40 rows 16.2 / 17.7 / 21.0.  (32 channels are one pass.)
+  // Where two warps make a second wave of a few CTAs, one is better: memory, 80 rows x 16 heads of 128 35.8 / 39.9, 96 rows 43.0 / 40.5.  Of 256 channels, eight tasks an SM are
+  // under way with one warp for each, four with two (memory, and wkv in 32 bits: six), whose wave takes 0.55 of the time: wkv, 8 heads, 80 rows 79.4 / 90.2, 200 rows 169 / 154, 256 rows 191 / 201;
+  // delta 82.7 / 92.8, 177 / 158, 195 / 205; memory 81.7 / 64.1, 152 / 142, 196 / 178, and 128 rows 96 / 107.
   auto by_parts = [&](auto taps) {
     if constexpr (DIM > 32) {
-      const int64_t tasks = static_cast<int64_t>(a.heads) * a.num_rows;
-      if (tasks <= 4 * sm_count()) return go(taps, four);
-      if (tasks <= 8 * sm_count() || DIM > 64) return go(taps, two);
+      const int64_t tasks = static_cast<int64_t>(a.heads) * a.num_rows, sms = sm_count();
+      constexpr bool memory = Rule::kKind == B200_RECURRENCE_MEMORY;
+      if (tasks <= 4 * sms) return go(taps, four);
+      if constexpr (DIM > 128) {
+        const int64_t one_waves = (tasks + 8 * sms - 1) / (8 * sms), per_wave = (memory || (sizeof(T) == 4 && Rule::kKind == B200_RECURRENCE_WKV) ? 6 : 4) * sms, two_waves = (tasks + per_wave - 1) / per_wave;
+        if (11 * two_waves < 20 * one_waves) return go(taps, two);
+      } else if (tasks <= 8 * sms || (DIM > 64 && !(memory && a.dim > 96 && tasks <= 9 * sms))) {
+        return go(taps, two);
+      }
     }
     return go(taps, one);
   };
