@@ -390,10 +390,17 @@ static int launch(const b200_residual_norm_args& a, cudaStream_t s) {
   if constexpr (sizeof(T) == 2) {
     // Without expert rows there is little to wait for, and CTAs of 512 threads lose (5952 rows of 4096 from the table: 47 us below, 55 here; of 2048: 33, 28).
     if (aligned && a.width % 8 == 0 && a.taps == 0 && a.rows > 2 * sm_count() && (a.expert_rows != nullptr || a.width <= 2048)) {
-      if (a.width > 512 && a.width <= 1024) return launch_pdl(residual_norm_rows_kernel<128, 8>, grid, dim3(128), 0, s, a);
-      if (a.width > 1024 && a.width <= 2048) return launch_pdl(residual_norm_rows_kernel<256, 4>, grid, dim3(256), 0, s, a);
+      // Of the time below, with four experts and two norms: up to 1024 wide 0.94 for 400 rows, 1.03 for 500, 0.93 for 592, 1.11 for 700, 0.8 from 800 on.  Wider than 4096, where
+      // one CTA of 1024 threads fits an SM here and three of 256 below, waves decide: 1.21, 0.87, 1.09, 0.78 and 1.01 for 400, 500, 800, 1000 and 3000 rows of 5120; 1.12, 0.81,
+      // 0.89, 0.73 and 0.91 of 6144 (eight experts: 0.91 for 400); 0.92, 0.62, 0.78, 0.68 and 0.79 of 8192.
+      const int sms = sm_count(), waves = (a.rows + sms - 1) / sms, waves_below = (a.rows + 3 * sms - 1) / (3 * sms);
+      const bool few = a.rows <= 4 * sms && a.table == nullptr;  // (from a table, 1024 wide, 500 rows 2.9 us below and 3.5 here)
+      if (a.width > 512 && a.width <= 1024 && (few || a.rows > 5 * sms))
+        return launch_pdl(residual_norm_rows_kernel<128, 8>, grid, dim3(128), 0, s, a);
+      if (a.width > 1024 && a.width <= 2048 && (few || a.rows > 4 * sms)) return launch_pdl(residual_norm_rows_kernel<256, 4>, grid, dim3(256), 0, s, a);
       if (a.width > 2048 && a.width <= 4096) return launch_pdl(residual_norm_rows_kernel<512, 2>, grid, dim3(512), 0, s, a);
-      if (a.width > 4096 && a.width <= 8192) return launch_pdl(residual_norm_rows_kernel<1024, 1>, grid, dim3(1024), 0, s, a);
+      if (a.width > 4096 && a.width <= 8192 && (a.width > 7168 || (a.width > 5120 ? a.top >= 8 || a.rows > 3 * sms : 4 * waves <= (a.width < 4608 ? 8 : 11) * waves_below)))
+        return launch_pdl(residual_norm_rows_kernel<1024, 1>, grid, dim3(1024), 0, s, a);
     }
   }
   if (aligned) {
