@@ -14,7 +14,7 @@
 //   delta_block_scan_kernel  rows of any length, heads of 33 to 128: one CTA per (row, head, 64 columns) walks the row's tokens four at a time.  Compute warps
 //                        hold two columns on four lanes (a vector is read from shared memory once for both); other warps prepare blocks of
 //                        four tokens (decays, unit key, removal vector, their products with one another) meanwhile.
-//   delta_scan_kernel    the same a token at a time, for the other sizes
+//   delta_scan_kernel    the same a token at a time, a column on two lanes, for the other sizes
 //   delta_finish_kernel  head norm + weight + output gate behind the scan (a head's columns may be spread over CTAs there).
 #include "common.cuh"
 
@@ -376,16 +376,15 @@ __device__ __forceinline__ int longest_first(const int32_t* cu_tokens, int rows,
   return __ffs(__ballot_sync(0xffffffffu, rank == k)) - 1;
 }
 
-template <int DIM, int COLS, int N, int LANES>
-struct ScanShape {  // COLS columns per CTA, N of them per thread, LANES lanes per column
+template <int DIM, int COLS, int LANES>
+struct ScanShape {  // COLS columns per CTA, LANES lanes for each
   static constexpr int I = DIM / LANES;
   static constexpr int NI = LANES;  // 32 / NI apart: neighbouring lanes read one address
   static constexpr int kStride = 32 / NI;
-  static constexpr int kComputeThreads = COLS / N * NI;
+  static constexpr int kComputeThreads = COLS * NI;
   static constexpr int kComputeWarps = kComputeThreads / 32;
   static constexpr int kPrepWarps = kComputeWarps < 2 ? 2 : kComputeWarps;
   static constexpr int kThreads = kComputeThreads + kPrepWarps * 32;
-  static constexpr int kGroups = COLS / N;                      // columns side by side
   static constexpr int kTokPerWarp = kScanTokens / kPrepWarps;  // tokens one warp prepares
   static constexpr int kBatch = kTokPerWarp < 4 ? kTokPerWarp : 4;  // of which this many at a time
   static constexpr int kElems = DIM / 32;                       // key channels per lane while preparing
@@ -394,10 +393,10 @@ struct ScanShape {  // COLS columns per CTA, N of them per thread, LANES lanes p
   static constexpr int kSmemBytes = 2 * kBufFloats * 4;
 };
 
-template <typename T, int DIM, int COLS, int N, int LANES>
-__global__ void __launch_bounds__(ScanShape<DIM, COLS, N, LANES>::kThreads)
+template <typename T, int DIM, int COLS, int LANES>
+__global__ void __launch_bounds__(ScanShape<DIM, COLS, LANES>::kThreads)
 delta_scan_kernel(b200_delta_args a) {
-  using Sh = ScanShape<DIM, COLS, N, LANES>;
+  using Sh = ScanShape<DIM, COLS, LANES>;
   constexpr int NI = Sh::NI, I = Sh::I, EL = Sh::kElems, VL = (COLS + 31) / 32;
   extern __shared__ __align__(16) float smem[];
   const int tid = threadIdx.x, lane = tid & 31;
@@ -483,19 +482,15 @@ delta_scan_kernel(b200_delta_args a) {
   const int in = a.state_in[row], out = a.state_out[row];
   const int64_t head_elems = static_cast<int64_t>(dim) * dim;
   constexpr int ST = Sh::kStride;
-  const int ni = lane / ST, group = (tid >> 5) * ST + lane % ST;  // this thread's columns: cb * COLS + n * kGroups + group
-  f32x2 s[N][I / 2];
+  const int ni = lane / ST, group = (tid >> 5) * ST + lane % ST, col = cb * COLS + group;  // this thread's column
+  f32x2 s[1][I / 2];
+  if (static_cast<unsigned>(in) < static_cast<unsigned>(a.state_slots) && col < dim) {
+    load_column<NI, I>(a.state + (static_cast<int64_t>(in) * a.heads + head) * head_elems + static_cast<int64_t>(col) * dim, dim, ni, full, s[0]);
+  } else {
 #pragma unroll
-  for (int n = 0; n < N; ++n) {
-    const int j = cb * COLS + n * Sh::kGroups + group;
-    if (static_cast<unsigned>(in) < static_cast<unsigned>(a.state_slots) && j < dim) {
-      load_column<NI, I>(a.state + (static_cast<int64_t>(in) * a.heads + head) * head_elems + static_cast<int64_t>(j) * dim, dim, ni, full, s[n]);
-    } else {
-#pragma unroll
-      for (int e = 0; e < I / 2; ++e) s[n][e] = 0ull;
-    }
+    for (int e = 0; e < I / 2; ++e) s[0][e] = 0ull;
   }
-  float* o_dst = a.o_f32 + static_cast<int64_t>(t_begin) * hd + head * dim + cb * COLS + group;
+  float* o_dst = a.o_f32 + static_cast<int64_t>(t_begin) * hd + head * dim + col;
   __syncthreads();  // chunk 0 is ready
   for (int c = 0; c < chunks; ++c) {
     const float* buf = smem + (c & 1) * Sh::kBufFloats;
@@ -505,25 +500,17 @@ delta_scan_kernel(b200_delta_args a) {
     for (int tt = 0; tt < cnt; ++tt) {
       const float* v0 = buf + tt * 5 * DIM;
       const TokenVectors tv{v0, v0 + DIM, v0 + 2 * DIM, v0 + 3 * DIM, v0 + 4 * DIM};
-      float v[N], o[N];
-#pragma unroll
-      for (int n = 0; n < N; ++n) v[n] = values[tt * COLS + n * Sh::kGroups];
-      step<NI, I, N, ST>(s, tv, v, ni, o);
-#pragma unroll
-      for (int n = 0; n < N; ++n) {
-        const float sum = lane_sum<NI, ST>(o[n]);
-        if (ni == 0 && cb * COLS + n * Sh::kGroups + group < dim) o_dst[n * Sh::kGroups] = sum;
-      }
+      const float v[1] = {values[tt * COLS]};
+      float o[1];
+      step<NI, I, 1, ST>(s, tv, v, ni, o);
+      const float sum = lane_sum<NI, ST>(o[0]);
+      if (ni == 0 && col < dim) *o_dst = sum;
       o_dst += hd;
     }
     __syncthreads();  // chunk c has been read, chunk c + 1 is ready
   }
-#pragma unroll
-  for (int n = 0; n < N; ++n) {
-    const int j = cb * COLS + n * Sh::kGroups + group;
-    if (static_cast<unsigned>(out) < static_cast<unsigned>(a.state_slots) && j < dim)
-      store_column<NI, I>(a.state + (static_cast<int64_t>(out) * a.heads + head) * head_elems + static_cast<int64_t>(j) * dim, dim, ni, full, s[n]);
-  }
+  if (static_cast<unsigned>(out) < static_cast<unsigned>(a.state_slots) && col < dim)
+    store_column<NI, I>(a.state + (static_cast<int64_t>(out) * a.heads + head) * head_elems + static_cast<int64_t>(col) * dim, dim, ni, full, s[0]);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -1014,15 +1001,15 @@ static int decode_by_dim(const b200_delta_args& a, cudaStream_t s) {
   if (a.dim <= 128) return launch_decode<T, 128>(a, s);
   return launch_decode<T, 256>(a, s);
 }
-template <typename T, int DIM, int COLS, int N, int LANES>
+template <typename T, int DIM, int COLS, int LANES>
 static int launch_scan(const b200_delta_args& a, cudaStream_t s) {
-  using Sh = ScanShape<DIM, COLS, N, LANES>;
+  using Sh = ScanShape<DIM, COLS, LANES>;
   static std::atomic<uint64_t> done{0};
-  if (ensure_dynamic_smem(delta_scan_kernel<T, DIM, COLS, N, LANES>, Sh::kSmemBytes, done) != B200_OK) return B200_ERR_LAUNCH;
+  if (ensure_dynamic_smem(delta_scan_kernel<T, DIM, COLS, LANES>, Sh::kSmemBytes, done) != B200_OK) return B200_ERR_LAUNCH;
   const int col_blocks = (a.dim + COLS - 1) / COLS;
   // Not a programmatic launch: CTAs that arrive while the previous kernel still holds most SMs would pile up on the others,
   // and a CTA stays where it is for the length of a prompt.
-  delta_scan_kernel<T, DIM, COLS, N, LANES><<<dim3(a.heads * col_blocks, a.num_rows), Sh::kThreads, Sh::kSmemBytes, s>>>(a);
+  delta_scan_kernel<T, DIM, COLS, LANES><<<dim3(a.heads * col_blocks, a.num_rows), Sh::kThreads, Sh::kSmemBytes, s>>>(a);
   return launch_status();
 }
 template <typename T, int DIM, int COLS, int BLOCKS>
@@ -1047,10 +1034,10 @@ template <typename T>
 static int scan_by_dim(const b200_delta_args& a, cudaStream_t s) {
   // Blocks of four tokens against one token at a time: 6208 tokens in 5 rows x 32 heads of 64 378 us, 581; 8 rows x 64 heads 764, 872; 16 heads of 128, 5448
   // tokens in 4 rows 711, 918; 64 rows x 32 heads of one token 42, 42.  256 channels do not fit the registers four times, 32 are not worth the preparation.
-  if (a.dim <= 32) return launch_scan<T, 32, 32, 1, 2>(a, s);
+  if (a.dim <= 32) return launch_scan<T, 32, 32, 2>(a, s);
   if (a.dim <= 64) return block_scan_by_size<T, 64>(a, s);
   if (a.dim <= 128) return block_scan_by_size<T, 128>(a, s);
-  return launch_scan<T, 256, 32, 1, 2>(a, s);
+  return launch_scan<T, 256, 32, 2>(a, s);
 }
 
 }  // namespace delta
