@@ -696,6 +696,92 @@ def test_splits_of_many_rows_merge_as_those_of_few(ops, nkv, G, D, recipe):
     assert recipe is not None or bool((run(T)[0][0] == 0).all())
 
 
+@pytest.mark.parametrize("nkv,G", [(2, 8), (4, 4)])
+def test_merged_splits_of_many_rows_have_the_scales_of_few(ops, nkv, G):
+    # the MXFP8 scale of every block of 32 outputs, where four heads share a CTA's merge
+    D, F = 128, nkv * G * 128
+    T = 3 * 1024 // (nkv * G) // 8 * 8
+    c = make_paged_case(T=T, nkv=nkv, G=G, D=D, chunk=64, kv_lens=[[1, 64, 65, 200, 257, 320, 385, 33][r * 5 % 8] for r in range(T)], seed=8)
+    cos, sin = (f(c["freqs"][:, : D // 2]).to(BF16).cuda() for f in (torch.cos, torch.sin))
+
+    def run(n):
+        kc, vc = c["k_cache"].cuda(), c["v_cache"].cuda()
+        d = {k: c[k][:n].contiguous().cuda() for k in ("qkv", "block_table", "kv_lens", "pos", "chunk_idx", "local")}
+        quantised = ops.quantized_like("mxfp8", n, F, "cuda")
+        ops.paged_attention(ops.make_attention_args(
+            qkv=d["qkv"], k_cache=kc, v_cache=vc, block_table=d["block_table"], kv_seq_lengths=d["kv_lens"], out=torch.zeros((n, F), dtype=BF16, device="cuda"),
+            num_q_heads=c["nq"], num_kv_heads=nkv, head_dim=D, chunk_size=c["chunk"], token_to_pos_ids=d["pos"], token_to_pos_in_request=d["pos"],
+            token_to_chunk_idx=d["chunk_idx"], token_to_local_pos=d["local"], rope_cos=cos, rope_sin=sin, num_splits=6, fuse_rope_append=True,
+            out_quantized=quantised))
+        torch.cuda.synchronize()
+        r, b = torch.arange(16)[:, None], torch.arange(F // 32)[None, :]  # (the place of row r's block b)
+        at = ((r // 128) * (F // 128) * 512 + (b // 4) * 512 + (r % 32) * 16 + ((r % 128) // 32) * 4 + b % 4).reshape(-1).cuda()
+        return quantised.q[:16].view(torch.uint8).cpu(), quantised.sf.view(-1)[at].cpu()
+
+    for many, few in zip(run(T), run(16)):
+        assert torch.equal(many, few)
+
+
+@pytest.mark.parametrize("sinks", [False, True])
+@pytest.mark.parametrize("gates", [False, True])
+@pytest.mark.parametrize("window,keep", [(0, 0), (150, 70)])
+def test_merged_splits_of_many_rows_with_sinks_gates_and_windows(ops, window, keep, gates, sinks):
+    # finished queries over a [keys | values] pool: four heads share a CTA's merge, and have the bits of a part of the rows alone (a CTA for each)
+    import ctypes
+
+    from megatron_mixtera_b200 import _lib
+
+    heads, groups, dim, vdim, chunk, T, splits = 16, 4, 64, 128, 64, 160, 5
+    assert T * heads > 16 * torch.cuda.get_device_properties(0).multi_processor_count >= 16 * heads
+    lens = [[0, 1, 64, 65, 200, 257, 320, 449][r * 3 % 8] for r in range(T)]
+    g = torch.Generator(device="cuda").manual_seed(9)
+    blocks = [-(-n // chunk) for n in lens]
+    width = groups * (dim + vdim)
+    pool = torch.randn(sum(blocks) + 1, chunk, width, generator=g, device="cuda").to(BF16)
+    table, at = torch.zeros(T, max(blocks), dtype=torch.int32), 0
+    for r, n in enumerate(blocks):
+        table[r, :n] = torch.arange(at, at + n)
+        at += n
+    table, kv = table.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda")
+    q = torch.randn(T, heads, dim, generator=g, device="cuda").to(BF16)
+    sink = torch.randn(heads, generator=g, device="cuda")
+    gate = torch.randn(T, heads, generator=g, device="cuda").to(BF16)
+
+    def run(n):
+        out = torch.full((n, heads * vdim), float("nan"), dtype=BF16, device="cuda")
+        work = torch.empty(n * heads * splits * (vdim + 1), device="cuda")
+        a = _lib.AttentionArgs()
+        a.qkv, a.k_cache, a.v_cache = q.data_ptr(), pool.data_ptr(), pool.data_ptr() + 2 * groups * dim
+        a.separate, a.value_dim, a.pool_row_elems, a.window, a.keep_first, a.out_scale = 2, vdim, width, window, keep, 0.75
+        if sinks:
+            a.sinks = sink.data_ptr()
+        if gates:
+            a.gate, a.gate_ld = gate.data_ptr(), heads
+        a.block_table, a.kv_seq_lengths, a.out, a.workspace, a.workspace_bytes = table.data_ptr(), kv.data_ptr(), out.data_ptr(), work.data_ptr(), work.numel() * 4
+        a.num_tokens, a.num_q_heads, a.num_kv_heads, a.head_dim, a.chunk_size = n, heads, groups, dim, chunk
+        a.num_chunks, a.max_chunks_per_row, a.num_splits = pool.shape[0], table.shape[1], splits
+        rc = _lib.load().b200_paged_attention(ctypes.byref(a), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert rc == 0 and ops.device_status() == 0
+        return out.view(n, heads, vdim).float()
+
+    many, few = run(T), run(16)
+    assert torch.equal(many[:16], few) and not bool(many.isnan().any())
+    for r in range(1, 16):  # (row 0 sees no key)
+        n = lens[r]
+        rows = torch.cat([pool[int(b)] for b in table[r]])[:n].double()
+        k, v = rows[:, : groups * dim].view(n, groups, dim).repeat_interleave(4, 1), rows[:, groups * dim:].view(n, groups, vdim).repeat_interleave(4, 1)
+        s = torch.einsum("hd,khd->hk", q[r].double(), k) * dim ** -0.5
+        if window:
+            i = torch.arange(n, device="cuda")
+            s = s.masked_fill(~((n - 1 - i < window) | (i < keep)), -math.inf)
+        s = torch.cat([s, sink.double()[:, None]], 1) if sinks else s
+        y = 0.75 * torch.einsum("hk,khv->hv", torch.softmax(s, -1)[:, :n], v)
+        if gates:
+            y = y * torch.sigmoid(gate[r].double())[:, None]
+        assert rel_l2(few[r], y.float()) < 3e-3
+
+
 @pytest.mark.parametrize("shards,vocab", [(2, 1000), (8, 128256), (4, 4096)])
 def test_shardwise_argmax_equals_argmax_of_the_gathered_rows(ops, shards, vocab):
     rows = 37

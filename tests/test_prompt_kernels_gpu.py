@@ -64,6 +64,25 @@ def test_pair_gemm_matches_the_fp32_product(ops, M, N, K):
     assert torch.equal(wide[:, :N], ops.gemm(x, w)) and not wide[:, N:].any()
 
 
+# Tiles are walked in groups of 16 token blocks, or of 8 where a token is more than 8 KB, every other group from the last features to the first: three groups of
+# each kind, the last one partial, features that end inside a tile.
+@pytest.mark.parametrize("M,N,K", [(4400, 1160, 4104), (8500, 1160, 1280)])
+def test_pair_gemm_walks_groups_of_tiles_to_and_fro(ops, M, N, K):
+    x, w = randn(M, K, seed=11), randn(N, K, seed=12, scale=K ** -0.5)
+    y = torch.full((M, N), float("nan"), dtype=BF16, device="cuda")
+    assert rel(ops.gemm(x, w, out=y), x.float() @ w.float().T) < 3e-3 and not bool(y.isnan().any())
+
+
+@pytest.mark.parametrize("M,N,K", [(4400, 1160, 8320), (8500, 1160, 1152)])
+def test_pair_gemm_mxfp8_walks_groups_of_tiles_to_and_fro(ops, M, N, K):
+    from oracle import decode_oracle as O
+
+    x, w = randn(M, K, seed=13), randn(N, K, seed=14)
+    xd, wd = (O.dequantize_mxfp8(*O.quantize_mxfp8(t.cpu())).cuda() for t in (x, w))
+    y = torch.full((M, N), float("nan"), dtype=BF16, device="cuda")
+    assert rel(ops.gemm_mxfp8(ops.quantize_mxfp8(x), ops.quantize_mxfp8_weight(w), out=y), xd.float() @ wd.float().T) < 3e-3 and not bool(y.isnan().any())
+
+
 @pytest.mark.parametrize("M,F,K", [(257, 7168, 256), (2048, 1280, 512), (1500, 3200, 72), (300, 9664, 1352)])
 def test_pair_gemm_swiglu_equals_gemm_then_activation(ops, M, F, K):
     x, w = randn(M, K, seed=4), randn(2 * F, K, seed=5, scale=K ** -0.5)
