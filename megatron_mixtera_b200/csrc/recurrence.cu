@@ -787,8 +787,10 @@ scan_kernel(b200_recurrence_args a, bool vec_k) {
 //   o_j = (r_j w[0..j-1]) . S + sum_(s<j) (r_j . k_s w[s+1..j-1]) v_s + (r_j . b k_j) v_j,   S <- w[0..3] S + sum_s (k_s w[s+1..3]) v_s
 //
 // nine passes over a column's registers and a vector each, where four tokens one after another take twelve, and one lane sum for four tokens.  Bound by the reads
-// of shared memory and the multiply-adds of the compute warps.  6016 tokens in 4 rows x 32 heads of 64 340 -> 218 us, 16 heads of 128 504 -> 343.  Decays are
-// only multiplied, so none can be too small.  (Delta in the same form, two dot products for each token, 16 heads of 128: 532 -> 527 us with four lanes for a
+// of shared memory and the multiply-adds of the compute warps.  6016 tokens in 4 rows x 32 heads of 64 340 -> 218 us, 16 heads of 128 504 -> 355.  Decays are
+// only multiplied, so none can be too small.  A state is rounded once for four tokens, behind the sum of what they write, and a product of four decays is rounded
+// once in effect: rounding errors are 0.89 to 0.99 of those of a token at a time in the state and 0.96 to 1.02 in the outputs (1.03 to 1.16 and 1.04 to 1.10 with the
+// state first and plain products; 16 heads of 128 344 us then).  (Delta in the same form, two dot products for each token, 16 heads of 128: 532 -> 527 us with four lanes for a
 // column, 464 with eight, and 8 % more rounding error: it stays with a token at a time.)
 constexpr int kBlockTokens = 4;
 // Of a block, in floats: r w[0..j-1] and k w[s+1..3] of its tokens and w[0..3], each [DIM]; the values [4][COLS]; the products of the tokens with one another
@@ -897,7 +899,7 @@ wkv_block_scan_kernel(b200_recurrence_args a, bool vec_k) {
       for (int i = 0; i < 16; ++i) sums[i] = 0.f;
 #pragma unroll
       for (int e = 0; e < EL; ++e) {
-        float kk[J], p = 1.f;  // keys on their way through the decays behind them; the decays so far
+        float kk[J], p = 1.f, rest = 0.f;  // keys on their way through the decays behind them; the decays so far, and what the roundings of their product left out
 #pragma unroll
         for (int j = 0; j < J; ++j) {
 #pragma unroll
@@ -907,12 +909,14 @@ wkv_block_scan_kernel(b200_recurrence_args a, bool vec_k) {
           }
           sums[j * (j + 1) / 2 + j] = fmaf(r[j][e] * bonus[e], k[j][e], sums[j * (j + 1) / 2 + j]);
           kk[j] = k[j][e];
-          buf[Sh::kR + j * DIM + lane * EL + e] = r[j][e] * p;
-          p *= w[j][e];
+          buf[Sh::kR + j * DIM + lane * EL + e] = r[j][e] * (p + rest);
+          const float next = p * w[j][e];
+          rest = fmaf(p, w[j][e], -next) + rest * w[j][e];
+          p = next;
         }
 #pragma unroll
         for (int s = 0; s < J; ++s) buf[Sh::kK + s * DIM + lane * EL + e] = kk[s];
-        buf[Sh::kW + lane * EL + e] = lane * EL + e < dim ? p : 0.f;
+        buf[Sh::kW + lane * EL + e] = lane * EL + e < dim ? p + rest : 0.f;
       }
       const float mine = delta::transposed_sum<16>(sums, lane);
       if (place >= 0) buf[Sh::kPairs + place] = mine;
@@ -988,24 +992,24 @@ wkv_block_scan_kernel(b200_recurrence_args a, bool vec_k) {
         for (int n = 0; n < N; ++n) write[j][n] = pack2(v[j][n], v[j][n]);
 #pragma unroll
       for (int q = 0; q < I / 4; ++q) {
-        const ulonglong2 w = piece(buf + Sh::kW + (q * NI + ni) * 4);
-#pragma unroll
-        for (int n = 0; n < N; ++n) {
-          s[n][q * 2] = mul2(w.x, s[n][q * 2]);
-          s[n][q * 2 + 1] = mul2(w.y, s[n][q * 2 + 1]);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < I / 4; ++q)
+        const int i = (q * NI + ni) * 4;
+        f32x2 x[N], y[N];  // what the four tokens write, before the state is added
 #pragma unroll
         for (int j = 0; j < J; ++j) {
-          const ulonglong2 k = piece(buf + Sh::kK + j * DIM + (q * NI + ni) * 4);
+          const ulonglong2 k = piece(buf + Sh::kK + j * DIM + i);
 #pragma unroll
           for (int n = 0; n < N; ++n) {
-            s[n][q * 2] = fma2(k.x, write[j][n], s[n][q * 2]);
-            s[n][q * 2 + 1] = fma2(k.y, write[j][n], s[n][q * 2 + 1]);
+            x[n] = j == 0 ? mul2(k.x, write[j][n]) : fma2(k.x, write[j][n], x[n]);
+            y[n] = j == 0 ? mul2(k.y, write[j][n]) : fma2(k.y, write[j][n], y[n]);
           }
         }
+        const ulonglong2 w = piece(buf + Sh::kW + i);
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          s[n][q * 2] = fma2(w.x, s[n][q * 2], x[n]);
+          s[n][q * 2 + 1] = fma2(w.y, s[n][q * 2 + 1], y[n]);
+        }
+      }
       // Token `mine`'s output: its partial sums from the lanes of the column, and what the block's tokens up to it wrote.
       const float4 rk = *reinterpret_cast<const float4*>(buf + Sh::kPairs + mine * J);
       const bool upper = ni & 4, high = ni & 2, odd = ni & 1;

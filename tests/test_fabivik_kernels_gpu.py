@@ -147,6 +147,30 @@ def test_wkv_scan_of_a_row_in_any_company(dim, dtype):
     assert bool(found[1][0].isfinite().all()) and bool(found[1][0][-n:].abs().max() > 0)
 
 
+@pytest.mark.parametrize("heads,dim,lens", [(8, 64, [401]), (4, 128, [401]), (8, 64, [30, 31, 33, 29]), (4, 128, [30, 31, 33, 29])])
+def test_wkv_states_are_rounded_no_more_than_a_token_at_a_time(heads, dim, lens):
+    """Against 64 bits, the states' error is no larger than that of S <- fma(w, S, k v) for every token in 32 bits with the same decays (which 64 bits restate: a
+    product of 24-bit numbers is exact there)."""
+    off = plain = 0.0
+    for seed in (1, 2, 3):
+        c = WkvCase(heads, dim, sum(lens), len(lens), torch.float32, seed)
+        c.z = c.z * 0.5 - 2
+        new, at = c.scan(lens)[1].double(), 0
+        k, v = (c.proj[:, i * c.n: (i + 1) * c.n].double().view(-1, heads, dim) for i in (1, 2))
+        w = torch.exp(-torch.exp(c.z[0].double() + c.bias.double())).view(-1, heads, dim)
+        w32 = torch.exp(-torch.exp(c.z[0] + c.bias)).double().view(-1, heads, dim)
+        for row, n in enumerate(lens):
+            S = c.state0[row].double().transpose(1, 2)
+            P = S
+            for t in range(at, at + n):
+                kv = k[t][:, :, None] * v[t][:, None, :]
+                S, P = w[t][:, :, None] * S + kv, (w32[t][:, :, None] * P + kv.float().double()).float().double()
+            off += float((new[row].transpose(1, 2) - S).square().sum())
+            plain += float((P - S).square().sum())
+            at += n
+    assert off <= plain, math.sqrt(off / plain)
+
+
 @pytest.mark.parametrize("kind", ["wkv", "delta", "memory"])
 @pytest.mark.parametrize("dim", [64, 48, 128])
 def test_recurrent_decode_shares_a_row_between_warps(kind, dim):
