@@ -984,11 +984,12 @@ static int launch_decode(const b200_delta_args& a, cudaStream_t s) {
     return launch_pdl(delta_decode_kernel<T, DIM, PARTS>, dim3(a.heads, (a.num_rows + kRows - 1) / kRows), dim3(D::kWarps * 32), bytes, s, a, w2_stride);
   };
   if constexpr (D::kPasses >= 4) {
-    // Tasks that a grid of two warps for each would have, rows that fill up its last CTA among them.
-    const int64_t tasks = static_cast<int64_t>(a.heads) * a.num_rows, in_twos = static_cast<int64_t>(a.heads) * ((a.num_rows + D::kWarps / 2 - 1) / (D::kWarps / 2) * (D::kWarps / 2));
+    const int64_t tasks = static_cast<int64_t>(a.heads) * a.num_rows;
+    // (Of 256 channels two CTAs of two rows fit an SM: four tasks, with rows that only fill a CTA up.)
+    const int64_t in_twos = DIM > 128 ? static_cast<int64_t>(a.heads) * (a.num_rows + a.num_rows % 2) : tasks;
     // Four warps for each of few tasks, two up to four tasks an SM; with more each of them has enough on its way, and the token would be prepared several times.
     // us, one / two / four: 32 heads of 64, one row 4.8 / 3.7 / 3.3, 8 rows 7.2 / 4.8 / 4.2, 16 rows 7.3 / 5.1 / 8.1, 32 rows 9.3 / 12.3 / 18.5; 16 heads of 128, one row 12.3 /
-    // 7.8 / 5.9, 64 rows 27 / 30 / 37; two rows x 4 heads of 256 43.5 / 25.6 / 15.2, 37 rows x 16, whose CTAs of two rows are eight too many for a wave, 76.6 / 81.5.
+    // 7.8 / 5.9, 64 rows 27 / 30 / 37; two rows x 4 heads of 256 43.5 / 25.6 / 15.2, 37 rows x 16, whose CTAs of two rows are eight too many for a wave, 76.6 / 81.5 (of 96 channels 20.1 / 18.7).
     if (tasks <= 2 * sm_count()) return go(std::integral_constant<int, 4>{});
     if (in_twos <= 4 * sm_count()) return go(std::integral_constant<int, 2>{});
   }
