@@ -855,9 +855,9 @@ delta_block_scan_kernel(b200_delta_args a) {
   }
 }
 
-// kFinishUnits (token, head) units in turn with all their loads in flight: LPH lanes of four channels each, in vectors, or (LPH == 0) a warp: channels 32 apart, up to
-// 128 of them in registers.  Bound by the bytes in flight: 6208 tokens x 32 heads of 64 55 us with a warp and single channels for each, 20 in vectors (floor 15);
-// 6000 x 32 heads of 66, which are no vectors, 63 us in registers, 87 in the loop.
+// kFinishUnits (token, head) units in turn with all their loads in flight: LPH lanes of four channels each, in vectors, or a warp, channels 32 apart: in registers
+// (LPH < 0, up to 128 of them) or (LPH == 0) not.  Bound by the bytes in flight: 6208 tokens x 32 heads of 64 55 us with a warp and single channels for each, 20 in vectors
+// (floor 15); 6000 x 32 heads of 66, which are no vectors, 60 us in registers, 87 in the loop; 8 heads of 256 54 in a kernel of its own, 74 behind the registers' code.
 constexpr int kFinishUnits = 4;
 template <typename T, int LPH>
 __global__ void __launch_bounds__(256, LPH > 0 ? 4 : 1)
@@ -898,7 +898,7 @@ delta_finish_kernel(b200_delta_args a) {
   }
   const int lane = threadIdx.x & 31;
   const uint32_t first = (blockIdx.x * 8 + (threadIdx.x >> 5)) * kFinishUnits;
-  if (dim <= 128) {  // heads in registers
+  if constexpr (LPH < 0) {  // heads in registers
     float v[kFinishUnits][4], w[kFinishUnits][4];
     T g[kFinishUnits][4];
 #pragma unroll
@@ -1086,6 +1086,7 @@ int b200_delta_finish(const b200_delta_args* a, b200_stream_t stream) {
     using T = decltype(zero);
     if (lanes == 16) return launch_pdl(delta::delta_finish_kernel<T, 16>, grid, dim3(256), 0, s, *a);
     if (lanes == 32) return launch_pdl(delta::delta_finish_kernel<T, 32>, grid, dim3(256), 0, s, *a);
+    if (a->dim <= 128) return launch_pdl(delta::delta_finish_kernel<T, -1>, grid, dim3(256), 0, s, *a);
     return launch_pdl(delta::delta_finish_kernel<T, 0>, grid, dim3(256), 0, s, *a);
   };
   return a->dtype == B200_DTYPE_F32 ? go(0.f) : go(__nv_bfloat16{});
