@@ -470,7 +470,8 @@ static int launch(Args& a, const CUtensorMap* mw, const CUtensorMap* mx_, const 
     a.tiles = a.m_tiles * a.n_tiles;
     // The weights are read once for each group, so long groups, while their tokens stay in L2 beside the weights in use: 16 blocks of up to 8 KB a token.  In
     // long runs at the power cap, us with 8 and 16 blocks, features always forwards: 7700 x 28672 x 4096 1420, 1397, x 14336 -> 4096 722, 732; MXFP8 15500 x 28672 x
-    // 4096 1830, 1804, x 14336 -> 4096 893, 902.  Every other group backwards: 0 to 1.2 % less.
+    // 4096 1830, 1804, x 14336 -> 4096 893, 902.  Every other group backwards: 0 to 1.2 % less.  (A group's size at run time costs a tile of a short K: MXFP8 1.7 % with K 512, 0.8 %
+    // up to 2048.)
     a.group_m = static_cast<int64_t>(a.p.K) * (MX ? 1 : 2) <= 8192 ? 16 : 8;
   }
   static std::atomic<uint64_t> smem_attr_done{0};
