@@ -1302,11 +1302,11 @@ static int launch_block_scan(const b200_recurrence_args& a, cudaStream_t s) {
 template <typename T, int DIM>
 static int block_scan_by_size(const b200_recurrence_args& a, cudaStream_t s) {
   // Rows of 64 tokens and more on average: two columns on four lanes, with eight preparing warps while there are few CTAs or the state leaves one CTA an SM anyway, and
-  // with four, two CTAs an SM, from eight CTAs an SM on.  us, eight / four / a token at a time, 32 heads of 64: 4 rows of 2048 tokens and less 214 / 262 / 286, 80 rows of
-  // 70 200 / 148 / 174, 64 of 256 405 / 344 / 419; 64 heads: 24 rows of 64 115 / 86 / 101.  What a long row has beside it slows it then: one of 2000 tokens and 20 of three,
-  // 32 heads 203 / 229 / 266, 64 heads 206 / 265 / 284 (24 rows of 64, 32 heads, 58 / 47 / 56, stay with eight for that).
-  // Shorter rows: four columns on eight lanes.  us, four lanes and eight warps / eight lanes and four warps / a token at a time: 60 rows of 20 71 / 49 / 57, 64 rows of one
-  // 46 / 25 / 33; 64 rows of 256 tokens x 16 heads of 128 658 / 754 / 847.
+  // with four, two CTAs an SM, from eight CTAs an SM on.  us, eight / four / a token at a time, 32 heads of 64: 4 rows of 2048 tokens and less 215 / 262 / 286, 80 rows of
+  // 70 203 / 153 / 174, 64 of 256 414 / 350 / 419; 64 heads: 24 rows of 64 117 / 88 / 101.  What a long row has beside it slows it then: one of 2000 tokens and 20 of three,
+  // 32 heads 207 / 229 / 266, 64 heads 210 / 272 / 285 (24 rows of 64, 32 heads, 59 / 47 / 56, stay with eight for that).
+  // Shorter rows: four columns on eight lanes.  us, four lanes and eight warps / eight lanes and four warps / a token at a time: 60 rows of 20 69 / 51 / 57, 64 rows of one
+  // 46 / 25 / 33; 64 rows of 256 tokens x 16 heads of 128 681 / 754 / 847.
   if (a.num_tokens / 64 < a.num_rows) return launch_block_scan<T, DIM, 8, 4>(a, s);
   if (DIM <= 64 && static_cast<int64_t>(a.num_rows) * a.heads * ((a.vdim + 63) / 64) > 8 * sm_count()) return launch_block_scan<T, DIM, 4, DIM <= 64 ? 4 : 8>(a, s);
   return launch_block_scan<T, DIM, 4, 8>(a, s);
